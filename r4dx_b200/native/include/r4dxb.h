@@ -56,6 +56,10 @@ int r4dxb_rotate_rows(void* x, const void* signs, long long T, int H, int mode, 
 int r4dxb_rotate_residual(void* x, const float* signs, const float* mix, long long T, int H, int B, int inverse, void* stream);
 int r4dxb_w4a16_gemv(const void* wq, const void* wsz, const void* x, void* y, int T, int N, int K, int group,
                      int out_f32, void* stream);
+/* The same product for up to 64 rows (16 rows a launch); R4DXB_UNSUPPORTED where the streaming kernel does not cover the
+ * shape. */
+int r4dxb_w4a16_rows(const void* wq, const void* wsz, const void* x, void* y, int T, int N, int K, int group, int out_f32,
+                     void* stream);
 /* y[T,N] (fp32) = x[T,K] (bf16) . W[N,K]^T (bf16): small dense projections (gates, router) */
 int r4dxb_bf16_gemv(const void* W, const void* x, float* y, int T, int N, int K, void* stream);
 /* same for T <= 8 rows of the residual stream with the zero-centred RMSNorm folded in */

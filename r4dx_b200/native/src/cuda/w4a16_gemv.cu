@@ -3,13 +3,17 @@
 //
 // w4a16: w = scale * (q - zero); a nibble n becomes fp16 (0x6400 | n) = 1024 + n, the stored
 // fp16 -(1024 + zero) makes n - zero exact, eight products are summed in fp16x2 and the group
-// sum is scaled in fp32 (the reference uses the same exact-nibble trick on its WMMA path:
+// sum is scaled in fp32 (shapes of whole 16-row tiles and whole chunks go to w4a16_mma.cu instead; the reference uses the same exact-nibble trick on its WMMA path:
 // reference third_party/libr4d/r4d_gemm_w4a16_nt_m64.hip:1-67).  One warp streams one weight
 // row with 16-byte loads (32 weights per lane per load); rows are independent, so there is no
 // cross-CTA reduction.
 #include "common.cuh"
 
 namespace r4dxb {
+
+bool W4MmaCovers(const void* wq, const void* x, int T, int N, int K, int group);       // w4a16_mma.cu
+int W4Mma(const void* wq, const void* wsz, const void* x, void* y, int T, int N, int K, int group, int out_f32, cudaStream_t s);
+
 namespace {
 
 constexpr int kThreads = 256;
@@ -324,10 +328,29 @@ int r4dxb_w4a16_gemv(const void* wq, const void* wsz, const void* x, void* y, in
                      int out_f32, void* stream) {
   if (T < 1 || T > 8 || K % 32 || (group != 32 && group != 64 && group != 128) || K % group) return R4DXB_BAD_ARG;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
+  // whole tiles and chunks stream through mma.sync (w4a16_mma.cu: 172 us for a 248320 x 5120 head at 1..8 rows, this file's
+  // kernel 218 us at one row and 2450 us at eight); the kernel here takes what is left over
+  if (W4MmaCovers(wq, x, T, N, K, group)) return W4Mma(wq, wsz, x, y, T, N, K, group, out_f32, s);
   if (T == 1) return LaunchW4<1>(wq, wsz, x, y, T, N, K, group, out_f32, s);
   if (T == 2) return LaunchW4<2>(wq, wsz, x, y, T, N, K, group, out_f32, s);
   if (T <= 4) return LaunchW4<4>(wq, wsz, x, y, T, N, K, group, out_f32, s);
   return LaunchW4<8>(wq, wsz, x, y, T, N, K, group, out_f32, s);
+}
+
+/* The same product for up to 64 rows, 16 rows a launch.  R4DXB_UNSUPPORTED where the streaming kernel does not cover the shape
+ * (the caller then takes the tensor-core GEMM, which covers any number of rows). */
+int r4dxb_w4a16_rows(const void* wq, const void* wsz, const void* x, void* y, int T, int N, int K, int group, int out_f32,
+                     void* stream) {
+  if (T < 1 || T > 64 || K % 32 || (group != 32 && group != 64 && group != 128) || K % group) return R4DXB_BAD_ARG;
+  const int parts = (T + 15) / 16;
+  for (int i = 0; i < parts; ++i) {
+    const int t0 = i * T / parts, rows = (i + 1) * T / parts - t0;
+    const unsigned char* xi = static_cast<const unsigned char*>(x) + static_cast<size_t>(t0) * K * 2;
+    if (!W4MmaCovers(wq, xi, rows, N, K, group)) return R4DXB_UNSUPPORTED;       // (the same answer for every part)
+    unsigned char* yi = static_cast<unsigned char*>(y) + static_cast<size_t>(t0) * N * (out_f32 ? 4 : 2);
+    if (int rc = W4Mma(wq, wsz, xi, yi, rows, N, K, group, out_f32, static_cast<cudaStream_t>(stream))) return rc;
+  }
+  return 0;
 }
 
 int r4dxb_bf16_gemv(const void* W, const void* x, float* y, int T, int N, int K, void* stream) {

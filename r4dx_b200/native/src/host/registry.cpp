@@ -29,6 +29,7 @@ const R4dxbConstraint c16[] = {{"K", R4DXB_C_DIV, 128, nullptr}};
 const R4dxbConstraint c17[] = {{"E", R4DXB_C_LE, 1024, nullptr}};
 const R4dxbConstraint c18[] = {{"N", R4DXB_C_DIV, 4, nullptr}, {"K", R4DXB_C_DIV, 8, nullptr}};
 const R4dxbConstraint c19[] = {{"T", R4DXB_C_LE, 8, nullptr}, {"group", R4DXB_C_IN, 0, "32 64 128"}};
+const R4dxbConstraint c19r[] = {{"T", R4DXB_C_LE, 64, nullptr}, {"N", R4DXB_C_DIV, 16, nullptr}, {"group", R4DXB_C_IN, 0, "32 64 128"}};
 const R4dxbConstraint c20[] = {{"T", R4DXB_C_LE, 8, nullptr}};
 const R4dxbConstraint c21[] = {{"K", R4DXB_C_DIV, 2, nullptr}};
 const R4dxbConstraint c22[] = {{"T", R4DXB_C_LE, 8, nullptr}, {"K", R4DXB_C_DIV, 2, nullptr}};
@@ -134,7 +135,9 @@ const R4dxbKernelInfo kKernels[] = {
     {"linear_tc", "gemm", "plain_linear_rows_any", "y = act(x W^T + bias) + residual: dense bf16 / fp16 W by TMA, or w4a16 W widened by the decode warps",
      "dense: N % 4, K % 8; w4a16: N, K % 128, group 32/64/128", "bf16 / fp16 / w4a16, bf16 or fp32 y", "tcgen05", c18, 2},
     {"w4a16_gemv", "gemm", "w4a16_linear_rows_le_8", "group-quantised 4-bit head product",
-     "rows * K * 2 <= 200 KB", "bf16 x, nibbles + fp16 scale / zero", "simt", c19, 2},
+     "rows * K * 2 <= 200 KB", "bf16 x, nibbles + fp16 scale / zero", "mma.sync", c19, 2},
+    {"w4a16_rows", "gemm", "w4a16_linear_rows_le_64", "the same, 16 rows a launch",
+     "K % (4 group), 16 rows * K * 2 <= 227 KB", "bf16 x, nibbles + fp16 scale / zero", "mma.sync", c19r, 3},
     {"w8a16_gemv", "gemm", "w8a16_linear_rows_le_8", "group-quantised 8-bit product",
      "", "bf16 x, u8 + fp16 scale", "simt", c20, 1},
     {"bf16_gemv", "gemm", "bf16_linear", "dense bf16 product, fp32 out (tiled above 8 rows)",

@@ -158,6 +158,31 @@ def test_w4a16_gemv_and_argmax(K, T):
     assert torch.equal(ids.cpu().long(), y.cpu().argmax(-1) + 7)
 
 
+@pytest.mark.parametrize("T", [1, 3, 8, 9, 16])
+@pytest.mark.parametrize("N,Kd,group", [(16, 128, 32), (48, 512, 64), (1040, 512, 128), (2384, 1280, 64), (40000, 1024, 128)])
+def test_w4a16_streaming_rows_match_fp64(K, T, N, Kd, group):
+    """Every shape class of the mma.sync streaming kernel (K split over 1..16 warps, one or many tiles per warp, both output
+    types).  (n - zero) * x is exact in fp32 (5 + 11 bits) and each sum of K terms rounds at most once per term, so the error
+    is below 2^-23 * sqrt(K) of the root sum of squares; 1e-5 of it leaves a factor of two at K = 1280."""
+    from r4dx_b200.quant import w4a16
+    g = torch.Generator().manual_seed(T + N)
+    q = w4a16.quantize(torch.randn(N, Kd, generator=g) * torch.rand(N, 1, generator=g), group)
+    Wd = w4a16.dequantize(q).double()
+    x = torch.randn(T, Kd, generator=g).to(BF)
+    ref = x.double() @ Wd.T
+    qd, xd = q.to("cuda"), x.cuda()
+    y = torch.full((T, N), float("nan"), device="cuda")
+    args = (K._p(qd.wq), K._p(qd.wsz), K._p(xd))
+    K._check(K._lib().r4dxb_w4a16_rows(*args, K._p(y), T, N, Kd, group, 1, K._stream()), "w4a16_rows")
+    bound = 1e-5 * (x.double() ** 2 @ (Wd ** 2).T).sqrt()
+    assert ((y.cpu().double() - ref).abs() <= bound).all()
+    yb = torch.empty(T, N, dtype=BF, device="cuda")
+    K._check(K._lib().r4dxb_w4a16_rows(*args, K._p(yb), T, N, Kd, group, 0, K._stream()), "w4a16_rows")
+    assert torch.equal(yb, y.to(BF))
+    if T <= 8:
+        assert torch.equal(K.w4a16_gemv(qd, xd), y)
+
+
 @pytest.mark.parametrize("T,N,Kd,group", [(16, 256, 512, 64), (40, 1024, 1024, 32), (300, 512, 2048, 128), (1100, 384, 640, 64)])
 def test_linear_tc_w4a16_matches_fp32_reference(K, T, N, Kd, group):
     """The tensor-core w4a16 product against x @ dequant(W)^T in fp32, with bias, residual and an fp32 output."""
