@@ -110,6 +110,13 @@ int r4dxb_attn_decode(const void* q, const void* qg, const void* cache, const in
 int r4dxb_trellis_gemv_siblings(int count, const void* const* words, const void* const* suh, const void* const* svh,
                                 void* const* y, const int* n, const void* x, const void* norm_w, float eps, int prologue, int T,
                                 int K, int kb, int ksplit, void* stream);
+/* One to three products of one K and bit width over the same 1..8 rows (weight i writes y[i] [T, n[i]]; a residual only with
+ * count 1), the rows transformed once per call into ws: count * T * (2 K + 64) bytes, 16-byte aligned.  Any ksplit of 1..8.
+ * R4DXB_TOO_LARGE where no split brings a slice into shared memory. */
+int r4dxb_trellis_gemv_rows(int count, const void* const* words, const void* const* suh, const void* const* svh, void* const* y,
+                            const int* n, const void* x, const void* residual, const void* norm_w, float eps, int prologue, int T,
+                            int K, int kb, int ksplit, void* ws, void* stream);
+
 
 /* A/B switch: one-token steps use the warp-autonomous decode-attention kernel (default on); off = the window kernel
  * for every row count, which makes one-row and many-row calls bit-identical. */

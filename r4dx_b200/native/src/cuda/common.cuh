@@ -103,12 +103,9 @@ __device__ __forceinline__ void WarpFwht128(float (&v)[4]) {
   }
 #pragma unroll
   for (int m = 1; m < 32; m <<= 1) {
-    const bool upper = lane & m;
+    const float sign = (lane & m) ? -1.f : 1.f;      // one multiply-add (exact product) instead of two sums and a select
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const float o = __shfl_xor_sync(0xffffffffu, v[i], m);
-      v[i] = upper ? (o - v[i]) : (v[i] + o);
-    }
+    for (int i = 0; i < 4; ++i) v[i] = fmaf(v[i], sign, __shfl_xor_sync(0xffffffffu, v[i], m));
   }
 }
 

@@ -81,6 +81,36 @@ __device__ __forceinline__ bool WarpMbarWait(uint64_t* bar, uint32_t parity, vol
   return __shfl_sync(0xffffffffu, ok, 0) != 0;
 }
 
+// The same operations on shared-memory addresses the caller keeps in registers: converting a generic pointer costs about ten
+// instructions each time, which a producer that issues several small copies per stage cannot afford.
+__device__ __forceinline__ void MbarArriveAt(uint32_t bar) {
+  asm volatile("{ .reg .b64 st; mbarrier.arrive.shared::cta.b64 st, [%0]; }" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ void MbarArriveExpectTxAt(uint32_t bar, uint32_t bytes) {
+  asm volatile("{ .reg .b64 st; mbarrier.arrive.expect_tx.shared::cta.b64 st, [%0], %1; }" ::"r"(bar), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ bool MbarTryWaitAt(uint32_t bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile("{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
+               : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+  return ok != 0;
+}
+__device__ __forceinline__ bool MbarWaitAt(uint32_t bar, uint32_t parity, volatile int* abort_flag, int code) {
+  if (MbarTryWaitAt(bar, parity)) return true;
+  const long long t0 = clock64();
+  for (;;) {
+    if (MbarTryWaitAt(bar, parity)) return true;
+    if (*abort_flag) return false;
+    if (clock64() - t0 > kWaitClocks) break;
+  }
+  *abort_flag = code;
+  return false;
+}
+__device__ __forceinline__ void BulkLoadAt(uint32_t smem_dst, const void* gsrc, uint32_t bytes, uint32_t bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+               ::"r"(smem_dst), "l"(reinterpret_cast<uint64_t>(gsrc)), "r"(bytes), "r"(bar) : "memory");
+}
+
 // ---- proxies / fences ------------------------------------------------------------------------------
 __device__ __forceinline__ void FenceProxyAsyncShared() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 __device__ __forceinline__ void TcFenceBefore() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }

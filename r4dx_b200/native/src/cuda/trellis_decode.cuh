@@ -74,4 +74,61 @@ __device__ __forceinline__ void TrellisDecode8(uint32_t hi, uint32_t lo, __half2
   w[3] = TrellisCode2(TrellisStateFromWindow<KB, 6>(hi, lo), TrellisStateFromWindow<KB, 7>(hi, lo));
 }
 
+// The 16 states of one row of a tile (positions 16 r .. 16 r + 15) out of a 96-bit window x2:x1:x0 that ends with the row's
+// last state (KB = 3 needs 64 bits of it).  Used where one lane owns whole rows (the integer tensor-core kernel).
+template <int KB>
+struct TrellisRow {
+  int i0, i1, i2, i3;   // word indices of the window inside a tile
+  int off;              // bit offset of the window inside word i0 (0 or 16)
+  __device__ __forceinline__ void Init(int row) {
+    constexpr int R = 256 * KB, NW = 8 * KB, W = KB == 3 ? 64 : 96;
+    int b0 = 16 * KB * (row + 1) - W;
+    if (b0 < 0) b0 += R;
+    i0 = b0 >> 5;
+    off = b0 & 31;
+    i1 = (i0 + 1) % NW;
+    i2 = (i0 + 2) % NW;
+    i3 = (i0 + 3) % NW;
+  }
+  __device__ __forceinline__ void Load(const uint32_t* tw, uint32_t& x2, uint32_t& x1, uint32_t& x0) const {
+    if constexpr (KB == 4) {               // word aligned for every row, and i1 = 2 row: one 8-byte load
+      x2 = tw[i0];
+      const uint2 v = *reinterpret_cast<const uint2*>(tw + i1);
+      x1 = v.x;
+      x0 = v.y;
+    } else if constexpr (KB == 3) {
+      const uint32_t a = tw[i0], b = tw[i1], c = tw[i2];
+      x2 = 0;
+      x1 = __funnelshift_l(b, a, off);
+      x0 = __funnelshift_l(c, b, off);
+    } else {
+      const uint32_t a = tw[i0], b = tw[i1], c = tw[i2], d = tw[i3];
+      x2 = __funnelshift_l(b, a, off);
+      x1 = __funnelshift_l(c, b, off);
+      x0 = __funnelshift_l(d, c, off);
+    }
+  }
+  // State J as a zero-extended word, in as few integer instructions as its bit position allows: whole bytes are one byte
+  // permute, a state inside one word is a left shift (which may run on the multiply pipe) and a byte permute.
+  template <int J>
+  static __device__ __forceinline__ uint32_t State(uint32_t x2, uint32_t x1, uint32_t x0) {
+    constexpr int sh = KB * (15 - J), q = sh >> 5, r = sh & 31;
+    const uint32_t lo = q == 0 ? x0 : (q == 1 ? x1 : x2);
+    const uint32_t hi = q == 0 ? x1 : x2;
+    if constexpr (KB == 4) {
+      // shifts 12, 20, 28 are byte positions of the word shifted by 12; 8, 16, 24 of the word shifted by 8
+      if constexpr (r == 0) return __byte_perm(lo, 0u, 0x4410);
+      else if constexpr (r == 4) return __byte_perm(lo << 12, 0u, 0x4432);
+      else if constexpr (r == 12 || r == 20 || r == 28) return __byte_perm(__funnelshift_r(lo, hi, 12), 0u, r == 12 ? 0x4410 : (r == 20 ? 0x4421 : 0x4432));
+      else return __byte_perm(__funnelshift_r(lo, hi, 8), 0u, r == 8 ? 0x4410 : (r == 16 ? 0x4421 : 0x4432));
+    } else {
+      if constexpr (r == 0) return __byte_perm(lo, 0u, 0x4410);
+      else if constexpr (r == 8) return __byte_perm(lo, 0u, 0x4421);
+      else if constexpr (r == 16) return __byte_perm(lo, 0u, 0x4432);
+      else if constexpr (r < 16) return __byte_perm(lo << (16 - r), 0u, 0x4432);
+      else return __funnelshift_r(lo, hi, r) & 0xFFFFu;
+    }
+  }
+};
+
 }  // namespace r4dxb

@@ -1,0 +1,575 @@
+// Trellis-decode weight-streaming product for 2..8 activation rows on mma.sync, with the hash bytes themselves as the operand.
+//
+//   y[t, n] = bf16( svh[n] * H128( sum_k Q[n, k] * xh[t, k] )[n] (+ residual[t, n]) ),  xh = H128(suh (.) act(x))
+//
+// A code value is  Q = scale * (1024 + b0 + b1 + b2 + b3) + bias  with the four bytes b of state * 0x83DCD12D.  A hash word is
+// therefore four consecutive K bytes of an unsigned 8-bit operand, and
+//     sum_k Q[n, k] x[k] = scale * sum_k (b0 + b1 + b2 + b3)[n, k] x[k] + (1024 scale + bias) * sum_k x[k]
+// needs no byte sum, no packing and no multiply-add on the CUDA cores: a weight costs its state's extraction, one multiply and
+// a quarter of an m16n8k32 instruction per four rows of x.  The rows are integers too: q = round(x * 32512 / max|x|) over the
+// CTA's K slice, split into two signed bytes that are two columns of the product; sums are exact in int32 (a slice of 32768
+// columns at the largest digits stays below 2^31).  Against 64 bits the product is closer than with fp16 rows and fp16 partial
+// sums (2.1e-4 against 6.1e-4 relative before the bf16 rounding; unrounded code values are most of what is left).
+//
+// What bounds it: the register-file ports.  Per 128 weights a scheduler issues about 14 instructions, one of them an MMA with
+// ten register operands, and a mix of 4 byte permutes, 4 multiplies and one MMA alone takes 13 to 17 clocks (8 if only the
+// pipes counted): about 20 weights per clock and SM, 2.8 TB/s of 4-bit codes, whatever the row count.  Measured against the
+// CUDA-core kernel (trellis_gemv.cu), 4 bits, us at 2 / 4 / 8 rows: 34816 x 5120 48 / 46 / 60 (70 / 90 / 136), 5120 x 17408
+// 32 / 32 / 40 (49 / 72 / 117), 16384 x 5120 30 / 30 / 36 (45 / 55 / 84), 5120 x 6144 17 / 19 / 22 (22 / 27 / 41).  One row stays
+// there: its CTAs are small enough to overlap with their neighbours' in a captured step, and 1410 against 1540 us a step was
+// the result of 8 layers at 8192 tokens of context.
+//
+// Two launches: TrellisDigitsKernel writes the rows' digits once (every CTA would otherwise repeat the transform: at 8 rows of
+// 5120 columns that was 74k of 103k clocks), then one CTA per (128-row block, K slice) streams words through a ring of bulk
+// copies - filled before the wait for the digits - and `ksplit` CTAs of a cluster add up over distributed shared memory in rank
+// order.
+#include <cooperative_groups.h>
+
+#include "sm100_ptx.cuh"
+#include "trellis_decode.cuh"
+
+namespace cg = cooperative_groups;
+
+namespace r4dxb {
+namespace {
+
+constexpr int kTeamWarps = 4;            // warps that share one K block
+constexpr int kTeams = 4;
+constexpr int kConsumerWarps = kTeamWarps * kTeams;
+constexpr int kThreads = (kConsumerWarps + 1) * 32;
+constexpr int kSums = 2 * kTeams;        // partial sums of a row inside a CTA
+constexpr int kMaxStages = 6;
+constexpr int kMaxSiblings = 3;
+
+// Digits of one row of x over one K slice: the slice's scale and sum.
+struct DigitMeta {
+  uint32_t amax;                         // bit pattern of the largest magnitude
+  int xsum;
+};
+
+struct RowsArgs {
+  const __nv_bfloat16* x;
+  const __nv_bfloat16* residual;
+  const __nv_bfloat16* norm_w;           // prologue mode 1
+  float eps;
+  int T, K, kblocks_per_cta, stages, act;
+  const unsigned char* digits;           // [siblings][2 T columns][K]
+  const DigitMeta* meta;                 // [siblings][ksplit][T]
+  // one to three weights that read the same rows through the same prologue; blockIdx.y runs over all their row blocks
+  int count;
+  struct Weight {
+    const uint32_t* words;
+    const __half* suh;
+    const __half* svh;
+    __nv_bfloat16* y;
+    int N, nb_end;                       // row blocks [previous nb_end, nb_end) belong to this weight
+  } w[kMaxSiblings];
+};
+
+struct Ctl {                             // control block at the start of dynamic shared memory
+  uint64_t full[kMaxStages], empty[kMaxStages];
+  uint64_t red_bar;                      // split-K partials have landed
+  uint64_t xfull;                        // digits have landed
+  int abort_flag;
+  int pad;
+  float unit[8];                         // value of one integer step of a row
+  int xsum[8];                           // sum of a row's integers
+  uint32_t fill[18];
+};
+static_assert(sizeof(Ctl) % 128 == 0, "what follows the control block is 128-byte aligned");
+constexpr float kDigitRange = 32512.f;   // 127 * 256: the high digit stays a signed byte after rounding the low one
+
+// bytes between two digit columns: neighbouring columns (and the two k-tile pairs of a quad) fall into different banks
+__host__ __device__ constexpr int XStride(int kslice) { return kslice + 32; }
+
+__device__ __forceinline__ void ConsumerSync() { asm volatile("bar.sync 1, %0;" ::"r"(kConsumerWarps * 32) : "memory"); }
+
+__device__ __forceinline__ void MmaU8S8(int (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm("mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+      : "+r"(d[0]), "+r"(d[1]), "+r"(d[2]), "+r"(d[3])
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
+__device__ __forceinline__ float SumSquares8(const uint4& v) {
+  return BfLo(v.x) * BfLo(v.x) + BfHi(v.x) * BfHi(v.x) + BfLo(v.y) * BfLo(v.y) + BfHi(v.y) * BfHi(v.y) +
+         BfLo(v.z) * BfLo(v.z) + BfHi(v.z) * BfHi(v.z) + BfLo(v.w) * BfLo(v.w) + BfHi(v.w) * BfHi(v.w);
+}
+
+// Sum of squares of one eighth of a row (warps 0..7 of a CTA); every kernel that needs the RMS of a row adds the eighths in order,
+// so that they all round alike.
+__device__ __forceinline__ float EighthSumSquares(const __nv_bfloat16* row, int K, int warp, int lane) {
+  const int kw = (K / 8 + 7) & ~7;    // columns per warp, a multiple of 8
+  const int k_lo = warp * kw, k_hi = min(K, k_lo + kw);
+  float ss = 0.f;
+  for (int k = k_lo + lane * 8; k < k_hi; k += 256) ss += SumSquares8(*reinterpret_cast<const uint4*>(row + k));
+  return WarpSum(ss);
+}
+__device__ __forceinline__ float RowRms(const float* eighths, int K, float eps) {
+  float ss = 0.f;
+#pragma unroll
+  for (int w = 0; w < 8; ++w) ss += eighths[w];
+  return rsqrtf(ss / K + eps);
+}
+
+// four columns of act(x) * suh, before the Hadamard transform
+template <int PRO>
+__device__ __forceinline__ void Activate(uint2 xv, uint2 uv, uint2 wv, uint2 sv, float r, int act, float (&v)[4]) {
+  if constexpr (PRO == 2) {
+    const uint32_t p01 = PackBf16(GateAct(BfLo(xv.x), act) * BfLo(uv.x), GateAct(BfHi(xv.x), act) * BfHi(uv.x));
+    const uint32_t p23 = PackBf16(GateAct(BfLo(xv.y), act) * BfLo(uv.y), GateAct(BfHi(xv.y), act) * BfHi(uv.y));
+    v[0] = BfLo(p01); v[1] = BfHi(p01); v[2] = BfLo(p23); v[3] = BfHi(p23);
+  } else {
+    v[0] = BfLo(xv.x); v[1] = BfHi(xv.x); v[2] = BfLo(xv.y); v[3] = BfHi(xv.y);
+    if constexpr (PRO == 1) {
+      // same rounding point as the standalone norm kernel: the normalised row is a bf16 tensor
+      const uint32_t p01 = PackBf16(v[0] * r * (1.f + BfLo(wv.x)), v[1] * r * (1.f + BfHi(wv.x)));
+      const uint32_t p23 = PackBf16(v[2] * r * (1.f + BfLo(wv.y)), v[3] * r * (1.f + BfHi(wv.y)));
+      v[0] = BfLo(p01); v[1] = BfHi(p01); v[2] = BfLo(p23); v[3] = BfHi(p23);
+    }
+  }
+  const __half2 s01 = *reinterpret_cast<const __half2*>(&sv.x), s23 = *reinterpret_cast<const __half2*>(&sv.y);
+  v[0] *= __low2float(s01); v[1] *= __high2float(s01); v[2] *= __low2float(s23); v[3] *= __high2float(s23);
+}
+
+// largest magnitude of a 128-column block as a bit pattern (a NaN is larger than infinity); v becomes the transformed block
+__device__ __forceinline__ uint32_t HadamardMax(float (&v)[4]) {
+  const float inv_sqrt = 0.08838834764831845f;   // 1 / sqrt(128)
+  WarpFwht128(v);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) v[i] *= inv_sqrt;
+  const uint32_t m01 = max(__float_as_uint(fabsf(v[0])), __float_as_uint(fabsf(v[1])));
+  const uint32_t m23 = max(__float_as_uint(fabsf(v[2])), __float_as_uint(fabsf(v[3])));
+  return __reduce_max_sync(0xffffffffu, max(m01, m23));
+}
+
+// 32512 / amax; zero for a row of zeros (or of values below 1e-30, where the quotient would overflow) and for a row with a NaN
+// or an infinity, whose scale is poisoned later
+__device__ __forceinline__ float DigitScale(uint32_t amax_bits) {
+  const float amax = __uint_as_float(amax_bits);
+  return amax > 1e-30f && amax < INFINITY ? kDigitRange / amax : 0.f;
+}
+// q = round(v * inv) = 256 hi + lo; returns the block's sum of q
+__device__ __forceinline__ int Digits(const float (&v)[4], float inv, uint32_t (&hi)[4], uint32_t (&lo)[4]) {
+  int sum = 0;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int q = __float2int_rn(v[i] * inv);
+    hi[i] = static_cast<uint32_t>((q + 128) >> 8) & 0xFFu;
+    lo[i] = static_cast<uint32_t>(q) & 0xFFu;
+    sum += q;
+  }
+  return __reduce_add_sync(0xffffffffu, sum);
+}
+__device__ __forceinline__ uint32_t PackBytes(const uint32_t (&b)[4]) { return b[0] | (b[1] << 8) | (b[2] << 16) | (b[3] << 24); }
+
+// The digits of T rows for a whole launch: grid (T, ksplit, weights), one CTA per (row, K slice, weight).
+constexpr int kDigitWarps = 16;
+template <int PRO>
+__global__ void __launch_bounds__(kDigitWarps * 32) TrellisDigitsKernel(RowsArgs a, unsigned char* digits, DigitMeta* meta) {
+  PdlEnter();
+  extern __shared__ __align__(16) float rowbuf[];      // the slice, transformed
+  __shared__ float red[8];
+  __shared__ uint32_t amax;
+  __shared__ int xsum;
+  const int t = blockIdx.x, krank = blockIdx.y, ksplit = gridDim.y, sib = blockIdx.z, T = a.T, K = a.K;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const __half* suh = a.w[sib].suh;
+  const int kb_lo = krank * (K / 128) / ksplit, my_blocks = (krank + 1) * (K / 128) / ksplit - kb_lo;
+  if (threadIdx.x == 0) { amax = 0u; xsum = 0; }
+  float r = 0.f;
+  if constexpr (PRO == 1) {
+    if (warp < 8) {
+      const float ss = EighthSumSquares(a.x + static_cast<size_t>(t) * K, K, warp, lane);
+      if (lane == 0) red[warp] = ss;
+    }
+    __syncthreads();
+    r = RowRms(red, K, a.eps);
+  }
+  __syncthreads();
+  uint32_t m = 0u;
+  for (int b = warp; b < my_blocks; b += kDigitWarps) {
+    const int k = (kb_lo + b) * 128 + lane * 4;
+    uint2 xv, uv = make_uint2(0u, 0u), wv = make_uint2(0u, 0u);
+    if constexpr (PRO == 2) {
+      xv = *reinterpret_cast<const uint2*>(a.x + static_cast<size_t>(t) * 2 * K + k);
+      uv = *reinterpret_cast<const uint2*>(a.x + static_cast<size_t>(t) * 2 * K + K + k);
+    } else {
+      xv = *reinterpret_cast<const uint2*>(a.x + static_cast<size_t>(t) * K + k);
+      if constexpr (PRO == 1) wv = *reinterpret_cast<const uint2*>(a.norm_w + k);
+    }
+    float v[4];
+    Activate<PRO>(xv, uv, wv, *reinterpret_cast<const uint2*>(suh + k), r, a.act, v);
+    m = max(m, HadamardMax(v));
+    *reinterpret_cast<float4*>(rowbuf + b * 128 + lane * 4) = make_float4(v[0], v[1], v[2], v[3]);
+  }
+  if (lane == 0) atomicMax(&amax, m);
+  __syncthreads();
+  int sum = 0;
+  const float inv = DigitScale(amax);
+  for (int b = warp; b < my_blocks; b += kDigitWarps) {
+    const float4 f = *reinterpret_cast<const float4*>(rowbuf + b * 128 + lane * 4);
+    const float v[4] = {f.x, f.y, f.z, f.w};
+    uint32_t hi[4], lo[4];
+    sum += Digits(v, inv, hi, lo);
+    unsigned char* c0 = digits + (static_cast<size_t>(sib) * 2 * T + 2 * t) * K + (kb_lo + b) * 128 + lane * 4;
+    *reinterpret_cast<uint32_t*>(c0) = PackBytes(hi);
+    *reinterpret_cast<uint32_t*>(c0 + K) = PackBytes(lo);
+  }
+  if (lane == 0) atomicAdd(&xsum, sum);
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    DigitMeta d;
+    d.amax = amax;
+    d.xsum = xsum;
+    meta[(sib * ksplit + krank) * T + t] = d;
+  }
+}
+
+template <int KB, int TMAX>
+__global__ void __launch_bounds__(kThreads, TMAX > 4 ? 1 : 2) TrellisRowsKernel(RowsArgs a) {
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  cg::cluster_group cluster = cg::this_cluster();
+  const int ksplit = gridDim.x;
+  const int krank = blockIdx.x;            // == rank inside the cluster
+  int nb = blockIdx.y;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  int sidx = 0;                            // the weight this CTA serves
+  while (sidx + 1 < a.count && nb >= a.w[sidx].nb_end) ++sidx;
+  if (sidx > 0) nb -= a.w[sidx - 1].nb_end;
+  const int N = a.w[sidx].N, K = a.K, T = a.T;
+  // K blocks are dealt out as evenly as the count allows (17 blocks over 4 CTAs: 4, 4, 4, 5); shared memory is laid
+  // out for the longest slice
+  const int kslice = a.kblocks_per_cta * 128;
+  const int kb_lo = krank * (K / 128) / ksplit;
+  const int my_blocks = (krank + 1) * (K / 128) / ksplit - kb_lo;
+  constexpr int NW = 8 * KB;
+  constexpr int kStageBytes = 8 * 8 * NW * 4;     // 8 k-tiles x 8 n-tiles
+  // A stage is two bulk copies of four k-tiles each, 64 bytes apart modulo the banks; a quad reads two k-tiles of either half, so
+  // its words spread over all banks.  (Padding every k-tile took eight copies of 1 KB, and the copy engine then delivered
+  // 8 bytes per clock and SM: 53k instead of 35k clocks for the main loop of 40 blocks.)
+  constexpr int kTileBytes = 8 * NW * 4;
+  constexpr int kHalfSlot = 4 * kTileBytes + 64;
+  constexpr int kStageSlot = 2 * kHalfSlot;
+  constexpr int NG = TMAX > 4 ? 2 : 1;            // column groups: 8 columns = 4 rows of x, two digits each
+
+  const int xstride = XStride(kslice);
+  Ctl* ctl = reinterpret_cast<Ctl*>(smem_raw);
+  float* loc = reinterpret_cast<float*>(smem_raw + sizeof(Ctl));                     // [kSums][TMAX][128] sums of (k-tile half, team)
+  float* part = loc + kSums * TMAX * 128;                                             // [ksplit][TMAX][128] (used on cluster rank 0)
+  unsigned char* xd = reinterpret_cast<unsigned char*>(part + (ksplit > 1 ? ksplit : 0) * TMAX * 128);   // digits: [2 TMAX columns][xstride]
+  unsigned char* wst = xd + static_cast<size_t>(2 * TMAX) * xstride;                 // [stages][kStageSlot]
+  uint64_t* red_bar = &ctl->red_bar;
+  volatile int* abort_flag = &ctl->abort_flag;
+  const uint32_t full_at = ptx::SmemAddr(ctl->full), wst_at = ptx::SmemAddr(wst);      // (the empty barriers follow the full ones)
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < a.stages; ++s) {
+      ptx::MbarInit(&ctl->full[s], 1);
+      ptx::MbarInit(&ctl->empty[s], kTeamWarps);
+    }
+    ptx::MbarInit(red_bar, ksplit * kConsumerWarps);
+    ptx::MbarInit(&ctl->xfull, 1);
+    *abort_flag = 0;
+    ptx::MbarFenceInit();
+  }
+  __syncthreads();
+  // Cluster rendezvous, split in two: arrive now, wait only just before the first remote write, so
+  // the weight stream overlaps with it.  It guarantees that rank 0's reduction
+  // barrier is initialised before any peer CTA touches it.
+  if (ksplit > 1) asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+  // let the next kernel in the stream begin its own launch and weight prefetch
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+
+  if (warp == kConsumerWarps) {
+    // ---------------- producer: this CTA's words through the stage ring, the digits once the ring is full ----------------
+    if (lane == 0) {
+      const unsigned char* src = reinterpret_cast<const unsigned char*>(a.w[sidx].words) +
+                                 (static_cast<size_t>(nb) * (K / 128) + static_cast<size_t>(kb_lo)) * kStageBytes;
+      int s = 0;
+      uint32_t phase = 1;          // parity to wait for on the "empty" barrier of stage s (fresh barriers pass parity 1)
+      for (int it = 0; it <= my_blocks; ++it) {
+        if (it == min(a.stages, my_blocks)) {
+          asm volatile("griddepcontrol.wait;" ::: "memory");
+          ptx::MbarArriveExpectTx(&ctl->xfull, 2 * T * my_blocks * 128);
+          const unsigned char* xsrc = a.digits + static_cast<size_t>(sidx) * 2 * T * K + kb_lo * 128;
+          for (int c = 0; c < 2 * T; ++c)
+            ptx::BulkLoad(xd + static_cast<size_t>(c) * xstride, xsrc + static_cast<size_t>(c) * K, my_blocks * 128, &ctl->xfull);
+        }
+        if (it == my_blocks) break;
+        if (!ptx::MbarWaitAt(full_at + (kMaxStages + s) * 8, phase, abort_flag, 1)) break;
+        ptx::MbarArriveExpectTxAt(full_at + s * 8, kStageBytes);
+        ptx::BulkLoadAt(wst_at + s * kStageSlot, src, kStageBytes / 2, full_at + s * 8);
+        ptx::BulkLoadAt(wst_at + s * kStageSlot + kHalfSlot, src + kStageBytes / 2, kStageBytes / 2, full_at + s * 8);
+        src += kStageBytes;
+        if (++s == a.stages) { s = 0; phase ^= 1u; }
+      }
+    }
+  } else {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (threadIdx.x < T) {
+      const DigitMeta m = a.meta[(sidx * ksplit + krank) * T + threadIdx.x];
+      // an infinity or a NaN anywhere in the slice makes the whole row one
+      ctl->unit[threadIdx.x] = m.amax < 0x7F800000u ? __uint_as_float(m.amax) / kDigitRange : __int_as_float(0x7FC00000);
+      ctl->xsum[threadIdx.x] = m.xsum;
+    }
+    bool ok = ptx::MbarWait(&ctl->xfull, 0, abort_flag, 3);
+    ConsumerSync();
+
+    // ---------------- main loop: a team of four warps takes every fourth K block; a warp = four of its k-tiles and four n-tiles ----------------
+    // lane (g, c): rows g and g + 8 of an n-tile, the 16 columns of its k-tile; column g of the product = row g / 2 of x, digit g % 2
+    const int team = warp / kTeamWarps, w4 = warp % kTeamWarps;
+    const int g = lane >> 2, c = lane & 3, kq = w4 & 1, nt0 = (w4 >> 1) * 4;
+    const int kt = (c >> 1) * 4 + kq * 2 + (c & 1);        // the lane's k-tile
+    TrellisRow<KB> ra, rb;
+    ra.Init(g);
+    rb.Init(g + 8);
+    int acc[4][NG][4];
+#pragma unroll
+    for (int n = 0; n < 4; ++n)
+#pragma unroll
+      for (int q = 0; q < NG; ++q)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) acc[n][q][i] = 0;
+    const bool two_groups = NG == 2 && T > 4;
+    // columns past the last row of x repeat it: a column of the product depends on its own column of x only
+    const unsigned char* xcol[NG];
+#pragma unroll
+    for (int q = 0; q < NG; ++q)
+      xcol[q] = xd + static_cast<size_t>(min(g + 8 * q, 2 * T - 1)) * xstride + kt * 16;
+    // stage index and barrier parity advance by counting: a division by the run-time ring depth per 128-wide
+    // K block would cost as much as decoding a dozen weights
+    int s = team;
+    uint32_t phase = 0;
+    while (s >= a.stages) { s -= a.stages; phase ^= 1u; }
+    for (int it = team; it < my_blocks && ok; it += kTeams) {
+      uint32_t bx[NG][16];
+#pragma unroll
+      for (int q = 0; q < NG; ++q) {
+        const uint4 v = *reinterpret_cast<const uint4*>(xcol[q] + it * 128);
+        const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int i = 0; i < 16; ++i) bx[q][i] = __byte_perm(w[i >> 2], 0u, 0x1111 * (i & 3));      // a byte four times over
+      }
+      ok = ptx::MbarWaitAt(full_at + s * 8, phase, abort_flag, 2);
+      if (!ok) break;
+      const unsigned char* st = wst + s * kStageSlot + (c >> 1) * kHalfSlot + (kq * 2 + (c & 1)) * kTileBytes + nt0 * (NW * 4);
+#pragma unroll
+      for (int n = 0; n < 4; ++n) {
+        const uint32_t* tw = reinterpret_cast<const uint32_t*>(st + n * (NW * 4));
+        uint32_t wa[3], wb[3];
+        ra.Load(tw, wa[2], wa[1], wa[0]);
+        rb.Load(tw, wb[2], wb[1], wb[0]);
+#define R4DXB_I8_STEP(I)                                                                                              \
+  {                                                                                                                   \
+    const uint32_t a0 = TrellisRow<KB>::template State<2 * I>(wa[2], wa[1], wa[0]) * R4DXB_TRELLIS_MUL;                \
+    const uint32_t a1 = TrellisRow<KB>::template State<2 * I>(wb[2], wb[1], wb[0]) * R4DXB_TRELLIS_MUL;                \
+    const uint32_t a2 = TrellisRow<KB>::template State<2 * I + 1>(wa[2], wa[1], wa[0]) * R4DXB_TRELLIS_MUL;            \
+    const uint32_t a3 = TrellisRow<KB>::template State<2 * I + 1>(wb[2], wb[1], wb[0]) * R4DXB_TRELLIS_MUL;            \
+    MmaU8S8(acc[n][0], a0, a1, a2, a3, bx[0][2 * I], bx[0][2 * I + 1]);                                               \
+    if (two_groups) MmaU8S8(acc[n][NG - 1], a0, a1, a2, a3, bx[NG - 1][2 * I], bx[NG - 1][2 * I + 1]);                \
+  }
+        R4DXB_I8_STEP(0) R4DXB_I8_STEP(1) R4DXB_I8_STEP(2) R4DXB_I8_STEP(3)
+        R4DXB_I8_STEP(4) R4DXB_I8_STEP(5) R4DXB_I8_STEP(6) R4DXB_I8_STEP(7)
+#undef R4DXB_I8_STEP
+      }
+      __syncwarp();
+      if (lane == 0) ptx::MbarArriveAt(full_at + (kMaxStages + s) * 8);
+      s += kTeams;
+      while (s >= a.stages) { s -= a.stages; phase ^= 1u; }
+    }
+    // the sums of a row (k-tile half, team) meet in shared memory
+    const float code_scale = __half2float(__ushort_as_half(R4DXB_TRELLIS_SCALE_F16));
+    const float code_zero = 1024.f * code_scale + __half2float(__ushort_as_half(R4DXB_TRELLIS_BIAS_F16));
+    float* mine = loc + (team * 2 + kq) * TMAX * 128 + nt0 * 16 + g;
+#pragma unroll
+    for (int q = 0; q < NG; ++q) {
+      const int t = c + 4 * q;
+      if (t < T) {
+        const float unit = ok ? ctl->unit[t] : __int_as_float(0x7FC00000);      // (a copy that never landed shows as NaN)
+        const float zero = team + kq == 0 ? code_zero * static_cast<float>(ctl->xsum[t]) : 0.f;
+#pragma unroll
+        for (int n = 0; n < 4; ++n)
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            const float v = fmaf(static_cast<float>(acc[n][q][2 * h]), 256.f, static_cast<float>(acc[n][q][2 * h + 1]));
+            mine[t * 128 + n * 16 + 8 * h] = unit * fmaf(code_scale, v, zero);
+          }
+      }
+    }
+    ConsumerSync();
+    if (ksplit > 1) {
+      // hand this CTA's rows to cluster rank 0: distributed-shared-memory stores + one remote mbarrier arrival per
+      // warp; only rank 0 waits, the other CTAs are done
+      asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+      float* dst = cluster.map_shared_rank(part, 0) + krank * TMAX * 128;
+      for (int i = threadIdx.x; i < T * 128; i += kConsumerWarps * 32) {
+        float v = 0.f;
+#pragma unroll
+        for (int r = 0; r < kSums; ++r) v += loc[r * TMAX * 128 + i];
+        dst[i] = v;
+      }
+      __syncwarp();
+      if (lane == 0) {
+        uint32_t remote_bar;
+        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote_bar) : "r"(ptx::SmemAddr(red_bar)), "r"(0));
+        asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(remote_bar) : "memory");
+      }
+    }
+  }
+  if (warp == kConsumerWarps) {
+    // lane 0 may still be feeding the ring while the other lanes are already here: reconverge first,
+    // and use the per-thread (non-.aligned) form of the barrier
+    __syncwarp();
+    if (ksplit > 1) asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+  }
+
+    // ---------------- epilogue (cluster rank 0): warp t finishes row t ----------------
+  if (krank == 0 && warp < T) {
+    bool landed = ksplit == 1;
+    if (ksplit > 1) {
+      // wait (bounded) until every consumer warp of every CTA of the cluster has delivered its partial rows
+      for (int i = 0; i < ptx::kSpinLimit && !landed; ++i) {
+        uint32_t okw;
+        asm volatile(
+            "{ .reg .pred p; mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
+            : "=r"(okw) : "r"(ptx::SmemAddr(red_bar)), "r"(0) : "memory");
+        landed = okw != 0;
+      }
+    }
+    const float inv_sqrt = 0.08838834764831845f;
+    const int t = warp, n = nb * 128 + lane * 4;
+    const float* from = ksplit > 1 ? part : loc;
+    const int parts = ksplit > 1 ? ksplit : kSums;
+    float v[4] = {0.f, 0.f, 0.f, 0.f};
+    for (int r = 0; r < parts; ++r) {          // fixed order: the result does not depend on timing
+      const float4 p = *reinterpret_cast<const float4*>(from + (r * TMAX + t) * 128 + lane * 4);
+      v[0] += p.x; v[1] += p.y; v[2] += p.z; v[3] += p.w;
+    }
+    if (!landed) v[0] = __int_as_float(0x7FC00000);      // a hand-off that never completes shows as NaN in the whole block
+    WarpFwht128(v);
+    const uint2 sv = *reinterpret_cast<const uint2*>(a.w[sidx].svh + n);
+    const __half2 s01 = *reinterpret_cast<const __half2*>(&sv.x), s23 = *reinterpret_cast<const __half2*>(&sv.y);
+    float o[4] = {v[0] * inv_sqrt * __low2float(s01), v[1] * inv_sqrt * __high2float(s01),
+                  v[2] * inv_sqrt * __low2float(s23), v[3] * inv_sqrt * __high2float(s23)};
+    if (a.residual != nullptr) {
+      const uint2 rv = *reinterpret_cast<const uint2*>(a.residual + static_cast<size_t>(t) * N + n);
+      o[0] += BfLo(rv.x); o[1] += BfHi(rv.x); o[2] += BfLo(rv.y); o[3] += BfHi(rv.y);
+    }
+    uint2 ov;
+    ov.x = PackBf16(o[0], o[1]);
+    ov.y = PackBf16(o[2], o[3]);
+    *reinterpret_cast<uint2*>(a.w[sidx].y + static_cast<size_t>(t) * N + n) = ov;
+  }
+}
+
+template <int KB, int TMAX>
+size_t SmemBytes(int kslice, int stages, int ksplit) {
+  return sizeof(Ctl) + static_cast<size_t>(kSums + (ksplit > 1 ? ksplit : 0)) * TMAX * 128 * 4 +
+         static_cast<size_t>(2 * TMAX) * XStride(kslice) + static_cast<size_t>(stages) * (2 * (4 * 8 * 8 * KB * 4 + 64));
+}
+
+size_t SmemOf(int kb, int T, int K, int ksplit) {
+  const int blocks = (K / 128 + ksplit - 1) / ksplit, stages = blocks < kMaxStages ? blocks : kMaxStages;
+  if (kb == 3) return T <= 4 ? SmemBytes<3, 4>(blocks * 128, stages, ksplit) : SmemBytes<3, 8>(blocks * 128, stages, ksplit);
+  if (kb == 4) return T <= 4 ? SmemBytes<4, 4>(blocks * 128, stages, ksplit) : SmemBytes<4, 8>(blocks * 128, stages, ksplit);
+  return T <= 4 ? SmemBytes<5, 4>(blocks * 128, stages, ksplit) : SmemBytes<5, 8>(blocks * 128, stages, ksplit);
+}
+
+template <int KB, int TMAX>
+int LaunchRows(RowsArgs a, int ksplit, cudaStream_t stream) {
+  a.kblocks_per_cta = (a.K / 128 + ksplit - 1) / ksplit;       // the longest slice
+  // ring depth: everything in flight for short slices, otherwise up to 6 stages (48-60 KiB)
+  a.stages = a.kblocks_per_cta < kMaxStages ? a.kblocks_per_cta : kMaxStages;
+  const size_t smem = SmemBytes<KB, TMAX>(a.kblocks_per_cta * 128, a.stages, ksplit);
+  auto kern = TrellisRowsKernel<KB, TMAX>;
+  const cudaError_t ea = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+  if (ea != cudaSuccess) return static_cast<int>(ea);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(ksplit, a.w[a.count - 1].nb_end, 1);
+  cfg.blockDim = dim3(kThreads, 1, 1);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = ksplit;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  // programmatic dependent launch: the CTAs fill their rings while the digits are still being written
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = g_use_pdl ? 2 : 1;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, a);
+  ++g_launch_count;
+  return static_cast<int>(e);
+}
+
+template <int PRO>
+int LaunchDigits(const RowsArgs& a, int ksplit, cudaStream_t stream) {
+  const size_t smem = static_cast<size_t>((a.K / 128 + ksplit - 1) / ksplit) * 512;
+  auto kern = TrellisDigitsKernel<PRO>;
+  const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+  if (e != cudaSuccess) return static_cast<int>(e);
+  return LaunchPdl(kern, dim3(a.T, ksplit, a.count), dim3(kDigitWarps * 32), smem, stream, a, const_cast<unsigned char*>(a.digits),
+                   const_cast<DigitMeta*>(a.meta));
+}
+
+template <int KB>
+int LaunchKb(const RowsArgs& a, int ksplit, cudaStream_t stream) {
+  if (a.T <= 4) return LaunchRows<KB, 4>(a, ksplit, stream);
+  return LaunchRows<KB, 8>(a, ksplit, stream);
+}
+
+}  // namespace
+}  // namespace r4dxb
+
+using namespace r4dxb;
+
+extern "C" {
+
+/* One to three trellis products over the same 1..8 rows (see the header).  The split of K widens beyond `ksplit` where a
+ * slice would not fit into shared memory. */
+int r4dxb_trellis_gemv_rows(int count, const void* const* words, const void* const* suh, const void* const* svh, void* const* y,
+                            const int* n, const void* x, const void* residual, const void* norm_w, float eps, int prologue, int T,
+                            int K, int kb, int ksplit, void* ws, void* stream) {
+  if (count < 1 || count > kMaxSiblings || T < 1 || T > 8 || K < 128 || K % 128 || ksplit < 1 || ksplit > 8 || K / 128 < ksplit ||
+      prologue < 0 || prologue > 3 || (prologue == 1 && norm_w == nullptr) || (residual != nullptr && count > 1) || ws == nullptr ||
+      (reinterpret_cast<uintptr_t>(ws) & 15) || kb < 3 || kb > 5)
+    return R4DXB_BAD_ARG;
+  RowsArgs a = {};
+  a.x = static_cast<const __nv_bfloat16*>(x);
+  a.residual = static_cast<const __nv_bfloat16*>(residual);
+  a.norm_w = static_cast<const __nv_bfloat16*>(norm_w);
+  a.eps = eps;
+  a.T = T;
+  a.K = K;
+  a.act = prologue == 3 ? 1 : 0;           // GeGLU: the SwiGLU prologue with a tanh-GELU gate
+  a.count = count;
+  int end = 0;
+  for (int i = 0; i < count; ++i) {
+    if (n[i] < 128 || n[i] % 128) return R4DXB_BAD_ARG;
+    end += n[i] / 128;
+    a.w[i].words = static_cast<const uint32_t*>(words[i]);
+    a.w[i].suh = static_cast<const __half*>(suh[i]);
+    a.w[i].svh = static_cast<const __half*>(svh[i]);
+    a.w[i].y = static_cast<__nv_bfloat16*>(y[i]);
+    a.w[i].N = n[i];
+    a.w[i].nb_end = end;
+  }
+  while (SmemOf(kb, T, K, ksplit) > 227 * 1024) {
+    if (ksplit == 8 || K / 128 <= ksplit) return R4DXB_TOO_LARGE;
+    ++ksplit;
+  }
+  a.digits = static_cast<unsigned char*>(ws);
+  a.meta = reinterpret_cast<const DigitMeta*>(a.digits + static_cast<size_t>(count) * 2 * T * K);
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  const int rc = prologue == 0 ? LaunchDigits<0>(a, ksplit, s) : (prologue == 1 ? LaunchDigits<1>(a, ksplit, s) : LaunchDigits<2>(a, ksplit, s));
+  if (rc) return rc;
+  switch (kb) {
+    case 3: return LaunchKb<3>(a, ksplit, s);
+    case 4: return LaunchKb<4>(a, ksplit, s);
+    default: return LaunchKb<5>(a, ksplit, s);
+  }
+}
+
+}  // extern "C"

@@ -198,6 +198,28 @@ def pick_ksplit(N: int, K: int, target_ctas: int = int(os.environ.get("R4DXB_KSP
     return best
 
 
+def pick_split(N: int, K: int) -> int:
+    """Cluster split of the weight-streaming kernel for several rows: the fewest 128-wide K blocks on the busiest of the 148
+    SMs, with three blocks' time for what a CTA does besides (setup, reduction).  A CTA of it keeps an SM busy by itself, so
+    more CTAs than SMs only help to even out the load.  Measured at two rows, 4 bits (us by split 1..8): 5120 x 17408
+    73 44 34 40 34 32 42 40; 34816 x 5120 48 52 60 62 68 75 81 85; 5120 x 6144 32 22 17 22 20 20 26 24; 1024 x 2048
+    17 13 13 11 11 11 11 11.  Clusters of seven fit badly into the chip's SM groups and are left out."""
+    rows, blocks = N // 128, K // 128
+    return min((c for c in (1, 2, 3, 4, 5, 6, 8) if c <= blocks),
+               key=lambda c: ((rows * c + 147) // 148) * ((blocks + c - 1) // c + 3))
+
+
+# Weights of a launch from which two and more rows take the rows kernel: below, its second launch costs what the contraction
+# saves (us at 4 / 8 rows, CUDA cores against rows kernel: 4096 x 1024 12 / 16 against 13 / 13, 1024 x 2048 10 / 12 against
+# 11 / 13; 5120 x 6144 27 / 41 against 19 / 22).
+ROWS_MIN_WEIGHTS = 1 << 23
+
+
+def rows_split(N: int, K: int) -> Optional[int]:
+    """Split of the rows kernel for a launch of N output rows, None where the CUDA-core kernel serves several rows too."""
+    return pick_split(N, K) if N * K >= ROWS_MIN_WEIGHTS else None
+
+
 _STATUS = {}
 
 
@@ -220,12 +242,10 @@ PRO_NONE, PRO_RMSNORM, PRO_SILU_MUL, PRO_GELU_MUL = 0, 1, 2, 3
 
 register_cuda_sig("r4dxb_trellis_gemv_mma", _I, [_P, _P, _P, _P, _P, _P, _P, _F, _I, _I, _I, _I, _I, _I, _P, _P])
 
-# Which weight-streaming kernel serves T <= 8 rows: "simt" = CUDA-core decode + fp16 FMA (default: the faster one
-# on the 27B shapes, 56-62 us vs 66-68 us on gate_up), "mma" = code values written to tensor memory and contracted
-# by tcgen05.mma kind::f16 (trellis_gemv_mma.cu).
-# "auto" (the default) takes the CUDA-core kernel for one to three rows and the tensor-memory kernel where it measured faster:
-# from six rows everywhere (gate_up at 8 rows: 95 against 121 us, down 69 against 97 us) and from four rows on the two large
-# MLP products (80 against 83 us, 57 against 67 us).
+# Which weight-streaming kernel serves T <= 8 rows: "simt" = CUDA-core decode + fp16 FMA (trellis_gemv.cu), "mma" = code values
+# written to tensor memory and contracted by tcgen05.mma kind::f16 (trellis_gemv_mma.cu), "auto" (the default) = the
+# CUDA-core kernel for one row and, from two rows, decode in registers with mma.sync on the hash bytes
+# (trellis_gemv_rows.cu; us at 2 / 4 / 8 rows on gate_up 48 / 46 / 60 against 70 / 80 / 95 for the better of the other two).
 GEMV_IMPL = os.environ.get("R4DXB_GEMV", "auto")
 
 
@@ -237,8 +257,10 @@ def set_gemv_impl(name: str) -> None:
 
 
 def use_mma_gemv(T: int, N: int, K: int, ksplit: int) -> bool:
-    """Whether a product of T rows goes to the tensor-memory weight-streaming kernel (it needs an even K split of at most
-    6144 columns per CTA)."""
+    """Whether a product that the rows kernel does not serve (the tensor-parallel launches, slices too long for it) goes to the
+    tensor-memory weight-streaming kernel (which needs an even K split of at most 6144 columns per CTA): where that measured
+    faster than the CUDA cores, from six rows (gate_up at 8 rows: 95 against 121 us, down 69 against 97 us) and from four
+    rows on the two large MLP products (80 against 83 us, 57 against 67 us)."""
     if GEMV_IMPL == "simt" or K // ksplit > 6144 or (K // 128) % ksplit:
         return False
     if GEMV_IMPL == "mma":
@@ -246,10 +268,29 @@ def use_mma_gemv(T: int, N: int, K: int, ksplit: int) -> bool:
     return T >= 6 or (T >= 4 and N * K >= (1 << 26))
 
 
+_TOO_LARGE = 10003
+
+register_cuda_sig("r4dxb_trellis_gemv_rows", _I, [_I, _P, _P, _P, _P, _P, _P, _P, _P, _F, _I, _I, _I, _I, _I, _P, _P])
+
+
+def _ptr1(t: torch.Tensor):
+    return (ctypes.c_void_p * 1)(t.data_ptr())
+
+
+def _gemv_rows(count: int, words, suh, svh, y, n, x, residual, norm_w, eps: float, prologue: int, T: int, K_: int, kb: int,
+               ksplit: int) -> int:
+    """The mma.sync weight-streaming kernel; its workspace (the rows' digits) lives for the call."""
+    ws = torch.empty(count * T * (2 * K_ + 64), dtype=torch.uint8, device=x.device)
+    return _lib().r4dxb_trellis_gemv_rows(count, words, suh, svh, y, n, _p(x), _p(residual), _p(norm_w), eps, prologue, T, K_, kb, ksplit,
+                                          _p(ws), _stream())
+
+
 def trellis_gemv(w: TrellisWeight, x: torch.Tensor, residual: Optional[torch.Tensor] = None,
                  out: Optional[torch.Tensor] = None, ksplit: Optional[int] = None, prologue: int = PRO_NONE,
-                 norm_w: Optional[torch.Tensor] = None, eps: float = 1e-6) -> torch.Tensor:
-    """y[T, N] = trellis linear of act(x) (T <= 8), optionally + residual (may alias out).
+                 norm_w: Optional[torch.Tensor] = None, eps: float = 1e-6, split_rows: Optional[int] = None) -> torch.Tensor:
+    """y[T, N] = trellis linear of act(x) (T <= 8), optionally + residual (may alias out).  ``ksplit``: cluster split of K
+    on the CUDA-core and tensor-memory kernels; ``split_rows``: two and more rows take the rows kernel with this split (by
+    shape unless given).
 
     prologue PRO_RMSNORM: x is the residual stream [T, K], act = zero-centred RMSNorm with ``norm_w``;
     PRO_SILU_MUL: x is fused [gate | up] rows [T, 2K].
@@ -257,6 +298,13 @@ def trellis_gemv(w: TrellisWeight, x: torch.Tensor, residual: Optional[torch.Ten
     _req(x, BF, "x")
     T = x.numel() // (2 * w.K if prologue in (PRO_SILU_MUL, PRO_GELU_MUL) else w.K)
     out = out if out is not None else torch.empty(T, w.N, dtype=BF, device=x.device)
+    split_rows = split_rows or rows_split(w.N, w.K)
+    if GEMV_IMPL == "auto" and T > 1 and split_rows is not None:
+        rc = _gemv_rows(1, _ptr1(w.words), _ptr1(w.suh), _ptr1(w.svh), _ptr1(out), (ctypes.c_int * 1)(w.N), x, residual, norm_w, eps,
+                        prologue, T, w.K, w.kb, split_rows)
+        if rc != _TOO_LARGE:
+            _check(rc, "trellis_gemv_rows")
+            return out
     ks = ksplit or pick_ksplit(w.N, w.K)
     if use_mma_gemv(T, w.N, w.K, ks):
         _check(_lib().r4dxb_trellis_gemv_mma(_p(w.words), _p(w.suh), _p(w.svh), _p(x), _p(out), _p(residual), _p(norm_w), eps,
@@ -287,6 +335,7 @@ class SiblingGroup:
         self._svh = arr([w.svh.data_ptr() for w in weights])
         self._n = (ctypes.c_int * len(weights))(*[w.N for w in weights])
         self.ksplit = pick_ksplit(sum(w.N for w in weights), w0.K)
+        self.split_rows = rows_split(sum(w.N for w in weights), w0.K)
         self._outs = {}
 
     def __call__(self, x: torch.Tensor, outs: Sequence[torch.Tensor], prologue: int = PRO_NONE,
@@ -297,6 +346,12 @@ class SiblingGroup:
         y = self._outs.get(key)
         if y is None:
             y = self._outs[key] = (ctypes.c_void_p * len(outs))(*key)
+        if GEMV_IMPL == "auto" and T > 1 and self.split_rows is not None:
+            rc = _gemv_rows(len(self.weights), self._words, self._suh, self._svh, y, self._n, x, None, norm_w, eps, prologue, T, self.K,
+                            self.kb, self.split_rows)
+            if rc != _TOO_LARGE:
+                _check(rc, "trellis_gemv_rows")
+                return
         _check(_lib().r4dxb_trellis_gemv_siblings(len(self.weights), self._words, self._suh, self._svh, y, self._n, _p(x),
                                                   _p(norm_w), eps, prologue, T, self.K, self.kb, self.ksplit, _stream()),
                "trellis_gemv_siblings")

@@ -98,6 +98,49 @@ def test_trellis_gemv_tensor_memory_path_against_reference_and_cuda_core_path(K,
     assert (y_mma - y_simt).abs().max().item() < 0.02 * scale + 1e-3
 
 
+@pytest.mark.parametrize("kb", [3, 4, 5])
+@pytest.mark.parametrize("T,N,Kd,split", [(2, 128, 128, 1), (3, 256, 384, 3), (4, 384, 1280, 2), (5, 128, 2176, 5), (7, 256, 1024, 8),
+                                          (8, 512, 5120, 1), (8, 128, 17408, 6)])
+def test_trellis_rows_kernel_against_fp64(K, kb, T, N, Kd, split):
+    """The integer tensor-core kernel (2..8 rows) at the edges of its stage ring, teams and splits, all prologues.  Its
+    product differs from the definition by the unrounded code values (half an fp16 ulp, 2.2e-4 rms of unit codes) and by
+    digits of 1/32512 of the row's largest value (below 1e-4 of the row's rms); the bf16 result adds 2^-9 of each value."""
+    from r4dx_b200.ops import reference as R
+    from r4dx_b200.quant import trellis
+    g = torch.Generator().manual_seed(T * 100 + kb)
+    tw = trellis.random_weight(N, Kd, kb, seed=kb + T, sigma=0.02)
+    W = trellis.reconstruct(tw).double()
+    twd = tw.to("cuda")
+    x = (torch.randn(T, Kd, generator=g) ** 3).to(BF)
+    ref = x.double() @ W.T
+    rms = (x.double() ** 2).mean(-1, keepdim=True).sqrt() * (W ** 2).sum(-1).sqrt()
+
+    def check(y, ref):
+        assert ((y.double().cpu() - ref).abs() <= 2.0 ** -8 * ref.abs() + 2e-3 * rms).all()
+
+    assert K.GEMV_IMPL == "auto"
+    check(K.trellis_gemv(twd, x.cuda(), split_rows=split), ref)
+    res = torch.randn(T, N, generator=g).to(BF)
+    check(K.trellis_gemv(twd, x.cuda(), residual=res.cuda(), split_rows=split), ref + res.double())
+    if Kd <= 12288:                               # (the norm kernel stages a row in 48 KB)
+        nw = (torch.randn(Kd, generator=g) * 0.1).to(BF).cuda()
+        h = K.rmsnorm(x.cuda(), nw)
+        # (the row's sum of squares is added up in another order than in the norm kernel: an entry of h may round the other way,
+        # which is 2^-8 of that entry, so the same bound holds around the product of h)
+        hd = h.double().cpu()
+        rms = (hd ** 2).mean(-1, keepdim=True).sqrt() * (W ** 2).sum(-1).sqrt()
+        check(K.trellis_gemv(twd, x.cuda(), split_rows=split, prologue=K.PRO_RMSNORM, norm_w=nw), hd @ W.T)
+    gu = torch.randn(T, 2 * Kd, generator=g).to(BF).cuda()
+    assert torch.equal(K.trellis_gemv(twd, gu, split_rows=split, prologue=K.PRO_SILU_MUL), K.trellis_gemv(twd, K.silu_mul(gu), split_rows=split))
+    # a row of zeros stays zero, a row with a NaN or an infinity becomes NaN, the others are not touched
+    bad = x.clone()
+    bad[0] = 0
+    bad[1, 5] = float("inf") if T % 2 else float("nan")
+    y = K.trellis_gemv(twd, bad.cuda(), split_rows=split)
+    assert (y[0] == 0).all() and y[1].isnan().all()
+    assert torch.equal(y[2:], K.trellis_gemv(twd, x.cuda(), split_rows=split)[2:])
+
+
 def test_trellis_gemv_one_hot_returns_decoded_rows(K):
     """x = e_k after undoing the input transform picks out column k of H Q H exactly (up to bf16)."""
     from r4dx_b200.quant import trellis
