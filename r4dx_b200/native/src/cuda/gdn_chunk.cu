@@ -8,11 +8,15 @@
 // so the work splits in two kernels:
 //   phase A (grid chunks x heads, no dependence on the state): A and P in fp32, then the triangular
 //           solve for U~ = (I + A)^-1 beta V and W = (I + A)^-1 beta gamma K by forward substitution,
-//           one right-hand-side column per thread with the 64 unknowns in registers;
-//   phase B (grid heads x 4 row blocks of the state, sequential over chunks): U = U~ - W S0^T,
+//           one right-hand-side column per thread with the 64 unknowns in registers.  The solve is right-looking (a
+//           solved unknown is subtracted from all later ones at once): the sums are independent, where adding up
+//           unknown i's terms when its turn comes is a chain of i multiply-adds behind a global load;
+//   phase B (grid heads x 2 row blocks of the state, sequential over chunks): U = U~ - W S0^T,
 //           O, and the state update as TF32 tensor-core products (mma.sync m16n8k8, fp32
-//           accumulate) out of shared memory; W, Q, P and K stream through two cp.async slots, each
-//           fetched one product ahead of its use.  The fp32 state block lives in shared memory for
+//           accumulate) out of shared memory; W, Q, P and K have a cp.async slot each that is refilled for the
+//           next chunk as soon as its product is done, three products ahead of its use (two shared slots fetched one
+//           product ahead left every one of the four products of a chunk waiting for its operand: 14k clocks a
+//           chunk where the products take about five).  The fp32 state block lives in shared memory for
 //           the whole sequence.
 // The per-token recurrence (gdn_prefill.cu) stays as the reference path and for D = 64
 // (reference: third_party/libr4d/r4d_gdn_chunk_scan_k128_v128_c64_bf16.hip:1-60 runs the same
@@ -32,10 +36,17 @@ constexpr int kLdA = kC + 4;
 struct PhaseASmem {
   float ks[kC][kLdK];
   float qs[kC][kLdK];
-  float As[kC][kLdA];
+  float At[kC][kLdA];     // -A transposed: row j holds the factors of unknown j
   float G[kC];
   float B[kC];
+  float BG[kC];           // beta gamma
 };
+
+__device__ __forceinline__ uint32_t Tf32(float x) {
+  uint32_t r;
+  asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r) : "f"(x));
+  return r;
+}
 
 __device__ __forceinline__ float Dot4(const float4& a, const float4& b, float acc) {
   acc = fmaf(a.x, b.x, acc);
@@ -74,12 +85,21 @@ __global__ void __launch_bounds__(256) GdnChunkPrepKernel(const float* __restric
     sm.G[tid] = t < T ? fmaxf(logf(eg[static_cast<size_t>(t) * H + h]), -80.f) : 0.f;
   }
   __syncthreads();
-  if (tid == 0) {
-    float acc = 0.f;
-    for (int i = 0; i < kC; ++i) {
-      acc += sm.G[i];
-      sm.G[i] = acc;
+  if (tid < 32) {
+    // running sum of the 64 log decays, two per lane
+    const float a = sm.G[2 * tid], b = a + sm.G[2 * tid + 1];
+    float sum = b;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const float up = __shfl_up_sync(0xffffffffu, sum, d);
+      if (tid >= d) sum += up;
     }
+    const float before = __shfl_up_sync(0xffffffffu, sum, 1);
+    const float base = tid > 0 ? before : 0.f;
+    sm.G[2 * tid] = base + a;
+    sm.G[2 * tid + 1] = sum;
+    sm.BG[2 * tid] = sm.B[2 * tid] * expf(base + a);
+    sm.BG[2 * tid + 1] = sm.B[2 * tid + 1] * expf(sum);
   }
   __syncthreads();
   if (tid < kC) ws_g[ch * kC + tid] = sm.G[tid];
@@ -115,8 +135,8 @@ __global__ void __launch_bounds__(256) GdnChunkPrepKernel(const float* __restric
       for (int cc = 0; cc < 4; ++cc) {
         const int i = ty + 16 * rr, j = tx + 16 * cc;
         const float decay = j <= i ? expf(sm.G[i] - sm.G[j]) : 0.f;
-        sm.As[i][j] = j < i ? sm.B[i] * decay * kk[rr][cc] : 0.f;
-        ws_p[(ch * kC + i) * kC + j] = decay * qk[rr][cc];
+        if (j < i) sm.At[j][i] = -(sm.B[i] * decay * kk[rr][cc]);
+        ws_p[(ch * kC + i) * kC + j] = __uint_as_float(Tf32(decay * qk[rr][cc]));     // (as phase B's product takes it)
       }
   }
   __syncthreads();
@@ -127,28 +147,28 @@ __global__ void __launch_bounds__(256) GdnChunkPrepKernel(const float* __restric
     const int col = is_u ? tid : tid - kD;
     float* dst = (is_u ? ws_ut : ws_w) + ch * kC * kD + col;
     float x[kC];
+    if (is_u) {
+      const float* src = v + (static_cast<size_t>(t0) * H + h) * kD + col;
 #pragma unroll
-    for (int i = 0; i < kC; ++i) {
-      float rhs;
-      if (is_u) {
-        const int t = t0 + i;
-        rhs = t < T ? sm.B[i] * v[(static_cast<size_t>(t) * H + h) * kD + col] : 0.f;
-      } else {
-        rhs = sm.B[i] * expf(sm.G[i]) * sm.ks[i][col];
+      for (int i = 0; i < kC; ++i) x[i] = t0 + i < T ? src[static_cast<size_t>(i) * H * kD] : 0.f;
+#pragma unroll
+      for (int i = 0; i < kC; ++i) x[i] *= sm.B[i];
+    } else {
+#pragma unroll
+      for (int i = 0; i < kC; ++i) x[i] = sm.BG[i] * sm.ks[i][col];
+    }
+#pragma unroll
+    for (int j = 0; j < kC; ++j) {
+#pragma unroll
+      for (int i4 = ((j + 1) / 4) * 4; i4 < kC; i4 += 4) {
+        const float4 a = *reinterpret_cast<const float4*>(&sm.At[j][i4]);
+        if (i4 > j) x[i4] = fmaf(a.x, x[j], x[i4]);
+        if (i4 + 1 > j) x[i4 + 1] = fmaf(a.y, x[j], x[i4 + 1]);
+        if (i4 + 2 > j) x[i4 + 2] = fmaf(a.z, x[j], x[i4 + 2]);
+        if (i4 + 3 > j) x[i4 + 3] = fmaf(a.w, x[j], x[i4 + 3]);
       }
-      float acc0 = rhs, acc1 = 0.f;
-#pragma unroll
-      for (int j = 0; j + 3 < i; j += 4) {
-        const float4 a = *reinterpret_cast<const float4*>(&sm.As[i][j]);
-        acc0 = fmaf(-a.x, x[j], acc0);
-        acc1 = fmaf(-a.y, x[j + 1], acc1);
-        acc0 = fmaf(-a.z, x[j + 2], acc0);
-        acc1 = fmaf(-a.w, x[j + 3], acc1);
-      }
-#pragma unroll
-      for (int j = (i / 4) * 4; j < i; ++j) acc0 = fmaf(-sm.As[i][j], x[j], acc0);
-      x[i] = acc0 + acc1;
-      dst[static_cast<size_t>(i) * kD] = x[i];
+      // W is an operand of phase B's tensor-core products only: rounded here instead of at every read
+      dst[static_cast<size_t>(j) * kD] = is_u ? x[j] : __uint_as_float(Tf32(x[j]));
     }
   }
 }
@@ -156,23 +176,22 @@ __global__ void __launch_bounds__(256) GdnChunkPrepKernel(const float* __restric
 // ---------------------------------------- phase B ----------------------------------------
 constexpr int kLd = kD + 8;       // W / Q / K / state rows: conflict-free 8-byte fragment reads and strided scalar reads
 constexpr int kLdP = kC + 4;      // P rows: conflict-free scalar fragment reads
-constexpr int kLdU = 32 + 8;      // U rows (this CTA's 32 value columns)
-constexpr int kSlotFloats = kC * kLd;
+static_assert(kC == 64, "the warps of a CTA tile 64 tokens by kRows columns");
+constexpr int kRows = 64;         // state rows (value columns) of a CTA
+constexpr int kLdU = kRows + 8;   // U rows
+constexpr int kScanThreads = kRows * 8;
 
 struct PhaseBSmem {
-  float slot[2][kSlotFloats];
-  float S[32][kLd];
+  float W[kC * kLd];
+  float Q[kC * kLd];
+  float K[kC * kLd];
+  float P[kC * kLdP];
+  float S[kRows][kLd];
   float U[2][kC][kLdU];
   float G[2][kC];
   float eG[kC];
   float fG[kC];
 };
-
-__device__ __forceinline__ uint32_t Tf32(float x) {
-  uint32_t r;
-  asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r) : "f"(x));
-  return r;
-}
 
 __device__ __forceinline__ void MmaTf32(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
                                         uint32_t b1) {
@@ -185,7 +204,8 @@ __device__ __forceinline__ void MmaTf32(float (&c)[4], uint32_t a0, uint32_t a1,
 // acc[nt] += A[m0 .. m0+16, 0 .. 128) * S[n0 + 8 nt .. +8, 0 .. 128)^T, both row-major along the contraction.
 // Inside every block of 8 contraction columns the hardware index t maps to column 2t and t + 4 to 2t + 1, so
 // that one 8-byte load feeds two fragment registers; A and B use the same map, so the product is unchanged.
-template <int NT>
+// kRounded: A already holds TF32 values.
+template <int NT, bool kRounded>
 __device__ __forceinline__ void MmaRowRow(float (&acc)[NT][4], const float* __restrict__ A, int m0, const float* __restrict__ S,
                                           int n0, int lane) {
   const int g = lane >> 2, t = lane & 3;
@@ -196,7 +216,8 @@ __device__ __forceinline__ void MmaRowRow(float (&acc)[NT][4], const float* __re
   for (int kb = 0; kb < kD / 8; ++kb) {
     const float2 lo = *reinterpret_cast<const float2*>(a_lo + kb * 8);
     const float2 hi = *reinterpret_cast<const float2*>(a_hi + kb * 8);
-    const uint32_t a0 = Tf32(lo.x), a2 = Tf32(lo.y), a1 = Tf32(hi.x), a3 = Tf32(hi.y);
+    const uint32_t a0 = kRounded ? __float_as_uint(lo.x) : Tf32(lo.x), a2 = kRounded ? __float_as_uint(lo.y) : Tf32(lo.y);
+    const uint32_t a1 = kRounded ? __float_as_uint(hi.x) : Tf32(hi.x), a3 = kRounded ? __float_as_uint(hi.y) : Tf32(hi.y);
 #pragma unroll
     for (int nt = 0; nt < NT; ++nt) {
       const float2 b = *reinterpret_cast<const float2*>(b_base + nt * 8 * kLd + kb * 8);
@@ -208,14 +229,14 @@ __device__ __forceinline__ void MmaRowRow(float (&acc)[NT][4], const float* __re
 __device__ __forceinline__ void CopyRows(float* dst, int ld_dst, const float* src, size_t src_stride, int rows, int row_floats,
                                          int tid) {
   const int per_row = row_floats / 4;
-  for (int i = tid; i < rows * per_row; i += 256) {
+  for (int i = tid; i < rows * per_row; i += kScanThreads) {
     const int r = i / per_row, o = (i % per_row) * 4;
     __pipeline_memcpy_async(dst + r * ld_dst + o, src + static_cast<size_t>(r) * src_stride + o, 16);
   }
 }
 
-// grid (H, 4), 256 threads: CTA (h, vb) owns state rows [32 vb, 32 vb + 32) of head h
-__global__ void __launch_bounds__(256, 2) GdnChunkScanKernel(const float* __restrict__ q, const float* __restrict__ k,
+// grid (H, 128 / kRows): CTA (h, vb) owns state rows [kRows vb, kRows vb + kRows) of head h
+__global__ void __launch_bounds__(kScanThreads, 1) GdnChunkScanKernel(const float* __restrict__ q, const float* __restrict__ k,
                                                              const float* __restrict__ ws_ut, const float* __restrict__ ws_w,
                                                              const float* __restrict__ ws_p, const float* __restrict__ ws_g,
                                                              float* __restrict__ state, float* __restrict__ o, int T, int H,
@@ -228,44 +249,55 @@ __global__ void __launch_bounds__(256, 2) GdnChunkScanKernel(const float* __rest
   const int chunks = (T + kC - 1) / kC;
   const float scale = rsqrtf(static_cast<float>(kD));
 
-  auto issue_wug = [&](int c, int buf) {      // W -> slot 0, U~ (this CTA's columns) and G
-    const size_t ch = static_cast<size_t>(c) * H + h;
-    CopyRows(sm.slot[0], kLd, ws_w + ch * kC * kD, kD, kC, kD, tid);
-    CopyRows(&sm.U[buf][0][0], kLdU, ws_ut + ch * kC * kD + vb * 32, kD, kC, 32, tid);
-    if (tid < kC / 4) __pipeline_memcpy_async(&sm.G[buf][tid * 4], ws_g + ch * kC + tid * 4, 16);
-    __pipeline_commit();
-  };
-  auto issue_qk = [&](const float* src, int c, int slot) {     // token rows of q or k (clamped past the end)
-    for (int i = tid; i < kC * (kD / 4); i += 256) {
-      const int r = i / (kD / 4), off = (i % (kD / 4)) * 4;
-      const int t = min(c * kC + r, T - 1);
-      __pipeline_memcpy_async(&sm.slot[slot][r * kLd + off], src + (static_cast<size_t>(t) * Hk + hk) * kD + off, 16);
+  // every call commits one copy group, an empty one past the last chunk, so that "all but the two newest" always names
+  // the operand of the next product
+  auto issue_wug = [&](int c) {               // W, U~ (this CTA's columns) and G
+    if (c < chunks) {
+      const size_t ch = static_cast<size_t>(c) * H + h;
+      CopyRows(sm.W, kLd, ws_w + ch * kC * kD, kD, kC, kD, tid);
+      CopyRows(&sm.U[c & 1][0][0], kLdU, ws_ut + ch * kC * kD + vb * kRows, kD, kC, kRows, tid);
+      if (tid < kC / 4) __pipeline_memcpy_async(&sm.G[c & 1][tid * 4], ws_g + ch * kC + tid * 4, 16);
     }
     __pipeline_commit();
   };
+  auto issue_rows = [&](float* dst, const float* src, int c) {     // token rows of q or k (clamped past the end)
+    if (c < chunks) {
+      for (int i = tid; i < kC * (kD / 4); i += kScanThreads) {
+        const int r = i / (kD / 4), off = (i % (kD / 4)) * 4;
+        const int t = min(c * kC + r, T - 1);
+        __pipeline_memcpy_async(dst + r * kLd + off, src + (static_cast<size_t>(t) * Hk + hk) * kD + off, 16);
+      }
+    }
+    __pipeline_commit();
+  };
+  auto issue_p = [&](int c) {
+    if (c < chunks) CopyRows(sm.P, kLdP, ws_p + (static_cast<size_t>(c) * H + h) * kC * kC, kC, kC, kC, tid);
+    __pipeline_commit();
+  };
 
-  issue_wug(0, 0);
-  for (int i = tid; i < 32 * (kD / 4); i += 256) {
+  issue_wug(0);
+  issue_rows(sm.Q, q, 0);
+  issue_p(0);
+  for (int i = tid; i < kRows * (kD / 4); i += kScanThreads) {
     const int r = i / (kD / 4), off = (i % (kD / 4)) * 4;
     *reinterpret_cast<float4*>(&sm.S[r][off]) =
-        *reinterpret_cast<const float4*>(state + (static_cast<size_t>(h) * kD + vb * 32 + r) * kD + off);
+        *reinterpret_cast<const float4*>(state + (static_cast<size_t>(h) * kD + vb * kRows + r) * kD + off);
   }
 
   for (int c = 0; c < chunks; ++c) {
     const int buf = c & 1;
-    const size_t ch = static_cast<size_t>(c) * H + h;
-    __pipeline_wait_prior(0);
-    __syncthreads();                       // W, U~, G of this chunk have landed; the state block is complete
-    issue_qk(q, c, 1);
+    __pipeline_wait_prior(2);
+    __syncthreads();                       // W, U~, G of this chunk have landed; the state block is complete, K no longer read
+    issue_rows(sm.K, k, c);
     if (tid < kC) {
       sm.eG[tid] = expf(sm.G[buf][tid]);
       sm.fG[tid] = expf(sm.G[buf][kC - 1] - sm.G[buf][tid]);
     }
-    // ---- 1: U = U~ - W S^T   (64 x 32; warp: 16 rows x 16 columns) ----
+    // ---- 1: U = U~ - W S^T   (64 x kRows; warp: 16 rows x 16 columns) ----
     const int m0 = (warp & 3) * 16, nh = (warp >> 2) * 16;
     {
       float acc[2][4] = {};
-      MmaRowRow<2>(acc, sm.slot[0], m0, &sm.S[0][0], nh, lane);
+      MmaRowRow<2, true>(acc, sm.W, m0, &sm.S[0][0], nh, lane);
 #pragma unroll
       for (int nt = 0; nt < 2; ++nt) {
         float2* lo = reinterpret_cast<float2*>(&sm.U[buf][m0 + g][nh + nt * 8 + 2 * t4]);
@@ -276,13 +308,12 @@ __global__ void __launch_bounds__(256, 2) GdnChunkScanKernel(const float* __rest
         *hi = b;
       }
     }
-    __pipeline_wait_prior(0);
+    __pipeline_wait_prior(2);
     __syncthreads();                       // U complete, Q landed, W no longer read
-    CopyRows(sm.slot[0], kLdP, ws_p + ch * kC * kC, kC, kC, kC, tid);
-    __pipeline_commit();
+    issue_wug(c + 1);
     // ---- 2a: O = diag(gamma) Q S^T ----
     float oacc[2][4] = {};
-    MmaRowRow<2>(oacc, sm.slot[1], m0, &sm.S[0][0], nh, lane);
+    MmaRowRow<2, false>(oacc, sm.Q, m0, &sm.S[0][0], nh, lane);
     {
       const float e_lo = sm.eG[m0 + g], e_hi = sm.eG[m0 + g + 8];
 #pragma unroll
@@ -290,16 +321,15 @@ __global__ void __launch_bounds__(256, 2) GdnChunkScanKernel(const float* __rest
         oacc[nt][0] *= e_lo; oacc[nt][1] *= e_lo; oacc[nt][2] *= e_hi; oacc[nt][3] *= e_hi;
       }
     }
-    __pipeline_wait_prior(0);
+    __pipeline_wait_prior(2);
     __syncthreads();                       // P landed, Q no longer read
-    issue_qk(k, c, 1);
-    // ---- 2b: O += P U ----
+    issue_rows(sm.Q, q, c + 1);
+    // ---- 2b: O += P U   (P was written rounded) ----
     {
-      const float* P = sm.slot[0];
-#pragma unroll 2
+#pragma unroll 4
       for (int kb = 0; kb < kC / 8; ++kb) {
-        const uint32_t a0 = Tf32(P[(m0 + g) * kLdP + kb * 8 + t4]), a1 = Tf32(P[(m0 + g + 8) * kLdP + kb * 8 + t4]);
-        const uint32_t a2 = Tf32(P[(m0 + g) * kLdP + kb * 8 + t4 + 4]), a3 = Tf32(P[(m0 + g + 8) * kLdP + kb * 8 + t4 + 4]);
+        const uint32_t a0 = __float_as_uint(sm.P[(m0 + g) * kLdP + kb * 8 + t4]), a1 = __float_as_uint(sm.P[(m0 + g + 8) * kLdP + kb * 8 + t4]);
+        const uint32_t a2 = __float_as_uint(sm.P[(m0 + g) * kLdP + kb * 8 + t4 + 4]), a3 = __float_as_uint(sm.P[(m0 + g + 8) * kLdP + kb * 8 + t4 + 4]);
 #pragma unroll
         for (int nt = 0; nt < 2; ++nt) {
           const uint32_t b0 = Tf32(sm.U[buf][kb * 8 + t4][nh + nt * 8 + g]);
@@ -309,7 +339,7 @@ __global__ void __launch_bounds__(256, 2) GdnChunkScanKernel(const float* __rest
       }
 #pragma unroll
       for (int nt = 0; nt < 2; ++nt) {
-        const int col = vb * 32 + nh + nt * 8 + 2 * t4;
+        const int col = vb * kRows + nh + nt * 8 + 2 * t4;
         const int t_lo = c * kC + m0 + g, t_hi = t_lo + 8;
         if (t_lo < T)
           *reinterpret_cast<float2*>(o + (static_cast<size_t>(t_lo) * H + h) * kD + col) =
@@ -319,12 +349,12 @@ __global__ void __launch_bounds__(256, 2) GdnChunkScanKernel(const float* __rest
               make_float2(oacc[nt][2] * scale, oacc[nt][3] * scale);
       }
     }
-    __pipeline_wait_prior(0);
+    __pipeline_wait_prior(2);
     __syncthreads();                       // K landed, P no longer read
-    if (c + 1 < chunks) issue_wug(c + 1, buf ^ 1);
-    // ---- 3: S = gamma_C S + U^T diag(gamma_C / gamma) K   (32 x 128; warp: 16 rows x 32 columns) ----
+    issue_p(c + 1);
+    // ---- 3: S = gamma_C S + U^T diag(gamma_C / gamma) K   (kRows x 128; warp: 16 rows x 32 columns) ----
     {
-      const int sm0 = (warp & 1) * 16, sn0 = (warp >> 1) * 32;
+      const int sm0 = (warp & 3) * 16, sn0 = (warp >> 2) * 32;
       const float e_c = sm.eG[kC - 1];
       float acc[4][4];
 #pragma unroll
@@ -333,7 +363,6 @@ __global__ void __launch_bounds__(256, 2) GdnChunkScanKernel(const float* __rest
         const float2 hi = *reinterpret_cast<const float2*>(&sm.S[sm0 + g + 8][sn0 + nt * 8 + 2 * t4]);
         acc[nt][0] = lo.x * e_c; acc[nt][1] = lo.y * e_c; acc[nt][2] = hi.x * e_c; acc[nt][3] = hi.y * e_c;
       }
-      const float* Kt = sm.slot[1];
 #pragma unroll 2
       for (int kb = 0; kb < kC / 8; ++kb) {
         const int j0 = kb * 8 + t4, j1 = j0 + 4;
@@ -342,7 +371,7 @@ __global__ void __launch_bounds__(256, 2) GdnChunkScanKernel(const float* __rest
         const uint32_t a2 = Tf32(sm.U[buf][j1][sm0 + g] * f1), a3 = Tf32(sm.U[buf][j1][sm0 + g + 8] * f1);
 #pragma unroll
         for (int nt = 0; nt < 4; ++nt) {
-          const uint32_t b0 = Tf32(Kt[j0 * kLd + sn0 + nt * 8 + g]), b1 = Tf32(Kt[j1 * kLd + sn0 + nt * 8 + g]);
+          const uint32_t b0 = Tf32(sm.K[j0 * kLd + sn0 + nt * 8 + g]), b1 = Tf32(sm.K[j1 * kLd + sn0 + nt * 8 + g]);
           MmaTf32(acc[nt], a0, a1, a2, a3, b0, b1);
         }
       }
@@ -355,9 +384,9 @@ __global__ void __launch_bounds__(256, 2) GdnChunkScanKernel(const float* __rest
   }
   __pipeline_wait_prior(0);
   __syncthreads();
-  for (int i = tid; i < 32 * (kD / 4); i += 256) {
+  for (int i = tid; i < kRows * (kD / 4); i += kScanThreads) {
     const int r = i / (kD / 4), off = (i % (kD / 4)) * 4;
-    *reinterpret_cast<float4*>(state + (static_cast<size_t>(h) * kD + vb * 32 + r) * kD + off) =
+    *reinterpret_cast<float4*>(state + (static_cast<size_t>(h) * kD + vb * kRows + r) * kD + off) =
         *reinterpret_cast<const float4*>(&sm.S[r][off]);
   }
 }
@@ -382,7 +411,7 @@ int LaunchGdnChunked(const float* q, const float* k, const float* v, const float
   GdnChunkPrepKernel<<<dim3(chunks, H), 256, sizeof(PhaseASmem), s>>>(q, k, v, eg, beta, ws_ut, ws_w, ws_p, ws_g, T, H, Hk);
   int e = FinishLaunch();
   if (e) return e;
-  GdnChunkScanKernel<<<dim3(H, 4), 256, sizeof(PhaseBSmem), s>>>(q, k, ws_ut, ws_w, ws_p, ws_g, state, o, T, H, Hk);
+  GdnChunkScanKernel<<<dim3(H, kD / kRows), kScanThreads, sizeof(PhaseBSmem), s>>>(q, k, ws_ut, ws_w, ws_p, ws_g, state, o, T, H, Hk);
   return FinishLaunch();
 }
 
