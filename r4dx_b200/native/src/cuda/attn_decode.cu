@@ -95,6 +95,76 @@ __global__ void PrecoreKernel(PrecoreArgs a) {
   }
 }
 
+// The same for many rows (prompt chunks): one CTA per token, a warp per head, PER = D / 32 consecutive elements per lane.  The
+// rotation angles are one table per token, where the kernel above evaluates them in double precision for every head: that was
+// most of its 492 us at 8192 tokens of 32 heads (the bytes take 40).
+template <int PER>
+__global__ void __launch_bounds__(256) PrecoreRowsKernel(PrecoreArgs a) {
+  constexpr int D = PER * 32;
+  extern __shared__ float row[];
+  const int t = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int half = a.rotary_dim / 2, pos = a.positions[t];
+  float* cs = row;                           // [half] cosines, [half] sines
+  float* hrow = row + a.rotary_dim + warp * D;
+  for (int i = threadIdx.x; i < half; i += 256) {
+    const double inv = exp2(-log2(static_cast<double>(a.theta)) * (2.0 * i / a.rotary_dim));
+    double s, c;
+    sincos(static_cast<double>(pos) * inv, &s, &c);
+    cs[i] = static_cast<float>(c);
+    cs[half + i] = static_cast<float>(s);
+  }
+  __syncthreads();
+  const int blk = a.block_table[pos / kBlockTokens], tok = pos % kBlockTokens;
+  for (int hh = warp; hh < a.Hq + 2 * a.Hkv; hh += 8) {
+    const int kind = hh < a.Hq ? 0 : (hh < a.Hq + a.Hkv ? 1 : 2);      // 0 = q, 1 = k, 2 = v
+    const int head = kind == 0 ? hh : (kind == 1 ? hh - a.Hq : hh - a.Hq - a.Hkv);
+    const __nv_bfloat16* src = kind == 0 ? a.qg + (static_cast<size_t>(t) * a.Hq + head) * a.q_stride
+                                         : (kind == 1 ? a.k : a.v) + (static_cast<size_t>(t) * a.Hkv + head) * D;
+    float x[PER];
+#pragma unroll
+    for (int i = 0; i < PER; i += 2) {
+      const uint32_t p = *reinterpret_cast<const uint32_t*>(src + lane * PER + i);
+      x[i] = BfLo(p);
+      x[i + 1] = BfHi(p);
+    }
+    if (kind != 2) {
+      const __nv_bfloat16* nw = kind == 0 ? a.q_norm : a.k_norm;
+      if (nw != nullptr) {        // families without per-head q/k normalisation pass null
+        float ss = 0.f;
+#pragma unroll
+        for (int i = 0; i < PER; ++i) ss += x[i] * x[i];
+        const float r = rsqrtf(WarpSum(ss) / D + a.eps);
+#pragma unroll
+        for (int i = 0; i < PER; ++i) x[i] = x[i] * r * (1.0f + __bfloat162float(nw[lane * PER + i]));
+      }
+      __syncwarp();
+#pragma unroll
+      for (int i = 0; i < PER; ++i) hrow[lane * PER + i] = x[i];
+      __syncwarp();
+#pragma unroll
+      for (int i = 0; i < PER; ++i) {
+        const int d = lane * PER + i;
+        if (d < a.rotary_dim) {
+          const int j = d < half ? d : d - half;
+          const float fc = cs[j], fs = cs[half + j];
+          x[i] = d < half ? hrow[d] * fc - hrow[d + half] * fs : hrow[d] * fc + hrow[d - half] * fs;
+        }
+      }
+    }
+    if (kind == 0) {
+      __nv_bfloat16* dst = a.q_out + (static_cast<size_t>(t) * a.Hq + head) * D + lane * PER;
+#pragma unroll
+      for (int i = 0; i < PER; i += 2) *reinterpret_cast<uint32_t*>(dst + i) = PackBf16(x[i], x[i + 1]);
+    } else {
+      const float ds = (kind == 1 ? a.k_descale : a.v_descale)[head];
+      uint8_t* dst = a.cache + ((static_cast<size_t>(blk) * a.Hkv + head) * 2 + (kind - 1)) * kBlockTokens * D + tok * D + lane * PER;
+#pragma unroll
+      for (int i = 0; i < PER; i += 2)
+        *reinterpret_cast<uint16_t*>(dst + i) = static_cast<uint16_t>(ToFp8(x[i] / ds)) | static_cast<uint16_t>(ToFp8(x[i + 1] / ds)) << 8;
+    }
+  }
+}
+
 struct DecodeArgs {
   const __nv_bfloat16* q;      // [T, Hq, D] (normed + roped)
   const uint8_t* cache;
@@ -635,6 +705,15 @@ int r4dxb_attn_precore(const void* qg, const void* k, const void* v, const void*
   a.T = T; a.Hq = Hq; a.Hkv = Hkv; a.D = D; a.rotary_dim = rotary_dim; a.theta = theta; a.eps = eps;
   a.row_slot = nullptr; a.table_stride = 0;
   a.q_stride = q_stride > 0 ? q_stride : 2 * D;
+  // more rows than a decode step has, and 4-byte bases for the pair loads (the head widths of every family here)
+  const uintptr_t bases = reinterpret_cast<uintptr_t>(qg) | reinterpret_cast<uintptr_t>(k) | reinterpret_cast<uintptr_t>(v) |
+                          reinterpret_cast<uintptr_t>(q_out) | reinterpret_cast<uintptr_t>(cache);
+  if (T > 8 && (D == 64 || D == 128 || D == 256) && (bases & 3) == 0 && a.q_stride % 2 == 0) {
+    const size_t smem = (rotary_dim + 8 * D) * sizeof(float);
+    auto kern = D == 64 ? PrecoreRowsKernel<2> : (D == 128 ? PrecoreRowsKernel<4> : PrecoreRowsKernel<8>);
+    kern<<<T, 256, smem, static_cast<cudaStream_t>(stream)>>>(a);
+    return FinishLaunch();
+  }
   return LaunchPdl(PrecoreKernel, dim3(Hq + 2 * Hkv, T), dim3(D), D * sizeof(float), static_cast<cudaStream_t>(stream), a);
 }
 
