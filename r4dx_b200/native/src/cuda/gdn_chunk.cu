@@ -16,7 +16,7 @@
 //           accumulate) out of shared memory; W, Q, P and K have a cp.async slot each that is refilled for the
 //           next chunk as soon as its product is done, three products ahead of its use (two shared slots fetched one
 //           product ahead left every one of the four products of a chunk waiting for its operand: 14k clocks a
-//           chunk where the products take about five).  The fp32 state block lives in shared memory for
+//           chunk where the products take about five).  The fp32 state block lives in registers for
 //           the whole sequence.
 // The per-token recurrence (gdn_prefill.cu) stays as the reference path and for D = 64
 // (reference: third_party/libr4d/r4d_gdn_chunk_scan_k128_v128_c64_bf16.hip:1-60 runs the same
@@ -193,6 +193,10 @@ struct PhaseBSmem {
   float fG[kC];
 };
 
+// The same rounding (half away from zero) in two integer instructions: conversions run at a quarter of their rate, and the scan
+// needs thousands of them per chunk.  (Only a NaN with all mantissa bits set would come out differently.)
+__device__ __forceinline__ uint32_t RoundTf32(float x) { return (__float_as_uint(x) + 0x1000u) & 0xFFFFE000u; }
+
 __device__ __forceinline__ void MmaTf32(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
                                         uint32_t b1) {
   asm volatile(
@@ -204,7 +208,7 @@ __device__ __forceinline__ void MmaTf32(float (&c)[4], uint32_t a0, uint32_t a1,
 // acc[nt] += A[m0 .. m0+16, 0 .. 128) * S[n0 + 8 nt .. +8, 0 .. 128)^T, both row-major along the contraction.
 // Inside every block of 8 contraction columns the hardware index t maps to column 2t and t + 4 to 2t + 1, so
 // that one 8-byte load feeds two fragment registers; A and B use the same map, so the product is unchanged.
-// kRounded: A already holds TF32 values.
+// kRounded: A already holds TF32 values (S always does).
 template <int NT, bool kRounded>
 __device__ __forceinline__ void MmaRowRow(float (&acc)[NT][4], const float* __restrict__ A, int m0, const float* __restrict__ S,
                                           int n0, int lane) {
@@ -216,12 +220,12 @@ __device__ __forceinline__ void MmaRowRow(float (&acc)[NT][4], const float* __re
   for (int kb = 0; kb < kD / 8; ++kb) {
     const float2 lo = *reinterpret_cast<const float2*>(a_lo + kb * 8);
     const float2 hi = *reinterpret_cast<const float2*>(a_hi + kb * 8);
-    const uint32_t a0 = kRounded ? __float_as_uint(lo.x) : Tf32(lo.x), a2 = kRounded ? __float_as_uint(lo.y) : Tf32(lo.y);
-    const uint32_t a1 = kRounded ? __float_as_uint(hi.x) : Tf32(hi.x), a3 = kRounded ? __float_as_uint(hi.y) : Tf32(hi.y);
+    const uint32_t a0 = kRounded ? __float_as_uint(lo.x) : RoundTf32(lo.x), a2 = kRounded ? __float_as_uint(lo.y) : RoundTf32(lo.y);
+    const uint32_t a1 = kRounded ? __float_as_uint(hi.x) : RoundTf32(hi.x), a3 = kRounded ? __float_as_uint(hi.y) : RoundTf32(hi.y);
 #pragma unroll
     for (int nt = 0; nt < NT; ++nt) {
       const float2 b = *reinterpret_cast<const float2*>(b_base + nt * 8 * kLd + kb * 8);
-      MmaTf32(acc[nt], a0, a1, a2, a3, Tf32(b.x), Tf32(b.y));
+      MmaTf32(acc[nt], a0, a1, a2, a3, __float_as_uint(b.x), __float_as_uint(b.y));
     }
   }
 }
@@ -278,11 +282,25 @@ __global__ void __launch_bounds__(kScanThreads, 1) GdnChunkScanKernel(const floa
   issue_wug(0);
   issue_rows(sm.Q, q, 0);
   issue_p(0);
-  for (int i = tid; i < kRows * (kD / 4); i += kScanThreads) {
-    const int r = i / (kD / 4), off = (i % (kD / 4)) * 4;
-    *reinterpret_cast<float4*>(&sm.S[r][off]) =
-        *reinterpret_cast<const float4*>(state + (static_cast<size_t>(h) * kD + vb * kRows + r) * kD + off);
+  // The fp32 state stays in registers in the accumulator layout of product 3 (a warp: 16 rows x 32 columns); shared memory
+  // holds its TF32 rounding, which is what products 1 and 2a read.
+  const int sm0 = (warp & 3) * 16, sn0 = (warp >> 2) * 32;
+  float* s_lo = state + (static_cast<size_t>(h) * kD + vb * kRows + sm0 + g) * kD + sn0 + 2 * t4;
+  float* s_hi = s_lo + 8 * kD;
+  float st[4][4];
+#pragma unroll
+  for (int nt = 0; nt < 4; ++nt) {
+    const float2 lo = *reinterpret_cast<const float2*>(s_lo + nt * 8), hi = *reinterpret_cast<const float2*>(s_hi + nt * 8);
+    st[nt][0] = lo.x; st[nt][1] = lo.y; st[nt][2] = hi.x; st[nt][3] = hi.y;
   }
+  auto publish = [&] {
+#pragma unroll
+    for (int nt = 0; nt < 4; ++nt) {
+      *reinterpret_cast<uint2*>(&sm.S[sm0 + g][sn0 + nt * 8 + 2 * t4]) = make_uint2(RoundTf32(st[nt][0]), RoundTf32(st[nt][1]));
+      *reinterpret_cast<uint2*>(&sm.S[sm0 + g + 8][sn0 + nt * 8 + 2 * t4]) = make_uint2(RoundTf32(st[nt][2]), RoundTf32(st[nt][3]));
+    }
+  };
+  publish();
 
   for (int c = 0; c < chunks; ++c) {
     const int buf = c & 1;
@@ -332,8 +350,8 @@ __global__ void __launch_bounds__(kScanThreads, 1) GdnChunkScanKernel(const floa
         const uint32_t a2 = __float_as_uint(sm.P[(m0 + g) * kLdP + kb * 8 + t4 + 4]), a3 = __float_as_uint(sm.P[(m0 + g + 8) * kLdP + kb * 8 + t4 + 4]);
 #pragma unroll
         for (int nt = 0; nt < 2; ++nt) {
-          const uint32_t b0 = Tf32(sm.U[buf][kb * 8 + t4][nh + nt * 8 + g]);
-          const uint32_t b1 = Tf32(sm.U[buf][kb * 8 + t4 + 4][nh + nt * 8 + g]);
+          const uint32_t b0 = RoundTf32(sm.U[buf][kb * 8 + t4][nh + nt * 8 + g]);
+          const uint32_t b1 = RoundTf32(sm.U[buf][kb * 8 + t4 + 4][nh + nt * 8 + g]);
           MmaTf32(oacc[nt], a0, a1, a2, a3, b0, b1);
         }
       }
@@ -354,40 +372,31 @@ __global__ void __launch_bounds__(kScanThreads, 1) GdnChunkScanKernel(const floa
     issue_p(c + 1);
     // ---- 3: S = gamma_C S + U^T diag(gamma_C / gamma) K   (kRows x 128; warp: 16 rows x 32 columns) ----
     {
-      const int sm0 = (warp & 3) * 16, sn0 = (warp >> 2) * 32;
       const float e_c = sm.eG[kC - 1];
-      float acc[4][4];
 #pragma unroll
-      for (int nt = 0; nt < 4; ++nt) {
-        const float2 lo = *reinterpret_cast<const float2*>(&sm.S[sm0 + g][sn0 + nt * 8 + 2 * t4]);
-        const float2 hi = *reinterpret_cast<const float2*>(&sm.S[sm0 + g + 8][sn0 + nt * 8 + 2 * t4]);
-        acc[nt][0] = lo.x * e_c; acc[nt][1] = lo.y * e_c; acc[nt][2] = hi.x * e_c; acc[nt][3] = hi.y * e_c;
-      }
+      for (int nt = 0; nt < 4; ++nt)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) st[nt][i] *= e_c;
 #pragma unroll 2
       for (int kb = 0; kb < kC / 8; ++kb) {
         const int j0 = kb * 8 + t4, j1 = j0 + 4;
         const float f0 = sm.fG[j0], f1 = sm.fG[j1];
-        const uint32_t a0 = Tf32(sm.U[buf][j0][sm0 + g] * f0), a1 = Tf32(sm.U[buf][j0][sm0 + g + 8] * f0);
-        const uint32_t a2 = Tf32(sm.U[buf][j1][sm0 + g] * f1), a3 = Tf32(sm.U[buf][j1][sm0 + g + 8] * f1);
+        const uint32_t a0 = RoundTf32(sm.U[buf][j0][sm0 + g] * f0), a1 = RoundTf32(sm.U[buf][j0][sm0 + g + 8] * f0);
+        const uint32_t a2 = RoundTf32(sm.U[buf][j1][sm0 + g] * f1), a3 = RoundTf32(sm.U[buf][j1][sm0 + g + 8] * f1);
 #pragma unroll
         for (int nt = 0; nt < 4; ++nt) {
-          const uint32_t b0 = Tf32(sm.K[j0 * kLd + sn0 + nt * 8 + g]), b1 = Tf32(sm.K[j1 * kLd + sn0 + nt * 8 + g]);
-          MmaTf32(acc[nt], a0, a1, a2, a3, b0, b1);
+          const uint32_t b0 = RoundTf32(sm.K[j0 * kLd + sn0 + nt * 8 + g]), b1 = RoundTf32(sm.K[j1 * kLd + sn0 + nt * 8 + g]);
+          MmaTf32(st[nt], a0, a1, a2, a3, b0, b1);
         }
       }
-#pragma unroll
-      for (int nt = 0; nt < 4; ++nt) {
-        *reinterpret_cast<float2*>(&sm.S[sm0 + g][sn0 + nt * 8 + 2 * t4]) = make_float2(acc[nt][0], acc[nt][1]);
-        *reinterpret_cast<float2*>(&sm.S[sm0 + g + 8][sn0 + nt * 8 + 2 * t4]) = make_float2(acc[nt][2], acc[nt][3]);
-      }
+      publish();
     }
   }
   __pipeline_wait_prior(0);
-  __syncthreads();
-  for (int i = tid; i < kRows * (kD / 4); i += kScanThreads) {
-    const int r = i / (kD / 4), off = (i % (kD / 4)) * 4;
-    *reinterpret_cast<float4*>(state + (static_cast<size_t>(h) * kD + vb * kRows + r) * kD + off) =
-        *reinterpret_cast<const float4*>(&sm.S[r][off]);
+#pragma unroll
+  for (int nt = 0; nt < 4; ++nt) {
+    *reinterpret_cast<float2*>(s_lo + nt * 8) = make_float2(st[nt][0], st[nt][1]);
+    *reinterpret_cast<float2*>(s_hi + nt * 8) = make_float2(st[nt][2], st[nt][3]);
   }
 }
 
