@@ -456,41 +456,110 @@ TrellisGemmKernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
 }
 
 // ---- input transform: Xh = fp16(H128(suh * x)) -------------------------------------------------------
-// one warp per 128-block; producer variants fold the preceding elementwise op into the transform
-// (reference: src/kernels/src/trellis_transform.hip:84-486 fuses the same producers).
+// Sixteen lanes per 128-column block, eight columns each (16-byte loads and stores); producer variants fold the preceding
+// elementwise op into the transform (reference: src/kernels/src/trellis_transform.hip:84-486 fuses the same producers).
 //   mode 0: x = in[t, k]                      (in: [T, K])
 //   mode 1: x = silu(in[t, k]) * in[t, K + k] (in: [T, 2K] fused gate|up rows); mode 2: the same with a tanh-GELU gate
-__global__ void TrellisInputKernel(const __nv_bfloat16* __restrict__ in, const __half* __restrict__ suh,
-                                   __half* __restrict__ out, int T, int K, int mode) {
-  const int lane = threadIdx.x & 31;
-  const int blocks_per_row = K / 128;
-  const long long item = static_cast<long long>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (item >= static_cast<long long>(T) * blocks_per_row) return;
-  const int t = static_cast<int>(item / blocks_per_row), b = static_cast<int>(item % blocks_per_row);
-  const int k = b * 128 + lane * 4;
-  float v[4];
-  if (mode == 0) {
-    const uint2 xv = *reinterpret_cast<const uint2*>(in + static_cast<size_t>(t) * K + k);
-    v[0] = BfLo(xv.x); v[1] = BfHi(xv.x); v[2] = BfLo(xv.y); v[3] = BfHi(xv.y);
+// Bound by memory; what costs is latency and instructions, so a half-warp takes R rows of one block (their loads are in flight
+// together, the signs are read once) and half of the Hadamard stages stay inside a lane: 115 -> 76 us on average over the
+// products of 8192 rows.
+__device__ __forceinline__ void Fwht128Half(float (&v)[8]) {
+  const int lane = threadIdx.x & 15;
+#pragma unroll
+  for (int m = 1; m < 8; m <<= 1)
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+      if (!(i & m)) {
+        const float a = v[i], b = v[i | m];
+        v[i] = a + b;
+        v[i | m] = a - b;
+      }
+#pragma unroll
+  for (int m = 1; m < 16; m <<= 1) {
+    const float sign = (lane & m) ? -1.f : 1.f;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[i] = fmaf(v[i], sign, __shfl_xor_sync(0xffffffffu, v[i], m));
+  }
+}
+
+// 16 bytes at p, as two halves where a base is only 8-byte aligned
+__device__ __forceinline__ uint4 Load16(const void* p, bool a16) {
+  if (a16) return *static_cast<const uint4*>(p);
+  const uint2 lo = static_cast<const uint2*>(p)[0], hi = static_cast<const uint2*>(p)[1];
+  return make_uint4(lo.x, lo.y, hi.x, hi.y);
+}
+__device__ __forceinline__ void Store16(void* p, const uint4& v, bool a16) {
+  if (a16) {
+    *static_cast<uint4*>(p) = v;
   } else {
-    const uint2 g = *reinterpret_cast<const uint2*>(in + static_cast<size_t>(t) * 2 * K + k);
-    const uint2 u = *reinterpret_cast<const uint2*>(in + static_cast<size_t>(t) * 2 * K + K + k);
+    static_cast<uint2*>(p)[0] = make_uint2(v.x, v.y);
+    static_cast<uint2*>(p)[1] = make_uint2(v.z, v.w);
+  }
+}
+
+__device__ __forceinline__ void Unpack8(const uint4& p, float (&v)[8]) {
+  v[0] = BfLo(p.x); v[1] = BfHi(p.x); v[2] = BfLo(p.y); v[3] = BfHi(p.y);
+  v[4] = BfLo(p.z); v[5] = BfHi(p.z); v[6] = BfLo(p.w); v[7] = BfHi(p.w);
+}
+
+// eight columns: act, signs, Hadamard, fp16
+__device__ __forceinline__ uint4 TransformBlock(const uint4& x, const uint4& u, const uint4& sv, int mode) {
+  float v[8];
+  Unpack8(x, v);
+  if (mode != 0) {
     // the product is rounded to bf16 exactly like the unfused silu_mul kernel rounds it
     const int act = mode == 2 ? 1 : 0;
-    const uint32_t p01 = PackBf16(GateAct(BfLo(g.x), act) * BfLo(u.x), GateAct(BfHi(g.x), act) * BfHi(u.x));
-    const uint32_t p23 = PackBf16(GateAct(BfLo(g.y), act) * BfLo(u.y), GateAct(BfHi(g.y), act) * BfHi(u.y));
-    v[0] = BfLo(p01); v[1] = BfHi(p01); v[2] = BfLo(p23); v[3] = BfHi(p23);
+    float w[8];
+    Unpack8(u, w);
+#pragma unroll
+    for (int i = 0; i < 8; i += 2) {
+      const uint32_t p = PackBf16(GateAct(v[i], act) * w[i], GateAct(v[i + 1], act) * w[i + 1]);
+      v[i] = BfLo(p);
+      v[i + 1] = BfHi(p);
+    }
   }
-  const uint2 sv = *reinterpret_cast<const uint2*>(suh + k);
-  const __half2 s01 = *reinterpret_cast<const __half2*>(&sv.x), s23 = *reinterpret_cast<const __half2*>(&sv.y);
-  v[0] *= __low2float(s01); v[1] *= __high2float(s01); v[2] *= __low2float(s23); v[3] *= __high2float(s23);
-  WarpFwht128(v);
+  const uint32_t s[4] = {sv.x, sv.y, sv.z, sv.w};
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const __half2 h = *reinterpret_cast<const __half2*>(&s[i]);
+    v[2 * i] *= __low2float(h);
+    v[2 * i + 1] *= __high2float(h);
+  }
+  Fwht128Half(v);
   const float inv_sqrt = 0.08838834764831845f;
-  __half2 o01 = __floats2half2_rn(v[0] * inv_sqrt, v[1] * inv_sqrt), o23 = __floats2half2_rn(v[2] * inv_sqrt, v[3] * inv_sqrt);
-  uint2 ov;
-  ov.x = *reinterpret_cast<uint32_t*>(&o01);
-  ov.y = *reinterpret_cast<uint32_t*>(&o23);
-  *reinterpret_cast<uint2*>(out + static_cast<size_t>(t) * K + k) = ov;
+  uint32_t o[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const __half2 h = __floats2half2_rn(v[2 * i] * inv_sqrt, v[2 * i + 1] * inv_sqrt);
+    o[i] = *reinterpret_cast<const uint32_t*>(&h);
+  }
+  return make_uint4(o[0], o[1], o[2], o[3]);
+}
+
+template <int R>
+__global__ void __launch_bounds__(256) TrellisInputKernel(const __nv_bfloat16* __restrict__ in, const __half* __restrict__ suh,
+                                                          __half* __restrict__ out, int T, int K, int mode, bool a16) {
+  const int blocks_per_row = K / 128;
+  const long long items = static_cast<long long>((T + R - 1) / R) * blocks_per_row;
+  long long item = (static_cast<long long>(blockIdx.x) * 256 + threadIdx.x) >> 4;
+  const bool live = item < items;                       // (both halves of a warp take part in its shuffles)
+  if (!live) item = items - 1;
+  const int t0 = static_cast<int>(item / blocks_per_row) * R;
+  const int k = static_cast<int>(item % blocks_per_row) * 128 + (threadIdx.x & 15) * 8;
+  const size_t stride = mode == 0 ? K : 2 * static_cast<size_t>(K);
+  const uint4 sv = Load16(suh + k, a16);
+  uint4 x[R], u[R];
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    const int t = min(t0 + r, T - 1);
+    x[r] = Load16(in + t * stride + k, a16);
+    u[r] = mode == 0 ? make_uint4(0u, 0u, 0u, 0u) : Load16(in + t * stride + K + k, a16);
+  }
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    const uint4 o = TransformBlock(x[r], u[r], sv, mode);
+    if (live && t0 + r < T) Store16(out + static_cast<size_t>(t0 + r) * K + k, o, a16);
+  }
 }
 
 // ---- grouped experts: tile list and per-expert input transform ---------------------------------------
@@ -520,46 +589,38 @@ __global__ void MoeTilesKernel(const int* __restrict__ offsets, int E, int tn, i
   if (e == 1023) *ntiles = min(scan[1023], max_tiles);
 }
 
-// xh[p] = fp16(H128(suh[e(p)] * act(in[perm[p] / xdiv]))) for every planned pair p (sorted by expert); one warp per
-// 128-block.  The expert of a sorted position is found by bisection of the offsets.
-__global__ void TrellisInputGroupedKernel(const __nv_bfloat16* __restrict__ in, const __half* __restrict__ suh,
-                                          __half* __restrict__ out, const int* __restrict__ offsets,
-                                          const int* __restrict__ perm, int E, int P, int K, int xdiv, int mode) {
-  const int lane = threadIdx.x & 31;
-  const int blocks_per_row = K / 128;
-  const long long item = static_cast<long long>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (item >= static_cast<long long>(P) * blocks_per_row) return;
-  const int p = static_cast<int>(item / blocks_per_row), b = static_cast<int>(item % blocks_per_row);
-  if (p >= __ldg(offsets + E)) return;
+// xh[p] = fp16(H128(suh[e(p)] * act(in[perm[p] / xdiv]))) for every planned pair p (sorted by expert); a warp takes
+// 2 * kPasses blocks of one pair (grid.y covers the rest of a row), so that the expert of the pair - found by bisection of the
+// offsets - and its row are looked up once and the loads of all its blocks are in flight together.
+constexpr int kPasses = 4;
+__global__ void __launch_bounds__(256) TrellisInputGroupedKernel(const __nv_bfloat16* __restrict__ in, const __half* __restrict__ suh,
+                                                                 __half* __restrict__ out, const int* __restrict__ offsets,
+                                                                 const int* __restrict__ perm, int E, int P, int K, int xdiv, int mode, bool a16) {
+  const int p = blockIdx.x * 8 + (threadIdx.x >> 5), half = (threadIdx.x >> 4) & 1;
+  if (p >= P || p >= __ldg(offsets + E)) return;
   int lo = 0, hi = E;                                  // largest e with offsets[e] <= p
   while (hi - lo > 1) {
     const int mid = (lo + hi) >> 1;
     if (__ldg(offsets + mid) <= p) lo = mid; else hi = mid;
   }
   const int t = __ldg(perm + p) / xdiv;
-  const int k = b * 128 + lane * 4;
-  float v[4];
-  if (mode == 0) {
-    const uint2 xv = *reinterpret_cast<const uint2*>(in + static_cast<size_t>(t) * K + k);
-    v[0] = BfLo(xv.x); v[1] = BfHi(xv.x); v[2] = BfLo(xv.y); v[3] = BfHi(xv.y);
-  } else {
-    const uint2 g = *reinterpret_cast<const uint2*>(in + static_cast<size_t>(t) * 2 * K + k);
-    const uint2 u = *reinterpret_cast<const uint2*>(in + static_cast<size_t>(t) * 2 * K + K + k);
-    const int act = mode == 2 ? 1 : 0;
-    const uint32_t p01 = PackBf16(GateAct(BfLo(g.x), act) * BfLo(u.x), GateAct(BfHi(g.x), act) * BfHi(u.x));
-    const uint32_t p23 = PackBf16(GateAct(BfLo(g.y), act) * BfLo(u.y), GateAct(BfHi(g.y), act) * BfHi(u.y));
-    v[0] = BfLo(p01); v[1] = BfHi(p01); v[2] = BfLo(p23); v[3] = BfHi(p23);
+  const __nv_bfloat16* row = in + static_cast<size_t>(t) * (mode == 0 ? K : 2 * static_cast<size_t>(K));
+  const __half* sg = suh + static_cast<size_t>(lo) * K;
+  const int b0 = blockIdx.y * 2 * kPasses + half, blocks = K / 128;
+  uint4 x[kPasses], u[kPasses], sv[kPasses];
+#pragma unroll
+  for (int i = 0; i < kPasses; ++i) {
+    const int k = min(b0 + 2 * i, blocks - 1) * 128 + (threadIdx.x & 15) * 8;
+    x[i] = Load16(row + k, a16);
+    u[i] = mode == 0 ? make_uint4(0u, 0u, 0u, 0u) : Load16(row + K + k, a16);
+    sv[i] = Load16(sg + k, a16);
   }
-  const uint2 sv = *reinterpret_cast<const uint2*>(suh + static_cast<size_t>(lo) * K + k);
-  const __half2 s01 = *reinterpret_cast<const __half2*>(&sv.x), s23 = *reinterpret_cast<const __half2*>(&sv.y);
-  v[0] *= __low2float(s01); v[1] *= __high2float(s01); v[2] *= __low2float(s23); v[3] *= __high2float(s23);
-  WarpFwht128(v);
-  const float inv_sqrt = 0.08838834764831845f;
-  __half2 o01 = __floats2half2_rn(v[0] * inv_sqrt, v[1] * inv_sqrt), o23 = __floats2half2_rn(v[2] * inv_sqrt, v[3] * inv_sqrt);
-  uint2 ov;
-  ov.x = *reinterpret_cast<uint32_t*>(&o01);
-  ov.y = *reinterpret_cast<uint32_t*>(&o23);
-  *reinterpret_cast<uint2*>(out + static_cast<size_t>(p) * K + k) = ov;
+#pragma unroll
+  for (int i = 0; i < kPasses; ++i) {
+    if (blockIdx.y * 2 * kPasses + 2 * i >= blocks) break;          // (uniform over the warp)
+    const uint4 o = TransformBlock(x[i], u[i], sv[i], mode);
+    if (b0 + 2 * i < blocks) Store16(out + static_cast<size_t>(p) * K + (b0 + 2 * i) * 128 + (threadIdx.x & 15) * 8, o, a16);
+  }
 }
 
 // ---- 8-bit activations: xq = e4m3(xh / scale), scale = rowmax |xh| / 448, one CTA per row ---------------------------
@@ -597,6 +658,10 @@ __global__ void __launch_bounds__(256) QuantizeRowsE4m3Kernel(const __half* __re
     }
     *reinterpret_cast<uint2*>(out + k) = make_uint2(o[0], o[1]);
   }
+}
+
+bool Aligned16(const void* a, const void* b, const void* c) {
+  return ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(c)) & 15) == 0;
 }
 
 int g_decode_warps = 16;
@@ -703,11 +768,11 @@ extern "C" {
 
 int r4dxb_trellis_input(const void* in, const void* suh, void* out, int T, int K, int mode, void* stream) {
   if (T < 1 || K % 128 || mode < 0 || mode > 2) return R4DXB_BAD_ARG;
-  const long long items = static_cast<long long>(T) * (K / 128);
-  const int warps_per_cta = 8;
-  TrellisInputKernel<<<static_cast<unsigned>((items + warps_per_cta - 1) / warps_per_cta), warps_per_cta * 32, 0,
-                       static_cast<cudaStream_t>(stream)>>>(static_cast<const __nv_bfloat16*>(in),
-                                                            static_cast<const __half*>(suh), static_cast<__half*>(out), T, K, mode);
+  // four rows per half-warp once there are enough of them to fill the machine that way (64 rows: 2.5 us with one, 4.4 with four)
+  const int r = T >= 512 ? 4 : 1;
+  const long long items = static_cast<long long>((T + r - 1) / r) * (K / 128);
+  (r == 4 ? TrellisInputKernel<4> : TrellisInputKernel<1>)<<<static_cast<unsigned>((items + 15) / 16), 256, 0, static_cast<cudaStream_t>(stream)>>>(
+      static_cast<const __nv_bfloat16*>(in), static_cast<const __half*>(suh), static_cast<__half*>(out), T, K, mode, Aligned16(in, suh, out));
   return FinishLaunch();
 }
 
@@ -795,10 +860,10 @@ int r4dxb_moe_tiles(const int* offsets, int E, int tn, int* tiles, int* ntiles, 
 int r4dxb_trellis_input_grouped(const void* in, const void* suh, void* out, const int* offsets, const int* perm, int E, int P,
                                 int K, int xdiv, int mode, void* stream) {
   if (P < 1 || K % 128 || xdiv < 1 || mode < 0 || mode > 2) return R4DXB_BAD_ARG;
-  const long long items = static_cast<long long>(P) * (K / 128);
-  TrellisInputGroupedKernel<<<static_cast<unsigned>((items + 7) / 8), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<const __nv_bfloat16*>(in), static_cast<const __half*>(suh), static_cast<__half*>(out), offsets, perm, E, P, K,
-      xdiv, mode);
+  const dim3 grid((P + 7) / 8, (K / 128 + 2 * kPasses - 1) / (2 * kPasses));
+  TrellisInputGroupedKernel<<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(
+      static_cast<const __nv_bfloat16*>(in), static_cast<const __half*>(suh), static_cast<__half*>(out), offsets, perm, E, P, K, xdiv, mode,
+      Aligned16(in, suh, out));
   return FinishLaunch();
 }
 

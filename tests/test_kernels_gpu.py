@@ -974,3 +974,73 @@ def test_linear_tc_w8a16_matches_fp32_reference(K, T, N, Kd, group):
     assert torch.allclose(y.cpu(), ref, atol=2e-2, rtol=1e-2)
     y2 = K.linear_tc(w.to("cuda"), x.cuda(), residual=res.cuda())
     assert torch.allclose(y2.float().cpu(), ref + res.float(), atol=6e-2, rtol=2e-2)
+
+
+@pytest.mark.parametrize("T,Kd", [(1, 128), (3, 384), (17, 2048), (515, 640), (1027, 128)])
+def test_trellis_input_bases_and_row_counts(K, T, Kd):
+    """The input transform over row counts that do not divide its row groups, and with bases that are only 8-byte aligned
+    (split loads): both give the bits of the aligned call, which match the reference to fp16."""
+    from r4dx_b200.ops import reference as R
+    g = torch.Generator().manual_seed(T)
+    x = torch.randn(T, 2 * Kd, generator=g).to(BF)
+    suh = torch.randn(Kd, generator=g).to(torch.float16)
+    for fused in (False, True):
+        xi = x if fused else x[:, :Kd].contiguous()
+        out = K.trellis_input(xi.cuda(), suh.cuda(), fused_silu_mul=fused)
+        act = R.silu_mul(x.float()).to(BF).float() if fused else xi.float()
+        assert torch.allclose(out.float().cpu(), R.fwht(act * suh.float()[None]), atol=2e-2, rtol=1e-2)
+        odd = torch.empty(xi.numel() + 4, dtype=BF, device="cuda")[4:].view(xi.shape)
+        odd.copy_(xi)
+        assert odd.data_ptr() % 16 == 8
+        assert torch.equal(K.trellis_input(odd, suh.cuda(), fused_silu_mul=fused), out)
+
+
+@pytest.mark.parametrize("D,T,pos0", [(64, 17, 0), (128, 35, 5), (128, 16, 3)])
+def test_gdn_prefill_odd_bases_equal_aligned_ones(K, D, T, pos0):
+    """Token counts around the 16-token groups of the convolution, a ring carried in, and bases of the bf16 operands that
+    rule vector loads out."""
+    g = torch.Generator().manual_seed(T)
+    H, Hk = 4, 2
+    conv_dim = 2 * Hk * D + H * D
+    mixed, z = torch.randn(T, conv_dim, generator=g).to(BF).cuda(), torch.randn(T, H * D, generator=g).to(BF).cuda()
+    ab = torch.randn(T, 2 * H, generator=g).cuda()
+    conv_w, nw = torch.randn(conv_dim, 4, generator=g).to(BF).cuda(), torch.rand(D, generator=g).to(BF).cuda()
+    A_log, dt = torch.randn(H, generator=g).cuda() * 0.2, torch.randn(H, generator=g).cuda()
+    ring0 = torch.randn(16, conv_dim, generator=g).to(BF).cuda()
+
+    def run(shift):
+        def at(t):
+            o = torch.empty(t.numel() + shift, dtype=t.dtype, device="cuda")[shift:].view(t.shape)
+            return o.copy_(t)
+        # (the fp32 scratch is copied asynchronously in 16-byte pieces and has to be aligned)
+        sc = {n: torch.zeros(T, h, D, device="cuda") for n, h in (("q", Hk), ("k", Hk), ("v", H), ("o", H))}
+        sc.update(eg=torch.zeros(T, H, device="cuda"), beta=torch.zeros(T, H, device="cuda"))
+        state, ring, out = torch.zeros(H, D, D, device="cuda"), at(ring0), at(torch.zeros(T, H * D, dtype=BF, device="cuda"))
+        K.gdn_prefill(at(mixed), at(z), ab, conv_w, A_log, dt, at(nw), ring, state, sc, out, T, H, Hk, D, pos0, 1e-6)
+        return sc["q"], sc["v"], state, ring, out
+
+    for a, b in zip(run(0), run(1 if D == 64 else 3)):
+        assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("D,Hq,Hkv,rot", [(256, 6, 2, 64), (128, 4, 1, 128), (64, 3, 3, 16)])
+def test_attention_precore_of_many_rows_equals_few_row_calls(K, D, Hq, Hkv, rot):
+    """The per-token kernel of prompt chunks against the per-head kernel of decode calls: same formulas, the sum of squares in
+    another order (a last-bit change of the norm factor: one bf16 / fp8 step where a value sits on a rounding edge)."""
+    g = torch.Generator().manual_seed(D)
+    T, nblk = 41, 4
+    qg, k, v = (torch.randn(T, n, generator=g).to(BF).cuda() for n in (Hq * 2 * D, Hkv * D, Hkv * D))
+    qn, kn = (torch.randn(D, generator=g) * 0.1).to(BF).cuda(), (torch.randn(D, generator=g) * 0.1).to(BF).cuda()
+    ds = torch.full((Hkv,), 0.02, device="cuda")
+    pos = torch.arange(7, 7 + T, dtype=torch.int32, device="cuda")
+    table = torch.arange(nblk, dtype=torch.int32, device="cuda").flip(0).contiguous()
+    outs = []
+    for step in (T, 8):
+        q, cache = torch.zeros(T, Hq * D, dtype=BF, device="cuda"), torch.zeros(nblk, Hkv, 2, 16, D, dtype=torch.uint8, device="cuda")
+        for s in range(0, T, step):
+            e = min(T, s + step)
+            K.attn_precore(qg[s:e], k[s:e], v[s:e], qn, kn, ds, ds, pos[s:e], table, q[s:e], cache, e - s, Hq, Hkv, D, rot, 1e6, 1e-6)
+        outs.append((q.float(), cache.view(torch.float8_e4m3fn).float()))
+    (q1, c1), (q8, c8) = outs
+    assert ((q1 - q8).abs() <= 2.0 ** -7 * q8.abs() + 1e-6).all() and (q1 != q8).float().mean() < 0.02
+    assert ((c1 - c8).abs() <= 2.0 ** -3 * c8.abs() + 2.0 ** -9).all() and (c1 != c8).float().mean() < 0.02
