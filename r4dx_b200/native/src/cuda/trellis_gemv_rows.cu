@@ -19,6 +19,12 @@
 // there: its CTAs are small enough to overlap with their neighbours' in a captured step, and 1410 against 1540 us a step was
 // the result of 8 layers at 8192 tokens of context.
 //
+// Grouped mode (mixture-of-experts blocks with a few rows per expert): a CTA serves one 128-row block of one tile of the routing
+// plan, up to four rows of one expert; the digits are those of the planned pairs in expert order.  A block of 512 experts
+// (top 10, hidden 2048) takes 266 / 463 / 734 us at 17 / 64 / 200 rows of x where the tcgen05 tiles of 16 rows take 364 / 644 /
+// 822: most experts have one or two rows, and decoding their weights is the work.  (Tiles of eight rows are slower at every
+// row count: twice the MMAs and one CTA per SM.)
+//
 // Two launches: TrellisDigitsKernel writes the rows' digits once (every CTA would otherwise repeat the transform: at 8 rows of
 // 5120 columns that was 74k of 103k clocks), then one CTA per (128-row block, K slice) streams words through a ring of bulk
 // copies - filled before the wait for the digits - and `ksplit` CTAs of a cluster add up over distributed shared memory in rank
@@ -56,6 +62,13 @@ struct RowsArgs {
   const unsigned char* digits;           // [siblings][2 T columns][K]
   const DigitMeta* meta;                 // [siblings][ksplit][T]
   // one to three weights that read the same rows through the same prologue; blockIdx.y runs over all their row blocks
+  // grouped mode
+  const int* g_offsets;                  // [E + 1] into g_perm
+  const int* g_perm;                     // pair of each sorted position = output row; its input row is pair / g_xdiv
+  const int* g_tiles;                    // (expert, first sorted position) per tile, *g_ntiles of them
+  const int* g_ntiles;
+  int g_experts, g_xdiv;
+  long long g_words;                     // words of one expert
   int count;
   struct Weight {
     const uint32_t* words;
@@ -164,7 +177,8 @@ __device__ __forceinline__ uint32_t PackBytes(const uint32_t (&b)[4]) { return b
 
 // The digits of T rows for a whole launch: grid (T, ksplit, weights), one CTA per (row, K slice, weight).
 constexpr int kDigitWarps = 16;
-template <int PRO>
+// Grouped: grid (pairs), t = sorted position.
+template <int PRO, bool kGrouped>
 __global__ void __launch_bounds__(kDigitWarps * 32) TrellisDigitsKernel(RowsArgs a, unsigned char* digits, DigitMeta* meta) {
   PdlEnter();
   extern __shared__ __align__(16) float rowbuf[];      // the slice, transformed
@@ -173,13 +187,25 @@ __global__ void __launch_bounds__(kDigitWarps * 32) TrellisDigitsKernel(RowsArgs
   __shared__ int xsum;
   const int t = blockIdx.x, krank = blockIdx.y, ksplit = gridDim.y, sib = blockIdx.z, T = a.T, K = a.K;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int warps = blockDim.x >> 5;
   const __half* suh = a.w[sib].suh;
+  int xrow = t;
+  if constexpr (kGrouped) {
+    if (t >= __ldg(a.g_offsets + a.g_experts)) return;       // (pairs of experts that live elsewhere)
+    int lo = 0, hi = a.g_experts;                            // largest e with offsets[e] <= t
+    while (hi - lo > 1) {
+      const int mid = (lo + hi) >> 1;
+      if (__ldg(a.g_offsets + mid) <= t) lo = mid; else hi = mid;
+    }
+    suh += static_cast<size_t>(lo) * K;
+    xrow = __ldg(a.g_perm + t) / a.g_xdiv;
+  }
   const int kb_lo = krank * (K / 128) / ksplit, my_blocks = (krank + 1) * (K / 128) / ksplit - kb_lo;
   if (threadIdx.x == 0) { amax = 0u; xsum = 0; }
   float r = 0.f;
   if constexpr (PRO == 1) {
     if (warp < 8) {
-      const float ss = EighthSumSquares(a.x + static_cast<size_t>(t) * K, K, warp, lane);
+      const float ss = EighthSumSquares(a.x + static_cast<size_t>(xrow) * K, K, warp, lane);
       if (lane == 0) red[warp] = ss;
     }
     __syncthreads();
@@ -187,14 +213,14 @@ __global__ void __launch_bounds__(kDigitWarps * 32) TrellisDigitsKernel(RowsArgs
   }
   __syncthreads();
   uint32_t m = 0u;
-  for (int b = warp; b < my_blocks; b += kDigitWarps) {
+  for (int b = warp; b < my_blocks; b += warps) {
     const int k = (kb_lo + b) * 128 + lane * 4;
     uint2 xv, uv = make_uint2(0u, 0u), wv = make_uint2(0u, 0u);
     if constexpr (PRO == 2) {
-      xv = *reinterpret_cast<const uint2*>(a.x + static_cast<size_t>(t) * 2 * K + k);
-      uv = *reinterpret_cast<const uint2*>(a.x + static_cast<size_t>(t) * 2 * K + K + k);
+      xv = *reinterpret_cast<const uint2*>(a.x + static_cast<size_t>(xrow) * 2 * K + k);
+      uv = *reinterpret_cast<const uint2*>(a.x + static_cast<size_t>(xrow) * 2 * K + K + k);
     } else {
-      xv = *reinterpret_cast<const uint2*>(a.x + static_cast<size_t>(t) * K + k);
+      xv = *reinterpret_cast<const uint2*>(a.x + static_cast<size_t>(xrow) * K + k);
       if constexpr (PRO == 1) wv = *reinterpret_cast<const uint2*>(a.norm_w + k);
     }
     float v[4];
@@ -206,12 +232,12 @@ __global__ void __launch_bounds__(kDigitWarps * 32) TrellisDigitsKernel(RowsArgs
   __syncthreads();
   int sum = 0;
   const float inv = DigitScale(amax);
-  for (int b = warp; b < my_blocks; b += kDigitWarps) {
+  for (int b = warp; b < my_blocks; b += warps) {
     const float4 f = *reinterpret_cast<const float4*>(rowbuf + b * 128 + lane * 4);
     const float v[4] = {f.x, f.y, f.z, f.w};
     uint32_t hi[4], lo[4];
     sum += Digits(v, inv, hi, lo);
-    unsigned char* c0 = digits + (static_cast<size_t>(sib) * 2 * T + 2 * t) * K + (kb_lo + b) * 128 + lane * 4;
+    unsigned char* c0 = digits + (static_cast<size_t>(sib) * 2 * T + 2 * static_cast<size_t>(t)) * K + (kb_lo + b) * 128 + lane * 4;
     *reinterpret_cast<uint32_t*>(c0) = PackBytes(hi);
     *reinterpret_cast<uint32_t*>(c0 + K) = PackBytes(lo);
   }
@@ -225,7 +251,7 @@ __global__ void __launch_bounds__(kDigitWarps * 32) TrellisDigitsKernel(RowsArgs
   }
 }
 
-template <int KB, int TMAX>
+template <int KB, int TMAX, bool kGrouped = false>
 __global__ void __launch_bounds__(kThreads, TMAX > 4 ? 1 : 2) TrellisRowsKernel(RowsArgs a) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   cg::cluster_group cluster = cg::this_cluster();
@@ -236,7 +262,18 @@ __global__ void __launch_bounds__(kThreads, TMAX > 4 ? 1 : 2) TrellisRowsKernel(
   int sidx = 0;                            // the weight this CTA serves
   while (sidx + 1 < a.count && nb >= a.w[sidx].nb_end) ++sidx;
   if (sidx > 0) nb -= a.w[sidx - 1].nb_end;
-  const int N = a.w[sidx].N, K = a.K, T = a.T;
+  const int N = a.w[sidx].N, K = a.K;
+  int T = a.T, start = 0;                  // rows of this CTA, the first one's place in the digits
+  const uint32_t* words = a.w[sidx].words;
+  const __half* svh = a.w[sidx].svh;
+  if constexpr (kGrouped) {
+    if (static_cast<int>(blockIdx.z) >= __ldg(a.g_ntiles)) return;       // the whole CTA (a cluster of one), before any barrier exists
+    const int e = __ldg(a.g_tiles + 2 * blockIdx.z);
+    start = __ldg(a.g_tiles + 2 * blockIdx.z + 1);
+    T = min(TMAX, __ldg(a.g_offsets + e + 1) - start);
+    words += static_cast<size_t>(e) * a.g_words;
+    svh += static_cast<size_t>(e) * N;
+  }
   // K blocks are dealt out as evenly as the count allows (17 blocks over 4 CTAs: 4, 4, 4, 5); shared memory is laid
   // out for the longest slice
   const int kslice = a.kblocks_per_cta * 128;
@@ -283,7 +320,7 @@ __global__ void __launch_bounds__(kThreads, TMAX > 4 ? 1 : 2) TrellisRowsKernel(
   if (warp == kConsumerWarps) {
     // ---------------- producer: this CTA's words through the stage ring, the digits once the ring is full ----------------
     if (lane == 0) {
-      const unsigned char* src = reinterpret_cast<const unsigned char*>(a.w[sidx].words) +
+      const unsigned char* src = reinterpret_cast<const unsigned char*>(words) +
                                  (static_cast<size_t>(nb) * (K / 128) + static_cast<size_t>(kb_lo)) * kStageBytes;
       int s = 0;
       uint32_t phase = 1;          // parity to wait for on the "empty" barrier of stage s (fresh barriers pass parity 1)
@@ -291,7 +328,7 @@ __global__ void __launch_bounds__(kThreads, TMAX > 4 ? 1 : 2) TrellisRowsKernel(
         if (it == min(a.stages, my_blocks)) {
           asm volatile("griddepcontrol.wait;" ::: "memory");
           ptx::MbarArriveExpectTx(&ctl->xfull, 2 * T * my_blocks * 128);
-          const unsigned char* xsrc = a.digits + static_cast<size_t>(sidx) * 2 * T * K + kb_lo * 128;
+          const unsigned char* xsrc = a.digits + (static_cast<size_t>(sidx) * 2 * T + 2 * static_cast<size_t>(start)) * K + kb_lo * 128;
           for (int c = 0; c < 2 * T; ++c)
             ptx::BulkLoad(xd + static_cast<size_t>(c) * xstride, xsrc + static_cast<size_t>(c) * K, my_blocks * 128, &ctl->xfull);
         }
@@ -307,7 +344,7 @@ __global__ void __launch_bounds__(kThreads, TMAX > 4 ? 1 : 2) TrellisRowsKernel(
   } else {
     asm volatile("griddepcontrol.wait;" ::: "memory");
     if (threadIdx.x < T) {
-      const DigitMeta m = a.meta[(sidx * ksplit + krank) * T + threadIdx.x];
+      const DigitMeta m = a.meta[(sidx * ksplit + krank) * T + start + threadIdx.x];
       // an infinity or a NaN anywhere in the slice makes the whole row one
       ctl->unit[threadIdx.x] = m.amax < 0x7F800000u ? __uint_as_float(m.amax) / kDigitRange : __int_as_float(0x7FC00000);
       ctl->xsum[threadIdx.x] = m.xsum;
@@ -447,7 +484,7 @@ __global__ void __launch_bounds__(kThreads, TMAX > 4 ? 1 : 2) TrellisRowsKernel(
     }
     if (!landed) v[0] = __int_as_float(0x7FC00000);      // a hand-off that never completes shows as NaN in the whole block
     WarpFwht128(v);
-    const uint2 sv = *reinterpret_cast<const uint2*>(a.w[sidx].svh + n);
+    const uint2 sv = *reinterpret_cast<const uint2*>(svh + n);
     const __half2 s01 = *reinterpret_cast<const __half2*>(&sv.x), s23 = *reinterpret_cast<const __half2*>(&sv.y);
     float o[4] = {v[0] * inv_sqrt * __low2float(s01), v[1] * inv_sqrt * __high2float(s01),
                   v[2] * inv_sqrt * __low2float(s23), v[3] * inv_sqrt * __high2float(s23)};
@@ -458,7 +495,8 @@ __global__ void __launch_bounds__(kThreads, TMAX > 4 ? 1 : 2) TrellisRowsKernel(
     uint2 ov;
     ov.x = PackBf16(o[0], o[1]);
     ov.y = PackBf16(o[2], o[3]);
-    *reinterpret_cast<uint2*>(a.w[sidx].y + static_cast<size_t>(t) * N + n) = ov;
+    const size_t out_row = kGrouped ? __ldg(a.g_perm + start + t) : t;
+    *reinterpret_cast<uint2*>(a.w[sidx].y + out_row * N + n) = ov;
   }
 }
 
@@ -504,10 +542,23 @@ int LaunchRows(RowsArgs a, int ksplit, cudaStream_t stream) {
   return static_cast<int>(e);
 }
 
+template <int KB, int TMAX>
+int LaunchGroupedRows(RowsArgs a, int max_tiles, cudaStream_t stream) {
+  a.kblocks_per_cta = a.K / 128;
+  a.stages = a.kblocks_per_cta < kMaxStages ? a.kblocks_per_cta : kMaxStages;
+  const size_t smem = SmemBytes<KB, TMAX>(a.K, a.stages, 1);
+  if (smem > 227 * 1024) return R4DXB_TOO_LARGE;
+  auto kern = TrellisRowsKernel<KB, TMAX, true>;
+  const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+  if (e != cudaSuccess) return static_cast<int>(e);
+  kern<<<dim3(1, a.w[0].N / 128, max_tiles), kThreads, smem, stream>>>(a);
+  return FinishLaunch();
+}
+
 template <int PRO>
 int LaunchDigits(const RowsArgs& a, int ksplit, cudaStream_t stream) {
   const size_t smem = static_cast<size_t>((a.K / 128 + ksplit - 1) / ksplit) * 512;
-  auto kern = TrellisDigitsKernel<PRO>;
+  auto kern = TrellisDigitsKernel<PRO, false>;
   const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
   if (e != cudaSuccess) return static_cast<int>(e);
   return LaunchPdl(kern, dim3(a.T, ksplit, a.count), dim3(kDigitWarps * 32), smem, stream, a, const_cast<unsigned char*>(a.digits),
@@ -570,6 +621,50 @@ int r4dxb_trellis_gemv_rows(int count, const void* const* words, const void* con
     case 4: return LaunchKb<4>(a, ksplit, s);
     default: return LaunchKb<5>(a, ksplit, s);
   }
+}
+
+/* Expert products with a few rows per expert: y[perm[p]] = svh[e] * H128(Q_e . H128(suh[e] * act(x[perm[p] / xdiv]))) for the
+ * planned pairs p (see the header). */
+int r4dxb_trellis_rows_grouped(const void* words, const void* suh, const void* svh, const void* x, void* y, const int* offsets,
+                               const int* perm, const int* tiles, const int* ntiles, int max_tiles, int xdiv, int mode, int P, int E,
+                               int N, int K, int kb, void* digits, void* meta, void* stream) {
+  if (P < 1 || E < 1 || N < 128 || N % 128 || K < 128 || K % 128 || max_tiles < 1 || max_tiles > 65535 || xdiv < 1 || mode < 0 || mode > 2 ||
+      digits == nullptr || meta == nullptr || (reinterpret_cast<uintptr_t>(digits) & 15) ||
+      (reinterpret_cast<uintptr_t>(meta) & 7))
+    return R4DXB_BAD_ARG;
+  RowsArgs a = {};
+  a.x = static_cast<const __nv_bfloat16*>(x);
+  a.T = P;
+  a.K = K;
+  a.act = mode == 2 ? 1 : 0;
+  a.count = 1;
+  a.w[0].words = static_cast<const uint32_t*>(words);
+  a.w[0].suh = static_cast<const __half*>(suh);
+  a.w[0].svh = static_cast<const __half*>(svh);
+  a.w[0].y = static_cast<__nv_bfloat16*>(y);
+  a.w[0].N = N;
+  a.w[0].nb_end = N / 128;
+  a.g_offsets = offsets;
+  a.g_perm = perm;
+  a.g_tiles = tiles;
+  a.g_ntiles = ntiles;
+  a.g_experts = E;
+  a.g_xdiv = xdiv;
+  a.g_words = static_cast<long long>(N / 16) * (K / 16) * 8 * kb;
+  a.digits = static_cast<unsigned char*>(digits);
+  a.meta = static_cast<const DigitMeta*>(meta);
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  const size_t smem = static_cast<size_t>(K) * 4;
+  if (smem > 200 * 1024) return R4DXB_TOO_LARGE;
+  auto digits_kernel = mode == 0 ? TrellisDigitsKernel<0, true> : TrellisDigitsKernel<2, true>;
+  const cudaError_t e = cudaFuncSetAttribute(digits_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+  if (e != cudaSuccess) return static_cast<int>(e);
+  digits_kernel<<<P, 32 * min(kDigitWarps, K / 128), smem, s>>>(a, static_cast<unsigned char*>(digits), static_cast<DigitMeta*>(meta));
+  if (int rc = FinishLaunch()) return rc;
+  if (kb == 3) return LaunchGroupedRows<3, 4>(a, max_tiles, s);
+  if (kb == 4) return LaunchGroupedRows<4, 4>(a, max_tiles, s);
+  if (kb == 5) return LaunchGroupedRows<5, 4>(a, max_tiles, s);
+  return R4DXB_BAD_ARG;
 }
 
 }  // extern "C"

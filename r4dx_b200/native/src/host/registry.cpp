@@ -96,6 +96,8 @@ const R4dxbKernelInfo kKernels[] = {
      "N, K multiples of 128; cluster split 1/2/4/8 of K; kb 3/4/5", "bf16 x, packed trellis words, bf16 y", "simt+bulk-copy", c0, 5},
     {"trellis_gemv_siblings", "gemm", "trellis_linear_rows_le_8", "2 or 3 weights of one K and bit width over the same rows in one launch",
      "as trellis_gemv_ex; no residual", "bf16 x, packed trellis words, bf16 y", "simt+bulk-copy", c1, 5},
+    {"trellis_rows_grouped", "gemm", "moe_experts_few_rows", "every expert's tiles of four planned rows, hash bytes times integer rows on mma.sync",
+     "N, K multiples of 128", "bf16 x, stacked trellis words, bf16 y", "mma.sync+bulk-copy", nullptr, 0},
     {"trellis_gemv_rows", "gemm", "trellis_linear_rows_le_8", "one to three weights over the same rows, hash bytes times integer rows on mma.sync",
      "as trellis_gemv_ex; any cluster split of 1..8", "bf16 x, packed trellis words, bf16 y", "mma.sync+bulk-copy", c1, 5},
     {"trellis_gemv_mma", "gemm", "trellis_linear_rows_le_8", "the same product with code values written to tensor memory and contracted by tcgen05.mma",

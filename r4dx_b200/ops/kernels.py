@@ -843,6 +843,21 @@ def trellis_gemm_grouped(words, svh, xh, y, offsets, perm, tiles, ntiles, P: int
     return y
 
 
+register_cuda_sig("r4dxb_trellis_rows_grouped", _I, [_P] * 9 + [_I] * 8 + [_P, _P, _P])
+
+
+def trellis_rows_grouped(words, suh, svh, x, y, offsets, perm, tiles, ntiles, xdiv: int, mode: int, P: int, E: int, N: int, Kd: int,
+                         kb: int, digits: torch.Tensor, meta: torch.Tensor):
+    """y[perm[p]] = expert e(p)'s trellis linear of act(x[perm[p] // xdiv]) for a few rows per expert (``moe_tiles`` of 4
+    rows); ``digits`` (2 Kd bytes per pair) and ``meta`` (8 bytes per pair) are workspace."""
+    if digits.numel() * digits.element_size() < 2 * Kd * P or meta.numel() * meta.element_size() < 8 * P:
+        raise KernelError("trellis_rows_grouped: workspace too small")
+    bound = min(tiles.numel() // 2, P // 4 + E)
+    _check(_lib().r4dxb_trellis_rows_grouped(_p(words), _p(suh), _p(svh), _p(x), _p(y), _p(offsets), _p(perm), _p(tiles), _p(ntiles), bound,
+                                             xdiv, mode, P, E, N, Kd, kb, _p(digits), _p(meta), _stream()), "trellis_rows_grouped")
+    return y
+
+
 register_cuda_sig("r4dxb_topk_lse", _I, [_P, _I, _I, _I, _F, _I, _P, _P, _P, _P, _P])
 register_cuda_sig("r4dxb_repetition_penalty", _I, [_P, _I, _P, _I, _F, _P])
 

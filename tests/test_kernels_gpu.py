@@ -1044,3 +1044,38 @@ def test_attention_precore_of_many_rows_equals_few_row_calls(K, D, Hq, Hkv, rot)
     (q1, c1), (q8, c8) = outs
     assert ((q1 - q8).abs() <= 2.0 ** -7 * q8.abs() + 1e-6).all() and (q1 != q8).float().mean() < 0.02
     assert ((c1 - c8).abs() <= 2.0 ** -3 * c8.abs() + 2.0 ** -9).all() and (c1 != c8).float().mean() < 0.02
+
+
+@pytest.mark.parametrize("kb,N,Kd,counts", [(3, 128, 128, (0, 1, 4, 5)), (4, 256, 640, (9, 0, 0, 2, 3)), (5, 128, 2176, (1, 8, 1)),
+                                            (3, 384, 2048, (4, 4, 4, 4, 0, 7))])
+def test_grouped_rows_kernel_matches_the_per_pair_reference(K, kb, N, Kd, counts):
+    """Experts with none, full and ragged tiles of four rows, both input forms, pairs of experts that live elsewhere left alone.
+    Bound as for the ungrouped kernel: unrounded codes and integer rows (2e-3 of the rms is ten times that) plus bf16."""
+    from r4dx_b200.quant import trellis
+    E, P, k = len(counts), sum(counts), 2
+    g = torch.Generator().manual_seed(N + Kd)
+    ws = [trellis.random_weight(N, Kd, kb, seed=e, sigma=0.05) for e in range(E)]
+    Wd = [trellis.reconstruct(w).double() for w in ws]
+    elsewhere = 3                                               # pairs past the plan's end
+    perm = torch.randperm(P + elsewhere, generator=g).to(torch.int32)
+    offsets = torch.tensor([0] + list(counts)).cumsum(0).to(torch.int32)
+    words, suh, svh = torch.cat([w.words for w in ws]).cuda(), torch.stack([w.suh for w in ws]).cuda(), torch.stack([w.svh for w in ws]).cuda()
+    total = P + elsewhere
+    tiles, ntiles = torch.zeros(2 * (total // 4 + E + 1), dtype=torch.int32, device="cuda"), torch.zeros(1, dtype=torch.int32, device="cuda")
+    od, pd = offsets.cuda(), perm.cuda()
+    K.moe_tiles(od, E, 4, tiles, ntiles)
+    assert int(ntiles) == sum((c + 3) // 4 for c in counts)
+    digits, meta = torch.empty(total * 2 * Kd, dtype=torch.uint8, device="cuda"), torch.empty(total, 2, dtype=torch.int32, device="cuda")
+    for mode, div in ((0, k), (1, 1)):
+        x = torch.randn((total + div - 1) // div, Kd * (mode + 1), generator=g).to(BF)
+        y = torch.full((total, N), 7.0, dtype=BF, device="cuda")
+        K.trellis_rows_grouped(words, suh, svh, x.cuda(), y, od, pd, tiles, ntiles, div, mode, total, E, N, Kd, kb, digits, meta)
+        act = K.silu_mul(x.cuda()).cpu().double() if mode else x.double()
+        for e in range(E):
+            for p in range(int(offsets[e]), int(offsets[e + 1])):
+                pair = int(perm[p])
+                xr = act[pair // div]
+                ref = Wd[e] @ xr
+                rms = xr.pow(2).mean().sqrt() * Wd[e].pow(2).sum(-1).sqrt()
+                assert ((y[pair].cpu().double() - ref).abs() <= 2.0 ** -8 * ref.abs() + 2e-3 * rms).all(), (e, p)
+        assert (y[perm[P:].long().cuda()] == 7.0).all()
