@@ -1,4 +1,4 @@
-// Trellis-decode weight-streaming product for 2..8 activation rows on mma.sync, with the hash bytes themselves as the operand.
+// Trellis-decode weight-streaming product for 1..8 activation rows on mma.sync, with the hash bytes themselves as the operand.
 //
 //   y[t, n] = bf16( svh[n] * H128( sum_k Q[n, k] * xh[t, k] )[n] (+ residual[t, n]) ),  xh = H128(suh (.) act(x))
 //
@@ -15,9 +15,9 @@
 // ten register operands, and a mix of 4 byte permutes, 4 multiplies and one MMA alone takes 13 to 17 clocks (8 if only the
 // pipes counted): about 20 weights per clock and SM, 2.8 TB/s of 4-bit codes, whatever the row count.  Measured against the
 // CUDA-core kernel (trellis_gemv.cu), 4 bits, us at 2 / 4 / 8 rows: 34816 x 5120 48 / 46 / 60 (70 / 90 / 136), 5120 x 17408
-// 32 / 32 / 40 (49 / 72 / 117), 16384 x 5120 30 / 30 / 36 (45 / 55 / 84), 5120 x 6144 17 / 19 / 22 (22 / 27 / 41).  One row stays
-// there: its CTAs are small enough to overlap with their neighbours' in a captured step, and 1410 against 1540 us a step was
-// the result of 8 layers at 8192 tokens of context.
+// 32 / 32 / 40 (49 / 72 / 117), 16384 x 5120 30 / 30 / 36 (45 / 55 / 84), 5120 x 6144 17 / 19 / 22 (22 / 27 / 41).  A step of one row
+// (8 layers, 8192 tokens of context) takes 1270 us with this kernel and 1435 with the other; that needed the digits kernel to be
+// quick (5.8 -> 3.4 us behind an RMSNorm, see there) and the CTAs of a cluster on SMs of their own (see the launch).
 //
 // Grouped mode (mixture-of-experts blocks with a few rows per expert): a CTA serves one 128-row block of one tile of the routing
 // plan, up to four rows of one expert; the digits are those of the planned pairs in expert order.  A block of 512 experts
@@ -26,7 +26,7 @@
 // row count: twice the MMAs and one CTA per SM.)
 //
 // Two launches: TrellisDigitsKernel writes the rows' digits once (every CTA would otherwise repeat the transform: at 8 rows of
-// 5120 columns that was 74k of 103k clocks), then one CTA per (128-row block, K slice) streams words through a ring of bulk
+// 5120 columns that was 74k of 103k clocks, at one row 8k of 50k), then one CTA per (128-row block, K slice) streams words through a ring of bulk
 // copies - filled before the wait for the digits - and `ksplit` CTAs of a cluster add up over distributed shared memory in rank
 // order.
 #include <cooperative_groups.h>
@@ -177,20 +177,24 @@ __device__ __forceinline__ uint32_t PackBytes(const uint32_t (&b)[4]) { return b
 
 // The digits of T rows for a whole launch: grid (T, ksplit, weights), one CTA per (row, K slice, weight).
 constexpr int kDigitWarps = 16;
-// Grouped: grid (pairs), t = sorted position.
+constexpr int kDigitBlocks = 4;          // 128-column blocks a warp keeps in registers
+// Grouped: grid (pairs), t = sorted position.  A chain of latencies: the signs and norm weights, which no kernel writes, are
+// requested before the wait for the previous kernel, all of a warp's activations at once after it, and the transformed values
+// stay in registers between the two barriers (slices of more than 64 blocks keep them in shared memory instead): 5.8 -> 3.4 us
+// behind an RMSNorm of 5120 columns in a captured window of four rows, against one block's loads at a time.
 template <int PRO, bool kGrouped>
 __global__ void __launch_bounds__(kDigitWarps * 32) TrellisDigitsKernel(RowsArgs a, unsigned char* digits, DigitMeta* meta) {
-  PdlEnter();
-  extern __shared__ __align__(16) float rowbuf[];      // the slice, transformed
+  extern __shared__ __align__(16) float rowbuf[];      // long slices: transformed columns
   __shared__ float red[8];
   __shared__ uint32_t amax;
   __shared__ int xsum;
   const int t = blockIdx.x, krank = blockIdx.y, ksplit = gridDim.y, sib = blockIdx.z, T = a.T, K = a.K;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int warps = blockDim.x >> 5;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
   const __half* suh = a.w[sib].suh;
   int xrow = t;
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   if constexpr (kGrouped) {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     if (t >= __ldg(a.g_offsets + a.g_experts)) return;       // (pairs of experts that live elsewhere)
     int lo = 0, hi = a.g_experts;                            // largest e with offsets[e] <= t
     while (hi - lo > 1) {
@@ -201,45 +205,79 @@ __global__ void __launch_bounds__(kDigitWarps * 32) TrellisDigitsKernel(RowsArgs
     xrow = __ldg(a.g_perm + t) / a.g_xdiv;
   }
   const int kb_lo = krank * (K / 128) / ksplit, my_blocks = (krank + 1) * (K / 128) / ksplit - kb_lo;
+  const bool in_regs = my_blocks <= kDigitBlocks * warps;
   if (threadIdx.x == 0) { amax = 0u; xsum = 0; }
+  uint2 sv[kDigitBlocks], nv[kDigitBlocks];
+  auto load_weights = [&](int i, int b) {
+    const int k = (kb_lo + b) * 128 + lane * 4;
+    sv[i] = *reinterpret_cast<const uint2*>(suh + k);
+    if constexpr (PRO == 1) nv[i] = *reinterpret_cast<const uint2*>(a.norm_w + k);
+    else nv[i] = make_uint2(0u, 0u);
+  };
+  const __nv_bfloat16* xin = a.x + static_cast<size_t>(xrow) * (PRO == 2 ? 2 * static_cast<size_t>(K) : K);
+  uint2 xv[kDigitBlocks], uv[kDigitBlocks];
+  auto load_x = [&](int i, int b) {
+    const int k = (kb_lo + b) * 128 + lane * 4;
+    xv[i] = *reinterpret_cast<const uint2*>(xin + k);
+    uv[i] = PRO == 2 ? *reinterpret_cast<const uint2*>(xin + K + k) : make_uint2(0u, 0u);
+  };
+#pragma unroll
+  for (int i = 0; i < kDigitBlocks; ++i)
+    if (in_regs && warp + i * warps < my_blocks) load_weights(i, warp + i * warps);
+  if constexpr (!kGrouped) asm volatile("griddepcontrol.wait;" ::: "memory");
+#pragma unroll
+  for (int i = 0; i < kDigitBlocks; ++i)
+    if (in_regs && warp + i * warps < my_blocks) load_x(i, warp + i * warps);
   float r = 0.f;
   if constexpr (PRO == 1) {
     if (warp < 8) {
-      const float ss = EighthSumSquares(a.x + static_cast<size_t>(xrow) * K, K, warp, lane);
+      const float ss = EighthSumSquares(xin, K, warp, lane);
       if (lane == 0) red[warp] = ss;
     }
     __syncthreads();
     r = RowRms(red, K, a.eps);
+  } else {
+    __syncthreads();
   }
-  __syncthreads();
+  float v[kDigitBlocks][4];
   uint32_t m = 0u;
-  for (int b = warp; b < my_blocks; b += warps) {
-    const int k = (kb_lo + b) * 128 + lane * 4;
-    uint2 xv, uv = make_uint2(0u, 0u), wv = make_uint2(0u, 0u);
-    if constexpr (PRO == 2) {
-      xv = *reinterpret_cast<const uint2*>(a.x + static_cast<size_t>(xrow) * 2 * K + k);
-      uv = *reinterpret_cast<const uint2*>(a.x + static_cast<size_t>(xrow) * 2 * K + K + k);
-    } else {
-      xv = *reinterpret_cast<const uint2*>(a.x + static_cast<size_t>(xrow) * K + k);
-      if constexpr (PRO == 1) wv = *reinterpret_cast<const uint2*>(a.norm_w + k);
+  if (in_regs) {
+#pragma unroll
+    for (int i = 0; i < kDigitBlocks; ++i)
+      if (warp + i * warps < my_blocks) {
+        Activate<PRO>(xv[i], uv[i], nv[i], sv[i], r, a.act, v[i]);
+        m = max(m, HadamardMax(v[i]));
+      }
+  } else {
+    for (int b = warp; b < my_blocks; b += warps) {
+      load_weights(0, b);
+      load_x(0, b);
+      Activate<PRO>(xv[0], uv[0], nv[0], sv[0], r, a.act, v[0]);
+      m = max(m, HadamardMax(v[0]));
+      *reinterpret_cast<float4*>(rowbuf + b * 128 + lane * 4) = make_float4(v[0][0], v[0][1], v[0][2], v[0][3]);
     }
-    float v[4];
-    Activate<PRO>(xv, uv, wv, *reinterpret_cast<const uint2*>(suh + k), r, a.act, v);
-    m = max(m, HadamardMax(v));
-    *reinterpret_cast<float4*>(rowbuf + b * 128 + lane * 4) = make_float4(v[0], v[1], v[2], v[3]);
   }
   if (lane == 0) atomicMax(&amax, m);
   __syncthreads();
   int sum = 0;
   const float inv = DigitScale(amax);
-  for (int b = warp; b < my_blocks; b += warps) {
-    const float4 f = *reinterpret_cast<const float4*>(rowbuf + b * 128 + lane * 4);
-    const float v[4] = {f.x, f.y, f.z, f.w};
+  auto write = [&](int b, const float (&x)[4]) {
     uint32_t hi[4], lo[4];
-    sum += Digits(v, inv, hi, lo);
+    sum += Digits(x, inv, hi, lo);
     unsigned char* c0 = digits + (static_cast<size_t>(sib) * 2 * T + 2 * static_cast<size_t>(t)) * K + (kb_lo + b) * 128 + lane * 4;
     *reinterpret_cast<uint32_t*>(c0) = PackBytes(hi);
     *reinterpret_cast<uint32_t*>(c0 + K) = PackBytes(lo);
+  };
+  if (in_regs) {
+#pragma unroll
+    for (int i = 0; i < kDigitBlocks; ++i)
+      if (warp + i * warps < my_blocks) write(warp + i * warps, v[i]);
+  } else {
+    for (int b = warp; b < my_blocks; b += warps) {
+      const float4 f = *reinterpret_cast<const float4*>(rowbuf + b * 128 + lane * 4);
+      v[0][0] = f.x; v[0][1] = f.y; v[0][2] = f.z; v[0][3] = f.w;
+      write(b, v[0]);
+    }
   }
   if (lane == 0) atomicAdd(&xsum, sum);
   __syncthreads();
@@ -518,7 +556,10 @@ int LaunchRows(RowsArgs a, int ksplit, cudaStream_t stream) {
   a.kblocks_per_cta = (a.K / 128 + ksplit - 1) / ksplit;       // the longest slice
   // ring depth: everything in flight for short slices, otherwise up to 6 stages (48-60 KiB)
   a.stages = a.kblocks_per_cta < kMaxStages ? a.kblocks_per_cta : kMaxStages;
-  const size_t smem = SmemBytes<KB, TMAX>(a.kblocks_per_cta * 128, a.stages, ksplit);
+  size_t smem = SmemBytes<KB, TMAX>(a.kblocks_per_cta * 128, a.stages, ksplit);
+  // a grid that fits one CTA per SM asks for more than half of the shared memory: a CTA keeps an SM busy by itself, and two of
+  // a cluster on one SM leave another idle (5120 x 17408 at two rows inside a captured step: 48 against 25 us)
+  if (ksplit * a.w[a.count - 1].nb_end <= 148 && smem < 116 * 1024) smem = 116 * 1024;
   auto kern = TrellisRowsKernel<KB, TMAX>;
   const cudaError_t ea = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
   if (ea != cudaSuccess) return static_cast<int>(ea);
@@ -557,7 +598,8 @@ int LaunchGroupedRows(RowsArgs a, int max_tiles, cudaStream_t stream) {
 
 template <int PRO>
 int LaunchDigits(const RowsArgs& a, int ksplit, cudaStream_t stream) {
-  const size_t smem = static_cast<size_t>((a.K / 128 + ksplit - 1) / ksplit) * 512;
+  const int blocks = (a.K / 128 + ksplit - 1) / ksplit;
+  const size_t smem = blocks <= kDigitBlocks * kDigitWarps ? 0 : static_cast<size_t>(blocks) * 512;
   auto kern = TrellisDigitsKernel<PRO, false>;
   const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
   if (e != cudaSuccess) return static_cast<int>(e);
@@ -654,7 +696,7 @@ int r4dxb_trellis_rows_grouped(const void* words, const void* suh, const void* s
   a.digits = static_cast<unsigned char*>(digits);
   a.meta = static_cast<const DigitMeta*>(meta);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  const size_t smem = static_cast<size_t>(K) * 4;
+  const size_t smem = K / 128 <= kDigitBlocks * min(kDigitWarps, K / 128) ? 0 : static_cast<size_t>(K) * 4;
   if (smem > 200 * 1024) return R4DXB_TOO_LARGE;
   auto digits_kernel = mode == 0 ? TrellisDigitsKernel<0, true> : TrellisDigitsKernel<2, true>;
   const cudaError_t e = cudaFuncSetAttribute(digits_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));

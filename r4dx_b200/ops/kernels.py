@@ -199,7 +199,7 @@ def pick_ksplit(N: int, K: int, target_ctas: int = int(os.environ.get("R4DXB_KSP
 
 
 def pick_split(N: int, K: int) -> int:
-    """Cluster split of the weight-streaming kernel for several rows: the fewest 128-wide K blocks on the busiest of the 148
+    """Cluster split of the rows kernel: the fewest 128-wide K blocks on the busiest of the 148
     SMs, with three blocks' time for what a CTA does besides (setup, reduction).  A CTA of it keeps an SM busy by itself, so
     more CTAs than SMs only help to even out the load.  Measured at two rows, 4 bits (us by split 1..8): 5120 x 17408
     73 44 34 40 34 32 42 40; 34816 x 5120 48 52 60 62 68 75 81 85; 5120 x 6144 32 22 17 22 20 20 26 24; 1024 x 2048
@@ -209,14 +209,14 @@ def pick_split(N: int, K: int) -> int:
                key=lambda c: ((rows * c + 147) // 148) * ((blocks + c - 1) // c + 3))
 
 
-# Weights of a launch from which two and more rows take the rows kernel: below, its second launch costs what the contraction
-# saves (us at 4 / 8 rows, CUDA cores against rows kernel: 4096 x 1024 12 / 16 against 13 / 13, 1024 x 2048 10 / 12 against
-# 11 / 13; 5120 x 6144 27 / 41 against 19 / 22).
+# Weights of a launch from which it takes the rows kernel: below, its second launch costs what the contraction saves (us at
+# 4 / 8 rows, CUDA cores against rows kernel: 4096 x 1024 12 / 16 against 13 / 13, 1024 x 2048 10 / 12 against 11 / 13;
+# 5120 x 6144 27 / 41 against 19 / 22).
 ROWS_MIN_WEIGHTS = 1 << 23
 
 
 def rows_split(N: int, K: int) -> Optional[int]:
-    """Split of the rows kernel for a launch of N output rows, None where the CUDA-core kernel serves several rows too."""
+    """Split of the rows kernel for a launch of N output rows, None where the CUDA-core kernel serves it."""
     return pick_split(N, K) if N * K >= ROWS_MIN_WEIGHTS else None
 
 
@@ -243,9 +243,9 @@ PRO_NONE, PRO_RMSNORM, PRO_SILU_MUL, PRO_GELU_MUL = 0, 1, 2, 3
 register_cuda_sig("r4dxb_trellis_gemv_mma", _I, [_P, _P, _P, _P, _P, _P, _P, _F, _I, _I, _I, _I, _I, _I, _P, _P])
 
 # Which weight-streaming kernel serves T <= 8 rows: "simt" = CUDA-core decode + fp16 FMA (trellis_gemv.cu), "mma" = code values
-# written to tensor memory and contracted by tcgen05.mma kind::f16 (trellis_gemv_mma.cu), "auto" (the default) = the
-# CUDA-core kernel for one row and, from two rows, decode in registers with mma.sync on the hash bytes
-# (trellis_gemv_rows.cu; us at 2 / 4 / 8 rows on gate_up 48 / 46 / 60 against 70 / 80 / 95 for the better of the other two).
+# written to tensor memory and contracted by tcgen05.mma kind::f16 (trellis_gemv_mma.cu), "auto" (the default) = decode in
+# registers with mma.sync on the hash bytes for large weights (trellis_gemv_rows.cu; us at 2 / 4 / 8 rows on gate_up
+# 48 / 46 / 60 against 70 / 80 / 95 for the better of the other two), else the CUDA-core kernel.
 GEMV_IMPL = os.environ.get("R4DXB_GEMV", "auto")
 
 
@@ -289,8 +289,7 @@ def trellis_gemv(w: TrellisWeight, x: torch.Tensor, residual: Optional[torch.Ten
                  out: Optional[torch.Tensor] = None, ksplit: Optional[int] = None, prologue: int = PRO_NONE,
                  norm_w: Optional[torch.Tensor] = None, eps: float = 1e-6, split_rows: Optional[int] = None) -> torch.Tensor:
     """y[T, N] = trellis linear of act(x) (T <= 8), optionally + residual (may alias out).  ``ksplit``: cluster split of K
-    on the CUDA-core and tensor-memory kernels; ``split_rows``: two and more rows take the rows kernel with this split (by
-    shape unless given).
+    on the CUDA-core and tensor-memory kernels; ``split_rows``: take the rows kernel with this split (by shape unless given).
 
     prologue PRO_RMSNORM: x is the residual stream [T, K], act = zero-centred RMSNorm with ``norm_w``;
     PRO_SILU_MUL: x is fused [gate | up] rows [T, 2K].
@@ -299,7 +298,7 @@ def trellis_gemv(w: TrellisWeight, x: torch.Tensor, residual: Optional[torch.Ten
     T = x.numel() // (2 * w.K if prologue in (PRO_SILU_MUL, PRO_GELU_MUL) else w.K)
     out = out if out is not None else torch.empty(T, w.N, dtype=BF, device=x.device)
     split_rows = split_rows or rows_split(w.N, w.K)
-    if GEMV_IMPL == "auto" and T > 1 and split_rows is not None:
+    if GEMV_IMPL == "auto" and split_rows is not None:
         rc = _gemv_rows(1, _ptr1(w.words), _ptr1(w.suh), _ptr1(w.svh), _ptr1(out), (ctypes.c_int * 1)(w.N), x, residual, norm_w, eps,
                         prologue, T, w.K, w.kb, split_rows)
         if rc != _TOO_LARGE:
@@ -346,7 +345,7 @@ class SiblingGroup:
         y = self._outs.get(key)
         if y is None:
             y = self._outs[key] = (ctypes.c_void_p * len(outs))(*key)
-        if GEMV_IMPL == "auto" and T > 1 and self.split_rows is not None:
+        if GEMV_IMPL == "auto" and self.split_rows is not None:
             rc = _gemv_rows(len(self.weights), self._words, self._suh, self._svh, y, self._n, x, None, norm_w, eps, prologue, T, self.K,
                             self.kb, self.split_rows)
             if rc != _TOO_LARGE:

@@ -99,10 +99,10 @@ def test_trellis_gemv_tensor_memory_path_against_reference_and_cuda_core_path(K,
 
 
 @pytest.mark.parametrize("kb", [3, 4, 5])
-@pytest.mark.parametrize("T,N,Kd,split", [(2, 128, 128, 1), (3, 256, 384, 3), (4, 384, 1280, 2), (5, 128, 2176, 5), (7, 256, 1024, 8),
+@pytest.mark.parametrize("T,N,Kd,split", [(1, 256, 640, 2), (2, 128, 128, 1), (3, 256, 384, 3), (4, 384, 1280, 2), (5, 128, 2176, 5), (7, 256, 1024, 8),
                                           (8, 512, 5120, 1), (8, 128, 17408, 6)])
 def test_trellis_rows_kernel_against_fp64(K, kb, T, N, Kd, split):
-    """The integer tensor-core kernel (2..8 rows) at the edges of its stage ring, teams and splits, all prologues.  Its
+    """The integer tensor-core kernel (1..8 rows) at the edges of its stage ring, teams and splits, all prologues.  Its
     product differs from the definition by the unrounded code values (half an fp16 ulp, 2.2e-4 rms of unit codes) and by
     digits of 1/32512 of the row's largest value (below 1e-4 of the row's rms); the bf16 result adds 2^-9 of each value."""
     from r4dx_b200.ops import reference as R
@@ -135,6 +135,9 @@ def test_trellis_rows_kernel_against_fp64(K, kb, T, N, Kd, split):
     # a row of zeros stays zero, a row with a NaN or an infinity becomes NaN, the others are not touched
     bad = x.clone()
     bad[0] = 0
+    if T == 1:
+        assert (K.trellis_gemv(twd, bad.cuda(), split_rows=split) == 0).all()
+        return
     bad[1, 5] = float("inf") if T % 2 else float("nan")
     y = K.trellis_gemv(twd, bad.cuda(), split_rows=split)
     assert (y[0] == 0).all() and y[1].isnan().all()
