@@ -26,9 +26,9 @@
 // row count: twice the MMAs and one CTA per SM.)
 //
 // Two launches: TrellisDigitsKernel writes the rows' digits once (every CTA would otherwise repeat the transform: at 8 rows of
-// 5120 columns that was 74k of 103k clocks, at one row 8k of 50k), then one CTA per (128-row block, K slice) streams words through a ring of bulk
-// copies - filled before the wait for the digits - and `ksplit` CTAs of a cluster add up over distributed shared memory in rank
-// order.
+// 5120 columns that was 74k of 103k clocks, at one row 8k of 50k), then one CTA per (128-row block, K slice) streams words
+// through a ring of bulk copies - filled before the wait for the digits - and `ksplit` CTAs of a cluster add up over
+// distributed shared memory in rank order.
 #include <cooperative_groups.h>
 
 #include "sm100_ptx.cuh"
@@ -390,7 +390,8 @@ __global__ void __launch_bounds__(kThreads, TMAX > 4 ? 1 : 2) TrellisRowsKernel(
     bool ok = ptx::MbarWait(&ctl->xfull, 0, abort_flag, 3);
     ConsumerSync();
 
-    // ---------------- main loop: a team of four warps takes every fourth K block; a warp = four of its k-tiles and four n-tiles ----------------
+    // ---------------- main loop: a team of four warps takes every fourth K block ----------------
+    // a warp has four of the block's k-tiles and four of its n-tiles;
     // lane (g, c): rows g and g + 8 of an n-tile, the 16 columns of its k-tile; column g of the product = row g / 2 of x, digit g % 2
     const int team = warp / kTeamWarps, w4 = warp % kTeamWarps;
     const int g = lane >> 2, c = lane & 3, kq = w4 & 1, nt0 = (w4 >> 1) * 4;
