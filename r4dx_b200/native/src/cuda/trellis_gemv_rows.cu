@@ -45,6 +45,12 @@ constexpr int kConsumerWarps = kTeamWarps * kTeams;
 constexpr int kThreads = (kConsumerWarps + 1) * 32;
 constexpr int kSums = 2 * kTeams;        // partial sums of a row inside a CTA
 constexpr int kMaxStages = 6;
+// The teams take the K blocks in turn, so with six stages a stage passes from one team to another.  A barrier per stage would then
+// alias: a team that never waited for a stage's phase 0 finds the parity of its phase 1 satisfied while the copies of phase 0 are
+// still on their way.  Block b therefore signals through barrier b % kBarriers: all blocks of a barrier belong to one team, which
+// (like the producer) waits for its phases in order.
+constexpr int kBarriers = 12;
+static_assert(kBarriers % kTeams == 0 && kBarriers >= kMaxStages, "the blocks of a barrier belong to one team, and at most one of them is in flight");
 constexpr int kMaxSiblings = 3;
 
 // Digits of one row of x over one K slice: the slice's scale and sum.
@@ -80,14 +86,14 @@ struct RowsArgs {
 };
 
 struct Ctl {                             // control block at the start of dynamic shared memory
-  uint64_t full[kMaxStages], empty[kMaxStages];
+  uint64_t full[kBarriers], empty[kBarriers];   // of block b % kBarriers
   uint64_t red_bar;                      // split-K partials have landed
   uint64_t xfull;                        // digits have landed
   int abort_flag;
   int pad;
   float unit[8];                         // value of one integer step of a row
   int xsum[8];                           // sum of a row's integers
-  uint32_t fill[18];
+  uint32_t fill[26];
 };
 static_assert(sizeof(Ctl) % 128 == 0, "what follows the control block is 128-byte aligned");
 constexpr float kDigitRange = 32512.f;   // 127 * 256: the high digit stays a signed byte after rounding the low one
@@ -338,7 +344,7 @@ __global__ void __launch_bounds__(kThreads, TMAX > 4 ? 1 : 2) TrellisRowsKernel(
   const uint32_t full_at = ptx::SmemAddr(ctl->full), wst_at = ptx::SmemAddr(wst);      // (the empty barriers follow the full ones)
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < a.stages; ++s) {
+    for (int s = 0; s < kBarriers; ++s) {
       ptx::MbarInit(&ctl->full[s], 1);
       ptx::MbarInit(&ctl->empty[s], kTeamWarps);
     }
@@ -360,8 +366,9 @@ __global__ void __launch_bounds__(kThreads, TMAX > 4 ? 1 : 2) TrellisRowsKernel(
     if (lane == 0) {
       const unsigned char* src = reinterpret_cast<const unsigned char*>(words) +
                                  (static_cast<size_t>(nb) * (K / 128) + static_cast<size_t>(kb_lo)) * kStageBytes;
-      int s = 0;
-      uint32_t phase = 1;          // parity to wait for on the "empty" barrier of stage s (fresh barriers pass parity 1)
+      int s = 0, b = 0;            // stage and barrier of block `it`
+      int eb = 0;                  // barrier of the block that held the stage before, and the parity of its release
+      uint32_t ephase = 0;
       for (int it = 0; it <= my_blocks; ++it) {
         if (it == min(a.stages, my_blocks)) {
           asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -371,12 +378,16 @@ __global__ void __launch_bounds__(kThreads, TMAX > 4 ? 1 : 2) TrellisRowsKernel(
             ptx::BulkLoad(xd + static_cast<size_t>(c) * xstride, xsrc + static_cast<size_t>(c) * K, my_blocks * 128, &ctl->xfull);
         }
         if (it == my_blocks) break;
-        if (!ptx::MbarWaitAt(full_at + (kMaxStages + s) * 8, phase, abort_flag, 1)) break;
-        ptx::MbarArriveExpectTxAt(full_at + s * 8, kStageBytes);
-        ptx::BulkLoadAt(wst_at + s * kStageSlot, src, kStageBytes / 2, full_at + s * 8);
-        ptx::BulkLoadAt(wst_at + s * kStageSlot + kHalfSlot, src + kStageBytes / 2, kStageBytes / 2, full_at + s * 8);
+        if (it >= a.stages) {
+          if (!ptx::MbarWaitAt(full_at + (kBarriers + eb) * 8, ephase, abort_flag, 1)) break;
+          if (++eb == kBarriers) { eb = 0; ephase ^= 1u; }
+        }
+        ptx::MbarArriveExpectTxAt(full_at + b * 8, kStageBytes);
+        ptx::BulkLoadAt(wst_at + s * kStageSlot, src, kStageBytes / 2, full_at + b * 8);
+        ptx::BulkLoadAt(wst_at + s * kStageSlot + kHalfSlot, src + kStageBytes / 2, kStageBytes / 2, full_at + b * 8);
         src += kStageBytes;
-        if (++s == a.stages) { s = 0; phase ^= 1u; }
+        if (++s == a.stages) s = 0;
+        if (++b == kBarriers) b = 0;
       }
     }
   } else {
@@ -414,9 +425,9 @@ __global__ void __launch_bounds__(kThreads, TMAX > 4 ? 1 : 2) TrellisRowsKernel(
       xcol[q] = xd + static_cast<size_t>(min(g + 8 * q, 2 * T - 1)) * xstride + kt * 16;
     // stage index and barrier parity advance by counting: a division by the run-time ring depth per 128-wide
     // K block would cost as much as decoding a dozen weights
-    int s = team;
+    int s = team, b = team;
     uint32_t phase = 0;
-    while (s >= a.stages) { s -= a.stages; phase ^= 1u; }
+    while (s >= a.stages) s -= a.stages;
     for (int it = team; it < my_blocks && ok; it += kTeams) {
       uint32_t bx[NG][16];
 #pragma unroll
@@ -426,7 +437,7 @@ __global__ void __launch_bounds__(kThreads, TMAX > 4 ? 1 : 2) TrellisRowsKernel(
 #pragma unroll
         for (int i = 0; i < 16; ++i) bx[q][i] = __byte_perm(w[i >> 2], 0u, 0x1111 * (i & 3));      // a byte four times over
       }
-      ok = ptx::MbarWaitAt(full_at + s * 8, phase, abort_flag, 2);
+      ok = ptx::MbarWaitAt(full_at + b * 8, phase, abort_flag, 2);
       if (!ok) break;
       const unsigned char* st = wst + s * kStageSlot + (c >> 1) * kHalfSlot + (kq * 2 + (c & 1)) * kTileBytes + nt0 * (NW * 4);
 #pragma unroll
@@ -449,9 +460,11 @@ __global__ void __launch_bounds__(kThreads, TMAX > 4 ? 1 : 2) TrellisRowsKernel(
 #undef R4DXB_I8_STEP
       }
       __syncwarp();
-      if (lane == 0) ptx::MbarArriveAt(full_at + (kMaxStages + s) * 8);
+      if (lane == 0) ptx::MbarArriveAt(full_at + (kBarriers + b) * 8);
       s += kTeams;
-      while (s >= a.stages) { s -= a.stages; phase ^= 1u; }
+      while (s >= a.stages) s -= a.stages;
+      b += kTeams;
+      if (b >= kBarriers) { b -= kBarriers; phase ^= 1u; }
     }
     // the sums of a row (k-tile half, team) meet in shared memory
     const float code_scale = __half2float(__ushort_as_half(R4DXB_TRELLIS_SCALE_F16));

@@ -144,6 +144,23 @@ def test_trellis_rows_kernel_against_fp64(K, kb, T, N, Kd, split):
     assert torch.equal(y[2:], K.trellis_gemv(twd, x.cuda(), split_rows=split)[2:])
 
 
+@pytest.mark.parametrize("kb", [3, 4, 5])
+@pytest.mark.parametrize("T", [4, 8])
+def test_trellis_rows_ring_that_wraps_many_times(K, kb, T):
+    """40 K blocks through six stages (every stage passes between the four teams) against slices of five blocks, which never
+    reuse a stage.  Both products are of the same rounded operands: one bf16 step of the result, and 1e-3 of the row's rms
+    for the order of the sums and the rows' own rounding.  Twelve launches give the same bits."""
+    from r4dx_b200.quant import trellis
+    N, Kd = 5120, 5120
+    w = trellis.random_weight(N, Kd, kb, seed=kb, sigma=0.02, device="cuda")
+    x = torch.randn(T, Kd, generator=torch.Generator().manual_seed(T)).to(BF).cuda()
+    ref = K.trellis_gemv(w, x, split_rows=8).float()
+    first = K.trellis_gemv(w, x, split_rows=1)
+    assert ((first.float() - ref).abs() <= 2.0 ** -7 * ref.abs() + 1e-3 * ref.pow(2).mean().sqrt()).all()
+    for _ in range(11):
+        assert torch.equal(K.trellis_gemv(w, x, split_rows=1), first)
+
+
 def test_trellis_gemv_one_hot_returns_decoded_rows(K):
     """x = e_k after undoing the input transform picks out column k of H Q H exactly (up to bf16)."""
     from r4dx_b200.quant import trellis
