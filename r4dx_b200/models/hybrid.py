@@ -36,7 +36,7 @@ class Linear:
         self.name = name
         if isinstance(w, TrellisWeight):
             self.N, self.K = w.N, w.K
-            self.ksplit, self.split_rows = K.pick_ksplit(w.N, w.K), K.rows_split(w.N, w.K)
+            self.ksplit = K.pick_ksplit(w.N, w.K)
         elif isinstance(w, (W4Weight, W8Weight)):
             self.N, self.K = w.N, w.K
         else:
@@ -47,7 +47,7 @@ class Linear:
         w = self.w
         if isinstance(w, TrellisWeight):
             return K.trellis_gemv(w, x, residual=residual, out=out, ksplit=self.ksplit, prologue=prologue,
-                                  norm_w=norm_w, eps=eps, split_rows=self.split_rows)
+                                  norm_w=norm_w, eps=eps)
         if isinstance(w, (W4Weight, W8Weight)):
             # group-quantised layouts: the streaming kernels have no prologue / residual modes, so the producer of the
             # activations and the residual add are kernels of their own (the w8a16 body of the dense and short-conv

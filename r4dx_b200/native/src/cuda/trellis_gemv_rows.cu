@@ -15,9 +15,8 @@
 // ten register operands, and a mix of 4 byte permutes, 4 multiplies and one MMA alone takes 13 to 17 clocks (8 if only the
 // pipes counted): about 20 weights per clock and SM, 2.8 TB/s of 4-bit codes, whatever the row count.  Measured against the
 // CUDA-core kernel (trellis_gemv.cu), 4 bits, us at 2 / 4 / 8 rows: 34816 x 5120 48 / 46 / 60 (70 / 90 / 136), 5120 x 17408
-// 32 / 32 / 40 (49 / 72 / 117), 16384 x 5120 30 / 30 / 36 (45 / 55 / 84), 5120 x 6144 17 / 19 / 22 (22 / 27 / 41).  A step of one row
-// (8 layers, 8192 tokens of context) takes 1270 us with this kernel and 1435 with the other; that needed the digits kernel to be
-// quick (5.8 -> 3.4 us behind an RMSNorm, see there) and the CTAs of a cluster on SMs of their own (see the launch).
+// 32 / 32 / 40 (49 / 72 / 117), 16384 x 5120 30 / 30 / 36 (45 / 55 / 84), 5120 x 6144 17 / 19 / 22 (22 / 27 / 41).  (One row
+// takes the other kernel: see ops/kernels.py:ROWS_MIN_ROWS.)
 //
 // Grouped mode (mixture-of-experts blocks with a few rows per expert): a CTA serves one 128-row block of one tile of the routing
 // plan, up to four rows of one expert; the digits are those of the planned pairs in expert order.  A block of 512 experts

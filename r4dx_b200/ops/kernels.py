@@ -6,6 +6,7 @@ fallback (a missing library raises).  Reference numerics for each op live in ``o
 from __future__ import annotations
 
 import ctypes
+import functools
 import os
 from typing import Optional, Sequence
 
@@ -214,10 +215,17 @@ def pick_split(N: int, K: int) -> int:
 # 5120 x 6144 27 / 41 against 19 / 22).
 ROWS_MIN_WEIGHTS = 1 << 23
 
+# Rows from which a launch takes the rows kernel.  One-row steps stay on the CUDA cores although a step of the 27B geometry (8
+# layers, 8192 tokens of context) takes 1435 us there and 1270 with the rows kernel: the two round differently (6.4e-4 and 2.2e-4
+# of a product against 64 bits, most of the first from fp16 partial sums), and over a run of steps, each fed from the recurrent
+# state of the last, the difference grows past 3 % of the logits.
+ROWS_MIN_ROWS = 2
 
-def rows_split(N: int, K: int) -> Optional[int]:
-    """Split of the rows kernel for a launch of N output rows, None where the CUDA-core kernel serves it."""
-    return pick_split(N, K) if N * K >= ROWS_MIN_WEIGHTS else None
+
+@functools.lru_cache(maxsize=None)
+def rows_split(N: int, K: int, T: int) -> Optional[int]:
+    """Split of the rows kernel for T rows of a launch of N outputs, None where one of the other kernels serves it."""
+    return pick_split(N, K) if T >= ROWS_MIN_ROWS and N * K >= ROWS_MIN_WEIGHTS else None
 
 
 _STATUS = {}
@@ -297,7 +305,7 @@ def trellis_gemv(w: TrellisWeight, x: torch.Tensor, residual: Optional[torch.Ten
     _req(x, BF, "x")
     T = x.numel() // (2 * w.K if prologue in (PRO_SILU_MUL, PRO_GELU_MUL) else w.K)
     out = out if out is not None else torch.empty(T, w.N, dtype=BF, device=x.device)
-    split_rows = split_rows or rows_split(w.N, w.K)
+    split_rows = split_rows or rows_split(w.N, w.K, T)
     if GEMV_IMPL == "auto" and split_rows is not None:
         rc = _gemv_rows(1, _ptr1(w.words), _ptr1(w.suh), _ptr1(w.svh), _ptr1(out), (ctypes.c_int * 1)(w.N), x, residual, norm_w, eps,
                         prologue, T, w.K, w.kb, split_rows)
@@ -334,7 +342,8 @@ class SiblingGroup:
         self._svh = arr([w.svh.data_ptr() for w in weights])
         self._n = (ctypes.c_int * len(weights))(*[w.N for w in weights])
         self.ksplit = pick_ksplit(sum(w.N for w in weights), w0.K)
-        self.split_rows = rows_split(sum(w.N for w in weights), w0.K)
+        self.split_rows = None           # split of the rows kernel (by shape and rows unless set)
+        self._N = sum(w.N for w in weights)
         self._outs = {}
 
     def __call__(self, x: torch.Tensor, outs: Sequence[torch.Tensor], prologue: int = PRO_NONE,
@@ -345,9 +354,10 @@ class SiblingGroup:
         y = self._outs.get(key)
         if y is None:
             y = self._outs[key] = (ctypes.c_void_p * len(outs))(*key)
-        if GEMV_IMPL == "auto" and self.split_rows is not None:
+        split_rows = self.split_rows or rows_split(self._N, self.K, T)
+        if GEMV_IMPL == "auto" and split_rows is not None:
             rc = _gemv_rows(len(self.weights), self._words, self._suh, self._svh, y, self._n, x, None, norm_w, eps, prologue, T, self.K,
-                            self.kb, self.split_rows)
+                            self.kb, split_rows)
             if rc != _TOO_LARGE:
                 _check(rc, "trellis_gemv_rows")
                 return

@@ -161,6 +161,32 @@ def test_trellis_rows_ring_that_wraps_many_times(K, kb, T):
         assert torch.equal(K.trellis_gemv(w, x, split_rows=1), first)
 
 
+def test_one_row_products_of_large_weights_have_the_bits_of_the_cuda_core_kernel(K):
+    """Whatever the size: the rounding of a one-row step decides the logits of all later ones."""
+    from r4dx_b200.quant import trellis
+    N, Kd = 4096, 2048
+    ws = [trellis.random_weight(N, Kd, 4, seed=i, sigma=0.02, device="cuda") for i in range(3)]
+    grp = K.SiblingGroup(ws)
+    g = torch.Generator().manual_seed(1)
+    x, gu, res = (torch.randn(1, n, generator=g).to(BF).cuda() for n in (Kd, 2 * Kd, N))
+    nw = (torch.randn(Kd, generator=g) * 0.1).to(BF).cuda()
+
+    def calls():
+        outs = [torch.empty(1, N, dtype=BF, device="cuda") for _ in ws]
+        grp(x, outs, prologue=K.PRO_RMSNORM, norm_w=nw)
+        return outs + [K.trellis_gemv(ws[0], x), K.trellis_gemv(ws[0], x, residual=res), K.trellis_gemv(ws[0], gu, prologue=K.PRO_SILU_MUL),
+                       K.trellis_gemv(ws[0], gu, prologue=K.PRO_GELU_MUL)]
+
+    assert K.GEMV_IMPL == "auto" and N * Kd >= K.ROWS_MIN_WEIGHTS
+    auto = calls()
+    K.set_gemv_impl("simt")
+    try:
+        for a, b in zip(auto, calls()):
+            assert torch.equal(a, b)
+    finally:
+        K.set_gemv_impl("auto")
+
+
 def test_trellis_gemv_one_hot_returns_decoded_rows(K):
     """x = e_k after undoing the input transform picks out column k of H Q H exactly (up to bf16)."""
     from r4dx_b200.quant import trellis
