@@ -94,6 +94,11 @@ __device__ __forceinline__ float GeluTanh(float x) {
 // gate activation of a gated MLP: 0 = SiLU (SwiGLU), 1 = tanh-GELU (GeGLU)
 __device__ __forceinline__ float GateAct(float x, int act) { return act == 0 ? Silu(x) : GeluTanh(x); }
 
+// x, a NaN as the one whose lower mantissa bits are zero (arithmetic produces 0x7FFFFFFF): integer rounding leaves it a NaN.
+__device__ __forceinline__ float PlainNan(float x) {
+  return __uint_as_float(fabsf(x) <= __uint_as_float(0x7F800000u) ? __float_as_uint(x) : 0x7FC00000u);
+}
+
 // 128-point Sylvester FWHT held by one warp: lane l owns elements 4l .. 4l+3 (unnormalised).
 __device__ __forceinline__ void WarpFwht128(float (&v)[4]) {
   const int lane = threadIdx.x & 31;

@@ -194,8 +194,11 @@ struct PhaseBSmem {
 };
 
 // The same rounding (half away from zero) in two integer instructions: conversions run at a quarter of their rate, and the scan
-// needs thousands of them per chunk.  (Only a NaN with all mantissa bits set would come out differently.)
+// needs thousands of them per chunk.  It would carry the NaN that arithmetic produces into the sign bit and leave a zero, so
+// the values it is applied to (q, k and U in shared memory) were written through PlainNan; RoundTf32Any takes any NaN.  (A
+// compare and a select at every rounding: 1674 against 1582 us for 8192 tokens of 48 heads.)
 __device__ __forceinline__ uint32_t RoundTf32(float x) { return (__float_as_uint(x) + 0x1000u) & 0xFFFFE000u; }
+__device__ __forceinline__ uint32_t RoundTf32Any(float x) { return RoundTf32(PlainNan(x)); }
 
 __device__ __forceinline__ void MmaTf32(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
                                         uint32_t b1) {
@@ -296,8 +299,8 @@ __global__ void __launch_bounds__(kScanThreads, 1) GdnChunkScanKernel(const floa
   auto publish = [&] {
 #pragma unroll
     for (int nt = 0; nt < 4; ++nt) {
-      *reinterpret_cast<uint2*>(&sm.S[sm0 + g][sn0 + nt * 8 + 2 * t4]) = make_uint2(RoundTf32(st[nt][0]), RoundTf32(st[nt][1]));
-      *reinterpret_cast<uint2*>(&sm.S[sm0 + g + 8][sn0 + nt * 8 + 2 * t4]) = make_uint2(RoundTf32(st[nt][2]), RoundTf32(st[nt][3]));
+      *reinterpret_cast<uint2*>(&sm.S[sm0 + g][sn0 + nt * 8 + 2 * t4]) = make_uint2(RoundTf32Any(st[nt][0]), RoundTf32Any(st[nt][1]));
+      *reinterpret_cast<uint2*>(&sm.S[sm0 + g + 8][sn0 + nt * 8 + 2 * t4]) = make_uint2(RoundTf32Any(st[nt][2]), RoundTf32Any(st[nt][3]));
     }
   };
   publish();
@@ -320,10 +323,9 @@ __global__ void __launch_bounds__(kScanThreads, 1) GdnChunkScanKernel(const floa
       for (int nt = 0; nt < 2; ++nt) {
         float2* lo = reinterpret_cast<float2*>(&sm.U[buf][m0 + g][nh + nt * 8 + 2 * t4]);
         float2* hi = reinterpret_cast<float2*>(&sm.U[buf][m0 + g + 8][nh + nt * 8 + 2 * t4]);
-        float2 a = *lo, b = *hi;
-        a.x -= acc[nt][0]; a.y -= acc[nt][1]; b.x -= acc[nt][2]; b.y -= acc[nt][3];
-        *lo = a;
-        *hi = b;
+        const float2 a = *lo, b = *hi;
+        *lo = make_float2(PlainNan(a.x - acc[nt][0]), PlainNan(a.y - acc[nt][1]));
+        *hi = make_float2(PlainNan(b.x - acc[nt][2]), PlainNan(b.y - acc[nt][3]));
       }
     }
     __pipeline_wait_prior(2);
@@ -381,8 +383,8 @@ __global__ void __launch_bounds__(kScanThreads, 1) GdnChunkScanKernel(const floa
       for (int kb = 0; kb < kC / 8; ++kb) {
         const int j0 = kb * 8 + t4, j1 = j0 + 4;
         const float f0 = sm.fG[j0], f1 = sm.fG[j1];
-        const uint32_t a0 = RoundTf32(sm.U[buf][j0][sm0 + g] * f0), a1 = RoundTf32(sm.U[buf][j0][sm0 + g + 8] * f0);
-        const uint32_t a2 = RoundTf32(sm.U[buf][j1][sm0 + g] * f1), a3 = RoundTf32(sm.U[buf][j1][sm0 + g + 8] * f1);
+        const uint32_t a0 = RoundTf32Any(sm.U[buf][j0][sm0 + g] * f0), a1 = RoundTf32Any(sm.U[buf][j0][sm0 + g + 8] * f0);
+        const uint32_t a2 = RoundTf32Any(sm.U[buf][j1][sm0 + g] * f1), a3 = RoundTf32Any(sm.U[buf][j1][sm0 + g + 8] * f1);
 #pragma unroll
         for (int nt = 0; nt < 4; ++nt) {
           const uint32_t b0 = RoundTf32(sm.K[j0 * kLd + sn0 + nt * 8 + g]), b1 = RoundTf32(sm.K[j1 * kLd + sn0 + nt * 8 + g]);

@@ -118,7 +118,7 @@ __global__ void __launch_bounds__(256) GdnPrepKernel(PrepArgs a) {
         ss = WarpSum(ss);
         const float inv = rsqrtf(ss + 1e-6f);
 #pragma unroll
-        for (int i = 0; i < PER; ++i) y.v[i] *= inv;
+        for (int i = 0; i < PER; ++i) y.v[i] = PlainNan(y.v[i] * inv);       // (as the chunked scan's rounding needs it)
       }
       StoreVec<kVec>(dst + t * dst_stride, y);
       h[0] = h[1]; h[1] = h[2]; h[2] = h[3]; h[3] = next;

@@ -567,6 +567,54 @@ def test_gdn_chunked_prefill_with_gates_of_thousands_of_nats_per_chunk(K):
     assert (states[0] - states[1]).norm() / states[1].norm() < 5e-3
 
 
+def _gdn_chunk_call(K, T, Hv, Hk, poison=None, A_log=None, decays=None):
+    D = 128
+    g = torch.Generator().manual_seed(T + Hv)
+    key_dim, conv_dim = Hk * D, 2 * Hk * D + Hv * D
+    mixed = (torch.randn(T, conv_dim, generator=g) * 0.5).to(BF)
+    z = torch.randn(T, Hv * D, generator=g).to(BF)
+    ab = torch.randn(T, 2 * Hv, generator=g)
+    if decays is not None:
+        ab[:, :Hv] = decays(T, Hv, g)
+    conv_w = (torch.randn(conv_dim, 4, generator=g) * 0.5).to(BF)
+    A_log = torch.zeros(Hv) if A_log is None else A_log
+    norm_w = torch.ones(D).to(BF)
+    state0 = torch.randn(Hv, D, D, generator=g) * 0.1
+    if poison is not None:
+        poison(mixed, state0)
+    runs = []
+    for use_ws in (True, False):
+        state, out = state0.cuda(), torch.zeros(T, Hv * D, dtype=BF, device="cuda")
+        sc = {n: torch.empty(T, h, D, device="cuda") for n, h in (("q", Hk), ("k", Hk), ("v", Hv), ("o", Hv))}
+        sc.update(eg=torch.empty(T, Hv, device="cuda"), beta=torch.empty(T, Hv, device="cuda"))
+        if use_ws:
+            sc["ws"] = torch.zeros(K.gdn_chunk_ws_floats(T, Hv), device="cuda")
+        K.gdn_prefill(mixed.cuda(), z.cuda(), ab.cuda(), conv_w.cuda(), A_log.cuda(), torch.zeros(Hv, device="cuda"), norm_w.cuda(),
+                      torch.zeros(16, conv_dim, dtype=BF, device="cuda"), state, sc, out, T, Hv, Hk, D, 0)
+        runs.append((out.view(T, Hv, D).float().cpu(), state.cpu(), sc))
+    return runs
+
+
+@pytest.mark.parametrize("where", ["q", "k", "v", "state", "v_last"])
+def test_gdn_chunked_prefill_keeps_nan(K, where):
+    """A NaN in one operand of head 0 (q / k: of its key head) is NaN wherever the token scan has it - in the output, in later
+    chunks and in the state - and the heads it does not reach keep the bits of a clean call."""
+    T, Hv, Hk, D = 200, 4, 2, 128
+    tok = T - 2 if where == "v_last" else 70
+
+    def poison(mixed, state):
+        if where == "state":
+            state[0, 5, 9] = float("nan")
+        else:
+            mixed[tok, {"q": 3, "k": Hk * D + 3}.get(where, 2 * Hk * D + 3)] = float("nan")
+
+    (out, state, _), (out_scan, state_scan, _) = _gdn_chunk_call(K, T, Hv, Hk, poison)
+    clean, clean_state, _ = _gdn_chunk_call(K, T, Hv, Hk)[0]
+    assert out_scan[tok:, 0].isnan().any() and (where == "q" or state_scan[0].isnan().any())
+    assert (out.isnan() | ~out_scan.isnan()).all() and (state.isnan() | ~state_scan.isnan()).all()
+    assert torch.equal(out[:, 2:], clean[:, 2:]) and torch.equal(state[2:], clean_state[2:])
+
+
 @pytest.mark.parametrize("D,Hv,Hk,T", [(128, 6, 2, 70), (64, 4, 2, 33)])
 def test_gdn_prefill_matches_recurrence_and_hands_over_to_decode(K, D, Hv, Hk, T):
     g = torch.Generator().manual_seed(D + T)
