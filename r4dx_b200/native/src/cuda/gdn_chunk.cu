@@ -85,21 +85,23 @@ __global__ void __launch_bounds__(256) GdnChunkPrepKernel(const float* __restric
     sm.G[tid] = t < T ? fmaxf(logf(eg[static_cast<size_t>(t) * H + h]), -80.f) : 0.f;
   }
   __syncthreads();
-  if (tid < 32) {
-    // running sum of the 64 log decays, two per lane
-    const float a = sm.G[2 * tid], b = a + sm.G[2 * tid + 1];
-    float sum = b;
+  // Running sum of the 64 log decays, each thread its own in token order: neighbouring sums then share all earlier roundings, so
+  // they never rise and exp(G_i - G_j) stays below 1 (a tree of partial sums doubled the error of a pair's decay).
+  float sum = 0.f;
+  if (tid < kC) {
 #pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-      const float up = __shfl_up_sync(0xffffffffu, sum, d);
-      if (tid >= d) sum += up;
+    for (int j = 0; j < kC; j += 4) {
+      const float4 g4 = *reinterpret_cast<const float4*>(&sm.G[j]);
+      if (j <= tid) sum += g4.x;
+      if (j + 1 <= tid) sum += g4.y;
+      if (j + 2 <= tid) sum += g4.z;
+      if (j + 3 <= tid) sum += g4.w;
     }
-    const float before = __shfl_up_sync(0xffffffffu, sum, 1);
-    const float base = tid > 0 ? before : 0.f;
-    sm.G[2 * tid] = base + a;
-    sm.G[2 * tid + 1] = sum;
-    sm.BG[2 * tid] = sm.B[2 * tid] * expf(base + a);
-    sm.BG[2 * tid + 1] = sm.B[2 * tid + 1] * expf(sum);
+  }
+  __syncthreads();
+  if (tid < kC) {
+    sm.G[tid] = sum;
+    sm.BG[tid] = sm.B[tid] * expf(sum);
   }
   __syncthreads();
   if (tid < kC) ws_g[ch * kC + tid] = sm.G[tid];

@@ -615,6 +615,16 @@ def test_gdn_chunked_prefill_keeps_nan(K, where):
     assert torch.equal(out[:, 2:], clean[:, 2:]) and torch.equal(state[2:], clean_state[2:])
 
 
+def test_gdn_chunk_log_decays_fall_monotonically(K):
+    """The running sums of a chunk's log decays never rise, so that exp(G_i - G_j) <= 1 for every pair: half of the gates at the
+    clamp of -80, where neighbouring sums that do not share their rounding can differ by more than a small decay."""
+    T, Hv = 640, 48
+    runs = _gdn_chunk_call(K, T, Hv, 48, A_log=torch.full((Hv,), 5.0),
+                           decays=lambda T, H, g: torch.where(torch.rand(T, H, generator=g) < 0.5, 3.0, -12.0 - 4 * torch.rand(T, H, generator=g)))
+    G = runs[0][2]["ws"][-(T // 64) * Hv * 64:].view(T // 64, Hv, 64).cpu()
+    assert (G[..., 1:] <= G[..., :-1]).all() and float(G.min()) < -2000
+
+
 @pytest.mark.parametrize("D,Hv,Hk,T", [(128, 6, 2, 70), (64, 4, 2, 33)])
 def test_gdn_prefill_matches_recurrence_and_hands_over_to_decode(K, D, Hv, Hk, T):
     g = torch.Generator().manual_seed(D + T)
