@@ -11,7 +11,7 @@
 //           one right-hand-side column per thread with the 64 unknowns in registers.  The solve is right-looking (a
 //           solved unknown is subtracted from all later ones at once): the sums are independent, where adding up
 //           unknown i's terms when its turn comes is a chain of i multiply-adds behind a global load;
-//   phase B (grid heads x 2 row blocks of the state, sequential over chunks): U = U~ - W S0^T,
+//   phase B (grid heads x 2 or 4 row blocks of the state, sequential over chunks): U = U~ - W S0^T,
 //           O, and the state update as TF32 tensor-core products (mma.sync m16n8k8, fp32
 //           accumulate) out of shared memory; W, Q, P and K have a cp.async slot each that is refilled for the
 //           next chunk as soon as its product is done, three products ahead of its use (two shared slots fetched one
@@ -179,11 +179,11 @@ __global__ void __launch_bounds__(256) GdnChunkPrepKernel(const float* __restric
 constexpr int kLd = kD + 8;       // W / Q / K / state rows: conflict-free 8-byte fragment reads and strided scalar reads
 constexpr int kLdP = kC + 4;      // P rows: conflict-free scalar fragment reads
 static_assert(kC == 64, "the warps of a CTA tile 64 tokens by kRows columns");
-constexpr int kRows = 64;         // state rows (value columns) of a CTA
-constexpr int kLdU = kRows + 8;   // U rows
-constexpr int kScanThreads = kRows * 8;
 
+// kRows: state rows (value columns) of a CTA, 32 or 64; kRows * 8 threads.
+template <int kRows>
 struct PhaseBSmem {
+  static constexpr int kLdU = kRows + 8;   // U rows
   float W[kC * kLd];
   float Q[kC * kLd];
   float K[kC * kLd];
@@ -235,23 +235,26 @@ __device__ __forceinline__ void MmaRowRow(float (&acc)[NT][4], const float* __re
   }
 }
 
+template <int kThreads>
 __device__ __forceinline__ void CopyRows(float* dst, int ld_dst, const float* src, size_t src_stride, int rows, int row_floats,
                                          int tid) {
   const int per_row = row_floats / 4;
-  for (int i = tid; i < rows * per_row; i += kScanThreads) {
+  for (int i = tid; i < rows * per_row; i += kThreads) {
     const int r = i / per_row, o = (i % per_row) * 4;
     __pipeline_memcpy_async(dst + r * ld_dst + o, src + static_cast<size_t>(r) * src_stride + o, 16);
   }
 }
 
 // grid (H, 128 / kRows): CTA (h, vb) owns state rows [kRows vb, kRows vb + kRows) of head h
-__global__ void __launch_bounds__(kScanThreads, 1) GdnChunkScanKernel(const float* __restrict__ q, const float* __restrict__ k,
+template <int kRows>
+__global__ void __launch_bounds__(kRows * 8, 1) GdnChunkScanKernel(const float* __restrict__ q, const float* __restrict__ k,
                                                              const float* __restrict__ ws_ut, const float* __restrict__ ws_w,
                                                              const float* __restrict__ ws_p, const float* __restrict__ ws_g,
                                                              float* __restrict__ state, float* __restrict__ o, int T, int H,
                                                              int Hk) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  PhaseBSmem& sm = *reinterpret_cast<PhaseBSmem*>(smem_raw);
+  PhaseBSmem<kRows>& sm = *reinterpret_cast<PhaseBSmem<kRows>*>(smem_raw);
+  constexpr int kScanThreads = kRows * 8, kLdU = PhaseBSmem<kRows>::kLdU;
   const int h = blockIdx.x, vb = blockIdx.y, hk = h / (H / Hk);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int g = lane >> 2, t4 = lane & 3;
@@ -263,8 +266,8 @@ __global__ void __launch_bounds__(kScanThreads, 1) GdnChunkScanKernel(const floa
   auto issue_wug = [&](int c) {               // W, U~ (this CTA's columns) and G
     if (c < chunks) {
       const size_t ch = static_cast<size_t>(c) * H + h;
-      CopyRows(sm.W, kLd, ws_w + ch * kC * kD, kD, kC, kD, tid);
-      CopyRows(&sm.U[c & 1][0][0], kLdU, ws_ut + ch * kC * kD + vb * kRows, kD, kC, kRows, tid);
+      CopyRows<kScanThreads>(sm.W, kLd, ws_w + ch * kC * kD, kD, kC, kD, tid);
+      CopyRows<kScanThreads>(&sm.U[c & 1][0][0], kLdU, ws_ut + ch * kC * kD + vb * kRows, kD, kC, kRows, tid);
       if (tid < kC / 4) __pipeline_memcpy_async(&sm.G[c & 1][tid * 4], ws_g + ch * kC + tid * 4, 16);
     }
     __pipeline_commit();
@@ -280,7 +283,7 @@ __global__ void __launch_bounds__(kScanThreads, 1) GdnChunkScanKernel(const floa
     __pipeline_commit();
   };
   auto issue_p = [&](int c) {
-    if (c < chunks) CopyRows(sm.P, kLdP, ws_p + (static_cast<size_t>(c) * H + h) * kC * kC, kC, kC, kC, tid);
+    if (c < chunks) CopyRows<kScanThreads>(sm.P, kLdP, ws_p + (static_cast<size_t>(c) * H + h) * kC * kC, kC, kC, kC, tid);
     __pipeline_commit();
   };
 
@@ -289,7 +292,7 @@ __global__ void __launch_bounds__(kScanThreads, 1) GdnChunkScanKernel(const floa
   issue_p(0);
   // The fp32 state stays in registers in the accumulator layout of product 3 (a warp: 16 rows x 32 columns); shared memory
   // holds its TF32 rounding, which is what products 1 and 2a read.
-  const int sm0 = (warp & 3) * 16, sn0 = (warp >> 2) * 32;
+  const int sm0 = (warp % (kRows / 16)) * 16, sn0 = (warp / (kRows / 16)) * 32;
   float* s_lo = state + (static_cast<size_t>(h) * kD + vb * kRows + sm0 + g) * kD + sn0 + 2 * t4;
   float* s_hi = s_lo + 8 * kD;
   float st[4][4];
@@ -418,13 +421,19 @@ int LaunchGdnChunked(const float* q, const float* k, const float* v, const float
   static bool configured = false;
   if (!configured) {
     cudaFuncSetAttribute(GdnChunkPrepKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sizeof(PhaseASmem)));
-    cudaFuncSetAttribute(GdnChunkScanKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sizeof(PhaseBSmem)));
+    cudaFuncSetAttribute(GdnChunkScanKernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sizeof(PhaseBSmem<32>)));
+    cudaFuncSetAttribute(GdnChunkScanKernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sizeof(PhaseBSmem<64>)));
     configured = true;
   }
   GdnChunkPrepKernel<<<dim3(chunks, H), 256, sizeof(PhaseASmem), s>>>(q, k, v, eg, beta, ws_ut, ws_w, ws_p, ws_g, T, H, Hk);
   int e = FinishLaunch();
   if (e) return e;
-  GdnChunkScanKernel<<<dim3(H, kD / kRows), kScanThreads, sizeof(PhaseBSmem), s>>>(q, k, ws_ut, ws_w, ws_p, ws_g, state, o, T, H, Hk);
+  // A CTA has an SM to itself.  32 state rows halve its four products and double the copies, so they pay while all CTAs of a
+  // launch run at once (4 H <= 148); with more heads the second half of them would wait for the first.
+  if (4 * H <= 148)
+    GdnChunkScanKernel<32><<<dim3(H, kD / 32), 32 * 8, sizeof(PhaseBSmem<32>), s>>>(q, k, ws_ut, ws_w, ws_p, ws_g, state, o, T, H, Hk);
+  else
+    GdnChunkScanKernel<64><<<dim3(H, kD / 64), 64 * 8, sizeof(PhaseBSmem<64>), s>>>(q, k, ws_ut, ws_w, ws_p, ws_g, state, o, T, H, Hk);
   return FinishLaunch();
 }
 

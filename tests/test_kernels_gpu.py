@@ -625,6 +625,27 @@ def test_gdn_chunk_log_decays_fall_monotonically(K):
     assert (G[..., 1:] <= G[..., :-1]).all() and float(G.min()) < -2000
 
 
+@pytest.mark.parametrize("T", [128, 333])
+def test_gdn_scan_of_37_heads_has_the_bits_of_38(K, T):
+    """37 heads run with 32 state rows per CTA, 38 with 64: the tile a state row falls into changes none of its sums."""
+    D, H = 128, 38
+    g = torch.Generator().manual_seed(T)
+    mixed, z, ab = torch.randn(T, 3, H, D, generator=g) * 0.5, torch.randn(T, H, D, generator=g), torch.randn(T, 2, H, generator=g)
+    conv_w, state0 = torch.randn(3, H, D, 4, generator=g) * 0.5, torch.randn(H, D, D, generator=g) * 0.1
+
+    def run(n):
+        sc = {s: torch.empty(T, n, D, device="cuda") for s in "qkvo"}
+        sc.update(eg=torch.empty(T, n, device="cuda"), beta=torch.empty(T, n, device="cuda"), ws=torch.zeros(K.gdn_chunk_ws_floats(T, n), device="cuda"))
+        state, out = state0[:n].contiguous().cuda(), torch.zeros(T, n * D, dtype=BF, device="cuda")
+        K.gdn_prefill(mixed[:, :, :n].reshape(T, -1).to(BF).cuda(), z[:, :n].reshape(T, -1).to(BF).cuda(), ab[..., :n].reshape(T, -1).contiguous().cuda(),
+                      conv_w[:, :n].reshape(-1, 4).to(BF).cuda(), torch.zeros(n, device="cuda"), torch.zeros(n, device="cuda"), torch.ones(D, device="cuda").to(BF),
+                      torch.zeros(16, 3 * n * D, dtype=BF, device="cuda"), state, sc, out, T, n, n, D, 0)
+        return out.view(T, n, D), state
+
+    (o37, s37), (o38, s38) = run(37), run(38)
+    assert torch.equal(o37, o38[:, :37]) and torch.equal(s37, s38[:37])
+
+
 @pytest.mark.parametrize("D,Hv,Hk,T", [(128, 6, 2, 70), (64, 4, 2, 33)])
 def test_gdn_prefill_matches_recurrence_and_hands_over_to_decode(K, D, Hv, Hk, T):
     g = torch.Generator().manual_seed(D + T)
