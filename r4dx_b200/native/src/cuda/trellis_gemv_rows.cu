@@ -1,32 +1,28 @@
-// Trellis-decode weight-streaming product for 1..8 activation rows on mma.sync, with the hash bytes themselves as the operand.
+// Trellis-decode weight-streaming product for 1..8 activation rows on mma.sync, the weights decoded straight into its operands.
 //
-//   y[t, n] = bf16( svh[n] * H128( sum_k Q[n, k] * xh[t, k] )[n] (+ residual[t, n]) ),  xh = H128(suh (.) act(x))
+//   y[t, n] = bf16( svh[n] * H128( sum_k Q[n, k] * xh[t, k] )[n] (+ residual[t, n]) ),  xh = fp16(H128(suh (.) act(x)))
 //
-// A code value is  Q = scale * (1024 + b0 + b1 + b2 + b3) + bias  with the four bytes b of state * 0x83DCD12D.  A hash word is
-// therefore four consecutive K bytes of an unsigned 8-bit operand, and
-//     sum_k Q[n, k] x[k] = scale * sum_k (b0 + b1 + b2 + b3)[n, k] x[k] + (1024 scale + bias) * sum_k x[k]
-// needs no byte sum, no packing and no multiply-add on the CUDA cores: a weight costs its state's extraction, one multiply and
-// a quarter of an m16n8k32 instruction per four rows of x.  The rows are integers too: q = round(x * 32512 / max|x|) over the
-// CTA's K slice, split into two signed bytes that are two columns of the product; sums are exact in int32 (a slice of 32768
-// columns at the largest digits stays below 2^31).  Against 64 bits the product is closer than with fp16 rows and fp16 partial
-// sums (2.1e-4 against 6.1e-4 relative before the bf16 rounding; unrounded code values are most of what is left).
+// Operands are those of the prompt path's tcgen05 product: code values as the format defines them (one fp16 rounding), fp16 rows,
+// products and sums in fp32.  One m16n8k16 takes 256 weights times up to eight rows, so a weight costs its state's extraction, a
+// multiply, a byte sum, half a byte permute and half a multiply-add, whatever the row count.
+// (The hash bytes themselves as 8-bit operands, with rows of two signed digits, need neither byte sum nor packing, but multiply
+// by code values that are not rounded, and the digits of a row share one exponent: 2.2e-4 of a product against 64 bits where this
+// form and the tcgen05 product have 2.0e-4.)
 //
-// What bounds it: the register-file ports.  Per 128 weights a scheduler issues about 14 instructions, one of them an MMA with
-// ten register operands, and a mix of 4 byte permutes, 4 multiplies and one MMA alone takes 13 to 17 clocks (8 if only the
-// pipes counted): about 20 weights per clock and SM, 2.8 TB/s of 4-bit codes, whatever the row count.  Measured against the
-// CUDA-core kernel (trellis_gemv.cu), 4 bits, us at 2 / 4 / 8 rows: 34816 x 5120 48 / 46 / 60 (70 / 90 / 136), 5120 x 17408
-// 32 / 32 / 40 (49 / 72 / 117), 16384 x 5120 30 / 30 / 36 (45 / 55 / 84), 5120 x 6144 17 / 19 / 22 (22 / 27 / 41).  (One row
-// takes the other kernel: see ops/kernels.py:ROWS_MIN_ROWS.)
+// What bounds it: instructions.  Per 256 weights a warp issues 8 extractions, 8 multiplies, 8 byte sums, 4 permutes, 4 multiply-adds
+// and one MMA, 41 clocks of a scheduler by themselves.  us at 2 / 4 / 8 rows, 4 bits, against the CUDA-core kernel
+// (trellis_gemv.cu): 34816 x 5120 52 / 52 / 54 (66 / 82 / 121), 5120 x 17408 34 / 36 / 34 (45 / 68 / 98), 16384 x 5120
+// 32 / 32 / 30 (39 / 47 / 71), 5120 x 6144 20 / 19 / 19 (23 / 27 / 39).  (The 8-bit form took 44 / 44 / 56, 32 / 32 / 36.)  One
+// row takes the other kernel: see ops/kernels.py:ROWS_MIN_ROWS.
 //
 // Grouped mode (mixture-of-experts blocks with a few rows per expert): a CTA serves one 128-row block of one tile of the routing
-// plan, up to four rows of one expert; the digits are those of the planned pairs in expert order.  A block of 512 experts
-// (top 10, hidden 2048) takes 266 / 463 / 734 us at 17 / 64 / 200 rows of x where the tcgen05 tiles of 16 rows take 364 / 644 /
-// 822: most experts have one or two rows, and decoding their weights is the work.  (Tiles of eight rows are slower at every
-// row count: twice the MMAs and one CTA per SM.)
+// plan, up to four rows of one expert; the rows are those of the planned pairs in expert order.  A block of 512
+// experts (top 10, hidden 2048) takes 261 / 478 / 755 us at 17 / 64 / 200 rows of x where the tcgen05 tiles of 16 rows take 338 /
+// 626 / 799: most experts have one or two rows, and decoding their weights is the work.
 //
-// Two launches: TrellisDigitsKernel writes the rows' digits once (every CTA would otherwise repeat the transform: at 8 rows of
-// 5120 columns that was 74k of 103k clocks, at one row 8k of 50k), then one CTA per (128-row block, K slice) streams words
-// through a ring of bulk copies - filled before the wait for the digits - and `ksplit` CTAs of a cluster add up over
+// Two launches: TrellisRowsInputKernel writes the transformed rows once (every CTA would otherwise repeat the transform: at 8 rows
+// of 5120 columns that was 74k of 103k clocks), then one CTA per (128-row block, K slice) streams words
+// through a ring of bulk copies - filled before the wait for the rows - and `ksplit` CTAs of a cluster add up over
 // distributed shared memory in rank order.
 #include <cooperative_groups.h>
 
@@ -52,20 +48,13 @@ constexpr int kBarriers = 12;
 static_assert(kBarriers % kTeams == 0 && kBarriers >= kMaxStages, "the blocks of a barrier belong to one team, and at most one of them is in flight");
 constexpr int kMaxSiblings = 3;
 
-// Digits of one row of x over one K slice: the slice's scale and sum.
-struct DigitMeta {
-  uint32_t amax;                         // bit pattern of the largest magnitude
-  int xsum;
-};
-
 struct RowsArgs {
   const __nv_bfloat16* x;
   const __nv_bfloat16* residual;
   const __nv_bfloat16* norm_w;           // prologue mode 1
   float eps;
   int T, K, kblocks_per_cta, stages, act;
-  const unsigned char* digits;           // [siblings][2 T columns][K]
-  const DigitMeta* meta;                 // [siblings][ksplit][T]
+  const __half* xh;                      // [siblings][T][K], the k-tiles of every 128 columns in StoredTile order
   // one to three weights that read the same rows through the same prologue; blockIdx.y runs over all their row blocks
   // grouped mode
   const int* g_offsets;                  // [E + 1] into g_perm
@@ -87,24 +76,25 @@ struct RowsArgs {
 struct Ctl {                             // control block at the start of dynamic shared memory
   uint64_t full[kBarriers], empty[kBarriers];   // of block b % kBarriers
   uint64_t red_bar;                      // split-K partials have landed
-  uint64_t xfull;                        // digits have landed
+  uint64_t xfull;                        // rows have landed
   int abort_flag;
   int pad;
-  float unit[8];                         // value of one integer step of a row
-  int xsum[8];                           // sum of a row's integers
-  uint32_t fill[26];
+  uint32_t fill[10];
 };
 static_assert(sizeof(Ctl) % 128 == 0, "what follows the control block is 128-byte aligned");
-constexpr float kDigitRange = 32512.f;   // 127 * 256: the high digit stays a signed byte after rounding the low one
 
-// bytes between two digit columns: neighbouring columns (and the two k-tile pairs of a quad) fall into different banks
-__host__ __device__ constexpr int XStride(int kslice) { return kslice + 32; }
+// Place of a k-tile inside its 128 columns of a stored row: the four k-tiles that a quad of lanes reads together (see the main
+// loop) lie side by side, 32 bytes each.
+__host__ __device__ constexpr int StoredTile(int kt) { return ((kt >> 1) & 1) * 4 + (kt >> 2) * 2 + (kt & 1); }
+
+// bytes between two rows in shared memory: neighbouring rows start 16 bytes apart modulo the banks
+__host__ __device__ constexpr int XStride(int kslice) { return kslice * 2 + 16; }
 
 __device__ __forceinline__ void ConsumerSync() { asm volatile("bar.sync 1, %0;" ::"r"(kConsumerWarps * 32) : "memory"); }
 
-__device__ __forceinline__ void MmaU8S8(int (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-  asm("mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
-      : "+r"(d[0]), "+r"(d[1]), "+r"(d[2]), "+r"(d[3])
+__device__ __forceinline__ void MmaF16(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
       : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
@@ -113,8 +103,8 @@ __device__ __forceinline__ float SumSquares8(const uint4& v) {
          BfLo(v.z) * BfLo(v.z) + BfHi(v.z) * BfHi(v.z) + BfLo(v.w) * BfLo(v.w) + BfHi(v.w) * BfHi(v.w);
 }
 
-// Sum of squares of one eighth of a row (warps 0..7 of a CTA); every kernel that needs the RMS of a row adds the eighths in order,
-// so that they all round alike.
+// Sum of squares of one eighth of a row (warps 0..7 of a CTA); the eighths are added in order, as in the CUDA-core kernel's
+// prologue.
 __device__ __forceinline__ float EighthSumSquares(const __nv_bfloat16* row, int K, int warp, int lane) {
   const int kw = (K / 8 + 7) & ~7;    // columns per warp, a multiple of 8
   const int k_lo = warp * kw, k_hi = min(K, k_lo + kw);
@@ -149,51 +139,16 @@ __device__ __forceinline__ void Activate(uint2 xv, uint2 uv, uint2 wv, uint2 sv,
   v[0] *= __low2float(s01); v[1] *= __high2float(s01); v[2] *= __low2float(s23); v[3] *= __high2float(s23);
 }
 
-// largest magnitude of a 128-column block as a bit pattern (a NaN is larger than infinity); v becomes the transformed block
-__device__ __forceinline__ uint32_t HadamardMax(float (&v)[4]) {
-  const float inv_sqrt = 0.08838834764831845f;   // 1 / sqrt(128)
-  WarpFwht128(v);
-#pragma unroll
-  for (int i = 0; i < 4; ++i) v[i] *= inv_sqrt;
-  const uint32_t m01 = max(__float_as_uint(fabsf(v[0])), __float_as_uint(fabsf(v[1])));
-  const uint32_t m23 = max(__float_as_uint(fabsf(v[2])), __float_as_uint(fabsf(v[3])));
-  return __reduce_max_sync(0xffffffffu, max(m01, m23));
-}
-
-// 32512 / amax; zero for a row of zeros (or of values below 1e-30, where the quotient would overflow) and for a row with a NaN
-// or an infinity, whose scale is poisoned later
-__device__ __forceinline__ float DigitScale(uint32_t amax_bits) {
-  const float amax = __uint_as_float(amax_bits);
-  return amax > 1e-30f && amax < INFINITY ? kDigitRange / amax : 0.f;
-}
-// q = round(v * inv) = 256 hi + lo; returns the block's sum of q
-__device__ __forceinline__ int Digits(const float (&v)[4], float inv, uint32_t (&hi)[4], uint32_t (&lo)[4]) {
-  int sum = 0;
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int q = __float2int_rn(v[i] * inv);
-    hi[i] = static_cast<uint32_t>((q + 128) >> 8) & 0xFFu;
-    lo[i] = static_cast<uint32_t>(q) & 0xFFu;
-    sum += q;
-  }
-  return __reduce_add_sync(0xffffffffu, sum);
-}
-__device__ __forceinline__ uint32_t PackBytes(const uint32_t (&b)[4]) { return b[0] | (b[1] << 8) | (b[2] << 16) | (b[3] << 24); }
-
-// The digits of T rows for a whole launch: grid (T, ksplit, weights), one CTA per (row, K slice, weight).
-constexpr int kDigitWarps = 16;
-constexpr int kDigitBlocks = 4;          // 128-column blocks a warp keeps in registers
-// Grouped: grid (pairs), t = sorted position.  A chain of latencies: the signs and norm weights, which no kernel writes, are
-// requested before the wait for the previous kernel, all of a warp's activations at once after it, and the transformed values
-// stay in registers between the two barriers (slices of more than 64 blocks keep them in shared memory instead): 5.8 -> 3.4 us
-// behind an RMSNorm of 5120 columns in a captured window of four rows, against one block's loads at a time.
+// The transformed rows of a launch: grid (T, parts, weights), a warp takes up to kInBlocks 128-column blocks.
+constexpr int kInWarps = 16;
+constexpr int kInBlocks = 2;
+inline int InputParts(int K) { return (K / 128 + kInWarps * kInBlocks - 1) / (kInWarps * kInBlocks); }
+// Grouped: grid (pairs, parts), t = sorted position.  A chain of latencies: the signs and norm weights, which no kernel writes,
+// are requested before the wait for the previous kernel and all of a warp's activations at once after it.
 template <int PRO, bool kGrouped>
-__global__ void __launch_bounds__(kDigitWarps * 32) TrellisDigitsKernel(RowsArgs a, unsigned char* digits, DigitMeta* meta) {
-  extern __shared__ __align__(16) float rowbuf[];      // long slices: transformed columns
+__global__ void __launch_bounds__(kInWarps * 32) TrellisRowsInputKernel(RowsArgs a, __half* xh) {
   __shared__ float red[8];
-  __shared__ uint32_t amax;
-  __shared__ int xsum;
-  const int t = blockIdx.x, krank = blockIdx.y, ksplit = gridDim.y, sib = blockIdx.z, T = a.T, K = a.K;
+  const int t = blockIdx.x, sib = blockIdx.z, T = a.T, K = a.K;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
   const __half* suh = a.w[sib].suh;
   int xrow = t;
@@ -209,30 +164,22 @@ __global__ void __launch_bounds__(kDigitWarps * 32) TrellisDigitsKernel(RowsArgs
     suh += static_cast<size_t>(lo) * K;
     xrow = __ldg(a.g_perm + t) / a.g_xdiv;
   }
-  const int kb_lo = krank * (K / 128) / ksplit, my_blocks = (krank + 1) * (K / 128) / ksplit - kb_lo;
-  const bool in_regs = my_blocks <= kDigitBlocks * warps;
-  if (threadIdx.x == 0) { amax = 0u; xsum = 0; }
-  uint2 sv[kDigitBlocks], nv[kDigitBlocks];
-  auto load_weights = [&](int i, int b) {
-    const int k = (kb_lo + b) * 128 + lane * 4;
-    sv[i] = *reinterpret_cast<const uint2*>(suh + k);
-    if constexpr (PRO == 1) nv[i] = *reinterpret_cast<const uint2*>(a.norm_w + k);
-    else nv[i] = make_uint2(0u, 0u);
-  };
-  const __nv_bfloat16* xin = a.x + static_cast<size_t>(xrow) * (PRO == 2 ? 2 * static_cast<size_t>(K) : K);
-  uint2 xv[kDigitBlocks], uv[kDigitBlocks];
-  auto load_x = [&](int i, int b) {
-    const int k = (kb_lo + b) * 128 + lane * 4;
-    xv[i] = *reinterpret_cast<const uint2*>(xin + k);
-    uv[i] = PRO == 2 ? *reinterpret_cast<const uint2*>(xin + K + k) : make_uint2(0u, 0u);
-  };
+  const int b0 = blockIdx.y * warps * kInBlocks + warp, blocks = K / 128;      // this warp's blocks: b0, b0 + warps, ..
+  uint2 sv[kInBlocks], nv[kInBlocks], xv[kInBlocks], uv[kInBlocks];
 #pragma unroll
-  for (int i = 0; i < kDigitBlocks; ++i)
-    if (in_regs && warp + i * warps < my_blocks) load_weights(i, warp + i * warps);
+  for (int i = 0; i < kInBlocks; ++i) {
+    const int k = min(b0 + i * warps, blocks - 1) * 128 + lane * 4;
+    sv[i] = *reinterpret_cast<const uint2*>(suh + k);
+    nv[i] = PRO == 1 ? *reinterpret_cast<const uint2*>(a.norm_w + k) : make_uint2(0u, 0u);
+  }
+  const __nv_bfloat16* xin = a.x + static_cast<size_t>(xrow) * (PRO == 2 ? 2 * static_cast<size_t>(K) : K);
   if constexpr (!kGrouped) asm volatile("griddepcontrol.wait;" ::: "memory");
 #pragma unroll
-  for (int i = 0; i < kDigitBlocks; ++i)
-    if (in_regs && warp + i * warps < my_blocks) load_x(i, warp + i * warps);
+  for (int i = 0; i < kInBlocks; ++i) {
+    const int k = min(b0 + i * warps, blocks - 1) * 128 + lane * 4;
+    xv[i] = *reinterpret_cast<const uint2*>(xin + k);
+    uv[i] = PRO == 2 ? *reinterpret_cast<const uint2*>(xin + K + k) : make_uint2(0u, 0u);
+  }
   float r = 0.f;
   if constexpr (PRO == 1) {
     if (warp < 8) {
@@ -241,57 +188,28 @@ __global__ void __launch_bounds__(kDigitWarps * 32) TrellisDigitsKernel(RowsArgs
     }
     __syncthreads();
     r = RowRms(red, K, a.eps);
-  } else {
-    __syncthreads();
   }
-  float v[kDigitBlocks][4];
-  uint32_t m = 0u;
-  if (in_regs) {
+  __half* dst = xh + (static_cast<size_t>(sib) * T + t) * K + StoredTile(lane >> 2) * 16 + (lane & 3) * 4;
 #pragma unroll
-    for (int i = 0; i < kDigitBlocks; ++i)
-      if (warp + i * warps < my_blocks) {
-        Activate<PRO>(xv[i], uv[i], nv[i], sv[i], r, a.act, v[i]);
-        m = max(m, HadamardMax(v[i]));
-      }
-  } else {
-    for (int b = warp; b < my_blocks; b += warps) {
-      load_weights(0, b);
-      load_x(0, b);
-      Activate<PRO>(xv[0], uv[0], nv[0], sv[0], r, a.act, v[0]);
-      m = max(m, HadamardMax(v[0]));
-      *reinterpret_cast<float4*>(rowbuf + b * 128 + lane * 4) = make_float4(v[0][0], v[0][1], v[0][2], v[0][3]);
-    }
+  for (int i = 0; i < kInBlocks; ++i) {
+    if (b0 + i * warps >= blocks) break;
+    float v[4];
+    Activate<PRO>(xv[i], uv[i], nv[i], sv[i], r, a.act, v);
+    WarpFwht128(v);
+    const float inv_sqrt = 0.08838834764831845f;   // 1 / sqrt(128)
+    const __half2 o01 = __floats2half2_rn(v[0] * inv_sqrt, v[1] * inv_sqrt), o23 = __floats2half2_rn(v[2] * inv_sqrt, v[3] * inv_sqrt);
+    uint2 ov;
+    ov.x = *reinterpret_cast<const uint32_t*>(&o01);
+    ov.y = *reinterpret_cast<const uint32_t*>(&o23);
+    *reinterpret_cast<uint2*>(dst + (b0 + i * warps) * 128) = ov;
   }
-  if (lane == 0) atomicMax(&amax, m);
-  __syncthreads();
-  int sum = 0;
-  const float inv = DigitScale(amax);
-  auto write = [&](int b, const float (&x)[4]) {
-    uint32_t hi[4], lo[4];
-    sum += Digits(x, inv, hi, lo);
-    unsigned char* c0 = digits + (static_cast<size_t>(sib) * 2 * T + 2 * static_cast<size_t>(t)) * K + (kb_lo + b) * 128 + lane * 4;
-    *reinterpret_cast<uint32_t*>(c0) = PackBytes(hi);
-    *reinterpret_cast<uint32_t*>(c0 + K) = PackBytes(lo);
-  };
-  if (in_regs) {
-#pragma unroll
-    for (int i = 0; i < kDigitBlocks; ++i)
-      if (warp + i * warps < my_blocks) write(warp + i * warps, v[i]);
-  } else {
-    for (int b = warp; b < my_blocks; b += warps) {
-      const float4 f = *reinterpret_cast<const float4*>(rowbuf + b * 128 + lane * 4);
-      v[0][0] = f.x; v[0][1] = f.y; v[0][2] = f.z; v[0][3] = f.w;
-      write(b, v[0]);
-    }
-  }
-  if (lane == 0) atomicAdd(&xsum, sum);
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    DigitMeta d;
-    d.amax = amax;
-    d.xsum = xsum;
-    meta[(sib * ksplit + krank) * T + t] = d;
-  }
+}
+
+// two code values of a row of a tile (positions J, J + 1) as an operand register
+template <int KB, int J>
+__device__ __forceinline__ uint32_t Code2(const uint32_t (&w)[3]) {
+  const __half2 q = TrellisCode2(TrellisRow<KB>::template State<J>(w[2], w[1], w[0]), TrellisRow<KB>::template State<J + 1>(w[2], w[1], w[0]));
+  return *reinterpret_cast<const uint32_t*>(&q);
 }
 
 template <int KB, int TMAX, bool kGrouped = false>
@@ -306,7 +224,7 @@ __global__ void __launch_bounds__(kThreads, TMAX > 4 ? 1 : 2) TrellisRowsKernel(
   while (sidx + 1 < a.count && nb >= a.w[sidx].nb_end) ++sidx;
   if (sidx > 0) nb -= a.w[sidx - 1].nb_end;
   const int N = a.w[sidx].N, K = a.K;
-  int T = a.T, start = 0;                  // rows of this CTA, the first one's place in the digits
+  int T = a.T, start = 0;                  // rows of this CTA, the first one's place in xh
   const uint32_t* words = a.w[sidx].words;
   const __half* svh = a.w[sidx].svh;
   if constexpr (kGrouped) {
@@ -330,14 +248,13 @@ __global__ void __launch_bounds__(kThreads, TMAX > 4 ? 1 : 2) TrellisRowsKernel(
   constexpr int kTileBytes = 8 * NW * 4;
   constexpr int kHalfSlot = 4 * kTileBytes + 64;
   constexpr int kStageSlot = 2 * kHalfSlot;
-  constexpr int NG = TMAX > 4 ? 2 : 1;            // column groups: 8 columns = 4 rows of x, two digits each
 
   const int xstride = XStride(kslice);
   Ctl* ctl = reinterpret_cast<Ctl*>(smem_raw);
   float* loc = reinterpret_cast<float*>(smem_raw + sizeof(Ctl));                     // [kSums][TMAX][128] sums of (k-tile half, team)
   float* part = loc + kSums * TMAX * 128;                                             // [ksplit][TMAX][128] (used on cluster rank 0)
-  unsigned char* xd = reinterpret_cast<unsigned char*>(part + (ksplit > 1 ? ksplit : 0) * TMAX * 128);   // digits: [2 TMAX columns][xstride]
-  unsigned char* wst = xd + static_cast<size_t>(2 * TMAX) * xstride;                 // [stages][kStageSlot]
+  unsigned char* xs = reinterpret_cast<unsigned char*>(part + (ksplit > 1 ? ksplit : 0) * TMAX * 128);   // rows: [TMAX][xstride]
+  unsigned char* wst = xs + static_cast<size_t>(TMAX) * xstride;                     // [stages][kStageSlot]
   uint64_t* red_bar = &ctl->red_bar;
   volatile int* abort_flag = &ctl->abort_flag;
   const uint32_t full_at = ptx::SmemAddr(ctl->full), wst_at = ptx::SmemAddr(wst);      // (the empty barriers follow the full ones)
@@ -361,7 +278,7 @@ __global__ void __launch_bounds__(kThreads, TMAX > 4 ? 1 : 2) TrellisRowsKernel(
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
   if (warp == kConsumerWarps) {
-    // ---------------- producer: this CTA's words through the stage ring, the digits once the ring is full ----------------
+    // ---------------- producer: this CTA's words through the stage ring, the rows once the ring is full ----------------
     if (lane == 0) {
       const unsigned char* src = reinterpret_cast<const unsigned char*>(words) +
                                  (static_cast<size_t>(nb) * (K / 128) + static_cast<size_t>(kb_lo)) * kStageBytes;
@@ -371,10 +288,10 @@ __global__ void __launch_bounds__(kThreads, TMAX > 4 ? 1 : 2) TrellisRowsKernel(
       for (int it = 0; it <= my_blocks; ++it) {
         if (it == min(a.stages, my_blocks)) {
           asm volatile("griddepcontrol.wait;" ::: "memory");
-          ptx::MbarArriveExpectTx(&ctl->xfull, 2 * T * my_blocks * 128);
-          const unsigned char* xsrc = a.digits + (static_cast<size_t>(sidx) * 2 * T + 2 * static_cast<size_t>(start)) * K + kb_lo * 128;
-          for (int c = 0; c < 2 * T; ++c)
-            ptx::BulkLoad(xd + static_cast<size_t>(c) * xstride, xsrc + static_cast<size_t>(c) * K, my_blocks * 128, &ctl->xfull);
+          ptx::MbarArriveExpectTx(&ctl->xfull, T * my_blocks * 256);
+          const __half* xsrc = a.xh + (static_cast<size_t>(sidx) * T + start) * K + kb_lo * 128;
+          for (int t = 0; t < T; ++t)
+            ptx::BulkLoad(xs + static_cast<size_t>(t) * xstride, xsrc + static_cast<size_t>(t) * K, my_blocks * 256, &ctl->xfull);
         }
         if (it == my_blocks) break;
         if (it >= a.stages) {
@@ -391,51 +308,32 @@ __global__ void __launch_bounds__(kThreads, TMAX > 4 ? 1 : 2) TrellisRowsKernel(
     }
   } else {
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    if (threadIdx.x < T) {
-      const DigitMeta m = a.meta[(sidx * ksplit + krank) * T + start + threadIdx.x];
-      // an infinity or a NaN anywhere in the slice makes the whole row one
-      ctl->unit[threadIdx.x] = m.amax < 0x7F800000u ? __uint_as_float(m.amax) / kDigitRange : __int_as_float(0x7FC00000);
-      ctl->xsum[threadIdx.x] = m.xsum;
-    }
     bool ok = ptx::MbarWait(&ctl->xfull, 0, abort_flag, 3);
-    ConsumerSync();
 
     // ---------------- main loop: a team of four warps takes every fourth K block ----------------
     // a warp has four of the block's k-tiles and four of its n-tiles;
-    // lane (g, c): rows g and g + 8 of an n-tile, the 16 columns of its k-tile; column g of the product = row g / 2 of x, digit g % 2
+    // lane (g, c): rows g and g + 8 of an n-tile, the 16 columns of its k-tile, four of them per MMA (the contraction index of
+    // the fragments maps to columns alike in both operands); column g of the product = row g of x
     const int team = warp / kTeamWarps, w4 = warp % kTeamWarps;
     const int g = lane >> 2, c = lane & 3, kq = w4 & 1, nt0 = (w4 >> 1) * 4;
-    const int kt = (c >> 1) * 4 + kq * 2 + (c & 1);        // the lane's k-tile
-    TrellisRow<KB> ra, rb;
+    TrellisRow<KB> ra, rb;                                 // (the lane's k-tile is (c >> 1) * 4 + kq * 2 + (c & 1))
     ra.Init(g);
     rb.Init(g + 8);
-    int acc[4][NG][4];
+    float acc[4][4];
 #pragma unroll
     for (int n = 0; n < 4; ++n)
 #pragma unroll
-      for (int q = 0; q < NG; ++q)
-#pragma unroll
-        for (int i = 0; i < 4; ++i) acc[n][q][i] = 0;
-    const bool two_groups = NG == 2 && T > 4;
+      for (int i = 0; i < 4; ++i) acc[n][i] = 0.f;
     // columns past the last row of x repeat it: a column of the product depends on its own column of x only
-    const unsigned char* xcol[NG];
-#pragma unroll
-    for (int q = 0; q < NG; ++q)
-      xcol[q] = xd + static_cast<size_t>(min(g + 8 * q, 2 * T - 1)) * xstride + kt * 16;
+    const unsigned char* xrow = xs + static_cast<size_t>(min(g, T - 1)) * xstride + (kq * 4 + c) * 32;
     // stage index and barrier parity advance by counting: a division by the run-time ring depth per 128-wide
     // K block would cost as much as decoding a dozen weights
     int s = team, b = team;
     uint32_t phase = 0;
     while (s >= a.stages) s -= a.stages;
     for (int it = team; it < my_blocks && ok; it += kTeams) {
-      uint32_t bx[NG][16];
-#pragma unroll
-      for (int q = 0; q < NG; ++q) {
-        const uint4 v = *reinterpret_cast<const uint4*>(xcol[q] + it * 128);
-        const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-        for (int i = 0; i < 16; ++i) bx[q][i] = __byte_perm(w[i >> 2], 0u, 0x1111 * (i & 3));      // a byte four times over
-      }
+      const uint4 xlo = *reinterpret_cast<const uint4*>(xrow + it * 256), xhi = *reinterpret_cast<const uint4*>(xrow + it * 256 + 16);
+      const uint32_t bx[8] = {xlo.x, xlo.y, xlo.z, xlo.w, xhi.x, xhi.y, xhi.z, xhi.w};
       ok = ptx::MbarWaitAt(full_at + b * 8, phase, abort_flag, 2);
       if (!ok) break;
       const unsigned char* st = wst + s * kStageSlot + (c >> 1) * kHalfSlot + (kq * 2 + (c & 1)) * kTileBytes + nt0 * (NW * 4);
@@ -445,18 +343,14 @@ __global__ void __launch_bounds__(kThreads, TMAX > 4 ? 1 : 2) TrellisRowsKernel(
         uint32_t wa[3], wb[3];
         ra.Load(tw, wa[2], wa[1], wa[0]);
         rb.Load(tw, wb[2], wb[1], wb[0]);
-#define R4DXB_I8_STEP(I)                                                                                              \
+#define R4DXB_STEP(I)                                                                                                  \
   {                                                                                                                   \
-    const uint32_t a0 = TrellisRow<KB>::template State<2 * I>(wa[2], wa[1], wa[0]) * R4DXB_TRELLIS_MUL;                \
-    const uint32_t a1 = TrellisRow<KB>::template State<2 * I>(wb[2], wb[1], wb[0]) * R4DXB_TRELLIS_MUL;                \
-    const uint32_t a2 = TrellisRow<KB>::template State<2 * I + 1>(wa[2], wa[1], wa[0]) * R4DXB_TRELLIS_MUL;            \
-    const uint32_t a3 = TrellisRow<KB>::template State<2 * I + 1>(wb[2], wb[1], wb[0]) * R4DXB_TRELLIS_MUL;            \
-    MmaU8S8(acc[n][0], a0, a1, a2, a3, bx[0][2 * I], bx[0][2 * I + 1]);                                               \
-    if (two_groups) MmaU8S8(acc[n][NG - 1], a0, a1, a2, a3, bx[NG - 1][2 * I], bx[NG - 1][2 * I + 1]);                \
+    const uint32_t a0 = Code2<KB, 4 * I>(wa), a1 = Code2<KB, 4 * I>(wb);                                               \
+    const uint32_t a2 = Code2<KB, 4 * I + 2>(wa), a3 = Code2<KB, 4 * I + 2>(wb);                                       \
+    MmaF16(acc[n], a0, a1, a2, a3, bx[2 * I], bx[2 * I + 1]);                                                          \
   }
-        R4DXB_I8_STEP(0) R4DXB_I8_STEP(1) R4DXB_I8_STEP(2) R4DXB_I8_STEP(3)
-        R4DXB_I8_STEP(4) R4DXB_I8_STEP(5) R4DXB_I8_STEP(6) R4DXB_I8_STEP(7)
-#undef R4DXB_I8_STEP
+        R4DXB_STEP(0) R4DXB_STEP(1) R4DXB_STEP(2) R4DXB_STEP(3)
+#undef R4DXB_STEP
       }
       __syncwarp();
       if (lane == 0) ptx::MbarArriveAt(full_at + (kBarriers + b) * 8);
@@ -466,24 +360,14 @@ __global__ void __launch_bounds__(kThreads, TMAX > 4 ? 1 : 2) TrellisRowsKernel(
       if (b >= kBarriers) { b -= kBarriers; phase ^= 1u; }
     }
     // the sums of a row (k-tile half, team) meet in shared memory
-    const float code_scale = __half2float(__ushort_as_half(R4DXB_TRELLIS_SCALE_F16));
-    const float code_zero = 1024.f * code_scale + __half2float(__ushort_as_half(R4DXB_TRELLIS_BIAS_F16));
     float* mine = loc + (team * 2 + kq) * TMAX * 128 + nt0 * 16 + g;
 #pragma unroll
-    for (int q = 0; q < NG; ++q) {
-      const int t = c + 4 * q;
-      if (t < T) {
-        const float unit = ok ? ctl->unit[t] : __int_as_float(0x7FC00000);      // (a copy that never landed shows as NaN)
-        const float zero = team + kq == 0 ? code_zero * static_cast<float>(ctl->xsum[t]) : 0.f;
+    for (int n = 0; n < 4; ++n)
 #pragma unroll
-        for (int n = 0; n < 4; ++n)
-#pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            const float v = fmaf(static_cast<float>(acc[n][q][2 * h]), 256.f, static_cast<float>(acc[n][q][2 * h + 1]));
-            mine[t * 128 + n * 16 + 8 * h] = unit * fmaf(code_scale, v, zero);
-          }
+      for (int i = 0; i < 4; ++i) {
+        const int t = 2 * c + (i & 1);
+        if (t < T) mine[t * 128 + n * 16 + 8 * (i >> 1)] = ok ? acc[n][i] : __int_as_float(0x7FC00000);      // (a copy that never landed shows as NaN)
       }
-    }
     ConsumerSync();
     if (ksplit > 1) {
       // hand this CTA's rows to cluster rank 0: distributed-shared-memory stores + one remote mbarrier arrival per
@@ -554,7 +438,7 @@ __global__ void __launch_bounds__(kThreads, TMAX > 4 ? 1 : 2) TrellisRowsKernel(
 template <int KB, int TMAX>
 size_t SmemBytes(int kslice, int stages, int ksplit) {
   return sizeof(Ctl) + static_cast<size_t>(kSums + (ksplit > 1 ? ksplit : 0)) * TMAX * 128 * 4 +
-         static_cast<size_t>(2 * TMAX) * XStride(kslice) + static_cast<size_t>(stages) * (2 * (4 * 8 * 8 * KB * 4 + 64));
+         static_cast<size_t>(TMAX) * XStride(kslice) + static_cast<size_t>(stages) * (2 * (4 * 8 * 8 * KB * 4 + 64));
 }
 
 size_t SmemOf(int kb, int T, int K, int ksplit) {
@@ -610,14 +494,9 @@ int LaunchGroupedRows(RowsArgs a, int max_tiles, cudaStream_t stream) {
 }
 
 template <int PRO>
-int LaunchDigits(const RowsArgs& a, int ksplit, cudaStream_t stream) {
-  const int blocks = (a.K / 128 + ksplit - 1) / ksplit;
-  const size_t smem = blocks <= kDigitBlocks * kDigitWarps ? 0 : static_cast<size_t>(blocks) * 512;
-  auto kern = TrellisDigitsKernel<PRO, false>;
-  const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-  if (e != cudaSuccess) return static_cast<int>(e);
-  return LaunchPdl(kern, dim3(a.T, ksplit, a.count), dim3(kDigitWarps * 32), smem, stream, a, const_cast<unsigned char*>(a.digits),
-                   const_cast<DigitMeta*>(a.meta));
+int LaunchInput(const RowsArgs& a, cudaStream_t stream) {
+  return LaunchPdl(TrellisRowsInputKernel<PRO, false>, dim3(a.T, InputParts(a.K), a.count), dim3(kInWarps * 32), 0, stream, a,
+                   const_cast<__half*>(a.xh));
 }
 
 template <int KB>
@@ -666,10 +545,9 @@ int r4dxb_trellis_gemv_rows(int count, const void* const* words, const void* con
     if (ksplit == 8 || K / 128 <= ksplit) return R4DXB_TOO_LARGE;
     ++ksplit;
   }
-  a.digits = static_cast<unsigned char*>(ws);
-  a.meta = reinterpret_cast<const DigitMeta*>(a.digits + static_cast<size_t>(count) * 2 * T * K);
+  a.xh = static_cast<const __half*>(ws);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  const int rc = prologue == 0 ? LaunchDigits<0>(a, ksplit, s) : (prologue == 1 ? LaunchDigits<1>(a, ksplit, s) : LaunchDigits<2>(a, ksplit, s));
+  const int rc = prologue == 0 ? LaunchInput<0>(a, s) : (prologue == 1 ? LaunchInput<1>(a, s) : LaunchInput<2>(a, s));
   if (rc) return rc;
   switch (kb) {
     case 3: return LaunchKb<3>(a, ksplit, s);
@@ -682,10 +560,9 @@ int r4dxb_trellis_gemv_rows(int count, const void* const* words, const void* con
  * planned pairs p (see the header). */
 int r4dxb_trellis_rows_grouped(const void* words, const void* suh, const void* svh, const void* x, void* y, const int* offsets,
                                const int* perm, const int* tiles, const int* ntiles, int max_tiles, int xdiv, int mode, int P, int E,
-                               int N, int K, int kb, void* digits, void* meta, void* stream) {
+                               int N, int K, int kb, void* xh, void* stream) {
   if (P < 1 || E < 1 || N < 128 || N % 128 || K < 128 || K % 128 || max_tiles < 1 || max_tiles > 65535 || xdiv < 1 || mode < 0 || mode > 2 ||
-      digits == nullptr || meta == nullptr || (reinterpret_cast<uintptr_t>(digits) & 15) ||
-      (reinterpret_cast<uintptr_t>(meta) & 7))
+      xh == nullptr || (reinterpret_cast<uintptr_t>(xh) & 15))
     return R4DXB_BAD_ARG;
   RowsArgs a = {};
   a.x = static_cast<const __nv_bfloat16*>(x);
@@ -706,15 +583,11 @@ int r4dxb_trellis_rows_grouped(const void* words, const void* suh, const void* s
   a.g_experts = E;
   a.g_xdiv = xdiv;
   a.g_words = static_cast<long long>(N / 16) * (K / 16) * 8 * kb;
-  a.digits = static_cast<unsigned char*>(digits);
-  a.meta = static_cast<const DigitMeta*>(meta);
+  a.xh = static_cast<const __half*>(xh);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  const size_t smem = K / 128 <= kDigitBlocks * min(kDigitWarps, K / 128) ? 0 : static_cast<size_t>(K) * 4;
-  if (smem > 200 * 1024) return R4DXB_TOO_LARGE;
-  auto digits_kernel = mode == 0 ? TrellisDigitsKernel<0, true> : TrellisDigitsKernel<2, true>;
-  const cudaError_t e = cudaFuncSetAttribute(digits_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-  if (e != cudaSuccess) return static_cast<int>(e);
-  digits_kernel<<<P, 32 * min(kDigitWarps, K / 128), smem, s>>>(a, static_cast<unsigned char*>(digits), static_cast<DigitMeta*>(meta));
+  auto input_kernel = mode == 0 ? TrellisRowsInputKernel<0, true> : TrellisRowsInputKernel<2, true>;
+  const int warps = min(kInWarps, K / 128), parts = (K / 128 + warps * kInBlocks - 1) / (warps * kInBlocks);
+  input_kernel<<<dim3(P, parts), 32 * warps, 0, s>>>(a, static_cast<__half*>(xh));
   if (int rc = FinishLaunch()) return rc;
   if (kb == 3) return LaunchGroupedRows<3, 4>(a, max_tiles, s);
   if (kb == 4) return LaunchGroupedRows<4, 4>(a, max_tiles, s);

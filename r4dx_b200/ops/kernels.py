@@ -252,8 +252,8 @@ register_cuda_sig("r4dxb_trellis_gemv_mma", _I, [_P, _P, _P, _P, _P, _P, _P, _F,
 
 # Which weight-streaming kernel serves T <= 8 rows: "simt" = CUDA-core decode + fp16 FMA (trellis_gemv.cu), "mma" = code values
 # written to tensor memory and contracted by tcgen05.mma kind::f16 (trellis_gemv_mma.cu), "auto" (the default) = decode in
-# registers with mma.sync on the hash bytes for large weights (trellis_gemv_rows.cu; us at 2 / 4 / 8 rows on gate_up
-# 48 / 46 / 60 against 70 / 80 / 95 for the better of the other two), else the CUDA-core kernel.
+# registers for mma.sync where rows and weights are many enough (trellis_gemv_rows.cu; us at 2 / 4 / 8 rows on gate_up
+# 52 / 52 / 54 against 66 / 78 / 94 for the better of the other two), else by row count one of the other two.
 GEMV_IMPL = os.environ.get("R4DXB_GEMV", "auto")
 
 
@@ -287,8 +287,8 @@ def _ptr1(t: torch.Tensor):
 
 def _gemv_rows(count: int, words, suh, svh, y, n, x, residual, norm_w, eps: float, prologue: int, T: int, K_: int, kb: int,
                ksplit: int) -> int:
-    """The mma.sync weight-streaming kernel; its workspace (the rows' digits) lives for the call."""
-    ws = torch.empty(count * T * (2 * K_ + 64), dtype=torch.uint8, device=x.device)
+    """The mma.sync weight-streaming kernel; its workspace (the transformed rows) lives for the call."""
+    ws = torch.empty(count * T * K_, dtype=torch.float16, device=x.device)
     return _lib().r4dxb_trellis_gemv_rows(count, words, suh, svh, y, n, _p(x), _p(residual), _p(norm_w), eps, prologue, T, K_, kb, ksplit,
                                           _p(ws), _stream())
 
@@ -852,18 +852,18 @@ def trellis_gemm_grouped(words, svh, xh, y, offsets, perm, tiles, ntiles, P: int
     return y
 
 
-register_cuda_sig("r4dxb_trellis_rows_grouped", _I, [_P] * 9 + [_I] * 8 + [_P, _P, _P])
+register_cuda_sig("r4dxb_trellis_rows_grouped", _I, [_P] * 9 + [_I] * 8 + [_P, _P])
 
 
 def trellis_rows_grouped(words, suh, svh, x, y, offsets, perm, tiles, ntiles, xdiv: int, mode: int, P: int, E: int, N: int, Kd: int,
-                         kb: int, digits: torch.Tensor, meta: torch.Tensor):
+                         kb: int, xh: torch.Tensor, meta: Optional[torch.Tensor] = None):
     """y[perm[p]] = expert e(p)'s trellis linear of act(x[perm[p] // xdiv]) for a few rows per expert (``moe_tiles`` of 4
-    rows); ``digits`` (2 Kd bytes per pair) and ``meta`` (8 bytes per pair) are workspace."""
-    if digits.numel() * digits.element_size() < 2 * Kd * P or meta.numel() * meta.element_size() < 8 * P:
+    rows); ``xh`` (2 Kd bytes per pair) is workspace.  (``meta`` was one for an earlier form of the kernel and is not read.)"""
+    if xh.numel() * xh.element_size() < 2 * Kd * P:
         raise KernelError("trellis_rows_grouped: workspace too small")
     bound = min(tiles.numel() // 2, P // 4 + E)
     _check(_lib().r4dxb_trellis_rows_grouped(_p(words), _p(suh), _p(svh), _p(x), _p(y), _p(offsets), _p(perm), _p(tiles), _p(ntiles), bound,
-                                             xdiv, mode, P, E, N, Kd, kb, _p(digits), _p(meta), _stream()), "trellis_rows_grouped")
+                                             xdiv, mode, P, E, N, Kd, kb, _p(xh), _stream()), "trellis_rows_grouped")
     return y
 
 

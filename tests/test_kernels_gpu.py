@@ -161,6 +161,22 @@ def test_trellis_rows_ring_that_wraps_many_times(K, kb, T):
         assert torch.equal(K.trellis_gemv(w, x, split_rows=1), first)
 
 
+@pytest.mark.parametrize("kb", [3, 4, 5])
+@pytest.mark.parametrize("T,N,Kd,split", [(2, 128, 128, 1), (5, 256, 640, 3), (8, 128, 2176, 1)])
+def test_trellis_rows_kernel_multiplies_the_formats_values(K, kb, T, N, Kd, split):
+    """Code values as the format defines them (one fp16 rounding) times the prompt path's fp16 rows.  Against that product in 64
+    bits only the fp32 sums and the bf16 result differ: half a bf16 step (2^-8 of the value at most) plus 2^-22 sqrt(K) of the
+    product's rms per element, 1.1e-5 at K = 2176; 2e-5 is allowed.  (Unrounded code values are 2.1e-4 off.)"""
+    from r4dx_b200.quant import trellis
+    w = trellis.random_weight(N, Kd, kb, seed=kb + T, sigma=0.02)
+    x = torch.randn(T, Kd, generator=torch.Generator().manual_seed(T)).to(BF).cuda()
+    wd = w.to("cuda")
+    xh = K.trellis_input(x, wd.suh).double().cpu()
+    ref = R.fwht(xh @ trellis.decode_codes(w).double().T) * w.svh.double()
+    y = K.trellis_gemv(wd, x, split_rows=split).double().cpu()
+    assert ((y - ref).abs() <= 2.0 ** -8 * ref.abs() + 2e-5 * ref.pow(2).mean().sqrt()).all()
+
+
 def test_one_row_products_of_large_weights_have_the_bits_of_the_cuda_core_kernel(K):
     """Whatever the size: the rounding of a one-row step decides the logits of all later ones."""
     from r4dx_b200.quant import trellis
