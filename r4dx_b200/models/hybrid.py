@@ -507,11 +507,11 @@ class HybridModel:
     def check_healthy(self, rows: int = 1) -> None:
         """Raises if a bounded device wait ran out since the last check: a timed-out collective leaves an un-reduced partial
         in the residual stream, so a token read after it must not be trusted (one small device-to-host read per call).
-        ``rows``: the row count of the call being checked (calls of four rows and more may have run the tensor-memory
-        weight-streaming kernel, whose waits report through the GEMM status word)."""
+        ``rows``: the row count of the call being checked (from ``K.ROWS_MIN_ROWS`` rows its products may have run on the
+        mma.sync or tensor-memory weight-streaming kernel, whose waits report through the GEMM status word)."""
         if self.comm is not None and self.comm.world > 1:
             self.comm.check_healthy()
-        if K.GEMV_IMPL == "mma" or (K.GEMV_IMPL == "auto" and rows >= 4):
+        if K.GEMV_IMPL == "mma" or (K.GEMV_IMPL == "auto" and rows >= K.ROWS_MIN_ROWS):
             K.check_gemm_status(self.device)
 
     def _read_token(self, idx: int) -> int:

@@ -112,10 +112,11 @@ int r4dxb_trellis_gemv_siblings(int count, const void* const* words, const void*
                                 int K, int kb, int ksplit, void* stream);
 /* One to three products of one K and bit width over the same 1..8 rows (weight i writes y[i] [T, n[i]]; a residual only with
  * count 1), the rows transformed once per call into ws: count * T * 2 K bytes, 16-byte aligned.  Any ksplit of 1..8.
- * R4DXB_TOO_LARGE where no split brings a slice into shared memory. */
+ * R4DXB_TOO_LARGE where no split brings a slice into shared memory.  status (may be null): device word that receives a code
+ * when a bounded wait ran out (the rows concerned are NaN). */
 int r4dxb_trellis_gemv_rows(int count, const void* const* words, const void* const* suh, const void* const* svh, void* const* y,
                             const int* n, const void* x, const void* residual, const void* norm_w, float eps, int prologue, int T,
-                            int K, int kb, int ksplit, void* ws, void* stream);
+                            int K, int kb, int ksplit, void* ws, int* status, void* stream);
 
 
 /* A/B switch: one-token steps use the warp-autonomous decode-attention kernel (default on); off = the window kernel
@@ -165,10 +166,10 @@ int r4dxb_trellis_gemm_grouped(const void* words, const void* svh, const void* x
                                int* status, void* stream);
 /* The same products for a few rows per expert, on the kernel of r4dxb_trellis_gemv_rows: tiles of four rows
  * (r4dxb_moe_tiles), input rows perm[p] / xdiv of x through mode (0: x, 1: SwiGLU of [2K], 2: GeGLU); workspace: xh
- * (P * 2 K bytes, 16-byte aligned). */
+ * (P * 2 K bytes, 16-byte aligned); status as above. */
 int r4dxb_trellis_rows_grouped(const void* words, const void* suh, const void* svh, const void* x, void* y, const int* offsets,
                                const int* perm, const int* tiles, const int* ntiles, int max_tiles, int xdiv, int mode, int P, int E,
-                               int N, int K, int kb, void* xh, void* stream);
+                               int N, int K, int kb, void* xh, int* status, void* stream);
 
 /* ---- batched decode (B sequences, one new token each; per-sequence state indexed by slot) ---------- */
 int r4dxb_gdn_decode_batch(const void* mixed, const void* z, const float* ab, const void* conv_w, const float* A_log,

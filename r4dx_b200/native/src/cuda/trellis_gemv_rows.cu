@@ -63,6 +63,7 @@ struct RowsArgs {
   const int* g_ntiles;
   int g_experts, g_xdiv;
   long long g_words;                     // words of one expert
+  int* status;                           // receives 700 + role code (390: split-K hand-off) when a bounded wait ran out
   int count;
   struct Weight {
     const uint32_t* words;
@@ -368,6 +369,7 @@ __global__ void __launch_bounds__(kThreads, TMAX > 4 ? 1 : 2) TrellisRowsKernel(
         const int t = 2 * c + (i & 1);
         if (t < T) mine[t * 128 + n * 16 + 8 * (i >> 1)] = ok ? acc[n][i] : __int_as_float(0x7FC00000);      // (a copy that never landed shows as NaN)
       }
+    if (!ok && lane == 0 && a.status != nullptr) atomicCAS(a.status, 0, 700 + *abort_flag);
     ConsumerSync();
     if (ksplit > 1) {
       // hand this CTA's rows to cluster rank 0: distributed-shared-memory stores + one remote mbarrier arrival per
@@ -417,7 +419,10 @@ __global__ void __launch_bounds__(kThreads, TMAX > 4 ? 1 : 2) TrellisRowsKernel(
       const float4 p = *reinterpret_cast<const float4*>(from + (r * TMAX + t) * 128 + lane * 4);
       v[0] += p.x; v[1] += p.y; v[2] += p.z; v[3] += p.w;
     }
-    if (!landed) v[0] = __int_as_float(0x7FC00000);      // a hand-off that never completes shows as NaN in the whole block
+    if (!landed) {
+      v[0] = __int_as_float(0x7FC00000);                 // a hand-off that never completes shows as NaN in the whole block
+      if (lane == 0 && a.status != nullptr) atomicCAS(a.status, 0, 390);
+    }
     WarpFwht128(v);
     const uint2 sv = *reinterpret_cast<const uint2*>(svh + n);
     const __half2 s01 = *reinterpret_cast<const __half2*>(&sv.x), s23 = *reinterpret_cast<const __half2*>(&sv.y);
@@ -516,7 +521,7 @@ extern "C" {
  * slice would not fit into shared memory. */
 int r4dxb_trellis_gemv_rows(int count, const void* const* words, const void* const* suh, const void* const* svh, void* const* y,
                             const int* n, const void* x, const void* residual, const void* norm_w, float eps, int prologue, int T,
-                            int K, int kb, int ksplit, void* ws, void* stream) {
+                            int K, int kb, int ksplit, void* ws, int* status, void* stream) {
   if (count < 1 || count > kMaxSiblings || T < 1 || T > 8 || K < 128 || K % 128 || ksplit < 1 || ksplit > 8 || K / 128 < ksplit ||
       prologue < 0 || prologue > 3 || (prologue == 1 && norm_w == nullptr) || (residual != nullptr && count > 1) || ws == nullptr ||
       (reinterpret_cast<uintptr_t>(ws) & 15) || kb < 3 || kb > 5)
@@ -530,6 +535,7 @@ int r4dxb_trellis_gemv_rows(int count, const void* const* words, const void* con
   a.K = K;
   a.act = prologue == 3 ? 1 : 0;           // GeGLU: the SwiGLU prologue with a tanh-GELU gate
   a.count = count;
+  a.status = status;
   int end = 0;
   for (int i = 0; i < count; ++i) {
     if (n[i] < 128 || n[i] % 128) return R4DXB_BAD_ARG;
@@ -560,7 +566,7 @@ int r4dxb_trellis_gemv_rows(int count, const void* const* words, const void* con
  * planned pairs p (see the header). */
 int r4dxb_trellis_rows_grouped(const void* words, const void* suh, const void* svh, const void* x, void* y, const int* offsets,
                                const int* perm, const int* tiles, const int* ntiles, int max_tiles, int xdiv, int mode, int P, int E,
-                               int N, int K, int kb, void* xh, void* stream) {
+                               int N, int K, int kb, void* xh, int* status, void* stream) {
   if (P < 1 || E < 1 || N < 128 || N % 128 || K < 128 || K % 128 || max_tiles < 1 || max_tiles > 65535 || xdiv < 1 || mode < 0 || mode > 2 ||
       xh == nullptr || (reinterpret_cast<uintptr_t>(xh) & 15))
     return R4DXB_BAD_ARG;
@@ -570,6 +576,7 @@ int r4dxb_trellis_rows_grouped(const void* words, const void* suh, const void* s
   a.K = K;
   a.act = mode == 2 ? 1 : 0;
   a.count = 1;
+  a.status = status;
   a.w[0].words = static_cast<const uint32_t*>(words);
   a.w[0].suh = static_cast<const __half*>(suh);
   a.w[0].svh = static_cast<const __half*>(svh);

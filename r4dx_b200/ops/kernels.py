@@ -232,7 +232,7 @@ _STATUS = {}
 
 
 def gemm_status(device) -> torch.Tensor:
-    """Device word that a tcgen05 kernel sets when one of its bounded waits runs out."""
+    """Device word that a tensor-core kernel sets when one of its bounded waits runs out."""
     key = torch.device(device).index or 0
     if key not in _STATUS:
         _STATUS[key] = torch.zeros(1, dtype=torch.int32, device=device)
@@ -243,7 +243,7 @@ def check_gemm_status(device) -> None:
     code = int(gemm_status(device).item())
     if code:
         gemm_status(device).zero_()
-        raise KernelError(f"tcgen05 GEMM gave up in a bounded wait (role code {code})")
+        raise KernelError(f"a tensor-core product gave up in a bounded wait (role code {code})")
 
 
 PRO_NONE, PRO_RMSNORM, PRO_SILU_MUL, PRO_GELU_MUL = 0, 1, 2, 3
@@ -278,7 +278,7 @@ def use_mma_gemv(T: int, N: int, K: int, ksplit: int) -> bool:
 
 _TOO_LARGE = 10003
 
-register_cuda_sig("r4dxb_trellis_gemv_rows", _I, [_I, _P, _P, _P, _P, _P, _P, _P, _P, _F, _I, _I, _I, _I, _I, _P, _P])
+register_cuda_sig("r4dxb_trellis_gemv_rows", _I, [_I, _P, _P, _P, _P, _P, _P, _P, _P, _F, _I, _I, _I, _I, _I, _P, _P, _P])
 
 
 def _ptr1(t: torch.Tensor):
@@ -290,7 +290,7 @@ def _gemv_rows(count: int, words, suh, svh, y, n, x, residual, norm_w, eps: floa
     """The mma.sync weight-streaming kernel; its workspace (the transformed rows) lives for the call."""
     ws = torch.empty(count * T * K_, dtype=torch.float16, device=x.device)
     return _lib().r4dxb_trellis_gemv_rows(count, words, suh, svh, y, n, _p(x), _p(residual), _p(norm_w), eps, prologue, T, K_, kb, ksplit,
-                                          _p(ws), _stream())
+                                          _p(ws), _p(gemm_status(x.device)), _stream())
 
 
 def trellis_gemv(w: TrellisWeight, x: torch.Tensor, residual: Optional[torch.Tensor] = None,
@@ -852,7 +852,7 @@ def trellis_gemm_grouped(words, svh, xh, y, offsets, perm, tiles, ntiles, P: int
     return y
 
 
-register_cuda_sig("r4dxb_trellis_rows_grouped", _I, [_P] * 9 + [_I] * 8 + [_P, _P])
+register_cuda_sig("r4dxb_trellis_rows_grouped", _I, [_P] * 9 + [_I] * 8 + [_P, _P, _P])
 
 
 def trellis_rows_grouped(words, suh, svh, x, y, offsets, perm, tiles, ntiles, xdiv: int, mode: int, P: int, E: int, N: int, Kd: int,
@@ -863,7 +863,8 @@ def trellis_rows_grouped(words, suh, svh, x, y, offsets, perm, tiles, ntiles, xd
         raise KernelError("trellis_rows_grouped: workspace too small")
     bound = min(tiles.numel() // 2, P // 4 + E)
     _check(_lib().r4dxb_trellis_rows_grouped(_p(words), _p(suh), _p(svh), _p(x), _p(y), _p(offsets), _p(perm), _p(tiles), _p(ntiles), bound,
-                                             xdiv, mode, P, E, N, Kd, kb, _p(xh), _stream()), "trellis_rows_grouped")
+                                             xdiv, mode, P, E, N, Kd, kb, _p(xh), _p(gemm_status(xh.device)), _stream()),
+           "trellis_rows_grouped")
     return y
 
 

@@ -1,0 +1,61 @@
+"""Which entry point of the kernel library a product takes, and with what (CPU: a library that only records the calls)."""
+from types import SimpleNamespace
+
+import pytest
+import torch
+
+from r4dx_b200.models.hybrid import HybridModel
+from r4dx_b200.ops import kernels as K
+from r4dx_b200.quant import trellis
+
+BF = torch.bfloat16
+
+
+class Recorder:
+    def __init__(self):
+        self.calls = []
+
+    def __getattr__(self, name):
+        def call(*args):
+            self.calls.append((name, args))
+            return 0
+        return call
+
+
+@pytest.fixture
+def lib(monkeypatch):
+    r = Recorder()
+    monkeypatch.setattr(K, "_lib", lambda: r)
+    monkeypatch.setattr(K, "_req", lambda *a: None)
+    monkeypatch.setattr(K, "_stream", lambda: None)
+    monkeypatch.setattr(K, "_STATUS", {})
+    assert K.GEMV_IMPL == "auto"
+    return r
+
+
+@pytest.fixture(scope="module")
+def large():
+    return trellis.random_weight(4096, 2048, 4, seed=1)
+
+
+def _address(arg):
+    return getattr(arg, "value", arg)
+
+
+def test_rows_kernel_reports_a_wait_that_ran_out(lib, large, monkeypatch):
+    """The launch is given the status word, and a call of as many rows reads it before its tokens are used."""
+    word = K.gemm_status("cpu").data_ptr()
+    K.trellis_gemv(large, torch.zeros(2, 2048, dtype=BF))
+    K.SiblingGroup([large, large])(torch.zeros(2, 2048, dtype=BF), [torch.zeros(2, 4096, dtype=BF)] * 2)
+    z = lambda *s, dtype=torch.int32: torch.zeros(*s, dtype=dtype)
+    K.trellis_rows_grouped(large.words, large.suh, large.svh, z(1, 2048, dtype=BF), z(1, 4096, dtype=BF), z(2), z(1), z(4), z(1), 1, 0, 1, 1,
+                           4096, 2048, 4, z(2048, dtype=torch.float16))
+    assert [n for n, _ in lib.calls] == ["r4dxb_trellis_gemv_rows"] * 2 + ["r4dxb_trellis_rows_grouped"]
+    assert all(_address(args[-2]) == word for _, args in lib.calls)
+    read = []
+    monkeypatch.setattr(K, "check_gemm_status", read.append)
+    m = SimpleNamespace(comm=None, device="cpu")
+    HybridModel.check_healthy(m, 1)
+    assert not read
+    HybridModel.check_healthy(m, K.ROWS_MIN_ROWS)
+    assert read == ["cpu"]
