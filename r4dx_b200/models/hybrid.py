@@ -46,8 +46,9 @@ class Linear:
                  prologue: int = 0, norm_w: Optional[torch.Tensor] = None, eps: float = 1e-6) -> torch.Tensor:
         w = self.w
         if isinstance(w, TrellisWeight):
+            T = x.numel() // (2 * self.K if prologue in (K.PRO_SILU_MUL, K.PRO_GELU_MUL) else self.K)
             return K.trellis_gemv(w, x, residual=residual, out=out, ksplit=self.ksplit, prologue=prologue,
-                                  norm_w=norm_w, eps=eps)
+                                  norm_w=norm_w, eps=eps, split_rows=K.rows_split(self.N, self.K, T))
         if isinstance(w, (W4Weight, W8Weight)):
             # group-quantised layouts: the streaming kernels have no prologue / residual modes, so the producer of the
             # activations and the residual add are kernels of their own (the w8a16 body of the dense and short-conv

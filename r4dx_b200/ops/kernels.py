@@ -296,8 +296,9 @@ def _gemv_rows(count: int, words, suh, svh, y, n, x, residual, norm_w, eps: floa
 def trellis_gemv(w: TrellisWeight, x: torch.Tensor, residual: Optional[torch.Tensor] = None,
                  out: Optional[torch.Tensor] = None, ksplit: Optional[int] = None, prologue: int = PRO_NONE,
                  norm_w: Optional[torch.Tensor] = None, eps: float = 1e-6, split_rows: Optional[int] = None) -> torch.Tensor:
-    """y[T, N] = trellis linear of act(x) (T <= 8), optionally + residual (may alias out).  ``ksplit``: cluster split of K
-    on the CUDA-core and tensor-memory kernels; ``split_rows``: take the rows kernel with this split (by shape unless given).
+    """y[T, N] = trellis linear of act(x) (T <= 8), optionally + residual (may alias out).  ``ksplit``: take the CUDA-core or
+    tensor-memory kernel with this cluster split of K; ``split_rows``: take the rows kernel with this one (in "auto" mode; a
+    slice too long for it falls back to the others).  With neither the kernel and its split go by shape.
 
     prologue PRO_RMSNORM: x is the residual stream [T, K], act = zero-centred RMSNorm with ``norm_w``;
     PRO_SILU_MUL: x is fused [gate | up] rows [T, 2K].
@@ -305,7 +306,8 @@ def trellis_gemv(w: TrellisWeight, x: torch.Tensor, residual: Optional[torch.Ten
     _req(x, BF, "x")
     T = x.numel() // (2 * w.K if prologue in (PRO_SILU_MUL, PRO_GELU_MUL) else w.K)
     out = out if out is not None else torch.empty(T, w.N, dtype=BF, device=x.device)
-    split_rows = split_rows or rows_split(w.N, w.K, T)
+    if split_rows is None and ksplit is None:
+        split_rows = rows_split(w.N, w.K, T)
     if GEMV_IMPL == "auto" and split_rows is not None:
         rc = _gemv_rows(1, _ptr1(w.words), _ptr1(w.suh), _ptr1(w.svh), _ptr1(out), (ctypes.c_int * 1)(w.N), x, residual, norm_w, eps,
                         prologue, T, w.K, w.kb, split_rows)

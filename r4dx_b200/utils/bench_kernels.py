@@ -55,9 +55,9 @@ def main() -> None:
     ap.add_argument("--ctx", type=int, default=8192)
     ap.add_argument("--decode-warps", type=int, default=0, help="4, 8 or 16; 0 leaves the library's own choice")
     ap.add_argument("--tn", type=int, default=0)
-    ap.add_argument("--ksplit", type=int, default=0, help="override the cluster split of the weight-streaming kernel")
+    ap.add_argument("--ksplit", type=int, default=0, help="time the CUDA-core / tensor-memory kernel with this cluster split (the rows kernel takes no override)")
     ap.add_argument("--f8", action="store_true", help="with --only trellis_gemm: also time the 8-bit (e4m3 x e4m3) product")
-    ap.add_argument("--impl", default="", help="weight-streaming kernel: mma (tensor memory, default) or simt (CUDA cores)")
+    ap.add_argument("--impl", default="", help="weight-streaming kernel: auto (by shape and rows, default), mma (tensor memory) or simt (CUDA cores)")
     a = ap.parse_args()
     from r4dx_b200.ops import kernels as K
     from r4dx_b200.quant import trellis, w4a16
@@ -76,10 +76,11 @@ def main() -> None:
                 w = trellis.random_weight(N, Kd, kb, seed=1, device=dev)
                 x = torch.randn(T, Kd, device=dev).to(BF)
                 y = torch.empty(T, N, dtype=BF, device=dev)
-                ks = a.ksplit or K.pick_ksplit(N, Kd)
-                if (Kd // 128) % ks:
+                split = K.rows_split(N, Kd, T) if K.GEMV_IMPL == "auto" and not a.ksplit else None
+                ks = split or a.ksplit or K.pick_ksplit(N, Kd)
+                if split is None and (Kd // 128) % ks:
                     continue
-                us = timed(lambda: K.trellis_gemv(w, x, out=y, ksplit=ks), a.iters, flush)
+                us = timed(lambda: K.trellis_gemv(w, x, out=y, ksplit=None if split else ks, split_rows=split), a.iters, flush)
                 gbs = w.nbytes / us / 1e3
                 K.check_gemm_status(dev)
                 print(f"trellis_gemv[{K.GEMV_IMPL}] {name:12s} N={N:6d} K={Kd:6d} kb={kb} T={T} ksplit={ks}: {us:8.1f} us  "

@@ -4,7 +4,7 @@ from types import SimpleNamespace
 import pytest
 import torch
 
-from r4dx_b200.models.hybrid import HybridModel
+from r4dx_b200.models.hybrid import HybridModel, Linear
 from r4dx_b200.ops import kernels as K
 from r4dx_b200.quant import trellis
 
@@ -59,3 +59,24 @@ def test_rows_kernel_reports_a_wait_that_ran_out(lib, large, monkeypatch):
     assert not read
     HybridModel.check_healthy(m, K.ROWS_MIN_ROWS)
     assert read == ["cpu"]
+
+
+@pytest.mark.parametrize("T,entry", [(1, "r4dxb_trellis_gemv_ex"), (2, "r4dxb_trellis_gemv_ex"), (8, "r4dxb_trellis_gemv_mma")])
+def test_an_explicit_split_of_k_is_the_one_that_runs(lib, large, T, entry):
+    """Tuning and benchmarking time the splits they ask for, whatever kernel the shape would go to by itself."""
+    x = torch.zeros(T, 2048, dtype=BF)
+    for ks in (1, 2, 4, 8):
+        K.trellis_gemv(large, x, ksplit=ks)
+    assert [n for n, _ in lib.calls] == [entry] * 4
+    at = -2 if entry.endswith("_ex") else -3
+    assert [args[at] for _, args in lib.calls] == [1, 2, 4, 8]
+
+
+@pytest.mark.parametrize("T,entry", [(1, "r4dxb_trellis_gemv_ex"), (2, "r4dxb_trellis_gemv_rows"), (8, "r4dxb_trellis_gemv_rows")])
+def test_a_models_linear_goes_by_shape_and_rows(lib, large, T, entry):
+    lin = Linear(large)
+    lin(torch.zeros(T, 2048, dtype=BF), torch.zeros(T, 4096, dtype=BF))
+    lin(torch.zeros(T, 4096, dtype=BF), torch.zeros(T, 4096, dtype=BF), prologue=K.PRO_SILU_MUL)
+    small = Linear(trellis.random_weight(256, 256, 4, seed=1))
+    small(torch.zeros(T, 256, dtype=BF), torch.zeros(T, 256, dtype=BF))
+    assert [n for n, _ in lib.calls] == [entry, entry, "r4dxb_trellis_gemv_mma" if T >= 6 else "r4dxb_trellis_gemv_ex"]
