@@ -343,10 +343,12 @@ int r4dxb_w4a16_rows(const void* wq, const void* wsz, const void* x, void* y, in
                      void* stream) {
   if (T < 1 || T > 64 || K % 32 || (group != 32 && group != 64 && group != 128) || K % group) return R4DXB_BAD_ARG;
   const int parts = (T + 15) / 16;
+  // before anything is launched, for the part with the most rows (parts differ by one, and whether they fit goes by the rows;
+  // they all start on a row, K * 2 bytes apart)
+  if (!W4MmaCovers(wq, x, (T + parts - 1) / parts, N, K, group)) return R4DXB_UNSUPPORTED;
   for (int i = 0; i < parts; ++i) {
     const int t0 = i * T / parts, rows = (i + 1) * T / parts - t0;
     const unsigned char* xi = static_cast<const unsigned char*>(x) + static_cast<size_t>(t0) * K * 2;
-    if (!W4MmaCovers(wq, xi, rows, N, K, group)) return R4DXB_UNSUPPORTED;       // (the same answer for every part)
     unsigned char* yi = static_cast<unsigned char*>(y) + static_cast<size_t>(t0) * N * (out_f32 ? 4 : 2);
     if (int rc = W4Mma(wq, wsz, xi, yi, rows, N, K, group, out_f32, static_cast<cudaStream_t>(stream))) return rc;
   }

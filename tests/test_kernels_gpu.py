@@ -288,6 +288,35 @@ def test_w4a16_streaming_rows_match_fp64(K, T, N, Kd, group):
         assert torch.equal(K.w4a16_gemv(qd, xd), y)
 
 
+@pytest.mark.parametrize("T", [17, 31, 32, 33, 64])
+def test_w4a16_streaming_rows_in_parts(K, T):
+    """More than 16 rows run in parts of nearly equal size: every row has the bits it has in a call of its own part size."""
+    from r4dx_b200.quant import w4a16
+    N, Kd, group = 1040, 512, 64
+    g = torch.Generator().manual_seed(T)
+    q = w4a16.quantize(torch.randn(N, Kd, generator=g), group).to("cuda")
+    x = torch.randn(T, Kd, generator=g).to(BF).cuda()
+
+    def rows(xs):
+        y = torch.full((len(xs), N), float("nan"), device="cuda")
+        K._check(K._lib().r4dxb_w4a16_rows(K._p(q.wq), K._p(q.wsz), K._p(xs), K._p(y), len(xs), N, Kd, group, 1, K._stream()), "w4a16_rows")
+        return y
+
+    assert torch.equal(rows(x), torch.cat([rows(x[s:s + 8].contiguous()) for s in range(0, T, 8)]))
+
+
+def test_w4a16_streaming_rows_refuse_before_they_write(K):
+    """17 rows run as 8 + 9; at K = 13312 eight rows fit into shared memory and nine do not."""
+    from r4dx_b200.quant import w4a16
+    T, N, Kd, group = 17, 16, 13312, 32
+    q = w4a16.quantize(torch.randn(N, Kd, generator=torch.Generator().manual_seed(0)), group).to("cuda")
+    x, y = torch.zeros(T, Kd, dtype=BF, device="cuda"), torch.full((T, N), 7.0, device="cuda")
+    rc = K._lib().r4dxb_w4a16_rows(K._p(q.wq), K._p(q.wsz), K._p(x), K._p(y), T, N, Kd, group, 1, K._stream())
+    assert rc == K._UNSUPPORTED and (y == 7.0).all()
+    assert K._lib().r4dxb_w4a16_rows(K._p(q.wq), K._p(q.wsz), K._p(x), K._p(y), 16, N, Kd, group, 1, K._stream()) == K._UNSUPPORTED
+    assert K._lib().r4dxb_w4a16_rows(K._p(q.wq), K._p(q.wsz), K._p(x), K._p(y), 8, N, Kd, group, 1, K._stream()) == 0 and (y[:8] == 0).all()
+
+
 @pytest.mark.parametrize("T,N,Kd,group", [(16, 256, 512, 64), (40, 1024, 1024, 32), (300, 512, 2048, 128), (1100, 384, 640, 64)])
 def test_linear_tc_w4a16_matches_fp32_reference(K, T, N, Kd, group):
     """The tensor-core w4a16 product against x @ dequant(W)^T in fp32, with bias, residual and an fp32 output."""
