@@ -48,6 +48,13 @@ inline int LaunchPdl(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem,
   return static_cast<int>(e);
 }
 
+// Lets launches of `kern` ask for any amount of dynamic shared memory up to an SM's 227 KB (the kernel declares none of its own).
+// Always the same value: a limit set to one call's size could be lowered by another host thread between the setting and the launch.
+template <typename... KArgs>
+inline cudaError_t AllowAllSharedMemory(void (*kern)(KArgs...)) {
+  return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+}
+
 // Status word of a communicator, read past the caches: non-zero means an earlier bounded wait ran out, and
 // every later wait gives up at once (the failure is sticky until the host has recovered and cleared it).
 __device__ __forceinline__ int StatusNow(const int* status) {

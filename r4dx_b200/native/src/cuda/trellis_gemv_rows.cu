@@ -463,7 +463,7 @@ int LaunchRows(RowsArgs a, int ksplit, cudaStream_t stream) {
   // a cluster on one SM leave another idle (5120 x 17408 at two rows inside a captured step: 48 against 25 us)
   if (ksplit * a.w[a.count - 1].nb_end <= 148 && smem < 116 * 1024) smem = 116 * 1024;
   auto kern = TrellisRowsKernel<KB, TMAX>;
-  const cudaError_t ea = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+  const cudaError_t ea = AllowAllSharedMemory(kern);
   if (ea != cudaSuccess) return static_cast<int>(ea);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(ksplit, a.w[a.count - 1].nb_end, 1);
@@ -492,7 +492,7 @@ int LaunchGroupedRows(RowsArgs a, int max_tiles, cudaStream_t stream) {
   const size_t smem = SmemBytes<KB, TMAX>(a.K, a.stages, 1);
   if (smem > 227 * 1024) return R4DXB_TOO_LARGE;
   auto kern = TrellisRowsKernel<KB, TMAX, true>;
-  const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+  const cudaError_t e = AllowAllSharedMemory(kern);
   if (e != cudaSuccess) return static_cast<int>(e);
   kern<<<dim3(1, a.w[0].N / 128, max_tiles), kThreads, smem, stream>>>(a);
   return FinishLaunch();

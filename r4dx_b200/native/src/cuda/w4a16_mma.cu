@@ -214,7 +214,7 @@ int LaunchW4Mma(const void* wq, const void* wsz, const void* x, void* y, int T, 
     slices *= 2;
   const size_t smem = xbytes + (slices > 1 ? red : 0);
   auto kern = W4MmaKernel<NT, G>;
-  const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+  const cudaError_t e = AllowAllSharedMemory(kern);
   if (e != cudaSuccess) return static_cast<int>(e);
   kern<<<grid, kW4Threads, smem, stream>>>(static_cast<const uint32_t*>(wq), static_cast<const uint32_t*>(wsz),
                                            static_cast<const __nv_bfloat16*>(x), y, T, N, K, out_f32, slices);

@@ -305,6 +305,38 @@ def test_w4a16_streaming_rows_in_parts(K, T):
     assert torch.equal(rows(x), torch.cat([rows(x[s:s + 8].contiguous()) for s in range(0, T, 8)]))
 
 
+def test_two_threads_with_calls_of_different_sizes(K):
+    """A call that needs 131 KB of shared memory beside one that needs 9: neither lowers the other's limit."""
+    import threading
+    from r4dx_b200.quant import trellis, w4a16
+    head = w4a16.quantize(torch.randn(16, 8192, generator=torch.Generator().manual_seed(0)), 32).to("cuda")
+    small = w4a16.quantize(torch.randn(16, 512, generator=torch.Generator().manual_seed(0)), 32).to("cuda")
+    body = trellis.random_weight(128, 8192, 4, seed=1, device="cuda")
+    calls = {"large": (lambda x: K.w4a16_gemv(head, x), lambda x: K.trellis_gemv(body, x, split_rows=1)),
+             "small": (lambda x: K.w4a16_gemv(small, x[:, :512].contiguous()), lambda x: K.trellis_gemv(body, x, split_rows=8))}
+    x = torch.ones(8, 8192, dtype=BF, device="cuda")
+    want = {n: [f(x) for f in fs] for n, fs in calls.items()}
+    failed = []
+
+    def loop(n):
+        try:
+            with torch.cuda.stream(torch.cuda.Stream()):
+                for _ in range(1500):
+                    got = [f(x) for f in calls[n]]
+                torch.cuda.current_stream().synchronize()
+            assert all(torch.equal(a, b) for a, b in zip(got, want[n]))
+        except Exception as e:
+            failed.append(e)
+
+    torch.cuda.synchronize()
+    threads = [threading.Thread(target=loop, args=(n,)) for n in calls]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not failed
+
+
 def test_w4a16_streaming_rows_refuse_before_they_write(K):
     """17 rows run as 8 + 9; at K = 13312 eight rows fit into shared memory and nine do not."""
     from r4dx_b200.quant import w4a16
