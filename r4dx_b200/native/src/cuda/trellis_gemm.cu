@@ -768,8 +768,10 @@ extern "C" {
 
 int r4dxb_trellis_input(const void* in, const void* suh, void* out, int T, int K, int mode, void* stream) {
   if (T < 1 || K % 128 || mode < 0 || mode > 2) return R4DXB_BAD_ARG;
-  // four rows per half-warp once there are enough of them to fill the machine that way (64 rows: 2.5 us with one, 4.4 with four)
-  const int r = T >= 512 ? 4 : 1;
+  // Four rows per half-warp once they still fill the machine that way; with a gate, twice the loads of a row are in flight as it
+  // is, and it takes more.  us with one / four: plain 512 x 5120 4.7 / 4.9, 512 x 6144 5.1 / 4.9, 1024 x 17408 19.3 / 16.0; gated
+  // 512 x 2048 4.3 / 6.1, 2048 x 5120 19.1 / 19.5, 1024 x 17408 33.5 / 32.2, 8192 x 5120 74 / 68.
+  const int r = static_cast<long long>(T) * K >= (mode == 0 ? 3LL << 20 : 1LL << 24) ? 4 : 1;
   const long long items = static_cast<long long>((T + r - 1) / r) * (K / 128);
   (r == 4 ? TrellisInputKernel<4> : TrellisInputKernel<1>)<<<static_cast<unsigned>((items + 15) / 16), 256, 0, static_cast<cudaStream_t>(stream)>>>(
       static_cast<const __nv_bfloat16*>(in), static_cast<const __half*>(suh), static_cast<__half*>(out), T, K, mode, Aligned16(in, suh, out));

@@ -1197,6 +1197,16 @@ def test_trellis_input_bases_and_row_counts(K, T, Kd):
         assert torch.equal(K.trellis_input(odd, suh.cuda(), fused_silu_mul=fused), out)
 
 
+@pytest.mark.parametrize("fused,T,Kd", [(False, 517, 6144), (True, 2051, 8320)])
+def test_trellis_input_of_many_rows_has_the_bits_of_few(K, fused, T, Kd):
+    """Calls large enough for four rows per half-warp (with a last group of less) against calls of one."""
+    g = torch.Generator().manual_seed(T)
+    x = torch.randn(T, Kd * (2 if fused else 1), generator=g).to(BF).cuda()
+    suh = torch.randn(Kd, generator=g).to(torch.float16).cuda()
+    out = K.trellis_input(x, suh, fused_silu_mul=fused)
+    assert torch.equal(out, torch.cat([K.trellis_input(x[s:s + 300], suh, fused_silu_mul=fused) for s in range(0, T, 300)]))
+
+
 @pytest.mark.parametrize("D,T,pos0", [(64, 17, 0), (128, 35, 5), (128, 16, 3)])
 def test_gdn_prefill_odd_bases_equal_aligned_ones(K, D, T, pos0):
     """Token counts around the 16-token groups of the convolution, a ring carried in, and bases of the bf16 operands that
