@@ -202,18 +202,20 @@ def pick_ksplit(N: int, K: int, target_ctas: int = int(os.environ.get("R4DXB_KSP
 def pick_split(N: int, K: int) -> int:
     """Cluster split of the rows kernel: the fewest 128-wide K blocks on the busiest of the 148
     SMs, with three blocks' time for what a CTA does besides (setup, reduction).  A CTA of it keeps an SM busy by itself, so
-    more CTAs than SMs only help to even out the load.  Measured at two rows, 4 bits (us by split 1..8): 5120 x 17408
-    73 44 34 40 34 32 42 40; 34816 x 5120 48 52 60 62 68 75 81 85; 5120 x 6144 32 22 17 22 20 20 26 24; 1024 x 2048
-    17 13 13 11 11 11 11 11.  Clusters of seven fit badly into the chip's SM groups and are left out."""
+    more CTAs than SMs only help to even out the load.  Measured at two rows, 4 bits (us by split 1 2 3 4 5 6 8): 5120 x 17408
+    77 44 34 44 40 36 44; 34816 x 5120 52 56 62 67 71 75 87; 5120 x 6144 34 24 20 24 22 19 26; 2048 x 4096 26 19 16 15 15 13 17.
+    Clusters of seven and eight fit badly into the chip's SM groups and are left out."""
     rows, blocks = N // 128, K // 128
-    return min((c for c in (1, 2, 3, 4, 5, 6, 8) if c <= blocks),
+    return min((c for c in (1, 2, 3, 4, 5, 6) if c <= blocks),
                key=lambda c: ((rows * c + 147) // 148) * ((blocks + c - 1) // c + 3))
 
 
-# Weights of a launch from which it takes the rows kernel: below, its second launch costs what the contraction saves (us at
-# 4 / 8 rows, CUDA cores against rows kernel: 4096 x 1024 12 / 16 against 13 / 13, 1024 x 2048 10 / 12 against 11 / 13;
-# 5120 x 6144 27 / 41 against 19 / 22).
+# Weights of a launch, and weights times rows, from which it takes the rows kernel: below, its second launch costs what the
+# contraction saves.  us at 2 / 3 / 4 / 6 / 8 rows, the better of the other two kernels against the rows kernel: 4096 x 2048
+# 12.3 / 12.4 / 12.3 / 14.4 / 14.3 against 11.6 / 13.3 / 13.3 / 13.3 / 13.3; 8192 x 2048 14.4 / 16.4 / 16.4 / 20.5 / 21.3 against 15.4
+# throughout; 5120 x 6144 22.6 / 26.6 / 26.6 / 32.8 / 32.8 against 19.5.
 ROWS_MIN_WEIGHTS = 1 << 23
+ROWS_MIN_WORK = 3 << 24
 
 # Rows from which a launch takes the rows kernel.  One-row steps stay on the CUDA cores although a step of the 27B geometry (8
 # layers, 8192 tokens of context) takes 1435 us there and 1270 with the rows kernel: the two round differently (6.4e-4 and 2.2e-4
@@ -225,7 +227,8 @@ ROWS_MIN_ROWS = 2
 @functools.lru_cache(maxsize=None)
 def rows_split(N: int, K: int, T: int) -> Optional[int]:
     """Split of the rows kernel for T rows of a launch of N outputs, None where one of the other kernels serves it."""
-    return pick_split(N, K) if T >= ROWS_MIN_ROWS and N * K >= ROWS_MIN_WEIGHTS else None
+    large = N * K >= ROWS_MIN_WEIGHTS and T * N * K >= ROWS_MIN_WORK
+    return pick_split(N, K) if T >= ROWS_MIN_ROWS and large else None
 
 
 _STATUS = {}

@@ -45,8 +45,8 @@ def _address(arg):
 def test_rows_kernel_reports_a_wait_that_ran_out(lib, large, monkeypatch):
     """The launch is given the status word, and a call of as many rows reads it before its tokens are used."""
     word = K.gemm_status("cpu").data_ptr()
-    K.trellis_gemv(large, torch.zeros(2, 2048, dtype=BF))
-    K.SiblingGroup([large, large])(torch.zeros(2, 2048, dtype=BF), [torch.zeros(2, 4096, dtype=BF)] * 2)
+    K.trellis_gemv(large, torch.zeros(6, 2048, dtype=BF))
+    K.SiblingGroup([large, large])(torch.zeros(3, 2048, dtype=BF), [torch.zeros(3, 4096, dtype=BF)] * 2)
     z = lambda *s, dtype=torch.int32: torch.zeros(*s, dtype=dtype)
     K.trellis_rows_grouped(large.words, large.suh, large.svh, z(1, 2048, dtype=BF), z(1, 4096, dtype=BF), z(2), z(1), z(4), z(1), 1, 0, 1, 1,
                            4096, 2048, 4, z(2048, dtype=torch.float16))
@@ -72,7 +72,7 @@ def test_an_explicit_split_of_k_is_the_one_that_runs(lib, large, T, entry):
     assert [args[at] for _, args in lib.calls] == [1, 2, 4, 8]
 
 
-@pytest.mark.parametrize("T,entry", [(1, "r4dxb_trellis_gemv_ex"), (2, "r4dxb_trellis_gemv_rows"), (8, "r4dxb_trellis_gemv_rows")])
+@pytest.mark.parametrize("T,entry", [(1, "r4dxb_trellis_gemv_ex"), (2, "r4dxb_trellis_gemv_ex"), (6, "r4dxb_trellis_gemv_rows"), (8, "r4dxb_trellis_gemv_rows")])
 def test_a_models_linear_goes_by_shape_and_rows(lib, large, T, entry):
     lin = Linear(large)
     lin(torch.zeros(T, 2048, dtype=BF), torch.zeros(T, 4096, dtype=BF))
