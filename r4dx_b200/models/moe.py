@@ -87,7 +87,7 @@ class MoeBlock:
         self.max_rows = R
         if R > GROUPED_MIN_ROWS:
             self.xh_pairs = z(R * k, max(H, I), dtype=torch.float16)
-            self.tiles = z(2 * (R * k // 4 + self.e_count + 1), dtype=torch.int32)
+            self.tiles = z(2 * (R * k // 8 + self.e_count + 1), dtype=torch.int32)
             self.ntiles = z(1, dtype=torch.int32)
         self.ks_gu = K.pick_ksplit(self.gate_up.N, self.gate_up.K, target_ctas=1)
         self.ks_dn = K.pick_ksplit(self.down.N, self.down.K, target_ctas=1)
@@ -144,9 +144,10 @@ class MoeBlock:
         K.trellis_gemv_grouped(d.words, d.suh, d.svh, self.gu_pairs, self.y_pairs, self.offsets, self.perm, 1, n_pass, tmax,
                                K.PRO_SILU_MUL, d.E, d.N, d.K, d.kb, ks_dn)
 
-    # Pairs per expert up to which the weight-streaming kernel on mma.sync (tiles of 4 rows) serves the grouped products: 512 experts
-    # of the hybrid geometry 463 against 644 us a block at 1.25, 734 against 822 at 3.9, 855 against 838 at 5; of the 4-stream
-    # geometry 619 / 905, 994 / 1153, 1167 / 1182.
+    # Pairs per expert up to which the weight-streaming kernel on mma.sync (tiles of 8 rows) serves the grouped products: 512 experts
+    # of the hybrid geometry 478 against 626 us a block at 1.25 and 620 against 798 at 3.9, of the 4-stream geometry 654 / 877 and
+    # 851 / 1118.  The line stays where tiles of 4 rows lost: uneven routing costs these tiles more than the others (all 200 rows on
+    # the same ten experts: 406 against 372 us).
     few_rows_avg = 4
 
     def _experts_grouped(self, h: torch.Tensor, T: int) -> None:
@@ -157,12 +158,12 @@ class MoeBlock:
         g, d = self.gate_up, self.down
         P = T * self.k
         experts = max(1, min(self.e_count, self.cfg.num_experts))
-        if P <= self.few_rows_avg * experts:
-            K.moe_tiles(self.offsets, self.e_count, 4, self.tiles, self.ntiles)
+        if P <= self.few_rows_avg * experts and max(g.K, d.K) <= K.GROUPED_ROWS_MAX_K:
+            K.moe_tiles(self.offsets, self.e_count, 8, self.tiles, self.ntiles)
             K.trellis_rows_grouped(g.words, g.suh, g.svh, h, self.gu_pairs, self.offsets, self.perm, self.tiles, self.ntiles, self.k, 0, P,
-                                   g.E, g.N, g.K, g.kb, self.xh_pairs)
+                                   g.E, g.N, g.K, g.kb, self.xh_pairs, tile_rows=8)
             K.trellis_rows_grouped(d.words, d.suh, d.svh, self.gu_pairs, self.y_pairs, self.offsets, self.perm, self.tiles, self.ntiles, 1, 1,
-                                   P, d.E, d.N, d.K, d.kb, self.xh_pairs)
+                                   P, d.E, d.N, d.K, d.kb, self.xh_pairs, tile_rows=8)
             return
         avg = max(1, P // experts)
         # the weights of an expert are decoded once per token tile, so a tile should hold all of an expert's rows

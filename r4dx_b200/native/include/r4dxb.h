@@ -164,12 +164,12 @@ int r4dxb_trellis_input_grouped(const void* in, const void* suh, void* out, cons
 int r4dxb_trellis_gemm_grouped(const void* words, const void* svh, const void* xh, void* y, const int* offsets, const int* perm,
                                const int* tiles, const int* ntiles, int max_tiles, int P, int E, int N, int K, int kb, int tn,
                                int* status, void* stream);
-/* The same products for a few rows per expert, on the kernel of r4dxb_trellis_gemv_rows: tiles of four rows
+/* The same products for a few rows per expert, on the kernel of r4dxb_trellis_gemv_rows: tiles of tile_rows (1..8) rows
  * (r4dxb_moe_tiles), input rows perm[p] / xdiv of x through mode (0: x, 1: SwiGLU of [2K], 2: GeGLU); workspace: xh
  * (P * 2 K bytes, 16-byte aligned); status as above. */
 int r4dxb_trellis_rows_grouped(const void* words, const void* suh, const void* svh, const void* x, void* y, const int* offsets,
-                               const int* perm, const int* tiles, const int* ntiles, int max_tiles, int xdiv, int mode, int P, int E,
-                               int N, int K, int kb, void* xh, int* status, void* stream);
+                               const int* perm, const int* tiles, const int* ntiles, int max_tiles, int tile_rows, int xdiv, int mode, int P,
+                               int E, int N, int K, int kb, void* xh, int* status, void* stream);
 
 /* ---- batched decode (B sequences, one new token each; per-sequence state indexed by slot) ---------- */
 int r4dxb_gdn_decode_batch(const void* mixed, const void* z, const float* ab, const void* conv_w, const float* A_log,

@@ -16,9 +16,10 @@
 // row takes the other kernel: see ops/kernels.py:ROWS_MIN_ROWS.
 //
 // Grouped mode (mixture-of-experts blocks with a few rows per expert): a CTA serves one 128-row block of one tile of the routing
-// plan, up to four rows of one expert; the rows are those of the planned pairs in expert order.  A block of 512
-// experts (top 10, hidden 2048) takes 261 / 478 / 755 us at 17 / 64 / 200 rows of x where the tcgen05 tiles of 16 rows take 338 /
-// 626 / 799: most experts have one or two rows, and decoding their weights is the work.
+// plan, up to eight rows of one expert; the rows are those of the planned pairs in expert order.  A block of 512
+// experts (top 10, hidden 2048) takes 261 / 478 / 620 us at 17 / 64 / 200 rows of x where the tcgen05 tiles of 16 rows take 339 /
+// 626 / 798: most experts have one or two rows, and decoding their weights is the work.  (Tiles of four rows: 261 / 478 / 755; with
+// most rows routed to a dozen experts they took 329 / 628 us at 64 / 200 rows, these 277 / 452, the tcgen05 tiles 320 / 458.)
 //
 // Two launches: TrellisRowsInputKernel writes the transformed rows once (every CTA would otherwise repeat the transform: at 8 rows
 // of 5120 columns that was 74k of 103k clocks), then one CTA per (128-row block, K slice) streams words
@@ -61,7 +62,7 @@ struct RowsArgs {
   const int* g_perm;                     // pair of each sorted position = output row; its input row is pair / g_xdiv
   const int* g_tiles;                    // (expert, first sorted position) per tile, *g_ntiles of them
   const int* g_ntiles;
-  int g_experts, g_xdiv;
+  int g_experts, g_xdiv, g_tile_rows;
   long long g_words;                     // words of one expert
   int* status;                           // receives 700 + role code (390: split-K hand-off) when a bounded wait ran out
   int count;
@@ -214,7 +215,7 @@ __device__ __forceinline__ uint32_t Code2(const uint32_t (&w)[3]) {
 }
 
 template <int KB, int TMAX, bool kGrouped = false>
-__global__ void __launch_bounds__(kThreads, TMAX > 4 ? 1 : 2) TrellisRowsKernel(RowsArgs a) {
+__global__ void __launch_bounds__(kThreads, TMAX > 4 && !kGrouped ? 1 : 2) TrellisRowsKernel(RowsArgs a) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   cg::cluster_group cluster = cg::this_cluster();
   const int ksplit = gridDim.x;
@@ -232,7 +233,7 @@ __global__ void __launch_bounds__(kThreads, TMAX > 4 ? 1 : 2) TrellisRowsKernel(
     if (static_cast<int>(blockIdx.z) >= __ldg(a.g_ntiles)) return;       // the whole CTA (a cluster of one), before any barrier exists
     const int e = __ldg(a.g_tiles + 2 * blockIdx.z);
     start = __ldg(a.g_tiles + 2 * blockIdx.z + 1);
-    T = min(TMAX, __ldg(a.g_offsets + e + 1) - start);
+    T = min(a.g_tile_rows, __ldg(a.g_offsets + e + 1) - start);
     words += static_cast<size_t>(e) * a.g_words;
     svh += static_cast<size_t>(e) * N;
   }
@@ -489,6 +490,8 @@ template <int KB, int TMAX>
 int LaunchGroupedRows(RowsArgs a, int max_tiles, cudaStream_t stream) {
   a.kblocks_per_cta = a.K / 128;
   a.stages = a.kblocks_per_cta < kMaxStages ? a.kblocks_per_cta : kMaxStages;
+  // a short slice: a shallower ring where that lets two CTAs share an SM
+  while (a.stages > 4 && SmemBytes<KB, TMAX>(a.K, a.stages, 1) > 113 * 1024) --a.stages;
   const size_t smem = SmemBytes<KB, TMAX>(a.K, a.stages, 1);
   if (smem > 227 * 1024) return R4DXB_TOO_LARGE;
   auto kern = TrellisRowsKernel<KB, TMAX, true>;
@@ -565,9 +568,9 @@ int r4dxb_trellis_gemv_rows(int count, const void* const* words, const void* con
 /* Expert products with a few rows per expert: y[perm[p]] = svh[e] * H128(Q_e . H128(suh[e] * act(x[perm[p] / xdiv]))) for the
  * planned pairs p (see the header). */
 int r4dxb_trellis_rows_grouped(const void* words, const void* suh, const void* svh, const void* x, void* y, const int* offsets,
-                               const int* perm, const int* tiles, const int* ntiles, int max_tiles, int xdiv, int mode, int P, int E,
-                               int N, int K, int kb, void* xh, int* status, void* stream) {
-  if (P < 1 || E < 1 || N < 128 || N % 128 || K < 128 || K % 128 || max_tiles < 1 || max_tiles > 65535 || xdiv < 1 || mode < 0 || mode > 2 ||
+                               const int* perm, const int* tiles, const int* ntiles, int max_tiles, int tile_rows, int xdiv, int mode, int P,
+                               int E, int N, int K, int kb, void* xh, int* status, void* stream) {
+  if (P < 1 || E < 1 || N < 128 || N % 128 || K < 128 || K % 128 || max_tiles < 1 || max_tiles > 65535 || tile_rows < 1 || tile_rows > 8 || xdiv < 1 || mode < 0 || mode > 2 ||
       xh == nullptr || (reinterpret_cast<uintptr_t>(xh) & 15))
     return R4DXB_BAD_ARG;
   RowsArgs a = {};
@@ -589,6 +592,7 @@ int r4dxb_trellis_rows_grouped(const void* words, const void* suh, const void* s
   a.g_ntiles = ntiles;
   a.g_experts = E;
   a.g_xdiv = xdiv;
+  a.g_tile_rows = tile_rows;
   a.g_words = static_cast<long long>(N / 16) * (K / 16) * 8 * kb;
   a.xh = static_cast<const __half*>(xh);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
@@ -596,9 +600,9 @@ int r4dxb_trellis_rows_grouped(const void* words, const void* suh, const void* s
   const int warps = min(kInWarps, K / 128), parts = (K / 128 + warps * kInBlocks - 1) / (warps * kInBlocks);
   input_kernel<<<dim3(P, parts), 32 * warps, 0, s>>>(a, static_cast<__half*>(xh));
   if (int rc = FinishLaunch()) return rc;
-  if (kb == 3) return LaunchGroupedRows<3, 4>(a, max_tiles, s);
-  if (kb == 4) return LaunchGroupedRows<4, 4>(a, max_tiles, s);
-  if (kb == 5) return LaunchGroupedRows<5, 4>(a, max_tiles, s);
+  if (kb == 3) return LaunchGroupedRows<3, 8>(a, max_tiles, s);
+  if (kb == 4) return LaunchGroupedRows<4, 8>(a, max_tiles, s);
+  if (kb == 5) return LaunchGroupedRows<5, 8>(a, max_tiles, s);
   return R4DXB_BAD_ARG;
 }
 

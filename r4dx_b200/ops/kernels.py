@@ -857,18 +857,21 @@ def trellis_gemm_grouped(words, svh, xh, y, offsets, perm, tiles, ntiles, P: int
     return y
 
 
-register_cuda_sig("r4dxb_trellis_rows_grouped", _I, [_P] * 9 + [_I] * 8 + [_P, _P, _P])
+# K up to which the rows of a tile and a ring of words fit into shared memory at every bit width.
+GROUPED_ROWS_MAX_K = 8192
+
+register_cuda_sig("r4dxb_trellis_rows_grouped", _I, [_P] * 9 + [_I] * 9 + [_P, _P, _P])
 
 
 def trellis_rows_grouped(words, suh, svh, x, y, offsets, perm, tiles, ntiles, xdiv: int, mode: int, P: int, E: int, N: int, Kd: int,
-                         kb: int, xh: torch.Tensor, meta: Optional[torch.Tensor] = None):
-    """y[perm[p]] = expert e(p)'s trellis linear of act(x[perm[p] // xdiv]) for a few rows per expert (``moe_tiles`` of 4
-    rows); ``xh`` (2 Kd bytes per pair) is workspace.  (``meta`` was one for an earlier form of the kernel and is not read.)"""
+                         kb: int, xh: torch.Tensor, meta: Optional[torch.Tensor] = None, tile_rows: int = 4):
+    """y[perm[p]] = expert e(p)'s trellis linear of act(x[perm[p] // xdiv]) for a few rows per expert (``moe_tiles`` of
+    ``tile_rows`` rows, 8 at most); ``xh`` (2 Kd bytes per pair) is workspace.  (``meta`` was one for an earlier form of the kernel and is not read.)"""
     if xh.numel() * xh.element_size() < 2 * Kd * P:
         raise KernelError("trellis_rows_grouped: workspace too small")
-    bound = min(tiles.numel() // 2, P // 4 + E)
+    bound = min(tiles.numel() // 2, P // tile_rows + E)
     _check(_lib().r4dxb_trellis_rows_grouped(_p(words), _p(suh), _p(svh), _p(x), _p(y), _p(offsets), _p(perm), _p(tiles), _p(ntiles), bound,
-                                             xdiv, mode, P, E, N, Kd, kb, _p(xh), _p(gemm_status(xh.device)), _stream()),
+                                             tile_rows, xdiv, mode, P, E, N, Kd, kb, _p(xh), _p(gemm_status(xh.device)), _stream()),
            "trellis_rows_grouped")
     return y
 

@@ -5,6 +5,7 @@ import pytest
 import torch
 
 from r4dx_b200.models.hybrid import HybridModel, Linear
+from r4dx_b200.models.moe import ExpertStack, MoeBlock
 from r4dx_b200.ops import kernels as K
 from r4dx_b200.quant import trellis
 
@@ -80,3 +81,18 @@ def test_a_models_linear_goes_by_shape_and_rows(lib, large, T, entry):
     small = Linear(trellis.random_weight(256, 256, 4, seed=1))
     small(torch.zeros(T, 256, dtype=BF), torch.zeros(T, 256, dtype=BF))
     assert [n for n, _ in lib.calls] == [entry, entry, "r4dxb_trellis_gemv_mma" if T >= 6 else "r4dxb_trellis_gemv_ex"]
+
+
+@pytest.mark.parametrize("H,I,few", [(2048, 512, True), (8192, 1024, True), (8320, 512, False), (512, 8320, False)])
+def test_experts_too_wide_for_the_rows_kernel_take_the_tiles(lib, H, I, few):
+    """Rows and a ring of words of either projection have to fit into shared memory."""
+    z = lambda *s, dtype=torch.int32: torch.zeros(*s, dtype=dtype)
+    stack = lambda N, Kd: ExpertStack(z(1), z(64, Kd, dtype=torch.float16), z(1, dtype=torch.float16), 64, N, Kd, 4)
+    P = 17 * 4
+    block = SimpleNamespace(gate_up=stack(2 * I, H), down=stack(H, I), k=4, e_count=64, cfg=SimpleNamespace(num_experts=64), few_rows_avg=4,
+                            offsets=z(65), perm=z(P), tiles=z(2 * (P + 65)), ntiles=z(1), xh_pairs=z(P, max(H, I), dtype=torch.float16),
+                            gu_pairs=z(P, 2 * I, dtype=BF), y_pairs=z(P, H, dtype=BF))
+    MoeBlock._experts_grouped(block, z(17, H, dtype=BF), 17)
+    names = [n for n, _ in lib.calls]
+    assert (names == ["r4dxb_moe_tiles", "r4dxb_trellis_rows_grouped", "r4dxb_trellis_rows_grouped"]) == few
+    assert few or "r4dxb_trellis_gemm_grouped" in names

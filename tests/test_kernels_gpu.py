@@ -1274,6 +1274,7 @@ def test_grouped_rows_kernel_matches_the_per_pair_reference(K, kb, N, Kd, counts
     words, suh, svh = torch.cat([w.words for w in ws]).cuda(), torch.stack([w.suh for w in ws]).cuda(), torch.stack([w.svh for w in ws]).cuda()
     total = P + elsewhere
     tiles, ntiles = torch.zeros(2 * (total // 4 + E + 1), dtype=torch.int32, device="cuda"), torch.zeros(1, dtype=torch.int32, device="cuda")
+    tiles8 = torch.zeros(2 * (total + E), dtype=torch.int32, device="cuda")
     od, pd = offsets.cuda(), perm.cuda()
     K.moe_tiles(od, E, 4, tiles, ntiles)
     assert int(ntiles) == sum((c + 3) // 4 for c in counts)
@@ -1291,3 +1292,9 @@ def test_grouped_rows_kernel_matches_the_per_pair_reference(K, kb, N, Kd, counts
                 rms = xr.pow(2).mean().sqrt() * Wd[e].pow(2).sum(-1).sqrt()
                 assert ((y[pair].cpu().double() - ref).abs() <= 2.0 ** -8 * ref.abs() + 2e-3 * rms).all(), (e, p)
         assert (y[perm[P:].long().cuda()] == 7.0).all()
+        for tile_rows in (1, 3, 8):                             # a row's sums do not depend on the rows beside it
+            K.moe_tiles(od, E, tile_rows, tiles8, ntiles)
+            y8 = torch.full((total, N), 7.0, dtype=BF, device="cuda")
+            K.trellis_rows_grouped(words, suh, svh, x.cuda(), y8, od, pd, tiles8, ntiles, div, mode, total, E, N, Kd, kb, digits, tile_rows=tile_rows)
+            assert torch.equal(y8, y)
+        K.moe_tiles(od, E, 4, tiles, ntiles)
