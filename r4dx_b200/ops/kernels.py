@@ -573,6 +573,9 @@ def _w4a16_rows(W: W4Weight, x: torch.Tensor, out_f32: bool, out: Optional[torch
         y = out
     else:
         return None
+    begin, end = xk.data_ptr(), xk.data_ptr() + xk.numel() * xk.element_size()
+    if y.data_ptr() < end and begin < y.data_ptr() + y.numel() * y.element_size():
+        return None                      # every CTA reads all rows while others already write theirs: the GEMM works on a copy of x
     rc = _lib().r4dxb_w4a16_rows(_p(W.wq), _p(W.wsz), _p(xk), _p(y), T, W.N, W.K, W.group, 1 if y.dtype == torch.float32 else 0,
                                  _stream())
     if rc == _UNSUPPORTED:

@@ -8,6 +8,7 @@ from r4dx_b200.models.hybrid import HybridModel, Linear
 from r4dx_b200.models.moe import ExpertStack, MoeBlock
 from r4dx_b200.ops import kernels as K
 from r4dx_b200.quant import trellis
+from r4dx_b200.quant.w4a16 import W4Weight
 
 BF = torch.bfloat16
 
@@ -96,3 +97,18 @@ def test_experts_too_wide_for_the_rows_kernel_take_the_tiles(lib, H, I, few):
     names = [n for n, _ in lib.calls]
     assert (names == ["r4dxb_moe_tiles", "r4dxb_trellis_rows_grouped", "r4dxb_trellis_rows_grouped"]) == few
     assert few or "r4dxb_trellis_gemm_grouped" in names
+
+
+def test_a_streamed_head_that_writes_over_its_rows_takes_the_gemm(lib):
+    """The GEMM reads a converted copy of the rows; the streaming kernel would read rows that it has already overwritten."""
+    z = lambda *s, dtype=torch.int32: torch.zeros(*s, dtype=dtype)
+    w = W4Weight(z(256, 32), z(256, 4), 256, 256, 64)
+    buf = z(5, 256, dtype=BF)
+    x = buf[1:4]
+    for out, entry in ((z(3, 256, dtype=BF), "w4a16_rows"), (x, "linear_tc"), (buf[:3], "linear_tc"), (buf[2:], "linear_tc")):
+        lib.calls.clear()
+        K.linear_tc(w, x, out=out)
+        assert [n for n, _ in lib.calls] == ["r4dxb_" + entry]
+    lib.calls.clear()
+    K.linear_tc(w, buf[:2], out=buf[2:4])
+    assert [n for n, _ in lib.calls] == ["r4dxb_w4a16_rows"]
