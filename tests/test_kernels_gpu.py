@@ -233,6 +233,44 @@ def test_sibling_launch_equals_separate_launches(K, T, ksplit):
         assert torch.equal(o, ref)
 
 
+@pytest.mark.parametrize("T,split,kb,widths", [(1, 1, 4, (384, 128)), (3, 3, 3, (384, 128, 256)), (5, 4, 5, (128, 128, 128)), (8, 1, 4, (128, 512, 256)),
+                                               (8, 8, 3, (256, 128))])
+def test_sibling_launch_on_the_rows_kernel_equals_separate_launches(K, T, split, kb, widths):
+    """Two and three weights in one launch (rows transformed per weight, row blocks back to back, uneven slices of nine K blocks)
+    have the bits of a launch per weight, with and without the norm prologue."""
+    from r4dx_b200.quant import trellis
+    Kd = 1152
+    ws = [trellis.random_weight(n, Kd, kb, seed=n + i, sigma=0.05).to("cuda") for i, n in enumerate(widths)]
+    g = torch.Generator().manual_seed(T)
+    x, gu = torch.randn(T, Kd, generator=g).to(BF).cuda(), torch.randn(T, 2 * Kd, generator=g).to(BF).cuda()
+    nw = (torch.randn(Kd, generator=g) * 0.1).to(BF).cuda()
+    grp = K.SiblingGroup(ws)
+    grp.split_rows = split
+    for pro, xs, norm in ((K.PRO_NONE, x, None), (K.PRO_RMSNORM, x, nw), (K.PRO_GELU_MUL, gu, None)):
+        outs = [torch.zeros(T, w.N, dtype=BF, device="cuda") for w in ws]
+        grp(xs, outs, prologue=pro, norm_w=norm)
+        for w, o in zip(ws, outs):
+            assert torch.equal(o, K.trellis_gemv(w, xs, split_rows=split, prologue=pro, norm_w=norm))
+
+
+def test_rows_kernel_grids_beyond_one_wave_and_widened_splits(K):
+    """160 row blocks (two CTAs on some SMs) against launches of two of them; a slice of 136 K blocks at eight rows, which
+    does not fit into shared memory, against the split that the launch widens to; the rule's own choice against the same split
+    given by hand."""
+    from r4dx_b200.quant import trellis
+    w = trellis.random_weight(160 * 128, 640, 4, seed=3, sigma=0.05, device="cuda")
+    x = torch.randn(4, 640, generator=torch.Generator().manual_seed(0)).to(BF).cuda()
+    y = K.trellis_gemv(w, x, split_rows=1)
+    per = w.words.numel() // 160
+    for b in (0, 73, 158):
+        part = trellis.TrellisWeight(w.words[b * per:(b + 2) * per], w.suh, w.svh[b * 128:(b + 2) * 128], 256, 640, 4)
+        assert torch.equal(y[:, b * 128:(b + 2) * 128], K.trellis_gemv(part, x, split_rows=1))
+    assert w.N * w.K >= K.ROWS_MIN_WEIGHTS and torch.equal(K.trellis_gemv(w, x), K.trellis_gemv(w, x, split_rows=K.pick_split(w.N, w.K)))
+    long = trellis.random_weight(128, 17408, 5, seed=3, sigma=0.05, device="cuda")
+    x = torch.randn(8, 17408, generator=torch.Generator().manual_seed(0)).to(BF).cuda()
+    assert torch.equal(K.trellis_gemv(long, x, split_rows=1), K.trellis_gemv(long, x, split_rows=2))
+
+
 @pytest.mark.parametrize("ksplit", [2, 4, 8])
 def test_trellis_gemv_uneven_k_split(K, ksplit):
     """17 K blocks over 2 / 4 / 8 CTAs of a cluster (uneven slices) against the unsplit launch and the reference."""
@@ -286,6 +324,24 @@ def test_w4a16_streaming_rows_match_fp64(K, T, N, Kd, group):
     assert torch.equal(yb, y.to(BF))
     if T <= 8:
         assert torch.equal(K.w4a16_gemv(qd, xd), y)
+
+
+@pytest.mark.parametrize("T", [1, 17, 32, 33])
+def test_linear_tc_of_a_w4a16_head_around_its_streaming_rows(K, T):
+    """Up to 32 rows the head streams its weights (fp32 scales and sums), from 33 it is the tcgen05 product (weights rounded to fp16
+    after scaling, 2^-11 each); both outputs, and an ``out`` that the caller owns."""
+    from r4dx_b200.quant import w4a16
+    N, Kd = 1280, 1024
+    g = torch.Generator().manual_seed(T)
+    q = w4a16.quantize(torch.randn(N, Kd, generator=g) * 0.05, 64)
+    W, x = w4a16.dequantize(q).double(), torch.randn(T, Kd, generator=g).to(BF)
+    ref, rms = x.double() @ W.T, (x.double() ** 2 @ (W ** 2).T).sqrt()
+    out = torch.full((T, N), float("nan"), device="cuda")
+    y = K.linear_tc(q.to("cuda"), x.cuda(), out=out)
+    assert y.data_ptr() == out.data_ptr()
+    assert ((y.cpu().double() - ref).abs() <= (1e-5 if T <= 32 else 2.0 ** -11 * 4) * rms).all()
+    yb = K.linear_tc(q.to("cuda"), x.cuda())
+    assert yb.dtype == BF and yb.shape == (T, N) and torch.equal(yb, y.to(BF))
 
 
 @pytest.mark.parametrize("T", [17, 31, 32, 33, 64])

@@ -284,6 +284,72 @@ def test_expert_parallel_exchange_in_one_gpu_matches_local_moe():
         assert torch.equal(xa, xb), (it, (xa.float() - xb.float()).abs().max())
 
 
+@pytest.mark.parametrize("T,skewed", [(17, False), (64, False), (64, True)])
+def test_experts_with_a_few_rows_each_match_the_tile_products(T, skewed):
+    """The block's two routes for more than 16 rows on the same plan: tiles of eight rows on mma.sync and tiles of 16 on tcgen05.
+    Both multiply the format's code values by the same fp16 rows; what differs is the order of fp32 sums, which can move the
+    bf16 result of either projection by a step.  Skewed: most pairs go to four experts."""
+    import dataclasses
+    from r4dx_b200.config import tiny_moe_config
+    from r4dx_b200.models.moe import MoeBlock
+    from r4dx_b200.models.oracle import init_weights
+    from r4dx_b200.quant.weights import moe_kb_rule, quantize_weight_set
+    cfg = dataclasses.replace(tiny_moe_config(), num_experts=64, num_hidden_layers=1, layer_types=["linear_attention"])
+    q = _to_dev(quantize_weight_set(cfg, init_weights(cfg, 0), kb_rule=moe_kb_rule))
+    g = torch.Generator().manual_seed(T)
+    h = torch.randn(T, cfg.hidden_size, generator=g).to(torch.bfloat16)
+    if skewed:
+        h += 3 * torch.randn(1, cfg.hidden_size, generator=g).to(torch.bfloat16)
+    h, outs = h.cuda(), []
+    for avg in (4, 0):
+        blk = MoeBlock(cfg, q, 0, "cuda", 64)
+        blk.few_rows_avg = avg
+        blk.route(h, T)
+        blk.experts(h, T)
+        outs.append((blk.gu_pairs[:T * blk.k].float(), blk.y_pairs[:T * blk.k].float()))
+        most = int(blk.offsets.diff().max())
+    assert T * blk.k <= 4 * cfg.num_experts and (most > 16) == skewed
+    for few, tiles, steps in zip(*outs, (1, 3)):            # (the second product's rows carry the first one's steps)
+        rms = tiles.pow(2).mean().sqrt()
+        assert ((few - tiles).abs() <= steps * (2.0 ** -7 * tiles.abs() + 2e-3 * rms)).all()
+
+
+def test_windows_of_large_weights_replay_as_they_run():
+    """Weights large enough for the rows kernel (the tiny geometries have none): a captured window of four rows gives the logits
+    and the state of an eager one, and those of the CUDA-core kernel up to rounding: the results of about thirty products in
+    series round to bf16 either way, 2^-9 of their value each, sqrt(30) 2^-9 = 1.1 % together; twice that is allowed."""
+    import dataclasses
+    from r4dx_b200.config import small_hybrid_config
+    from r4dx_b200.models.hybrid import HybridModel
+    from r4dx_b200.ops import kernels as K
+    from r4dx_b200.quant.weights import synthetic_weight_set
+    cfg = dataclasses.replace(small_hybrid_config(4), hidden_size=2048, intermediate_size=4096, linear_num_key_heads=8, linear_num_value_heads=16)
+    w = synthetic_weight_set(cfg, device="cuda", seed=3)
+    prompt = torch.randint(0, cfg.vocab_size, (70,), generator=torch.Generator().manual_seed(0), dtype=torch.int32)
+
+    def windows(graph):
+        m = HybridModel(cfg, w, max_ctx=256, device="cuda")
+        m.prefill(prompt)
+        if graph:
+            m.enable_graphs((4,))
+        logits = []
+        for i in range(3):
+            m.verify_window(5 + i, [7, 11, 13 + i])
+            logits.append(m.logits_rows(4).clone())
+        return torch.cat(logits), [m.gdn_state[i].clone() for i in sorted(m.gdn_state)]
+
+    assert K.GEMV_IMPL == "auto" and K.rows_split(2 * cfg.intermediate_size, cfg.hidden_size, 4)
+    eager, eager_state = windows(False)
+    replayed, replayed_state = windows(True)
+    assert torch.equal(eager, replayed) and all(torch.equal(a, b) for a, b in zip(eager_state, replayed_state))
+    K.set_gemv_impl("simt")
+    try:
+        simt, _ = windows(False)
+    finally:
+        K.set_gemv_impl("auto")
+    assert not torch.equal(simt, eager) and (simt - eager).norm() < 0.022 * eager.norm()
+
+
 def test_batched_decode_matches_independent_sequences(tiny):
     from r4dx_b200.models.batch import BatchModel
     from r4dx_b200.models.hybrid import HybridModel
