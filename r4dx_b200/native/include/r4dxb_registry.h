@@ -28,7 +28,7 @@ typedef struct R4dxbKernelInfo {
   const char* computes; /* for a human */
   const char* shape;    /* geometry, for a human */
   const char* dtypes;
-  const char* engine;   /* tcgen05 | mma.sync | simt, "+bulk-copy" / "+peer-stores" where they apply */
+  const char* engine;   /* tcgen05 | mma.sync | simt, "+bulk-copy" / "+peer-stores" / "+simt" where they apply */
   const R4dxbConstraint* constraints;
   int n_constraints;
 } R4dxbKernelInfo;

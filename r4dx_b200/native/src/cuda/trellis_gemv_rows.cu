@@ -476,7 +476,7 @@ int LaunchRows(RowsArgs a, int ksplit, cudaStream_t stream) {
   attr[0].val.clusterDim.x = ksplit;
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
-  // programmatic dependent launch: the CTAs fill their rings while the digits are still being written
+  // programmatic dependent launch: the CTAs fill their rings while the rows are still being written
   attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;

@@ -12,6 +12,7 @@ namespace {
 
 const R4dxbConstraint c0[] = {{"T", R4DXB_C_LE, 8, nullptr}, {"N", R4DXB_C_DIV, 128, nullptr}, {"K", R4DXB_C_DIV, 128, nullptr}, {"kb", R4DXB_C_IN, 0, "3 4 5"}, {"ksplit", R4DXB_C_IN, 0, "1 2 4 8"}};
 const R4dxbConstraint c1[] = {{"T", R4DXB_C_LE, 8, nullptr}, {"count", R4DXB_C_LE, 3, nullptr}, {"count", R4DXB_C_GE, 2, nullptr}, {"K", R4DXB_C_DIV, 128, nullptr}, {"kb", R4DXB_C_IN, 0, "3 4 5"}};
+const R4dxbConstraint c1r[] = {{"T", R4DXB_C_LE, 8, nullptr}, {"count", R4DXB_C_LE, 3, nullptr}, {"K", R4DXB_C_DIV, 128, nullptr}, {"kb", R4DXB_C_IN, 0, "3 4 5"}};
 const R4dxbConstraint c2[] = {{"T", R4DXB_C_LE, 8, nullptr}, {"N", R4DXB_C_DIV, 128, nullptr}, {"K", R4DXB_C_DIV, 128, nullptr}, {"kb", R4DXB_C_IN, 0, "3 4 5"}};
 const R4dxbConstraint c3[] = {{"T", R4DXB_C_LE, 8, nullptr}, {"world", R4DXB_C_LE, 8, nullptr}, {"world", R4DXB_C_GE, 2, nullptr}, {"N", R4DXB_C_DIV, 128, nullptr}, {"K", R4DXB_C_DIV, 128, nullptr}};
 const R4dxbConstraint c4[] = {{"N", R4DXB_C_DIV, 128, nullptr}, {"K", R4DXB_C_DIV, 128, nullptr}, {"kb", R4DXB_C_IN, 0, "3 4 5"}, {"tmax", R4DXB_C_IN, 0, "2 8"}};
@@ -96,10 +97,10 @@ const R4dxbKernelInfo kKernels[] = {
      "N, K multiples of 128; cluster split 1/2/4/8 of K; kb 3/4/5", "bf16 x, packed trellis words, bf16 y", "simt+bulk-copy", c0, 5},
     {"trellis_gemv_siblings", "gemm", "trellis_linear_rows_le_8", "2 or 3 weights of one K and bit width over the same rows in one launch",
      "as trellis_gemv_ex; no residual", "bf16 x, packed trellis words, bf16 y", "simt+bulk-copy", c1, 5},
-    {"trellis_rows_grouped", "gemm", "moe_experts_few_rows", "every expert's tiles of four planned rows, hash bytes times integer rows on mma.sync",
+    {"trellis_rows_grouped", "gemm", "moe_experts_few_rows", "every expert's tiles of four planned rows, decoded into mma.sync operands",
      "N, K multiples of 128", "bf16 x, stacked trellis words, bf16 y", "mma.sync+bulk-copy", nullptr, 0},
-    {"trellis_gemv_rows", "gemm", "trellis_linear_rows_le_8", "one to three weights over the same rows, hash bytes times integer rows on mma.sync",
-     "as trellis_gemv_ex; any cluster split of 1..8", "bf16 x, packed trellis words, bf16 y", "mma.sync+bulk-copy", c1, 5},
+    {"trellis_gemv_rows", "gemm", "trellis_linear_rows_le_8", "one to three weights over the same rows, decoded into mma.sync operands",
+     "as trellis_gemv_ex; any cluster split of 1..8; residual with one weight", "bf16 x, packed trellis words, bf16 y", "mma.sync+bulk-copy", c1r, 4},
     {"trellis_gemv_mma", "gemm", "trellis_linear_rows_le_8", "the same product with code values written to tensor memory and contracted by tcgen05.mma",
      "K / ksplit <= 6144", "bf16 x, packed trellis words, bf16 y", "tcgen05", c2, 4},
     {"trellis_gemv_allreduce", "gemm+collective", "row_parallel_linear_allreduce", "row-parallel product whose epilogue pushes (value, sequence) pairs to every peer and sums them in rank order",
@@ -139,7 +140,7 @@ const R4dxbKernelInfo kKernels[] = {
     {"linear_tc", "gemm", "plain_linear_rows_any", "y = act(x W^T + bias) + residual: dense bf16 / fp16 W by TMA, or w4a16 W widened by the decode warps",
      "dense: N % 4, K % 8; w4a16: N, K % 128, group 32/64/128", "bf16 / fp16 / w4a16, bf16 or fp32 y", "tcgen05", c18, 2},
     {"w4a16_gemv", "gemm", "w4a16_linear_rows_le_8", "group-quantised 4-bit head product",
-     "rows * K * 2 <= 200 KB", "bf16 x, nibbles + fp16 scale / zero", "mma.sync", c19, 2},
+     "rows * K * 2 <= 200 KB; mma.sync where N % 16 and K % (4 group) are 0, else CUDA cores", "bf16 x, nibbles + fp16 scale / zero", "mma.sync+simt", c19, 2},
     {"w4a16_rows", "gemm", "w4a16_linear_rows_le_64", "the same, 16 rows a launch",
      "K % (4 group), 16 rows * K * 2 <= 227 KB", "bf16 x, nibbles + fp16 scale / zero", "mma.sync", c19r, 3},
     {"w8a16_gemv", "gemm", "w8a16_linear_rows_le_8", "group-quantised 8-bit product",

@@ -268,10 +268,10 @@ def set_gemv_impl(name: str) -> None:
 
 
 def use_mma_gemv(T: int, N: int, K: int, ksplit: int) -> bool:
-    """Whether a product that the rows kernel does not serve (the tensor-parallel launches, slices too long for it) goes to the
-    tensor-memory weight-streaming kernel (which needs an even K split of at most 6144 columns per CTA): where that measured
-    faster than the CUDA cores, from six rows (gate_up at 8 rows: 95 against 121 us, down 69 against 97 us) and from four
-    rows on the two large MLP products (80 against 83 us, 57 against 67 us)."""
+    """Whether a product that the rows kernel does not serve (small weights, the tensor-parallel launches, slices too long for it)
+    goes to the tensor-memory weight-streaming kernel (which needs an even K split of at most 6144 columns per CTA): where that
+    measured faster than the CUDA cores, from six rows (gate_up at 8 rows: 95 against 121 us, down 69 against 97 us) and from
+    four rows on the two large MLP products (80 against 83 us, 57 against 67 us)."""
     if GEMV_IMPL == "simt" or K // ksplit > 6144 or (K // 128) % ksplit:
         return False
     if GEMV_IMPL == "mma":
@@ -333,7 +333,8 @@ register_cuda_sig("r4dxb_trellis_gemv_siblings", _I, [_I, _P, _P, _P, _P, _P, _P
 
 class SiblingGroup:
     """Trellis weights that read the same rows through the same prologue (q / k / v; the GDN qkv / z pair), served by
-    one launch of the weight-streaming kernel.  Holds the pointer tables so a call allocates nothing."""
+    one launch of the weight-streaming kernel.  Holds the pointer tables, so that a call allocates nothing but (on the rows
+    kernel) its workspace."""
 
     def __init__(self, weights: Sequence[TrellisWeight]):
         w0 = weights[0]

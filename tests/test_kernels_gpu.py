@@ -102,9 +102,9 @@ def test_trellis_gemv_tensor_memory_path_against_reference_and_cuda_core_path(K,
 @pytest.mark.parametrize("T,N,Kd,split", [(1, 256, 640, 2), (2, 128, 128, 1), (3, 256, 384, 3), (4, 384, 1280, 2), (5, 128, 2176, 5), (7, 256, 1024, 8),
                                           (8, 512, 5120, 1), (8, 128, 17408, 6)])
 def test_trellis_rows_kernel_against_fp64(K, kb, T, N, Kd, split):
-    """The integer tensor-core kernel (1..8 rows) at the edges of its stage ring, teams and splits, all prologues.  Its
-    product differs from the definition by the unrounded code values (half an fp16 ulp, 2.2e-4 rms of unit codes) and by
-    digits of 1/32512 of the row's largest value (below 1e-4 of the row's rms); the bf16 result adds 2^-9 of each value."""
+    """The mma.sync kernel (1..8 rows) at the edges of its stage ring, teams and splits, all prologues.  Its product differs from
+    the definition by the fp16 rounding of the rows (2^-11 of each entry at most, 2.0e-4 rms of the product; 2e-3 is ten
+    times that); the bf16 result adds 2^-9 of each value."""
     from r4dx_b200.ops import reference as R
     from r4dx_b200.quant import trellis
     g = torch.Generator().manual_seed(T * 100 + kb)
@@ -1318,7 +1318,7 @@ def test_attention_precore_of_many_rows_equals_few_row_calls(K, D, Hq, Hkv, rot)
                                             (3, 384, 2048, (4, 4, 4, 4, 0, 7))])
 def test_grouped_rows_kernel_matches_the_per_pair_reference(K, kb, N, Kd, counts):
     """Experts with none, full and ragged tiles of four rows, both input forms, pairs of experts that live elsewhere left alone.
-    Bound as for the ungrouped kernel: unrounded codes and integer rows (2e-3 of the rms is ten times that) plus bf16."""
+    Bound as for the ungrouped kernel: fp16 rows (2e-3 of the rms is ten times their rounding) plus bf16."""
     from r4dx_b200.quant import trellis
     E, P, k = len(counts), sum(counts), 2
     g = torch.Generator().manual_seed(N + Kd)
