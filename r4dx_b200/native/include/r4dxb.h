@@ -139,6 +139,9 @@ int r4dxb_tp_reduce_push(void* const* x, void* const* xflag, const void* recv, c
 int r4dxb_tp_wait(const void* flag, unsigned target, int spin_limit, int code, int* status, void* stream);
 int r4dxb_trellis_gemm(const void* w, const void* svh, const void* xh, void* y, const void* residual, int T, int N, int K,
                        int kb, int tn, int* status, void* stream);
+/* The same with K split over the ksplit (1..8) CTAs of a cluster; 192 and 384 are token tiles as well. */
+int r4dxb_trellis_gemm_split(const void* w, const void* svh, const void* xh, void* y, const void* residual, int T, int N, int K,
+                             int kb, int tn, int ksplit, int* status, void* stream);
 
 /* Plain linear on the same tensor-core kernel, any T: y[T,N] = x[T,K] W^T (+ bias[N] bf16) (+ residual[T,N] bf16).
  * kind 0: dense 16-bit W[N,K] (bf16 != 0: W and x bf16, else fp16); kind 1: w4a16 (w = nibbles [N][K/8] u32,
@@ -146,6 +149,9 @@ int r4dxb_trellis_gemm(const void* w, const void* svh, const void* xh, void* y, 
  * K % 8 == 0.  out_f32 bit 0: y fp32; bits 8-15: activation after the bias (0 none, 1 tanh-GELU, 2 erf-GELU). */
 int r4dxb_linear_tc(const void* w, const void* wsz, int kind, int group, int bf16, const void* x, void* y, int out_f32,
                     const void* bias, const void* residual, int T, int N, int K, int tn, int* status, void* stream);
+/* The same with K split over the ksplit (1..8) CTAs of a cluster. */
+int r4dxb_linear_tc_split(const void* w, const void* wsz, int kind, int group, int bf16, const void* x, void* y, int out_f32,
+                          const void* bias, const void* residual, int T, int N, int K, int tn, int ksplit, int* status, void* stream);
 
 /* 8-bit prefill product (opt-in): r4dxb_quantize_rows_e4m3 turns fp16 rows [T, K] into e4m3 rows + one fp32 scale per row
  * (scale = rowmax / 448); r4dxb_trellis_gemm_f8 multiplies them with e4m3 code values on tcgen05.mma kind::f8f6f4

@@ -95,6 +95,12 @@ __device__ __forceinline__ bool MbarTryWaitAt(uint32_t bar, uint32_t parity) {
                : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
   return ok != 0;
 }
+__device__ __forceinline__ bool MbarTestWaitAt(uint32_t bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile("{ .reg .pred p; mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
+               : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+  return ok != 0;
+}
 __device__ __forceinline__ bool MbarWaitAt(uint32_t bar, uint32_t parity, volatile int* abort_flag, int code) {
   if (MbarTryWaitAt(bar, parity)) return true;
   const long long t0 = clock64();
@@ -109,6 +115,50 @@ __device__ __forceinline__ bool MbarWaitAt(uint32_t bar, uint32_t parity, volati
 __device__ __forceinline__ void BulkLoadAt(uint32_t smem_dst, const void* gsrc, uint32_t bytes, uint32_t bar) {
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
                ::"r"(smem_dst), "l"(reinterpret_cast<uint64_t>(gsrc)), "r"(bytes), "r"(bar) : "memory");
+}
+
+// ---- pairs of floats ------------------------------------------------------------------------------------
+__device__ __forceinline__ float2 Add2(float2 a, float2 b) {
+  float2 d;
+  asm("{ .reg .b64 x, y, z; mov.b64 x, {%2, %3}; mov.b64 y, {%4, %5}; add.rn.f32x2 z, x, y; mov.b64 {%0, %1}, z; }"
+      : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return d;
+}
+__device__ __forceinline__ float2 Fma2(float2 a, float2 b, float2 c) {
+  float2 d;
+  asm("{ .reg .b64 x, y, z, w; mov.b64 x, {%2, %3}; mov.b64 y, {%4, %5}; mov.b64 z, {%6, %7}; fma.rn.f32x2 w, x, y, z; mov.b64 {%0, %1}, w; }"
+      : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+  return d;
+}
+
+// ---- clusters ------------------------------------------------------------------------------------------
+// Barrier over every thread of the cluster; shared-memory writes before it are visible to the peers after it.
+__device__ __forceinline__ void ClusterSync() {
+  asm volatile("barrier.cluster.arrive.release;\n barrier.cluster.wait.acquire;" ::: "memory");
+}
+__device__ __forceinline__ uint32_t ClusterRank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+// The shared-memory address `addr` (of this CTA's window) in CTA `rank` of the cluster.
+__device__ __forceinline__ uint32_t MapToRank(uint32_t addr, uint32_t rank) {
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+  return r;
+}
+// Arrival at a barrier of another CTA (`bar` from MapToRank).  With the default scope: what the arrival announces are operands of a
+// paired product, which the writers have handed to the async proxy (fence.proxy.async) or which a TMA load has written; an arrival
+// with cluster scope took 1300 to 1900 clocks in the product's main loop.
+__device__ __forceinline__ void MbarArriveRemote(uint32_t bar) {
+  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+// 16 bytes at the shared-memory address `addr` (of this CTA's window) in CTA `rank` of the cluster.
+__device__ __forceinline__ float4 LoadRemote4(uint32_t addr, uint32_t rank) {
+  float4 v;
+  asm volatile("{ .reg .b32 a; mapa.shared::cluster.u32 a, %4, %5; ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [a]; }"
+               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr), "r"(rank) : "memory");
+  return v;
 }
 
 // ---- proxies / fences ------------------------------------------------------------------------------
@@ -128,6 +178,12 @@ __device__ __forceinline__ void TmaLoad2D(void* smem_dst, const CUtensorMap* map
       ::"r"(SmemAddr(smem_dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(SmemAddr(bar)), "r"(x), "r"(y)
       : "memory");
 }
+__device__ __forceinline__ void TmaLoad2DAt(uint32_t smem_dst, const CUtensorMap* map, uint32_t bar, int x, int y) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
+      ::"r"(smem_dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(x), "r"(y)
+      : "memory");
+}
 // Untiled bulk copy global -> shared; both addresses 16-byte aligned, bytes a multiple of 16.
 __device__ __forceinline__ void BulkLoad(void* smem_dst, const void* gsrc, uint32_t bytes, uint64_t* bar) {
   asm volatile(
@@ -135,6 +191,16 @@ __device__ __forceinline__ void BulkLoad(void* smem_dst, const void* gsrc, uint3
       ::"r"(SmemAddr(smem_dst)), "l"(reinterpret_cast<uint64_t>(gsrc)), "r"(bytes), "r"(SmemAddr(bar))
       : "memory");
 }
+
+// Untiled bulk copy shared -> global (of this GPU), both 16-byte aligned, in the issuing thread's bulk groups; the generic writes it
+// reads were made visible with FenceProxyAsyncShared.
+__device__ __forceinline__ void BulkStore(void* gdst, uint32_t smem_src, uint32_t bytes) {
+  asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;"
+               ::"l"(reinterpret_cast<uint64_t>(gdst)), "r"(smem_src), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void BulkStoreCommit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void BulkStoreWaitRead() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
+__device__ __forceinline__ void BulkStoreWait() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 
 // ---- tensor memory ------------------------------------------------------------------------------------
 // Whole-warp calls (.sync.aligned).  Columns: power of two, 32..512.
@@ -147,6 +213,18 @@ __device__ __forceinline__ void TmemRelinquish() {
 }
 __device__ __forceinline__ void TmemDealloc(uint32_t taddr, uint32_t columns) {
   asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(columns) : "memory");
+}
+
+// The same for a pair of CTAs (cta_group::2): a warp of each takes part, and both get the same columns.
+__device__ __forceinline__ void TmemAllocPair(uint32_t* smem_result, uint32_t columns) {
+  asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(SmemAddr(smem_result)), "r"(columns)
+               : "memory");
+}
+__device__ __forceinline__ void TmemRelinquishPair() {
+  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void TmemDeallocPair(uint32_t taddr, uint32_t columns) {
+  asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(columns) : "memory");
 }
 
 // ---- UMMA --------------------------------------------------------------------------------------------------
@@ -174,6 +252,15 @@ __device__ __forceinline__ void UmmaF16(uint32_t tmem_d, uint64_t desc_a, uint64
       ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
       : "memory");
 }
+// The same over a pair of CTAs, issued by ONE thread of the first: A rows 0..127 and the first half of the B rows come from the
+// first CTA's shared memory, the others from the second's (same addresses); each CTA's tensor memory gets its 128 rows of D.
+__device__ __forceinline__ void UmmaF16Pair(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{ .reg .pred p; setp.ne.b32 p, %4, 0;\n"
+      "  tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p; }"
+      ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
 // kind::f8f6f4 with e4m3 A and B (format code 0 for both), both K-major, fp32 accumulate; K = 32 per instruction.
 __host__ __device__ constexpr uint32_t UmmaInstrDescE4m3(int M, int N) {
   return (1u << 4) | (static_cast<uint32_t>(N >> 3) << 17) | (static_cast<uint32_t>(M >> 4) << 24);
@@ -188,6 +275,14 @@ __device__ __forceinline__ void UmmaF8(uint32_t tmem_d, uint64_t desc_a, uint64_
 // Arrives once on `bar` when every MMA issued so far by this thread has finished.
 __device__ __forceinline__ void UmmaCommit(uint64_t* bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(SmemAddr(bar)) : "memory");
+}
+__device__ __forceinline__ void UmmaCommitAt(uint32_t bar) {
+  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+}
+// For a pair: arrives on the barrier at the same address in every CTA of the mask (bit = rank in the cluster).
+__device__ __forceinline__ void UmmaCommitPairAt(uint32_t bar, uint16_t ctas) {
+  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
+               ::"r"(bar), "h"(ctas) : "memory");
 }
 // 32 lanes x 32 consecutive fp32 columns: thread t of the warp reads TMEM lane (base lane + t).
 __device__ __forceinline__ void TmemLoad32x32(uint32_t taddr, uint32_t (&r)[32]) {

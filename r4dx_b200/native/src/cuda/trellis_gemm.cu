@@ -1,26 +1,21 @@
-// Trellis-decode GEMM on the 5th-generation tensor cores (tcgen05 + TMEM), for T >= 16 rows.
+// Plain linears (dense 16-bit, w4a16, w8a16) and the 8-bit trellis product on the 5th-generation tensor cores (tcgen05 + TMEM), the
+// input transforms of the trellis products, and the tile list of the grouped ones.  The 16-bit trellis product is in trellis_product.cu.
 //
-//   Y[t, n] = bf16( svh[n] * H128( sum_k Q[n, k] * Xh[t, k] )[n] (+ residual[t, n]) )
+// "Swap-AB": the weight block is the UMMA A operand (M = 128 weight rows = the span of one output Hadamard), the activations are the B
+// operand (N = TN tokens), so the fp32 accumulator sits in TMEM as [lane = weight row][column = token].  Weights are widened or
+// decoded exactly once per CTA and reused by all TN tokens of the tile.
 //
-// "Swap-AB": the decoded weight block is the UMMA A operand (M = 128 weight rows = the span of one
-// output Hadamard), the activations are the B operand (N = TN tokens), so the fp32 accumulator
-// sits in TMEM as [lane = weight row][column = token].  Weights are decoded exactly once per CTA
-// and reused by all TN tokens of the tile.
-//
-// Warp roles (DW + 2 warps, DW = 4, 8 or 16 decode warps):
-//   warps 0..DW-1  decode: packed words (shared memory) -> fp16 codes -> A tile in the canonical
+// Warp roles (DW + 3 warps, DW = 8 or 16 decode warps):
+//   warps 0..DW-1  decode: packed words or 4- / 8-bit weights -> A tile in the canonical
 //              K-major 128-byte-swizzled UMMA layout; later the epilogue (TMEM -> registers ->
-//              shared transpose -> FWHT128 over the weight rows -> svh, residual -> bf16 rows).
-//              The decode chain (shift, multiply, byte-sum) is dependent integer work at ~0.3 IPC
-//              per warp, so several warps per scheduler are what keeps the tensor pipe fed.
-//   warp DW    producer: TMA tile of Xh [TN x 64] (128B swizzle) + bulk copy of the slab's words
+//              shared transpose -> (trellis: FWHT128 over the weight rows -> svh) -> residual -> rows).
+//   warp DW    producer: TMA tile of the activations [TN x 64] (128B swizzle)
 //   warp DW+1  MMA issuer: one elected thread issues 4 x tcgen05.mma (K = 16) per 64-wide K slab
 //              and commits to the stage's "empty" barrier; it also owns the TMEM allocation.
-// A dense mode (KB == 0) takes A from a plain fp16 [N, K] matrix instead of decoding: that is the
-// bf16/fp16-layout linear and the bisecting aid for the tensor-core plumbing.
-//
-// The reference engine's counterparts are WMMA kernels whose decoded fragments are shared through
-// LDS (reference: third_party/libr4d/r4d_gemm_trellis_nt_m256.hip:1-60); nothing is shared with them.
+//   warp DW+2  producer: packed words, or the tiles of a dense A
+// A Hadamard mode with a dense A (MODE 0) takes A from a plain fp16 [N, K] matrix: the bisecting aid for the tensor-core plumbing.
+// K may be split over the CTAs of a cluster (plain modes): a router or an a / b projection has so few outputs that its row blocks
+// alone occupy a few SMs.
 #include <cuda_fp8.h>
 
 #include "sm100_ptx.cuh"
@@ -50,21 +45,14 @@ struct GemmSmem {
   static constexpr int kXBytes = XST * kXTileBytes;
   static constexpr int kEpiStride = 132;                                     // floats per staged token row
   static constexpr int kEpiBytes = 32 * kEpiStride * 4;                      // per group of four epilogue warps
-  // the epilogue staging reuses the (by then drained) rings: it must hold one buffer per warp group
+  static constexpr bool kSplits = KB == 0 && TN <= 256;                      // whether the CTAs of a cluster may split K
+  // the epilogue staging reuses the (by then drained) rings: it must hold one buffer per warp group, or all sums where K is split
   static constexpr int kRingsRaw = kABytes + kXBytes + WST * kWordsSlot;
-  static constexpr int kRing = kRingsRaw > 4 * kEpiBytes ? kRingsRaw : 4 * kEpiBytes;
+  static constexpr int kSums = kSplits ? TN * kEpiStride * 4 : 0;
+  static constexpr int kEpiAll = kSums > 4 * kEpiBytes ? kSums : 4 * kEpiBytes;
+  static constexpr int kRing = kRingsRaw > kEpiAll ? kRingsRaw : kEpiAll;
   static constexpr int kBars = 2 * WST + 2 * AST + 2 * XST + 1;
   static constexpr int kTotal = kRing + 1024 /*alignment slack*/ + 512 /*barriers*/;
-};
-
-// Reduce-scatter epilogue (tensor-parallel prefill): instead of its own output tensor, the row-parallel product
-// stores every partial row into the receive buffer of the rank that owns the row (rows are dealt out in
-// contiguous blocks of rows_per_rank), over NVLink peer mappings, tile by tile as the epilogue produces them;
-// one system-scope counter per owner collects the arrivals of every CTA on every rank.
-struct RsArgs {
-  __nv_bfloat16* recv[8];      // peer-mapped receive buffers, indexed by owner rank: [world(src)][rows_per_rank][N]
-  unsigned* cnt[8];            // peer-mapped arrival counters, indexed by owner rank
-  int world, rank, rows_per_rank;
 };
 
 // Plain linear modes of the same kernel (MODE 1: dense 16-bit A matrix, MODE 2: w4a16 group-quantised A): y = x W^T
@@ -83,14 +71,6 @@ struct PlainArgs {
   int bf16;                    // the 16-bit operands are bf16 (MODE 1 only)
   int out_f32;                 // y is fp32 [T, N] instead of bf16
   int act;                     // after the bias: 0 none, 1 tanh-GELU, 2 erf-GELU
-  // MODE 3, grouped experts: the rows of xh are the (row, expert) pairs sorted by expert; a token tile is one expert's
-  // next TN rows.  offsets [E + 1] and perm [pairs] come from the routing plan, tiles/ntiles from MoeTilesKernel.
-  const int* g_offsets;
-  const int* g_perm;           // sorted position -> pair id = output row
-  const int* g_tiles;          // [2 * max_tiles]: (local expert, first sorted row)
-  const int* g_ntiles;
-  long long g_words;           // packed words per expert
-  int g_max_tiles;             // grid height: an upper bound on the tile count
   // MODE 4, 8-bit operands: the decode warps emit e4m3 code values, the activations are e4m3 rows with one fp32 scale per
   // row (xh = scale * e4m3); K per slab is 128 and the products run at the 8-bit rate with half the activation bytes
   const float* x_scale;        // [T]
@@ -101,8 +81,7 @@ __global__ void __launch_bounds__((DW + 3) * 32, 1)
 TrellisGemmKernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_a,
                   const void* __restrict__ wsrc,
                   const __half* __restrict__ svh, __nv_bfloat16* __restrict__ y,
-                  const __nv_bfloat16* __restrict__ residual, int T, int N, int K, int* __restrict__ status, RsArgs rs,
-                  PlainArgs pl) {
+                  const __nv_bfloat16* __restrict__ residual, int T, int N, int K, int* __restrict__ status, PlainArgs pl) {
   using S = GemmSmem<KB, TN, MODE == 4>;
   constexpr int kSlabElems = MODE == 4 ? 2 * kSlabK : kSlabK;      // K values per slab (one 128-byte row per operand row)
   constexpr int kKTiles = S::kKTiles;
@@ -126,17 +105,12 @@ TrellisGemmKernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int nb = blockIdx.x;                 // 128-row weight block
-  int t0 = blockIdx.y * TN;                  // first token of the tile
-  int t_end = T;                             // rows at and past t_end are not stored
-  if constexpr (MODE == 3) {
-    if (static_cast<int>(blockIdx.y) >= __ldg(pl.g_ntiles)) return;       // the whole CTA, before any barrier exists
-    const int e = __ldg(pl.g_tiles + 2 * blockIdx.y);
-    t0 = __ldg(pl.g_tiles + 2 * blockIdx.y + 1);
-    t_end = __ldg(pl.g_offsets + e + 1);
-    wsrc = static_cast<const uint32_t*>(wsrc) + static_cast<long long>(e) * pl.g_words;
-    svh += static_cast<size_t>(e) * N;
-  }
-  const int slabs = (K + kSlabElems - 1) / kSlabElems;   // a ragged last slab only in the dense plain mode (TMA zero-fills X)
+  const int t0 = blockIdx.y * TN;            // first token of the tile
+  // this CTA's K slabs: all, or an even share where the CTAs of a cluster split K (a ragged last slab only in the dense plain
+  // mode: TMA zero-fills X)
+  const int ksplit = gridDim.z, krank = blockIdx.z;
+  const int slabs_all = (K + kSlabElems - 1) / kSlabElems;
+  const int slab0 = krank * slabs_all / ksplit, slabs = (krank + 1) * slabs_all / ksplit - slab0;
   constexpr uint32_t kTmemCols = TN < 32 ? 32 : TN;
   constexpr int kHalves = TN > 256 ? TN / 256 : 1;     // one MMA covers at most 256 token columns
   constexpr int kMmaN = TN > 256 ? 256 : TN;
@@ -177,7 +151,7 @@ TrellisGemmKernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
         ptx::MbarArriveExpectTx(&xfull[s], S::kXTileBytes);
 #pragma unroll
         for (int h = 0; h < kHalves; ++h)
-          ptx::TmaLoad2D(x_ring + s * S::kXTileBytes + h * (kMmaN * kSlabK * 2), &tmap_x, &xfull[s], it * kSlabElems, t0 + h * kMmaN);
+          ptx::TmaLoad2D(x_ring + s * S::kXTileBytes + h * (kMmaN * kSlabK * 2), &tmap_x, &xfull[s], (slab0 + it) * kSlabElems, t0 + h * kMmaN);
       }
     }
   } else if (warp == DW + 2) {
@@ -189,7 +163,7 @@ TrellisGemmKernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
         const int s = it % AST, round = it / AST;
         if (!ptx::MbarWait(&aempty[s], (round & 1) ^ 1, abort_flag, 5)) break;
         ptx::MbarArriveExpectTx(&afull[s], kATileBytes);
-        ptx::TmaLoad2D(a_ring + s * kATileBytes, &tmap_a, &afull[s], it * kSlabK, nb * 128);
+        ptx::TmaLoad2D(a_ring + s * kATileBytes, &tmap_a, &afull[s], (slab0 + it) * kSlabK, nb * 128);
       }
     }
     if (KB != 0 && lane == 0) {
@@ -204,27 +178,33 @@ TrellisGemmKernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
     }
   } else if (warp == DW + 1) {
     // ---------------- MMA issuer ----------------
-    if (lane == 0) {
+    // (one thread's instruction latencies add up: addresses and ring positions are counted up, not derived at each use)
+    if (ptx::ElectOne()) {
       const uint32_t idesc = MODE == 4 ? ptx::UmmaInstrDescE4m3(128, kMmaN) : ptx::UmmaInstrDescF16(128, kMmaN, MODE == 1 && pl.bf16 != 0);
+      const uint32_t xfull_at = ptx::SmemAddr(xfull), xempty_at = ptx::SmemAddr(xempty), afull_at = ptx::SmemAddr(afull), aempty_at = ptx::SmemAddr(aempty);
+      const uint64_t da0 = ptx::UmmaDescSw128(ptx::SmemAddr(a_ring)), db0 = ptx::UmmaDescSw128(ptx::SmemAddr(x_ring));      // (the address is the low field, in units of 16 bytes)
+      int sa = 0, sx = 0;
+      uint32_t pa = 0, px = 0, accumulate = 0;
       bool ok = true;
-      for (int it = 0; it < slabs && ok; ++it) {
-        const int sa = it % AST, ra = it / AST, sx = it % XST, rx = it / XST;
-        ok = ptx::MbarWait(&xfull[sx], rx & 1, abort_flag, 2) && ptx::MbarWait(&afull[sa], ra & 1, abort_flag, 3);
+      for (int it = 0; it < slabs; ++it) {
+        ok = ptx::MbarWaitAt(xfull_at + sx * 8, px, abort_flag, 2) && ptx::MbarWaitAt(afull_at + sa * 8, pa, abort_flag, 3);
         if (!ok) break;
         ptx::TcFenceAfter();
-        const uint32_t a_addr = ptx::SmemAddr(a_ring + sa * kATileBytes), b_addr = ptx::SmemAddr(x_ring + sx * S::kXTileBytes);
+        const uint64_t da = da0 + sa * (kATileBytes >> 4), db = db0 + sx * (S::kXTileBytes >> 4);
 #pragma unroll
         for (int h = 0; h < kHalves; ++h) {
 #pragma unroll
           for (int k = 0; k < kSlabK / 16; ++k) {
-            const uint64_t da = ptx::UmmaDescSw128(a_addr + k * 32);
-            const uint64_t db = ptx::UmmaDescSw128(b_addr + h * (kMmaN * kSlabK * 2) + k * 32);
-            if constexpr (MODE == 4) ptx::UmmaF8(tmem_base + h * kMmaN, da, db, idesc, (it > 0 || k > 0) ? 1u : 0u);
-            else ptx::UmmaF16(tmem_base + h * kMmaN, da, db, idesc, (it > 0 || k > 0) ? 1u : 0u);
+            const uint64_t dbk = db + h * (kMmaN * kSlabK * 2 >> 4) + k * 2;
+            if constexpr (MODE == 4) ptx::UmmaF8(tmem_base + h * kMmaN, da + k * 2, dbk, idesc, k > 0 ? 1u : accumulate);
+            else ptx::UmmaF16(tmem_base + h * kMmaN, da + k * 2, dbk, idesc, k > 0 ? 1u : accumulate);
           }
         }
-        ptx::UmmaCommit(&aempty[sa]);         // frees the A tile and the X tile once these MMAs have read them
-        ptx::UmmaCommit(&xempty[sx]);
+        accumulate = 1;
+        ptx::UmmaCommitAt(aempty_at + sa * 8);         // frees the A tile and the X tile once these MMAs have read them
+        ptx::UmmaCommitAt(xempty_at + sx * 8);
+        if (++sa == AST) { sa = 0; pa ^= 1u; }
+        if (++sx == XST) { sx = 0; px ^= 1u; }
       }
       if (ok) ptx::UmmaCommit(accum);         // accumulator complete
     }
@@ -248,7 +228,7 @@ TrellisGemmKernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
         for (int idx = warp; idx < 8; idx += DW) {
           const int r = idx * 16 + (lane >> 1), half = lane & 1;
           const size_t n = static_cast<size_t>(nb) * 128 + r;
-          const int kbase = it * kSlabK + half * 32;
+          const int kbase = (slab0 + it) * kSlabK + half * 32;
           const uint4* src = reinterpret_cast<const uint4*>(static_cast<const uint8_t*>(wsrc) + n * K + kbase);
           const uint4 q0 = __ldg(src), q1 = __ldg(src + 1);
           const __half sc = __ldg(reinterpret_cast<const __half*>(pl.wsz) + n * (K / pl.group) + kbase / pl.group);
@@ -274,7 +254,7 @@ TrellisGemmKernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
         for (int idx = warp; idx < 8; idx += DW) {
           const int r = idx * 16 + (lane >> 1), half = lane & 1;
           const size_t n = static_cast<size_t>(nb) * 128 + r;
-          const int kbase = it * kSlabK + half * 32;
+          const int kbase = (slab0 + it) * kSlabK + half * 32;
           const uint4 q = __ldg(reinterpret_cast<const uint4*>(static_cast<const uint32_t*>(wsrc) + n * (K / 8) + kbase / 8));
           const uint32_t sz = __ldg(pl.wsz + n * (K / pl.group) + kbase / pl.group);
           const uint32_t scb = (sz & 0xFFFFu) | (sz << 16), nzb = (sz >> 16) | (sz & 0xFFFF0000u);
@@ -336,7 +316,7 @@ TrellisGemmKernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
           packed.w = *reinterpret_cast<uint32_t*>(&w[3]);
         } else {
           const __half* dense = static_cast<const __half*>(wsrc);
-          const int n = nb * 128 + r, k = it * kSlabK + kt * 16 + khalf * 8;
+          const int n = nb * 128 + r, k = (slab0 + it) * kSlabK + kt * 16 + khalf * 8;
           if (MODE == 0 || (n < N && k < K))
             packed = __ldg(reinterpret_cast<const uint4*>(dense + static_cast<size_t>(n) * K + k));
           else
@@ -364,84 +344,98 @@ TrellisGemmKernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
     const int q = warp & 3, grp = warp >> 2;
     float* epi = reinterpret_cast<float*>(smem + grp * S::kEpiBytes);
     constexpr int CW = TN < 32 ? 16 : 32;   // columns per TMEM load
-    for (int c0 = grp * 32; c0 < TN; c0 += kGroups * 32) {
-      if (ok) {
-        uint32_t v[32];
-        if constexpr (CW == 32) {
-          ptx::TmemLoad32x32(tmem_base + (static_cast<uint32_t>(q * 32) << 16) + c0, v);
-        } else {
-          uint32_t v16[16];
-          ptx::TmemLoad32x16(tmem_base + (static_cast<uint32_t>(q * 32) << 16) + c0, v16);
-#pragma unroll
-          for (int i = 0; i < 16; ++i) v[i] = v16[i];
+    auto load_columns = [&](int c0, uint32_t (&v)[CW]) {
+      const uint32_t taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + c0;
+      if constexpr (CW == 32) ptx::TmemLoad32x32(taddr, v);
+      else ptx::TmemLoad32x16(taddr, v);
+      ptx::TmemLoadWait();
+    };
+    // four outputs of token t out of their sums
+    auto finish = [&](int t, float (&f)[4]) {
+      const int n = nb * 128 + lane * 4;
+      if (MODE == 1 && n >= N) return;
+      float o0, o1, o2, o3;
+      if constexpr (MODE == 0 || MODE == 4) {
+        if constexpr (MODE == 4) {
+          const float xs = __ldg(pl.x_scale + t);               // the row's activation scale
+          f[0] *= xs; f[1] *= xs; f[2] *= xs; f[3] *= xs;
         }
-        ptx::TmemLoadWait();
-#pragma unroll
-        for (int c = 0; c < CW; ++c) epi[c * S::kEpiStride + q * 32 + lane] = __uint_as_float(v[c]);
+        WarpFwht128(f);
+        const uint2 sv = *reinterpret_cast<const uint2*>(svh + n);
+        const __half2 s01 = *reinterpret_cast<const __half2*>(&sv.x), s23 = *reinterpret_cast<const __half2*>(&sv.y);
+        o0 = f[0] * inv_sqrt * __low2float(s01); o1 = f[1] * inv_sqrt * __high2float(s01);
+        o2 = f[2] * inv_sqrt * __low2float(s23); o3 = f[3] * inv_sqrt * __high2float(s23);
+      } else {
+        o0 = f[0]; o1 = f[1]; o2 = f[2]; o3 = f[3];
+        if (pl.bias != nullptr) {
+          const uint2 bv = *reinterpret_cast<const uint2*>(pl.bias + n);
+          o0 += BfLo(bv.x); o1 += BfHi(bv.x); o2 += BfLo(bv.y); o3 += BfHi(bv.y);
+        }
+        if (pl.act == 1) {
+          o0 = GeluTanh(o0); o1 = GeluTanh(o1); o2 = GeluTanh(o2); o3 = GeluTanh(o3);
+        } else if (pl.act == 2) {
+          o0 = GeluErf(o0); o1 = GeluErf(o1); o2 = GeluErf(o2); o3 = GeluErf(o3);
+        }
       }
-      asm volatile("bar.sync %0, 128;" ::"r"(1 + grp) : "memory");
-      if (ok) {
-        for (int c = q; c < CW; c += 4) {
-          const int t = t0 + c0 + c;
-          if (t < t_end && (MODE != 1 || nb * 128 + lane * 4 < N)) {
-            const float4 p = *reinterpret_cast<const float4*>(epi + c * S::kEpiStride + lane * 4);
-            float f[4] = {p.x, p.y, p.z, p.w};
-            const int n = nb * 128 + lane * 4;
-            float o0, o1, o2, o3;
-            if constexpr (MODE == 0 || MODE == 3 || MODE == 4) {
-              if constexpr (MODE == 4) {
-                const float xs = __ldg(pl.x_scale + t);               // the row's activation scale
-                f[0] *= xs; f[1] *= xs; f[2] *= xs; f[3] *= xs;
-              }
-              WarpFwht128(f);
-              const uint2 sv = *reinterpret_cast<const uint2*>(svh + n);
-              const __half2 s01 = *reinterpret_cast<const __half2*>(&sv.x), s23 = *reinterpret_cast<const __half2*>(&sv.y);
-              o0 = f[0] * inv_sqrt * __low2float(s01); o1 = f[1] * inv_sqrt * __high2float(s01);
-              o2 = f[2] * inv_sqrt * __low2float(s23); o3 = f[3] * inv_sqrt * __high2float(s23);
-            } else {
-              o0 = f[0]; o1 = f[1]; o2 = f[2]; o3 = f[3];
-              if (pl.bias != nullptr) {
-                const uint2 bv = *reinterpret_cast<const uint2*>(pl.bias + n);
-                o0 += BfLo(bv.x); o1 += BfHi(bv.x); o2 += BfLo(bv.y); o3 += BfHi(bv.y);
-              }
-              if (pl.act == 1) {
-                o0 = GeluTanh(o0); o1 = GeluTanh(o1); o2 = GeluTanh(o2); o3 = GeluTanh(o3);
-              } else if (pl.act == 2) {
-                o0 = GeluErf(o0); o1 = GeluErf(o1); o2 = GeluErf(o2); o3 = GeluErf(o3);
-              }
-            }
-            if (residual != nullptr) {
-              const uint2 rv = *reinterpret_cast<const uint2*>(residual + static_cast<size_t>(t) * N + n);
-              o0 += BfLo(rv.x); o1 += BfHi(rv.x); o2 += BfLo(rv.y); o3 += BfHi(rv.y);
-            }
-            uint2 ov;
-            ov.x = PackBf16(o0, o1);
-            ov.y = PackBf16(o2, o3);
-            if ((MODE == 1 || MODE == 2 || MODE == 5) && pl.out_f32) {
-              *reinterpret_cast<float4*>(reinterpret_cast<float*>(y) + static_cast<size_t>(t) * N + n) = make_float4(o0, o1, o2, o3);
-            } else if (rs.world > 0) {
-              const int owner = t / rs.rows_per_rank, tl = t - owner * rs.rows_per_rank;
-              *reinterpret_cast<uint2*>(rs.recv[owner] + (static_cast<size_t>(rs.rank) * rs.rows_per_rank + tl) * N + n) = ov;
-            } else if (MODE == 3) {
-              *reinterpret_cast<uint2*>(y + static_cast<size_t>(__ldg(pl.g_perm + t)) * N + n) = ov;
-            } else {
-              *reinterpret_cast<uint2*>(y + static_cast<size_t>(t) * N + n) = ov;
+      if (residual != nullptr) {
+        const uint2 rv = *reinterpret_cast<const uint2*>(residual + static_cast<size_t>(t) * N + n);
+        o0 += BfLo(rv.x); o1 += BfHi(rv.x); o2 += BfLo(rv.y); o3 += BfHi(rv.y);
+      }
+      if ((MODE == 1 || MODE == 2 || MODE == 5) && pl.out_f32)
+        *reinterpret_cast<float4*>(reinterpret_cast<float*>(y) + static_cast<size_t>(t) * N + n) = make_float4(o0, o1, o2, o3);
+      else
+        *reinterpret_cast<uint2*>(y + static_cast<size_t>(t) * N + n) = make_uint2(PackBf16(o0, o1), PackBf16(o2, o3));
+    };
+    if (S::kSplits && ksplit > 1) {
+      // K was split: the CTAs of the cluster lay their sums side by side in shared memory, and each finishes its share of the
+      // tokens, adding up over distributed shared memory in rank order
+      const int tile_end = min(TN, T - t0);
+      float* sums = reinterpret_cast<float*>(smem);
+      const uint32_t sums_at = ptx::SmemAddr(sums);
+      for (int c0 = grp * CW; c0 < tile_end; c0 += kGroups * CW) {
+        uint32_t v[CW];
+        if (ok) load_columns(c0, v);
+#pragma unroll
+        for (int c = 0; c < CW; ++c)         // (a wait that ran out shows as NaN)
+          sums[(c0 + c) * S::kEpiStride + q * 32 + lane] = ok ? __uint_as_float(v[c]) : __int_as_float(0x7FC00000);
+      }
+      ptx::ClusterSync();
+      for (int c = warp * ksplit + krank; c < tile_end; c += DW * ksplit) {
+        float f[4] = {0.f, 0.f, 0.f, 0.f};
+        for (int r = 0; r < ksplit; ++r) {
+          const float4 p = ptx::LoadRemote4(sums_at + (c * S::kEpiStride + lane * 4) * 4, r);
+          f[0] += p.x; f[1] += p.y; f[2] += p.z; f[3] += p.w;
+        }
+        finish(t0 + c, f);
+      }
+      ptx::ClusterSync();
+    } else {
+      for (int c0 = grp * 32; c0 < TN; c0 += kGroups * 32) {
+        if (ok) {
+          uint32_t v[CW];
+          load_columns(c0, v);
+#pragma unroll
+          for (int c = 0; c < CW; ++c) epi[c * S::kEpiStride + q * 32 + lane] = __uint_as_float(v[c]);
+        }
+        asm volatile("bar.sync %0, 128;" ::"r"(1 + grp) : "memory");
+        if (ok) {
+          for (int c = q; c < CW; c += 4) {
+            const int t = t0 + c0 + c;
+            if (t < T) {
+              const float4 p = *reinterpret_cast<const float4*>(epi + c * S::kEpiStride + lane * 4);
+              float f[4] = {p.x, p.y, p.z, p.w};
+              finish(t, f);
             }
           }
         }
-      }
-      asm volatile("bar.sync %0, 128;" ::"r"(1 + grp) : "memory");
-    }
-    if (rs.world > 0) {
-      // every partial row of this tile is on its way: publish them, then count this CTA in at each owner it wrote to
-      // (also when a wait ran out: the peers must not wait for a CTA that gave up; the status word tells the host)
-      __threadfence_system();
-      asm volatile("bar.sync 6, %0;" ::"r"(DW * 32) : "memory");
-      if (threadIdx.x == 0) {
-        const int t_last = min(t0 + TN, T) - 1;
-        for (int o = t0 / rs.rows_per_rank; o <= t_last / rs.rows_per_rank; ++o) atomicAdd_system(rs.cnt[o], 1u);
+        asm volatile("bar.sync %0, 128;" ::"r"(1 + grp) : "memory");
       }
     }
+  }
+  if (S::kSplits && warp >= DW && ksplit > 1) {
+    __syncwarp();
+    ptx::ClusterSync();                      // the other warps take part in the cluster's barriers
+    ptx::ClusterSync();
   }
 
   // ---------------- teardown ----------------
@@ -665,11 +659,10 @@ bool Aligned16(const void* a, const void* b, const void* c) {
 }
 
 int g_decode_warps = 16;
-int g_grouped_decode_warps = 0;      // 0: by tile size
 
 template <int KB, int TN, int DW, int MODE = 0>
 int LaunchGemm(const void* wsrc, const void* svh, const void* xh, void* y, const void* residual, int T, int N, int K,
-               int* status, cudaStream_t stream, const RsArgs& rs, const PlainArgs& pl = PlainArgs{}) {
+               int* status, cudaStream_t stream, const PlainArgs& pl, int ksplit = 1) {
   using S = GemmSmem<KB, TN, MODE == 4>;
   static_assert(S::kTotal <= 227 * 1024, "shared memory budget");
   static_assert(S::kBars * 8 + 16 <= 512, "barrier block");
@@ -686,80 +679,60 @@ int LaunchGemm(const void* wsrc, const void* svh, const void* xh, void* y, const
   auto kern = TrellisGemmKernel<KB, TN, DW, MODE>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, S::kTotal);
   if (e != cudaSuccess) return static_cast<int>(e);
-  dim3 grid((N + 127) / 128, MODE == 3 ? pl.g_max_tiles : (T + TN - 1) / TN);
-  kern<<<grid, (DW + 3) * 32, S::kTotal, stream>>>(tmap, tmap_a, wsrc, static_cast<const __half*>(svh),
-                                                   static_cast<__nv_bfloat16*>(y),
-                                                   static_cast<const __nv_bfloat16*>(residual), T, N, K, status, rs, pl);
-  return FinishLaunch();
-}
-
-template <int KB>
-int LaunchGrouped(const void* w, const void* svh, const void* xh, void* y, int P, int N, int K, int tn, int* status,
-                  cudaStream_t s, const PlainArgs& pl) {
-  const RsArgs rs = {};
-  // measured on the 512-expert block: 1745 -> 1308 us at 2048 rows (tile 64), but 4178 -> 4519 us at 8192 rows (tile 128)
-  const int dw = g_grouped_decode_warps ? g_grouped_decode_warps : (tn <= 64 ? 8 : 16);
-  if (dw == 8) {
-    // eight decode warps: 352 threads per CTA, so two CTAs share an SM and one tile's prologue and epilogue overlap the
-    // other's main loop (an expert tile has little K: the fixed part of a CTA is most of its time)
-    switch (tn) {
-      case 16: return LaunchGemm<KB, 16, 8, 3>(w, svh, xh, y, nullptr, P, N, K, status, s, rs, pl);
-      case 32: return LaunchGemm<KB, 32, 8, 3>(w, svh, xh, y, nullptr, P, N, K, status, s, rs, pl);
-      case 64: return LaunchGemm<KB, 64, 8, 3>(w, svh, xh, y, nullptr, P, N, K, status, s, rs, pl);
-      case 128: return LaunchGemm<KB, 128, 8, 3>(w, svh, xh, y, nullptr, P, N, K, status, s, rs, pl);
-      default: return R4DXB_BAD_ARG;
-    }
-  }
-  switch (tn) {
-    case 16: return LaunchGemm<KB, 16, 16, 3>(w, svh, xh, y, nullptr, P, N, K, status, s, rs, pl);
-    case 32: return LaunchGemm<KB, 32, 16, 3>(w, svh, xh, y, nullptr, P, N, K, status, s, rs, pl);
-    case 64: return LaunchGemm<KB, 64, 16, 3>(w, svh, xh, y, nullptr, P, N, K, status, s, rs, pl);
-    case 128: return LaunchGemm<KB, 128, 16, 3>(w, svh, xh, y, nullptr, P, N, K, status, s, rs, pl);
-    case 256: return LaunchGemm<KB, 256, 16, 3>(w, svh, xh, y, nullptr, P, N, K, status, s, rs, pl);
-    default: return R4DXB_BAD_ARG;
-  }
+  if (ksplit > 1 && !S::kSplits) return R4DXB_BAD_ARG;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((N + 127) / 128, (T + TN - 1) / TN, ksplit);
+  cfg.blockDim = dim3((DW + 3) * 32, 1, 1);
+  cfg.dynamicSmemBytes = S::kTotal;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 1;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = ksplit;
+  cfg.attrs = attr;
+  cfg.numAttrs = ksplit > 1 ? 1 : 0;
+  e = cudaLaunchKernelEx(&cfg, kern, tmap, tmap_a, wsrc, static_cast<const __half*>(svh), static_cast<__nv_bfloat16*>(y),
+                         static_cast<const __nv_bfloat16*>(residual), T, N, K, status, pl);
+  ++g_launch_count;
+  return static_cast<int>(e);
 }
 
 template <int MODE>
-int LaunchPlain(const void* w, const void* xh, void* y, const void* residual, int T, int N, int K, int tn, int* status,
+int LaunchPlain(const void* w, const void* xh, void* y, const void* residual, int T, int N, int K, int tn, int ksplit, int* status,
                 cudaStream_t s, const PlainArgs& pl) {
-  const RsArgs rs = {};
   switch (tn) {
-    case 16: return LaunchGemm<0, 16, 8, MODE>(w, nullptr, xh, y, residual, T, N, K, status, s, rs, pl);
-    case 32: return LaunchGemm<0, 32, 8, MODE>(w, nullptr, xh, y, residual, T, N, K, status, s, rs, pl);
-    case 64: return LaunchGemm<0, 64, 8, MODE>(w, nullptr, xh, y, residual, T, N, K, status, s, rs, pl);
-    case 128: return LaunchGemm<0, 128, 8, MODE>(w, nullptr, xh, y, residual, T, N, K, status, s, rs, pl);
-    case 256: return LaunchGemm<0, 256, 8, MODE>(w, nullptr, xh, y, residual, T, N, K, status, s, rs, pl);
-    case 512: return LaunchGemm<0, 512, 8, MODE>(w, nullptr, xh, y, residual, T, N, K, status, s, rs, pl);
+    case 16: return LaunchGemm<0, 16, 8, MODE>(w, nullptr, xh, y, residual, T, N, K, status, s, pl, ksplit);
+    case 32: return LaunchGemm<0, 32, 8, MODE>(w, nullptr, xh, y, residual, T, N, K, status, s, pl, ksplit);
+    case 64: return LaunchGemm<0, 64, 8, MODE>(w, nullptr, xh, y, residual, T, N, K, status, s, pl, ksplit);
+    case 128: return LaunchGemm<0, 128, 8, MODE>(w, nullptr, xh, y, residual, T, N, K, status, s, pl, ksplit);
+    case 256: return LaunchGemm<0, 256, 8, MODE>(w, nullptr, xh, y, residual, T, N, K, status, s, pl, ksplit);
+    case 512: return LaunchGemm<0, 512, 8, MODE>(w, nullptr, xh, y, residual, T, N, K, status, s, pl, ksplit);
     default: return R4DXB_BAD_ARG;
   }
 }
 
-template <int KB, int DW>
-int LaunchGemmTN(const void* wsrc, const void* svh, const void* xh, void* y, const void* residual, int T, int N, int K,
-                 int tn, int* status, cudaStream_t s, const RsArgs& rs) {
+template <int DW>
+int LaunchDense(const void* w, const void* svh, const void* xh, void* y, const void* residual, int T, int N, int K, int tn,
+                int* status, cudaStream_t s) {
+  const PlainArgs pl = {};
   switch (tn) {
-    case 16: return LaunchGemm<KB, 16, DW>(wsrc, svh, xh, y, residual, T, N, K, status, s, rs);
-    case 32: return LaunchGemm<KB, 32, DW>(wsrc, svh, xh, y, residual, T, N, K, status, s, rs);
-    case 64: return LaunchGemm<KB, 64, DW>(wsrc, svh, xh, y, residual, T, N, K, status, s, rs);
-    case 128: return LaunchGemm<KB, 128, DW>(wsrc, svh, xh, y, residual, T, N, K, status, s, rs);
-    case 256: return LaunchGemm<KB, 256, DW>(wsrc, svh, xh, y, residual, T, N, K, status, s, rs);
-    case 512: return LaunchGemm<KB, 512, DW>(wsrc, svh, xh, y, residual, T, N, K, status, s, rs);
+    case 16: return LaunchGemm<0, 16, DW>(w, svh, xh, y, residual, T, N, K, status, s, pl);
+    case 32: return LaunchGemm<0, 32, DW>(w, svh, xh, y, residual, T, N, K, status, s, pl);
+    case 64: return LaunchGemm<0, 64, DW>(w, svh, xh, y, residual, T, N, K, status, s, pl);
+    case 128: return LaunchGemm<0, 128, DW>(w, svh, xh, y, residual, T, N, K, status, s, pl);
+    case 256: return LaunchGemm<0, 256, DW>(w, svh, xh, y, residual, T, N, K, status, s, pl);
+    case 512: return LaunchGemm<0, 512, DW>(w, svh, xh, y, residual, T, N, K, status, s, pl);
     default: return R4DXB_BAD_ARG;
-  }
-}
-
-template <int KB>
-int LaunchGemmDW(const void* wsrc, const void* svh, const void* xh, void* y, const void* residual, int T, int N, int K,
-                 int tn, int* status, cudaStream_t s, const RsArgs& rs) {
-  switch (g_decode_warps) {
-    case 4: return LaunchGemmTN<KB, 4>(wsrc, svh, xh, y, residual, T, N, K, tn, status, s, rs);
-    case 8: return LaunchGemmTN<KB, 8>(wsrc, svh, xh, y, residual, T, N, K, tn, status, s, rs);
-    default: return LaunchGemmTN<KB, 16>(wsrc, svh, xh, y, residual, T, N, K, tn, status, s, rs);
   }
 }
 
 }  // namespace
+
+int TrellisProduct(const void* w, const void* svh, const void* xh, void* y, const void* residual, int T, int N, int K, int kb, int tn,
+                   int ksplit, int* status, cudaStream_t s);         // trellis_product.cu
+extern int g_grouped_decode_warps;
+
 }  // namespace r4dxb
 
 using namespace r4dxb;
@@ -782,7 +755,8 @@ int r4dxb_trellis_input(const void* in, const void* suh, void* out, int T, int K
  * matrix (svh still applies; pass ones and set hadamard-free weights accordingly); kb in {3,4,5}: packed
  * trellis words.  tn = token tile (16/32/64/128/256/512).  status: device int, set non-zero if a bounded wait
  * inside the kernel ran out. */
-/* decode warps per CTA of the tensor-core GEMM (4, 8 or 16): a tuning and A/B-measurement switch */
+/* decode warps per CTA of the dense Hadamard mode (4, 8 or 16) and of the grouped trellis product (8 or 16, 4: by tile size): a
+ * tuning and A/B-measurement switch */
 void r4dxb_set_gemm_decode_warps(int n) {
   g_decode_warps = (n == 4 || n == 8) ? n : 16;
   g_grouped_decode_warps = n == 8 ? 8 : (n == 16 ? 16 : 0);
@@ -790,15 +764,21 @@ void r4dxb_set_gemm_decode_warps(int n) {
 
 int r4dxb_trellis_gemm(const void* w, const void* svh, const void* xh, void* y, const void* residual, int T, int N, int K,
                        int kb, int tn, int* status, void* stream) {
-  if (T < 1 || N % 128 || K % 128) return R4DXB_BAD_ARG;
+  return r4dxb_trellis_gemm_split(w, svh, xh, y, residual, T, N, K, kb, tn, 1, status, stream);
+}
+
+/* The same with K split over the `ksplit` (1..8, trellis weights only) CTAs of a cluster, which add up in rank order; 192 and 384
+ * are token tiles of a trellis product as well. */
+int r4dxb_trellis_gemm_split(const void* w, const void* svh, const void* xh, void* y, const void* residual, int T, int N, int K,
+                             int kb, int tn, int ksplit, int* status, void* stream) {
+  if (T < 1 || N % 128 || K % 128 || ksplit < 1 || ksplit > 8 || K / 128 < ksplit) return R4DXB_BAD_ARG;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  RsArgs rs = {};
-  switch (kb) {
-    case 0: return LaunchGemmDW<0>(w, svh, xh, y, residual, T, N, K, tn, status, s, rs);
-    case 3: return LaunchGemmDW<3>(w, svh, xh, y, residual, T, N, K, tn, status, s, rs);
-    case 4: return LaunchGemmDW<4>(w, svh, xh, y, residual, T, N, K, tn, status, s, rs);
-    case 5: return LaunchGemmDW<5>(w, svh, xh, y, residual, T, N, K, tn, status, s, rs);
-    default: return R4DXB_BAD_ARG;
+  if (kb != 0) return TrellisProduct(w, svh, xh, y, residual, T, N, K, kb, tn, ksplit, status, s);
+  if (ksplit > 1) return R4DXB_BAD_ARG;
+  switch (g_decode_warps) {
+    case 4: return LaunchDense<4>(w, svh, xh, y, residual, T, N, K, tn, status, s);
+    case 8: return LaunchDense<8>(w, svh, xh, y, residual, T, N, K, tn, status, s);
+    default: return LaunchDense<16>(w, svh, xh, y, residual, T, N, K, tn, status, s);
   }
 }
 
@@ -809,7 +789,13 @@ int r4dxb_trellis_gemm(const void* w, const void* svh, const void* xh, void* y, 
  * out_f32: y is fp32 instead of bf16.  act (low byte of out_f32 >> 8): 0 none, 1 tanh-GELU, 2 erf-GELU after the bias. */
 int r4dxb_linear_tc(const void* w, const void* wsz, int kind, int group, int bf16, const void* x, void* y, int out_f32,
                     const void* bias, const void* residual, int T, int N, int K, int tn, int* status, void* stream) {
-  if (T < 1 || N < 4 || K < 8 || kind < 0 || kind > 2) return R4DXB_BAD_ARG;
+  return r4dxb_linear_tc_split(w, wsz, kind, group, bf16, x, y, out_f32, bias, residual, T, N, K, tn, 1, status, stream);
+}
+
+/* The same with K split over the `ksplit` (1..8, tiles up to 256) CTAs of a cluster, which add up in rank order. */
+int r4dxb_linear_tc_split(const void* w, const void* wsz, int kind, int group, int bf16, const void* x, void* y, int out_f32,
+                          const void* bias, const void* residual, int T, int N, int K, int tn, int ksplit, int* status, void* stream) {
+  if (T < 1 || N < 4 || K < 8 || kind < 0 || kind > 2 || ksplit < 1 || ksplit > 8 || (K + 63) / 64 < ksplit) return R4DXB_BAD_ARG;
   if (kind == 0 && (N % 4 || K % 8)) return R4DXB_BAD_ARG;
   if (kind >= 1 && (N % 128 || K % 128 || wsz == nullptr || (group != 32 && group != 64 && group != 128) || bf16))
     return R4DXB_BAD_ARG;
@@ -821,9 +807,9 @@ int r4dxb_linear_tc(const void* w, const void* wsz, int kind, int group, int bf1
   pl.out_f32 = out_f32 & 1;
   pl.act = (out_f32 >> 8) & 0xFF;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (kind == 2) return LaunchPlain<5>(w, x, y, residual, T, N, K, tn, status, s, pl);
-  return kind == 0 ? LaunchPlain<1>(w, x, y, residual, T, N, K, tn, status, s, pl)
-                   : LaunchPlain<2>(w, x, y, residual, T, N, K, tn, status, s, pl);
+  if (kind == 2) return LaunchPlain<5>(w, x, y, residual, T, N, K, tn, ksplit, status, s, pl);
+  return kind == 0 ? LaunchPlain<1>(w, x, y, residual, T, N, K, tn, ksplit, status, s, pl)
+                   : LaunchPlain<2>(w, x, y, residual, T, N, K, tn, ksplit, status, s, pl);
 }
 
 /* 8-bit prefill product: rows of fp16 transformed activations -> e4m3 rows + one fp32 scale per row, then the trellis GEMM
@@ -838,11 +824,10 @@ int r4dxb_quantize_rows_e4m3(const void* xh, void* xq, float* scale, int T, int 
 int r4dxb_trellis_gemm_f8(const void* w, const void* svh, const void* xq, const float* x_scale, void* y, const void* residual,
                           int T, int N, int K, int kb, int tn, int* status, void* stream) {
   if (T < 1 || N % 128 || K % 128 || x_scale == nullptr) return R4DXB_BAD_ARG;
-  const RsArgs rs = {};
   PlainArgs pl = {};
   pl.x_scale = x_scale;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-#define R4DXB_F8(KBV, TNV) if (kb == KBV && tn == TNV) return LaunchGemm<KBV, TNV, 16, 4>(w, svh, xq, y, residual, T, N, K, status, s, rs, pl);
+#define R4DXB_F8(KBV, TNV) if (kb == KBV && tn == TNV) return LaunchGemm<KBV, TNV, 16, 4>(w, svh, xq, y, residual, T, N, K, status, s, pl);
   R4DXB_F8(3, 128) R4DXB_F8(3, 256) R4DXB_F8(3, 512) R4DXB_F8(4, 128) R4DXB_F8(4, 256) R4DXB_F8(4, 512)
   R4DXB_F8(5, 128) R4DXB_F8(5, 256) R4DXB_F8(5, 512)
 #undef R4DXB_F8
@@ -852,7 +837,7 @@ int r4dxb_trellis_gemm_f8(const void* w, const void* svh, const void* xq, const 
 /* Grouped experts on the tensor cores (prefill and wide batches of the mixture-of-experts block).
  * r4dxb_moe_tiles: tile list of the routing plan for token tiles of tn rows (E <= 1024 local experts).
  * r4dxb_trellis_input_grouped: xh[p] = fp16(H128(suh[e(p)] * act(in[perm[p] / xdiv]))) for the planned pairs in expert order.
- * r4dxb_trellis_gemm_grouped: y[perm[p]] = svh[e] * H128(xh[p] Q_e^T); max_tiles >= P / tn + E bounds the grid. */
+ * (the product itself: trellis_product.cu). */
 int r4dxb_moe_tiles(const int* offsets, int E, int tn, int* tiles, int* ntiles, int max_tiles, void* stream) {
   if (E < 1 || E > 1024 || tn < 1 || max_tiles < 1) return R4DXB_BAD_ARG;
   MoeTilesKernel<<<1, 1024, 0, static_cast<cudaStream_t>(stream)>>>(offsets, E, tn, tiles, ntiles, max_tiles);
@@ -867,49 +852,6 @@ int r4dxb_trellis_input_grouped(const void* in, const void* suh, void* out, cons
       static_cast<const __nv_bfloat16*>(in), static_cast<const __half*>(suh), static_cast<__half*>(out), offsets, perm, E, P, K, xdiv, mode,
       Aligned16(in, suh, out));
   return FinishLaunch();
-}
-
-int r4dxb_trellis_gemm_grouped(const void* words, const void* svh, const void* xh, void* y, const int* offsets, const int* perm,
-                               const int* tiles, const int* ntiles, int max_tiles, int P, int E, int N, int K, int kb, int tn,
-                               int* status, void* stream) {
-  if (P < 1 || E < 1 || N % 128 || K % 128 || max_tiles < 1 || max_tiles > 65535) return R4DXB_BAD_ARG;
-  PlainArgs pl = {};
-  pl.g_offsets = offsets;
-  pl.g_perm = perm;
-  pl.g_tiles = tiles;
-  pl.g_ntiles = ntiles;
-  pl.g_words = static_cast<long long>(N / 16) * (K / 16) * 8 * kb;
-  pl.g_max_tiles = max_tiles;
-  cudaStream_t s = static_cast<cudaStream_t>(stream);
-  switch (kb) {
-    case 3: return LaunchGrouped<3>(words, svh, xh, y, P, N, K, tn, status, s, pl);
-    case 4: return LaunchGrouped<4>(words, svh, xh, y, P, N, K, tn, status, s, pl);
-    case 5: return LaunchGrouped<5>(words, svh, xh, y, P, N, K, tn, status, s, pl);
-    default: return R4DXB_BAD_ARG;
-  }
-}
-
-/* Row-parallel product with the reduce-scatter in its epilogue: partial row t goes to rank t / rows_per_rank, into
- * recv[owner] + (rank * rows_per_rank + t % rows_per_rank) * N (bf16), and every CTA adds 1 to cnt[owner] for each
- * owner its token tile touches, after its rows are visible at system scope.  recv / cnt: `world` peer-mapped pointers. */
-int r4dxb_trellis_gemm_rs(const void* w, const void* svh, const void* xh, int T, int N, int K, int kb, int tn, int* status,
-                          void* const* recv, void* const* cnt, int world, int rank, int rows_per_rank, void* stream) {
-  if (T < 1 || N % 128 || K % 128 || world < 2 || world > 8 || rank < 0 || rank >= world || rows_per_rank < 1 ||
-      static_cast<long long>(rows_per_rank) * world < T)
-    return R4DXB_BAD_ARG;
-  cudaStream_t s = static_cast<cudaStream_t>(stream);
-  RsArgs rs = {};
-  for (int p = 0; p < world; ++p) {
-    rs.recv[p] = static_cast<__nv_bfloat16*>(recv[p]);
-    rs.cnt[p] = static_cast<unsigned*>(cnt[p]);
-  }
-  rs.world = world; rs.rank = rank; rs.rows_per_rank = rows_per_rank;
-  switch (kb) {
-    case 3: return LaunchGemmDW<3>(w, svh, xh, nullptr, nullptr, T, N, K, tn, status, s, rs);
-    case 4: return LaunchGemmDW<4>(w, svh, xh, nullptr, nullptr, T, N, K, tn, status, s, rs);
-    case 5: return LaunchGemmDW<5>(w, svh, xh, nullptr, nullptr, T, N, K, tn, status, s, rs);
-    default: return R4DXB_BAD_ARG;
-  }
 }
 
 }  // extern "C"

@@ -117,6 +117,8 @@ const R4dxbKernelInfo kKernels[] = {
      "K multiple of 128", "bf16 in, fp16 out", "simt", c6, 1},
     {"trellis_gemm", "gemm", "trellis_linear_rows_ge_16", "prefill product on tcgen05 with the output Hadamard in the epilogue",
      "token tiles 16..512", "fp16 xh (TMA), packed trellis words, bf16 y", "tcgen05", c7, 4},
+    {"trellis_gemm_split", "gemm", "trellis_linear_rows_ge_16_split_k", "the same product with K shared by the 1..8 CTAs of a cluster",
+     "token tiles 16..512", "fp16 xh (TMA), packed trellis words, bf16 y", "tcgen05", c7, 4},
     {"trellis_gemm_f8", "gemm", "trellis_linear_rows_ge_16_8bit", "the same product with e4m3 code values and e4m3 activations (one scale per row), kind::f8f6f4",
      "token tiles 128/256/512", "e4m3 xq + fp32 row scales, bf16 y", "tcgen05", c8, 4},
     {"quantize_rows_e4m3", "quant", "activation_quantizer", "fp16 rows -> e4m3 rows + one fp32 scale per row",
@@ -138,6 +140,8 @@ const R4dxbKernelInfo kKernels[] = {
     {"moe_tiles", "moe", "moe_tile_list", "token tiles of a routing plan built on the device",
      "E <= 1024", "int32", "simt", c17, 1},
     {"linear_tc", "gemm", "plain_linear_rows_any", "y = act(x W^T + bias) + residual: dense bf16 / fp16 W by TMA, or w4a16 W widened by the decode warps",
+     "dense: N % 4, K % 8; w4a16: N, K % 128, group 32/64/128", "bf16 / fp16 / w4a16, bf16 or fp32 y", "tcgen05", c18, 2},
+    {"linear_tc_split", "gemm", "plain_linear_rows_any_split_k", "the same linear with K shared by the 1..8 CTAs of a cluster (tiles up to 256)",
      "dense: N % 4, K % 8; w4a16: N, K % 128, group 32/64/128", "bf16 / fp16 / w4a16, bf16 or fp32 y", "tcgen05", c18, 2},
     {"w4a16_gemv", "gemm", "w4a16_linear_rows_le_8", "group-quantised 4-bit head product",
      "rows * K * 2 <= 200 KB; mma.sync where N % 16 and K % (4 group) are 0, else CUDA cores", "bf16 x, nibbles + fp16 scale / zero", "mma.sync+simt", c19, 2},

@@ -455,6 +455,7 @@ def attn_decode(q, qg, cache, block_table, positions, k_descale, v_descale, part
 
 register_cuda_sig("r4dxb_trellis_input", _I, [_P, _P, _P, _I, _I, _I, _P])
 register_cuda_sig("r4dxb_trellis_gemm", _I, [_P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _P, _P])
+register_cuda_sig("r4dxb_trellis_gemm_split", _I, [_P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _P, _P])
 
 def trellis_input(x: torch.Tensor, suh: torch.Tensor, out: Optional[torch.Tensor] = None, fused_silu_mul: bool = False,
                   gelu: bool = False) -> torch.Tensor:
@@ -468,11 +469,11 @@ def trellis_input(x: torch.Tensor, suh: torch.Tensor, out: Optional[torch.Tensor
     return out
 
 
-_TILE_COST = {128: 0.60, 256: 0.62, 512: 1.0}   # relative time of one CTA's K loop (decode-bound below 512 columns)
+_TILE_COST = {128: 0.60, 256: 0.62, 512: 1.0}   # relative time of one CTA's K loop
 
 
 def pick_token_tile(T: int, N: int = 0, K: int = 0) -> int:
-    """Token-tile width of the tensor-core GEMM: the smallest tile that covers T below 512 rows; above,
+    """Token-tile width of the plain and 8-bit tensor-core products and of the reduce-scatter: the smallest tile that covers T below 512 rows; above,
     the width whose CTA count wastes the fewest of the 148 SMs' waves (one CTA per SM)."""
     for tn in (16, 32, 64, 128):
         if T <= tn:
@@ -493,15 +494,53 @@ def pick_token_tile(T: int, N: int = 0, K: int = 0) -> int:
     return best
 
 
+# us that a CTA of the trellis product takes per 64 columns of K, by token tile: of one CTA (up to 128 tokens the decode warps, above
+# the X stream bounds it) and of a CTA of a pair, which loads half of the tile.  Fitted to 34816 / 16384 / 5120 outputs at 16 to
+# 8192 tokens.
+_SLAB_US = {16: 0.31, 32: 0.33, 64: 0.35, 128: 0.37, 192: 0.46, 256: 0.50, 384: 0.75, 512: 0.90}
+_SLAB_US_PAIR = {256: 0.46, 384: 0.62, 512: 0.74}
+# CTAs that run at a time, by cluster size (one CTA per SM; large clusters fit badly into the chip's SM groups)
+_CLUSTER_SLOTS = {1: 148, 2: 148, 3: 144, 4: 136, 6: 126, 8: 112}
+
+
+@functools.lru_cache(maxsize=None)
+def pick_product(T: int, N: int, K: int) -> tuple:
+    """(token tile, split of K) of the trellis product: the fewest us by waves of CTAs, each with a fixed part (start, first loads,
+    epilogue) and its share of K.  Short N and few tokens leave SMs idle without a split: 5120 x 17408 at 16 tokens 98 us with one
+    CTA per row block and 44 with three (145 with the kernel before), at 333 tokens 139 and 72 (170)."""
+    hit = TUNING.get(("gemm", str(N), str(K), str(T)))
+    if hit is not None:
+        return hit, 1
+    blocks, slabs = N // 128, K // 64
+    best, best_cost = (16, 1), None
+    for tn in _SLAB_US:
+        if tn > 16 and tn >= 2 * T and T <= 256:
+            continue                         # (a smaller tile holds all rows)
+        pair = tn in _SLAB_US_PAIR and blocks % 2 == 0
+        c = _SLAB_US_PAIR[tn] if pair else _SLAB_US[tn]
+        for ks in (1, 2, 3, 4) if pair else (1, 2, 3, 4, 6, 8):
+            if K // 128 < ks:
+                break
+            ctas = blocks * ((T + tn - 1) // tn) * ks
+            slots = _CLUSTER_SLOTS[2 * ks if pair else ks]
+            cost = (ctas + slots - 1) // slots * (8 + 0.012 * tn + (slabs + ks - 1) // ks * c + (5 + 0.02 * min(tn, T) if ks > 1 else 0))
+            if best_cost is None or cost < best_cost - 1e-9:
+                best, best_cost = (tn, ks), cost
+    return best
+
+
 def trellis_gemm(w: TrellisWeight, xh: torch.Tensor, residual: Optional[torch.Tensor] = None,
-                 out: Optional[torch.Tensor] = None, tn: Optional[int] = None) -> torch.Tensor:
-    """y[T, N] from input-transformed xh[T, K] on the tcgen05 path."""
+                 out: Optional[torch.Tensor] = None, tn: Optional[int] = None, ksplit: Optional[int] = None) -> torch.Tensor:
+    """y[T, N] from input-transformed xh[T, K] on the tcgen05 path; ``tn``: token tile, ``ksplit``: CTAs that share K."""
     _req(xh, torch.float16, "xh")
     T = xh.numel() // w.K
     out = out if out is not None else torch.empty(T, w.N, dtype=BF, device=xh.device)
-    tn = tn or pick_token_tile(T, w.N, w.K)
-    _check(_lib().r4dxb_trellis_gemm(_p(w.words), _p(w.svh), _p(xh), _p(out), _p(residual), T, w.N, w.K, w.kb, tn,
-                                     _p(gemm_status(xh.device)), _stream()), "trellis_gemm")
+    if tn is None:
+        tn, ksplit = pick_product(T, w.N, w.K)
+    head = (_p(w.words), _p(w.svh), _p(xh), _p(out), _p(residual), T, w.N, w.K, w.kb, tn)
+    tail = (_p(gemm_status(xh.device)), _stream())
+    rc = _lib().r4dxb_trellis_gemm_split(*head, ksplit, *tail) if ksplit and ksplit > 1 else _lib().r4dxb_trellis_gemm(*head, *tail)
+    _check(rc, "trellis_gemm")
     return out
 
 
@@ -560,6 +599,7 @@ W4_STREAM_ROWS = 32
 _UNSUPPORTED = 10002
 
 register_cuda_sig("r4dxb_linear_tc", _I, [_P, _P, _I, _I, _I, _P, _P, _I, _P, _P, _I, _I, _I, _I, _P, _P])
+register_cuda_sig("r4dxb_linear_tc_split", _I, [_P, _P, _I, _I, _I, _P, _P, _I, _P, _P, _I, _I, _I, _I, _I, _P, _P])
 
 
 def _w4a16_rows(W: W4Weight, x: torch.Tensor, out_f32: bool, out: Optional[torch.Tensor]) -> Optional[torch.Tensor]:
@@ -585,9 +625,33 @@ def _w4a16_rows(W: W4Weight, x: torch.Tensor, out_f32: bool, out: Optional[torch
     return y
 
 
+@functools.lru_cache(maxsize=None)
+def pick_plain(T: int, N: int, K: int) -> tuple:
+    """(token tile, split of K) of a plain linear.  Where row blocks and tiles leave most SMs idle - a router, the a / b projections -
+    narrower tiles and CTAs that share K: 96 x 5120 at 333 / 8192 rows 49 / 104 us with 256- and 512-row tiles, 12 / 33 so; 512 x
+    2048 at 64 rows 18 and 10."""
+    blocks, slabs = (N + 127) // 128, (K + 63) // 64
+    tn = pick_token_tile(T, N)
+    if blocks * ((T + tn - 1) // tn) >= 74:
+        return tn, 1
+    best, best_cost = (tn, 1), None
+    for t, c in ((16, 0.25), (32, 0.26), (64, 0.28), (128, 0.33), (256, 0.50)):
+        if t > 16 and t >= 2 * T:
+            continue
+        slots = 296 if t <= 64 else 148      # (narrow tiles: two CTAs share an SM)
+        for ks in (1, 2, 4, 8):
+            if slabs < ks:
+                break
+            ctas = blocks * ((T + t - 1) // t) * ks
+            cost = (ctas + slots - 1) // slots * (6 + (slabs + ks - 1) // ks * c) + (3 if ks > 1 else 0)
+            if best_cost is None or cost < best_cost - 1e-9:
+                best, best_cost = (t, ks), cost
+    return best
+
+
 def linear_tc(W, x: torch.Tensor, bias: Optional[torch.Tensor] = None, residual: Optional[torch.Tensor] = None,
               out_f32: bool = False, out: Optional[torch.Tensor] = None, tn: Optional[int] = None,
-              act: int = 0) -> torch.Tensor:
+              act: int = 0, ksplit: Optional[int] = None) -> torch.Tensor:
     """y[T, N] = act(x W^T + bias) + residual on the tcgen05 kernel for any number of rows.
 
     ``W``: a dense bf16 / fp16 [N, K] matrix (x must have the same dtype; N % 4 == 0, K % 8 == 0), a ``W4Weight`` or a
@@ -628,9 +692,12 @@ def linear_tc(W, x: torch.Tensor, bias: Optional[torch.Tensor] = None, residual:
         _req(bias, BF, "bias")
     if residual is not None:
         _req(residual, BF, "residual")
-    tn = tn or pick_token_tile(T, N)
-    _check(_lib().r4dxb_linear_tc(_p(wp), _p(szp), kind, group, is_bf, _p(xk), _p(out), (1 if out_f32 else 0) | (act << 8),
-                                  _p(bias), _p(residual), T, N, K_, tn, _p(gemm_status(dev)), _stream()), "linear_tc")
+    if tn is None:
+        tn, ksplit = pick_plain(T, N, K_)
+    head = (_p(wp), _p(szp), kind, group, is_bf, _p(xk), _p(out), (1 if out_f32 else 0) | (act << 8), _p(bias), _p(residual), T, N, K_, tn)
+    tail = (_p(gemm_status(dev)), _stream())
+    rc = _lib().r4dxb_linear_tc_split(*head, ksplit, *tail) if ksplit and ksplit > 1 else _lib().r4dxb_linear_tc(*head, *tail)
+    _check(rc, "linear_tc")
     return out
 
 

@@ -112,3 +112,18 @@ def test_a_streamed_head_that_writes_over_its_rows_takes_the_gemm(lib):
     lib.calls.clear()
     K.linear_tc(w, buf[:2], out=buf[2:4])
     assert [n for n, _ in lib.calls] == ["r4dxb_w4a16_rows"]
+
+
+def test_products_get_a_tile_and_a_split_that_the_kernel_has():
+    """Token tile and split of K by shape: a tile of the kernel, at most eight CTAs in a cluster (a pair counts twice), at least 128
+    columns of K for each; a plain linear that fills the chip keeps its tile and is not split."""
+    from r4dx_b200.ops import kernels as K
+    for N in (128, 256, 640, 1024, 5120, 16384, 34816):
+        for Kd in (128, 256, 512, 2048, 5120, 17408):
+            for T in (1, 9, 16, 17, 64, 65, 128, 200, 256, 257, 333, 512, 1000, 8192):
+                tn, ks = K.pick_product(T, N, Kd)
+                assert tn in (16, 32, 64, 128, 192, 256, 384, 512) and 1 <= ks <= max(1, Kd // 128)
+                assert ks * (2 if tn >= 256 and N % 256 == 0 else 1) <= 8
+                tp, kp = K.pick_plain(T, N, Kd)
+                assert tp in (16, 32, 64, 128, 256, 512) and 1 <= kp <= (Kd + 63) // 64 and (kp == 1 or tp <= 256)
+    assert K.pick_plain(4096, 4096, 4096) == (K.pick_token_tile(4096, 4096), 1)

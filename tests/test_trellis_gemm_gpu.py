@@ -65,6 +65,56 @@ def test_trellis_gemm_matches_reference_and_gemv(K, kb, T, tn):
     assert (y8.float() - y[:8].float()).abs().max().item() < 0.02 * scale + 1e-3
 
 
+@pytest.mark.parametrize("kb", [3, 4, 5])
+@pytest.mark.parametrize("T,tn,ksplit", [(9, 16, 3), (16, 16, 1), (33, 64, 8), (65, 128, 2), (129, 192, 1), (191, 192, 4), (255, 256, 1), (257, 256, 3),
+                                         (333, 384, 2), (385, 384, 1), (511, 512, 3), (513, 512, 1)])
+@pytest.mark.parametrize("N", [128, 256, 640])
+def test_trellis_product_tiles_pairs_and_splits(K, kb, T, tn, ksplit, N):
+    """Edges of every token tile, with an even number of row blocks (from 256 tokens in pairs of CTAs) and an odd one, and with K
+    split unevenly (9 blocks); against fp64 sums of the transformed rows that both sides share.  What differs is the rounding of the
+    result to bf16 (at most 2^-9 of each value) and fp32 sums of 1152 products: below 2^-8 in the norm."""
+    from r4dx_b200.quant import trellis
+    Kd = 1152
+    tw = trellis.random_weight(N, Kd, kb, seed=kb, sigma=0.02)
+    g = torch.Generator().manual_seed(T)
+    x = torch.randn(T, Kd, generator=g).to(BF).cuda()
+    res = torch.randn(T, N, generator=g).to(BF).cuda()
+    twd = tw.to("cuda")
+    ref = x.double() @ trellis.reconstruct(tw).double().cuda().T
+    xh = K.trellis_input(x, twd.suh)
+    y = K.trellis_gemm(twd, xh, tn=tn, ksplit=ksplit)
+    z = res.clone()
+    K.trellis_gemm(twd, xh, residual=z, out=z, tn=tn, ksplit=ksplit)
+    K.check_gemm_status("cuda")
+    assert ((y.double() - ref).norm() / ref.norm()).item() < 2 ** -8
+    assert ((z.double() - ref - res.double()).norm() / (ref + res.double()).norm()).item() < 2 ** -8
+
+
+def test_trellis_product_writes_rows_that_are_not_16_byte_aligned(K):
+    """An output whose base is 8-byte aligned only takes the lane stores instead of the bulk copies."""
+    from r4dx_b200.quant import trellis
+    tw = trellis.random_weight(256, 512, 4, seed=2).to("cuda")
+    xh = torch.randn(300, 512, device="cuda").half()
+    buf = torch.zeros(300 * 256 + 8, dtype=BF, device="cuda")
+    y = K.trellis_gemm(tw, xh, out=buf[4:4 + 300 * 256].view(300, 256), tn=256)
+    assert torch.equal(y, K.trellis_gemm(tw, xh, tn=256))
+    assert not buf[:4].any() and not buf[4 + 300 * 256:].any()
+
+
+@pytest.mark.parametrize("N,Kd,T,tn,ksplit", [(96, 5120, 333, 16, 8), (100, 72, 40, 32, 2), (512, 2048, 65, 64, 3), (1000, 200, 257, 256, 4)])
+def test_plain_linear_with_a_split_of_k(K, N, Kd, T, tn, ksplit):
+    """fp32 results of bf16 operands with K shared by a cluster (ragged last slab, remainders of tokens and outputs): sums of K
+    products in fp32, 2^-24 sqrt(K) of their norm and far below 1e-5."""
+    g = torch.Generator().manual_seed(N)
+    W, x = torch.randn(N, Kd, generator=g).to(BF).cuda(), torch.randn(T, Kd, generator=g).to(BF).cuda()
+    ref = x.double() @ W.double().T
+    y = K.linear_tc(W, x, out_f32=True, tn=tn, ksplit=ksplit)
+    auto = K.linear_tc(W, x, out_f32=True)
+    K.check_gemm_status("cuda")
+    assert ((y.double() - ref).norm() / ref.norm()).item() < 1e-5
+    assert ((auto.double() - ref).norm() / ref.norm()).item() < 1e-5
+
+
 @pytest.mark.parametrize("kb,T,N,Kd,tn", [(4, 300, 256, 512, 128), (5, 1024, 384, 1024, 512), (3, 700, 128, 256, 256)])
 def test_trellis_gemm_8bit_operands_match_the_reference_within_their_rounding(kb, T, N, Kd, tn):
     """e4m3 activations (one scale per row) times e4m3 code values against the fp32 reference of the same weights.
