@@ -509,7 +509,8 @@ class HybridModel:
         """Raises if a bounded device wait ran out since the last check: a timed-out collective leaves an un-reduced partial
         in the residual stream, so a token read after it must not be trusted (one small device-to-host read per call).
         ``rows``: the row count of the call being checked (from ``K.ROWS_MIN_ROWS`` rows its products may have run on the
-        mma.sync or tensor-memory weight-streaming kernel, whose waits report through the GEMM status word)."""
+        mma.sync or tensor-memory weight-streaming kernel, whose waits report through the GEMM status word; a one-row step does not
+        read it: a wait that ran out there leaves NaN in its logits, and the word set for the next call that reads it)."""
         if self.comm is not None and self.comm.world > 1:
             self.comm.check_healthy()
         if K.GEMV_IMPL == "mma" or (K.GEMV_IMPL == "auto" and rows >= K.ROWS_MIN_ROWS):

@@ -12,8 +12,13 @@
 // What bounds it: instructions.  Per 256 weights a warp issues 8 extractions, 8 multiplies, 8 byte sums, 4 permutes, 4 multiply-adds
 // and one MMA, 41 clocks of a scheduler by themselves.  us at 2 / 4 / 8 rows, 4 bits, against the CUDA-core kernel
 // (trellis_gemv.cu): 34816 x 5120 52 / 52 / 54 (66 / 82 / 121), 5120 x 17408 34 / 36 / 34 (45 / 68 / 98), 16384 x 5120
-// 32 / 32 / 30 (39 / 47 / 71), 5120 x 6144 20 / 19 / 19 (23 / 27 / 39).  (The 8-bit form took 44 / 44 / 56, 32 / 32 / 36.)  One
-// row takes the other kernel: see ops/kernels.py:ROWS_MIN_ROWS.
+// 32 / 32 / 30 (39 / 47 / 71), 5120 x 6144 20 / 19 / 19 (23 / 27 / 39).  (The 8-bit form took 44 / 44 / 56, 32 / 32 / 36.)
+//
+// One row: no MMA but fp16 multiply-adds in the order of the CUDA-core kernel, whose rounding it keeps (up to 3 of 34816 outputs
+// differ, by one bf16 step: the fp32 sums are added up in another order).  Multiplies, byte sums and fp16 multiply-adds share a pipe,
+// 24 of them per 256 weights at two clocks: 48 of the 60 clocks it takes.  us at one row, 4 / 5 bits (CUDA-core kernel): 34816 x 5120
+// 50 / 54 (57 / 64), 5120 x 17408 34 / 36 (39 / 43), 16384 x 5120 30 / 32 (34 / 39), 5120 x 6144 20 / 20 (18 / 21, but inside a
+// step the next product no longer waits for a transform in every CTA).
 //
 // Grouped mode (mixture-of-experts blocks with a few rows per expert): a CTA serves one 128-row block of one tile of the routing
 // plan, up to eight rows of one expert; the rows are those of the planned pairs in expert order.  A block of 512
@@ -214,6 +219,20 @@ __device__ __forceinline__ uint32_t Code2(const uint32_t (&w)[3]) {
   return *reinterpret_cast<const uint32_t*>(&q);
 }
 
+// The 16 code values of a row of a tile times the 16 columns x, onto the partial sums of its two halves: one fp16 multiply-add per
+// pair, the eight columns of a half in order.
+template <int KB>
+__device__ __forceinline__ void RowDot(const uint32_t (&w)[3], const uint4& xlo, const uint4& xhi, __half2 (&h)[2]) {
+  const uint32_t x[8] = {xlo.x, xlo.y, xlo.z, xlo.w, xhi.x, xhi.y, xhi.z, xhi.w};
+#define R4DXB_STEP(I)                                                                                          \
+  {                                                                                                           \
+    const uint32_t q = Code2<KB, 2 * I>(w);                                                                    \
+    h[I / 4] = __hfma2(*reinterpret_cast<const __half2*>(&q), *reinterpret_cast<const __half2*>(&x[I]), h[I / 4]); \
+  }
+  R4DXB_STEP(0) R4DXB_STEP(1) R4DXB_STEP(2) R4DXB_STEP(3) R4DXB_STEP(4) R4DXB_STEP(5) R4DXB_STEP(6) R4DXB_STEP(7)
+#undef R4DXB_STEP
+}
+
 template <int KB, int TMAX, bool kGrouped = false>
 __global__ void __launch_bounds__(kThreads, TMAX > 4 && !kGrouped ? 1 : 2) TrellisRowsKernel(RowsArgs a) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -317,59 +336,97 @@ __global__ void __launch_bounds__(kThreads, TMAX > 4 && !kGrouped ? 1 : 2) Trell
     // lane (g, c): rows g and g + 8 of an n-tile, the 16 columns of its k-tile, four of them per MMA (the contraction index of
     // the fragments maps to columns alike in both operands); column g of the product = row g of x
     const int team = warp / kTeamWarps, w4 = warp % kTeamWarps;
-    const int g = lane >> 2, c = lane & 3, kq = w4 & 1, nt0 = (w4 >> 1) * 4;
-    TrellisRow<KB> ra, rb;                                 // (the lane's k-tile is (c >> 1) * 4 + kq * 2 + (c & 1))
-    ra.Init(g);
-    rb.Init(g + 8);
-    float acc[4][4];
-#pragma unroll
-    for (int n = 0; n < 4; ++n)
-#pragma unroll
-      for (int i = 0; i < 4; ++i) acc[n][i] = 0.f;
-    // columns past the last row of x repeat it: a column of the product depends on its own column of x only
-    const unsigned char* xrow = xs + static_cast<size_t>(min(g, T - 1)) * xstride + (kq * 4 + c) * 32;
+    const int kq = w4 & 1, nt0 = (w4 >> 1) * 4;
     // stage index and barrier parity advance by counting: a division by the run-time ring depth per 128-wide
     // K block would cost as much as decoding a dozen weights
     int s = team, b = team;
     uint32_t phase = 0;
     while (s >= a.stages) s -= a.stages;
-    for (int it = team; it < my_blocks && ok; it += kTeams) {
-      const uint4 xlo = *reinterpret_cast<const uint4*>(xrow + it * 256), xhi = *reinterpret_cast<const uint4*>(xrow + it * 256 + 16);
-      const uint32_t bx[8] = {xlo.x, xlo.y, xlo.z, xlo.w, xhi.x, xhi.y, xhi.z, xhi.w};
-      ok = ptx::MbarWaitAt(full_at + b * 8, phase, abort_flag, 2);
-      if (!ok) break;
-      const unsigned char* st = wst + s * kStageSlot + (c >> 1) * kHalfSlot + (kq * 2 + (c & 1)) * kTileBytes + nt0 * (NW * 4);
-#pragma unroll
-      for (int n = 0; n < 4; ++n) {
-        const uint32_t* tw = reinterpret_cast<const uint32_t*>(st + n * (NW * 4));
-        uint32_t wa[3], wb[3];
-        ra.Load(tw, wa[2], wa[1], wa[0]);
-        rb.Load(tw, wb[2], wb[1], wb[0]);
-#define R4DXB_STEP(I)                                                                                                  \
-  {                                                                                                                   \
-    const uint32_t a0 = Code2<KB, 4 * I>(wa), a1 = Code2<KB, 4 * I>(wb);                                               \
-    const uint32_t a2 = Code2<KB, 4 * I + 2>(wa), a3 = Code2<KB, 4 * I + 2>(wb);                                       \
-    MmaF16(acc[n], a0, a1, a2, a3, bx[2 * I], bx[2 * I + 1]);                                                          \
-  }
-        R4DXB_STEP(0) R4DXB_STEP(1) R4DXB_STEP(2) R4DXB_STEP(3)
-#undef R4DXB_STEP
-      }
+    auto next_block = [&] {
       __syncwarp();
       if (lane == 0) ptx::MbarArriveAt(full_at + (kBarriers + b) * 8);
       s += kTeams;
       while (s >= a.stages) s -= a.stages;
       b += kTeams;
       if (b >= kBarriers) { b -= kBarriers; phase ^= 1u; }
-    }
-    // the sums of a row (k-tile half, team) meet in shared memory
-    float* mine = loc + (team * 2 + kq) * TMAX * 128 + nt0 * 16 + g;
+    };
+    float* mine = loc + (team * 2 + kq) * TMAX * 128 + nt0 * 16;
+    if constexpr (TMAX == 1) {
+      // One row: nothing to contract, so a lane takes a row of an n-tile (lanes 16..31 that of the next n-tile) times the 64 columns
+      // of half a K block.  Sums of 16 products in fp16 (the even or the odd columns of one half of four k-tiles), the rest in fp32.
+      TrellisRow<KB> row;
+      row.Init(lane & 15);
+      float acc[2] = {0.f, 0.f};
+      const unsigned char* xrow = xs + kq * 64;
+      for (int it = team; it < my_blocks && ok; it += kTeams) {
+        ok = ptx::MbarWaitAt(full_at + b * 8, phase, abort_flag, 2);
+        if (!ok) break;
+        const unsigned char* st = wst + s * kStageSlot + kq * kHalfSlot + (nt0 + (lane >> 4)) * (NW * 4);
+        __half2 h[2][2];
 #pragma unroll
-    for (int n = 0; n < 4; ++n)
+        for (int i = 0; i < 2; ++i) h[i][0] = h[i][1] = __float2half2_rn(0.f);
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const int t = 2 * c + (i & 1);
-        if (t < T) mine[t * 128 + n * 16 + 8 * (i >> 1)] = ok ? acc[n][i] : __int_as_float(0x7FC00000);      // (a copy that never landed shows as NaN)
+        for (int j = 0; j < 4; ++j) {
+          const uint4* xt = reinterpret_cast<const uint4*>(xrow + it * 256 + StoredTile(j) * 32);
+          const uint4 xlo = xt[0], xhi = xt[1];
+#pragma unroll
+          for (int i = 0; i < 2; ++i) {
+            uint32_t w[3];
+            row.Load(reinterpret_cast<const uint32_t*>(st + j * kTileBytes + i * 2 * (NW * 4)), w[2], w[1], w[0]);
+            RowDot<KB>(w, xlo, xhi, h[i]);
+          }
+        }
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+          acc[i] += (__low2float(h[i][0]) + __high2float(h[i][0])) + (__low2float(h[i][1]) + __high2float(h[i][1]));
+        next_block();
       }
+#pragma unroll
+      for (int i = 0; i < 2; ++i) mine[i * 32 + lane] = ok ? acc[i] : __int_as_float(0x7FC00000);      // (a copy that never landed shows as NaN)
+    } else {
+      const int g = lane >> 2, c = lane & 3;
+      TrellisRow<KB> ra, rb;                                 // (the lane's k-tile is (c >> 1) * 4 + kq * 2 + (c & 1))
+      ra.Init(g);
+      rb.Init(g + 8);
+      float acc[4][4];
+#pragma unroll
+      for (int n = 0; n < 4; ++n)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) acc[n][i] = 0.f;
+      // columns past the last row of x repeat it: a column of the product depends on its own column of x only
+      const unsigned char* xrow = xs + static_cast<size_t>(min(g, T - 1)) * xstride + (kq * 4 + c) * 32;
+      for (int it = team; it < my_blocks && ok; it += kTeams) {
+        const uint4 xlo = *reinterpret_cast<const uint4*>(xrow + it * 256), xhi = *reinterpret_cast<const uint4*>(xrow + it * 256 + 16);
+        const uint32_t bx[8] = {xlo.x, xlo.y, xlo.z, xlo.w, xhi.x, xhi.y, xhi.z, xhi.w};
+        ok = ptx::MbarWaitAt(full_at + b * 8, phase, abort_flag, 2);
+        if (!ok) break;
+        const unsigned char* st = wst + s * kStageSlot + (c >> 1) * kHalfSlot + (kq * 2 + (c & 1)) * kTileBytes + nt0 * (NW * 4);
+#pragma unroll
+        for (int n = 0; n < 4; ++n) {
+          const uint32_t* tw = reinterpret_cast<const uint32_t*>(st + n * (NW * 4));
+          uint32_t wa[3], wb[3];
+          ra.Load(tw, wa[2], wa[1], wa[0]);
+          rb.Load(tw, wb[2], wb[1], wb[0]);
+#define R4DXB_STEP(I)                                                                                                  \
+    {                                                                                                                   \
+      const uint32_t a0 = Code2<KB, 4 * I>(wa), a1 = Code2<KB, 4 * I>(wb);                                               \
+      const uint32_t a2 = Code2<KB, 4 * I + 2>(wa), a3 = Code2<KB, 4 * I + 2>(wb);                                       \
+      MmaF16(acc[n], a0, a1, a2, a3, bx[2 * I], bx[2 * I + 1]);                                                          \
+    }
+          R4DXB_STEP(0) R4DXB_STEP(1) R4DXB_STEP(2) R4DXB_STEP(3)
+#undef R4DXB_STEP
+        }
+        next_block();
+      }
+      // the sums of a row (k-tile half, team) meet in shared memory
+#pragma unroll
+      for (int n = 0; n < 4; ++n)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const int t = 2 * c + (i & 1);
+          if (t < T) mine[t * 128 + n * 16 + g + 8 * (i >> 1)] = ok ? acc[n][i] : __int_as_float(0x7FC00000);      // (a copy that never landed shows as NaN)
+        }
+    }
     if (!ok && lane == 0 && a.status != nullptr) atomicCAS(a.status, 0, 700 + *abort_flag);
     ConsumerSync();
     if (ksplit > 1) {
@@ -449,6 +506,7 @@ size_t SmemBytes(int kslice, int stages, int ksplit) {
 
 size_t SmemOf(int kb, int T, int K, int ksplit) {
   const int blocks = (K / 128 + ksplit - 1) / ksplit, stages = blocks < kMaxStages ? blocks : kMaxStages;
+  if (T == 1) return kb == 3 ? SmemBytes<3, 1>(blocks * 128, stages, ksplit) : (kb == 4 ? SmemBytes<4, 1>(blocks * 128, stages, ksplit) : SmemBytes<5, 1>(blocks * 128, stages, ksplit));
   if (kb == 3) return T <= 4 ? SmemBytes<3, 4>(blocks * 128, stages, ksplit) : SmemBytes<3, 8>(blocks * 128, stages, ksplit);
   if (kb == 4) return T <= 4 ? SmemBytes<4, 4>(blocks * 128, stages, ksplit) : SmemBytes<4, 8>(blocks * 128, stages, ksplit);
   return T <= 4 ? SmemBytes<5, 4>(blocks * 128, stages, ksplit) : SmemBytes<5, 8>(blocks * 128, stages, ksplit);
@@ -509,6 +567,7 @@ int LaunchInput(const RowsArgs& a, cudaStream_t stream) {
 
 template <int KB>
 int LaunchKb(const RowsArgs& a, int ksplit, cudaStream_t stream) {
+  if (a.T == 1) return LaunchRows<KB, 1>(a, ksplit, stream);
   if (a.T <= 4) return LaunchRows<KB, 4>(a, ksplit, stream);
   return LaunchRows<KB, 8>(a, ksplit, stream);
 }

@@ -217,18 +217,20 @@ def pick_split(N: int, K: int) -> int:
 ROWS_MIN_WEIGHTS = 1 << 23
 ROWS_MIN_WORK = 3 << 24
 
-# Rows from which a launch takes the rows kernel.  One-row steps stay on the CUDA cores although a step of the 27B geometry (8
-# layers, 8192 tokens of context) takes 1435 us there and 1270 with the rows kernel: the two round differently (6.4e-4 and 2.2e-4
-# of a product against 64 bits, most of the first from fp16 partial sums), and over a run of steps, each fed from the recurrent
-# state of the last, the difference grows past 3 % of the logits.
+# Rows from which a launch takes the rows kernel's mma.sync form, and weights from which one row takes its other form, which rounds as
+# the CUDA-core kernel does (fp16 sums of 32 products, whose error decides the logits of all later steps) and transforms the row once
+# per launch instead of once per CTA.  us of a step of the 27B geometry (8 layers, 8192 tokens of context), one-row products on the
+# CUDA cores / on the rows kernel from 64M / from 28M weights: 1425 / 1279 / 1241.  Smaller ones stay: 8192 x 2048 14.3 and 15.4 us.
 ROWS_MIN_ROWS = 2
+ONE_ROW_MIN_WEIGHTS = 7 << 22
 
 
 @functools.lru_cache(maxsize=None)
 def rows_split(N: int, K: int, T: int) -> Optional[int]:
     """Split of the rows kernel for T rows of a launch of N outputs, None where one of the other kernels serves it."""
-    large = N * K >= ROWS_MIN_WEIGHTS and T * N * K >= ROWS_MIN_WORK
-    return pick_split(N, K) if T >= ROWS_MIN_ROWS and large else None
+    if T < ROWS_MIN_ROWS:
+        return pick_split(N, K) if N * K >= ONE_ROW_MIN_WEIGHTS else None
+    return pick_split(N, K) if N * K >= ROWS_MIN_WEIGHTS and T * N * K >= ROWS_MIN_WORK else None
 
 
 _STATUS = {}
@@ -255,7 +257,7 @@ register_cuda_sig("r4dxb_trellis_gemv_mma", _I, [_P, _P, _P, _P, _P, _P, _P, _F,
 
 # Which weight-streaming kernel serves T <= 8 rows: "simt" = CUDA-core decode + fp16 FMA (trellis_gemv.cu), "mma" = code values
 # written to tensor memory and contracted by tcgen05.mma kind::f16 (trellis_gemv_mma.cu), "auto" (the default) = decode in
-# registers for mma.sync where rows and weights are many enough (trellis_gemv_rows.cu; us at 2 / 4 / 8 rows on gate_up
+# registers for mma.sync (one row: for fp16 FMA) where rows and weights are many enough (trellis_gemv_rows.cu; us at 2 / 4 / 8 rows on gate_up
 # 52 / 52 / 54 against 66 / 78 / 94 for the better of the other two), else by row count one of the other two.
 GEMV_IMPL = os.environ.get("R4DXB_GEMV", "auto")
 

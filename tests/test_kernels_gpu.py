@@ -1354,3 +1354,20 @@ def test_grouped_rows_kernel_matches_the_per_pair_reference(K, kb, N, Kd, counts
             K.trellis_rows_grouped(words, suh, svh, x.cuda(), y8, od, pd, tiles8, ntiles, div, mode, total, E, N, Kd, kb, digits, tile_rows=tile_rows)
             assert torch.equal(y8, y)
         K.moe_tiles(od, E, 4, tiles, ntiles)
+
+
+@pytest.mark.parametrize("kb", [3, 4, 5])
+@pytest.mark.parametrize("N,Kd,split", [(128, 128, 1), (256, 640, 3), (640, 2176, 2), (5120, 6144, 3), (5760, 5120, 1)])
+def test_one_row_on_the_rows_kernel_rounds_as_the_cuda_core_kernel(K, kb, N, Kd, split):
+    """The same fp16 sums of 16 products; only the fp32 sums of those are added up in another order (a few 2^-24 of their norm), which
+    moves the bf16 result of an output by one step now and then: at most one output in 500 here, by at most 2^-7 of its value."""
+    from r4dx_b200.quant import trellis
+    w = trellis.random_weight(N, Kd, kb, seed=N + kb, sigma=0.02).to("cuda")
+    g = torch.Generator().manual_seed(Kd)
+    x, gu, res = (torch.randn(1, n, generator=g).to(BF).cuda() for n in (Kd, 2 * Kd, N))
+    nw = (torch.randn(Kd, generator=g) * 0.1).to(BF).cuda()
+    for args in ({}, {"residual": res}, {"prologue": K.PRO_RMSNORM, "norm_w": nw}, {"prologue": K.PRO_SILU_MUL}, {"prologue": K.PRO_GELU_MUL}):
+        xs = gu if args.get("prologue") in (K.PRO_SILU_MUL, K.PRO_GELU_MUL) else x
+        y, ref = K.trellis_gemv(w, xs, split_rows=split, **args).float(), K.trellis_gemv(w, xs, ksplit=1, **args).float()
+        assert int((y != ref).sum()) <= max(1, N // 500)
+        assert ((y - ref).abs() <= 2.0 ** -7 * ref.abs() + 2.0 ** -14 * ref.abs().max()).all()
