@@ -15,6 +15,9 @@ extern "C" {
 #define R4DXB_UNSUPPORTED 10002
 #define R4DXB_TOO_LARGE 10003
 
+/* A non-blocking stream of the current device (null: none could be created), and its release. */
+void* r4dxb_stream_create(void);
+unsigned r4dxb_stream_destroy(void* stream);
 unsigned long long r4dxb_launch_count(void);
 void r4dxb_launch_count_reset(void);
 

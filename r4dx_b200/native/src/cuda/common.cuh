@@ -86,6 +86,19 @@ __device__ __forceinline__ float BlockSum(float v, float* red) {
   return r;
 }
 
+// The largest e < n with sorted[e] <= p (sorted[0] <= p), by a whole warp for one p: 32 probes a round, so two rounds of loads for
+// 1024 entries where a bisection is a chain of ten.
+__device__ __forceinline__ int LastAtOrBelow(const int* __restrict__ sorted, int n, int p) {
+  int lo = 0, len = n;                       // the answer lies in [lo, lo + len)
+  while (len > 1) {
+    const int step = (len + 31) / 32, at = lo + (threadIdx.x & 31) * step;
+    const int below = __popc(__ballot_sync(0xffffffffu, at < lo + len && __ldg(sorted + at) <= p));
+    lo += (below - 1) * step;
+    len = min(step, n - lo);
+  }
+  return lo;
+}
+
 __device__ __forceinline__ float Bf16Bits(uint16_t b) { return __uint_as_float(static_cast<uint32_t>(b) << 16); }
 __device__ __forceinline__ float BfLo(uint32_t p) { return __uint_as_float(p << 16); }
 __device__ __forceinline__ float BfHi(uint32_t p) { return __uint_as_float(p & 0xFFFF0000u); }

@@ -162,6 +162,12 @@ extern "C" {
 unsigned long long r4dxb_launch_count() { return g_launch_count; }
 void r4dxb_launch_count_reset() { g_launch_count = 0; }
 
+void* r4dxb_stream_create(void) {
+  cudaStream_t s = nullptr;
+  return cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking) == cudaSuccess ? s : nullptr;
+}
+unsigned r4dxb_stream_destroy(void* stream) { return static_cast<unsigned>(cudaStreamDestroy(static_cast<cudaStream_t>(stream))); }
+
 int r4dxb_embed_gather_bf16(const int* ids, const void* table, void* out, int T, int H, int V, void* stream) {
   if (H % 8 || T <= 0) return R4DXB_BAD_ARG;
   EmbedGatherKernel<<<T, 128, 0, static_cast<cudaStream_t>(stream)>>>(

@@ -584,35 +584,33 @@ __global__ void MoeTilesKernel(const int* __restrict__ offsets, int E, int tn, i
 }
 
 // xh[p] = fp16(H128(suh[e(p)] * act(in[perm[p] / xdiv]))) for every planned pair p (sorted by expert); a warp takes
-// 2 * kPasses blocks of one pair (grid.y covers the rest of a row), so that the expert of the pair - found by bisection of the
-// offsets - and its row are looked up once and the loads of all its blocks are in flight together.
-constexpr int kPasses = 4;
-__global__ void __launch_bounds__(256) TrellisInputGroupedKernel(const __nv_bfloat16* __restrict__ in, const __half* __restrict__ suh,
+// 2 * kPasses blocks of one pair (grid.y covers the rest of a row), so that the expert of the pair and its row are looked up once and
+// the loads of all its blocks are in flight together; with a gate, half as many blocks, so that four CTAs share an SM either way
+// (40960 pairs, 2048 columns / gated 512: 81 / 71 -> 72 / 43 us; the first is bound by 500 MB through the L2).
+template <bool kGated, int kPasses>
+__global__ void __launch_bounds__(256, 4) TrellisInputGroupedKernel(const __nv_bfloat16* __restrict__ in, const __half* __restrict__ suh,
                                                                  __half* __restrict__ out, const int* __restrict__ offsets,
                                                                  const int* __restrict__ perm, int E, int P, int K, int xdiv, int mode, bool a16) {
   const int p = blockIdx.x * 8 + (threadIdx.x >> 5), half = (threadIdx.x >> 4) & 1;
   if (p >= P || p >= __ldg(offsets + E)) return;
-  int lo = 0, hi = E;                                  // largest e with offsets[e] <= p
-  while (hi - lo > 1) {
-    const int mid = (lo + hi) >> 1;
-    if (__ldg(offsets + mid) <= p) lo = mid; else hi = mid;
-  }
+  const int lo = LastAtOrBelow(offsets, E, p);
   const int t = __ldg(perm + p) / xdiv;
-  const __nv_bfloat16* row = in + static_cast<size_t>(t) * (mode == 0 ? K : 2 * static_cast<size_t>(K));
+  const __nv_bfloat16* row = in + static_cast<size_t>(t) * (kGated ? 2 * static_cast<size_t>(K) : K);
   const __half* sg = suh + static_cast<size_t>(lo) * K;
   const int b0 = blockIdx.y * 2 * kPasses + half, blocks = K / 128;
-  uint4 x[kPasses], u[kPasses], sv[kPasses];
+  uint4 x[kPasses], u[kGated ? kPasses : 1], sv[kPasses];
+  u[0] = make_uint4(0u, 0u, 0u, 0u);
 #pragma unroll
   for (int i = 0; i < kPasses; ++i) {
     const int k = min(b0 + 2 * i, blocks - 1) * 128 + (threadIdx.x & 15) * 8;
     x[i] = Load16(row + k, a16);
-    u[i] = mode == 0 ? make_uint4(0u, 0u, 0u, 0u) : Load16(row + K + k, a16);
+    if constexpr (kGated) u[i] = Load16(row + K + k, a16);
     sv[i] = Load16(sg + k, a16);
   }
 #pragma unroll
   for (int i = 0; i < kPasses; ++i) {
     if (blockIdx.y * 2 * kPasses + 2 * i >= blocks) break;          // (uniform over the warp)
-    const uint4 o = TransformBlock(x[i], u[i], sv[i], mode);
+    const uint4 o = TransformBlock(x[i], u[kGated ? i : 0], sv[i], kGated ? mode : 0);
     if (b0 + 2 * i < blocks) Store16(out + static_cast<size_t>(p) * K + (b0 + 2 * i) * 128 + (threadIdx.x & 15) * 8, o, a16);
   }
 }
@@ -847,8 +845,9 @@ int r4dxb_moe_tiles(const int* offsets, int E, int tn, int* tiles, int* ntiles, 
 int r4dxb_trellis_input_grouped(const void* in, const void* suh, void* out, const int* offsets, const int* perm, int E, int P,
                                 int K, int xdiv, int mode, void* stream) {
   if (P < 1 || K % 128 || xdiv < 1 || mode < 0 || mode > 2) return R4DXB_BAD_ARG;
-  const dim3 grid((P + 7) / 8, (K / 128 + 2 * kPasses - 1) / (2 * kPasses));
-  TrellisInputGroupedKernel<<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(
+  const int per_warp = mode == 0 ? 8 : 4;            // 128-column blocks
+  const dim3 grid((P + 7) / 8, (K / 128 + per_warp - 1) / per_warp);
+  (mode == 0 ? TrellisInputGroupedKernel<false, 4> : TrellisInputGroupedKernel<true, 2>)<<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(
       static_cast<const __nv_bfloat16*>(in), static_cast<const __half*>(suh), static_cast<__half*>(out), offsets, perm, E, P, K, xdiv, mode,
       Aligned16(in, suh, out));
   return FinishLaunch();

@@ -163,11 +163,7 @@ __global__ void __launch_bounds__(kInWarps * 32) TrellisRowsInputKernel(RowsArgs
   if constexpr (kGrouped) {
     asm volatile("griddepcontrol.wait;" ::: "memory");
     if (t >= __ldg(a.g_offsets + a.g_experts)) return;       // (pairs of experts that live elsewhere)
-    int lo = 0, hi = a.g_experts;                            // largest e with offsets[e] <= t
-    while (hi - lo > 1) {
-      const int mid = (lo + hi) >> 1;
-      if (__ldg(a.g_offsets + mid) <= t) lo = mid; else hi = mid;
-    }
+    const int lo = LastAtOrBelow(a.g_offsets, a.g_experts, t);
     suh += static_cast<size_t>(lo) * K;
     xrow = __ldg(a.g_perm + t) / a.g_xdiv;
   }

@@ -8,6 +8,7 @@ from __future__ import annotations
 import ctypes
 import functools
 import os
+import weakref
 from typing import Optional, Sequence
 
 import torch
@@ -81,6 +82,21 @@ def launch_count() -> int:
 
 def launch_count_reset() -> None:
     _lib().r4dxb_launch_count_reset()
+
+
+register_cuda_sig("r4dxb_stream_create", _P, [])
+register_cuda_sig("r4dxb_stream_destroy", ctypes.c_uint, [_P])
+
+
+def own_stream(owner, device) -> "torch.cuda.ExternalStream":
+    """A stream that lives as long as ``owner``.  Not one of torch's pool, which hands the same 32 streams to everybody: work that
+    another thread puts on a stream which a capture has forked into would become part of that capture."""
+    with torch.cuda.device(device):
+        handle = _lib().r4dxb_stream_create()
+    if not handle:
+        raise KernelError("no stream could be created")
+    weakref.finalize(owner, _lib().r4dxb_stream_destroy, handle).atexit = False
+    return torch.cuda.ExternalStream(handle, device=device)
 
 
 BF = torch.bfloat16

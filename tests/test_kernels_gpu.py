@@ -1371,3 +1371,48 @@ def test_one_row_on_the_rows_kernel_rounds_as_the_cuda_core_kernel(K, kb, N, Kd,
         y, ref = K.trellis_gemv(w, xs, split_rows=split, **args).float(), K.trellis_gemv(w, xs, ksplit=1, **args).float()
         assert int((y != ref).sum()) <= max(1, N // 500)
         assert ((y - ref).abs() <= 2.0 ** -7 * ref.abs() + 2.0 ** -14 * ref.abs().max()).all()
+
+
+@pytest.mark.parametrize("E,k,T", [(16, 4, 3), (33, 16, 8), (257, 10, 40), (512, 10, 102), (1000, 8, 129), (1024, 16, 64), (512, 10, 700)])
+def test_router_and_plan_at_the_edges_of_their_groups(K, E, k, T):
+    """Ties, both zeros and minus infinity among the logits (larger value first, then the lower id), experts in groups of 256 and pairs on
+    both sides of 1024, against a sort on the host."""
+    g = torch.Generator().manual_seed(E + T)
+    logits = torch.randint(-6, 7, (T, E), generator=g).float() * 0.5
+    logits[:, 3] = -0.0
+    logits[0, E // 2:] = float("-inf")
+    order = torch.sort(logits + 0.0, dim=-1, descending=True, stable=True).indices[:, :k].to(torch.int32)
+    ids, w = torch.empty(T, k, dtype=torch.int32, device="cuda"), torch.empty(T, k, device="cuda")
+    K.moe_router(logits.cuda(), k, True, ids, w)
+    assert torch.equal(ids.cpu(), order)
+    flat = order.flatten().long()
+    offs = torch.cat([torch.zeros(1, dtype=torch.long), torch.bincount(flat, minlength=E).cumsum(0)]).to(torch.int32)
+    perm = torch.sort(flat, stable=True).indices.to(torch.int32)
+    for route in (False, True):
+        if route and T > 8:
+            continue
+        off, pm = torch.zeros(E + 1, dtype=torch.int32, device="cuda"), torch.zeros(T * k, dtype=torch.int32, device="cuda")
+        if route:
+            K.moe_route_plan(logits.cuda(), None, k, True, False, 1.0, ids, w, 0, E, off, pm)
+            assert torch.equal(ids.cpu(), order)
+        else:
+            K.moe_plan(ids, T * k, E, 0, E, off, pm)
+        assert torch.equal(off.cpu(), offs) and torch.equal(pm.cpu(), perm)
+
+
+@pytest.mark.parametrize("T,H,shift", [(1, 2048, 0), (600, 2048, 0), (600, 2048, 2), (1100, 1000, 0), (1100, 1026, 0)])
+def test_moe_combine_wide_and_narrow(K, T, H, shift):
+    """Sixteen-byte and four-byte columns, aligned and not, give the same sums: products in ascending expert id, one bf16 rounding."""
+    g = torch.Generator().manual_seed(H)
+    k = 10
+    ids = torch.stack([torch.randperm(64, generator=g)[:k] for _ in range(T)]).to(torch.int32)
+    w = torch.rand(T, k, generator=g).to(BF).float()
+    y = torch.randn(T * k, H, generator=g).to(BF)
+    res = torch.randn(T * H + 8, generator=g).to(BF).cuda()
+    x = res[shift:shift + T * H].view(T, H)
+    ref = x.float().cpu().double()
+    for t in range(T):
+        ref[t] += (w[t].double()[:, None] * y[t * k:(t + 1) * k].double()).sum(0)
+    out = torch.empty(T, H, dtype=BF, device="cuda")
+    K.moe_combine(y.cuda(), ids.cuda(), w.cuda(), None, None, x, out, T, H, k)
+    assert ((out.double().cpu() - ref).abs() <= 2.0 ** -8 * ref.abs() + 1e-5 * ref.abs().max()).all()

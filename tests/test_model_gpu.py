@@ -621,3 +621,27 @@ def test_llama_family_in_the_w8a16_layout_matches_its_oracle():
     a = HybridModel(cfg, qd, max_ctx=128).generate_greedy(ids.to(torch.int32), 6, use_graph=True)
     b = HybridModel(cfg, qd, max_ctx=128).generate_greedy(ids.to(torch.int32), 6, use_graph=False)
     assert a == b
+
+
+@pytest.mark.parametrize("T", [1, 2, 8])
+def test_captured_moe_block_runs_its_shared_expert_beside_the_routed_ones(T):
+    """The captured block (shared expert on a stream of its own) has the bits of the eager one, replay after replay, on new rows."""
+    from r4dx_b200.config import tiny_moe_config
+    from r4dx_b200.models.moe import MoeBlock
+    from r4dx_b200.models.oracle import init_weights
+    from r4dx_b200.quant.weights import moe_kb_rule, quantize_weight_set
+    cfg = tiny_moe_config()
+    blk = MoeBlock(cfg, _to_dev(quantize_weight_set(cfg, init_weights(cfg, 0), kb_rule=moe_kb_rule)), 0, "cuda", 8)
+    g = torch.Generator().manual_seed(T)
+    h, x = (torch.randn(T, cfg.hidden_size, generator=g).to(torch.bfloat16).cuda() for _ in range(2))
+    blk.forward(h, x.clone(), T)
+    graph, y = torch.cuda.CUDAGraph(), x.clone()
+    with torch.cuda.graph(graph):
+        blk.forward(h, y, T)
+    for _ in range(5):
+        h.copy_(torch.randn(T, cfg.hidden_size, generator=g).to(torch.bfloat16))
+        y.copy_(x)
+        graph.replay()
+        z = x.clone()
+        blk.forward(h, z, T)
+        assert torch.equal(y, z)
