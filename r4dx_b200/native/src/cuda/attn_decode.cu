@@ -333,6 +333,285 @@ __global__ void __launch_bounds__(256) DecodeKernel(DecodeArgs a) {
   }
 }
 
+// ---- several query rows per KV head on mma.sync: speculative windows ---------------------------------------------
+// The same splits, tiles and partials as DecodeKernel for D = 64, 128 or 256 and up to 64 rows (MT tiles of 16), contracted with
+// m16n8k16: scores from the fp16 rows and the cache's fp8 values (exact in fp16) with fp32 sums; probabilities, which are fp32
+// values, as the sum of two fp16 ones (scaled by 2^10, their error is 2^-35 of the largest probability), each times the fp8 values.
+// DecodeKernel works row by row on the CUDA cores: with the merge of the splits, 8 x 6 rows over 4099 / 12000 keys took 122 / 271 us
+// and take 27.6 / 44.0, 4 x 6 rows over 2048 keys 46 and 19.5; the partial results are 1e-6 off (64 bits) where sums of
+// four fp16 products left 6e-4.  What bounds it: with 148 / 4 splits a CTA has two tiles of 64 keys, so the chain of a tile (copy,
+// scores, softmax, values: 17 us with the start at 8 x 6 rows) and the merge, 12 us.
+//   scores: warp w has keys 8 w .. 8 w + 7 of the tile; a lane's share of 64 columns is 16 consecutive ones (one 16-byte load of K),
+//           four contraction steps - the order of the columns is the same in both operands
+//   values: warp w has columns 32 w .. 32 w + 31; a lane loads four columns of four keys and turns them with byte permutes
+constexpr float kProbScaleLog2 = 10.f;
+
+__device__ __forceinline__ void MmaF16(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ void LoadMatrix4(uint32_t (&r)[4], const __half* p) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(static_cast<uint32_t>(__cvta_generic_to_shared(p))) : "memory");
+}
+__device__ __forceinline__ uint32_t Fp8x2Bits(uint32_t two) {
+  const __half2 h = Fp8x2ToHalf2(static_cast<uint16_t>(two));
+  return *reinterpret_cast<const uint32_t*>(&h);
+}
+
+template <int D, int MT>
+struct TcShape {
+  static constexpr int kRows = 16 * MT;
+  // strides: what the lanes of one load phase read lies in different banks
+  static constexpr int kK = D + 64, kV = D + 32;           // bytes between keys
+  static constexpr int kQ = D + 4, kP = 72, kH = 72;       // elements between rows of q (fp16), of the scores (fp32), of the probabilities (fp16)
+  static constexpr int kKBytes = kTileTokens * kK, kVBytes = kTileTokens * kV;
+  static constexpr size_t kSmem = 2 * (kKBytes + kVBytes) + kRows * (2 * kQ + 4 * kP + 2 * 2 * kH + 4 * 4);
+};
+
+template <int D, int MT>
+__global__ void __launch_bounds__(256) DecodeTcKernel(DecodeArgs a) {
+  PdlEnter();
+  using S = TcShape<D, MT>;
+  extern __shared__ __align__(16) unsigned char smem[];
+  if (a.row_slot != nullptr) {
+    const int b = blockIdx.z;
+    a.q += static_cast<size_t>(b) * a.Hq * D;
+    a.positions += b;
+    a.block_table += static_cast<size_t>(a.row_slot[b]) * a.table_stride;
+    const size_t per = static_cast<size_t>(a.splits) * a.Hkv * (a.Hq / a.Hkv);
+    a.part_acc += b * per * D;
+    a.part_ml += b * per * 2;
+  }
+  const int gqa = a.Hq / a.Hkv, G = gqa * a.T;
+  const int split = blockIdx.x, hkv = blockIdx.y, tid = threadIdx.x;
+  const int lane = tid & 31, warp = tid >> 5, g = lane >> 2, c = lane & 3;
+  uint8_t* Kt = smem;                                                // [2][64][kK]
+  uint8_t* Vt = Kt + 2 * S::kKBytes;                                 // [2][64][kV]
+  float* P = reinterpret_cast<float*>(Vt + 2 * S::kVBytes);          // [rows][kP]
+  __half* Ph = reinterpret_cast<__half*>(P + S::kRows * S::kP);      // [rows][kH]: leading halves, the 16 keys of a step in fragment order
+  __half* Pl = Ph + S::kRows * S::kH;                                // what they leave
+  __half* qs = Pl + S::kRows * S::kH;                                // [rows][kQ]
+  float* mrow = reinterpret_cast<float*>(qs + S::kRows * S::kQ);     // [rows]
+  float* lrow = mrow + S::kRows;
+  float* arow = lrow + S::kRows;                                     // per-tile rescale factor
+  int* qpos = reinterpret_cast<int*>(arow + S::kRows);               // position of each query row
+
+  const int seqlen = a.positions[a.T - 1] + 1;
+  const int nblocks = (seqlen + kBlockTokens - 1) / kBlockTokens;
+  const int first_blk = a.window > 0 ? max(0, a.positions[0] - a.window + 1) / kBlockTokens : 0;
+  const int per = ((((nblocks - first_blk) + a.splits - 1) / a.splits) + 3) & ~3;     // blocks per split, whole tiles
+  const int b0 = first_blk + split * per, b1 = min(nblocks, b0 + per);
+  const int ntiles = b1 > b0 ? (b1 - b0 + 3) / 4 : 0;
+
+  auto issue = [&](int tile, int buf) {
+    // 64 keys x D bytes of K and of V, 16 bytes a copy: D / 16 threads take a key's row
+    constexpr int kPer = D / 16, kKeys = 256 / kPer;
+    const int v = tid % kPer;
+#pragma unroll
+    for (int k0 = 0; k0 < kTileTokens; k0 += kKeys) {
+      const int key = k0 + tid / kPer, b = b0 + tile * 4 + key / kBlockTokens;
+      uint8_t* kd = Kt + buf * S::kKBytes + key * S::kK + v * 16;
+      uint8_t* vd = Vt + buf * S::kVBytes + key * S::kV + v * 16;
+      if (b < b1) {
+        const uint8_t* src = a.cache + ((static_cast<size_t>(a.block_table[b]) * a.Hkv + hkv) * 2) * kBlockTokens * D + (key % kBlockTokens) * D + v * 16;
+        __pipeline_memcpy_async(kd, src, 16);
+        __pipeline_memcpy_async(vd, src + kBlockTokens * D, 16);
+      } else {
+        *reinterpret_cast<uint4*>(kd) = make_uint4(0, 0, 0, 0);       // past the end: zeros (masked, but never NaN)
+        *reinterpret_cast<uint4*>(vd) = make_uint4(0, 0, 0, 0);
+      }
+    }
+    __pipeline_commit();
+  };
+  if (ntiles > 0) issue(0, 0);
+
+  const float sm_scale = rsqrtf(static_cast<float>(D)) * a.k_descale[hkv] * 1.4426950408889634f;  // into log2 domain
+  constexpr int kQLoads = S::kRows * D / 4 / 256;           // four elements a load, all of a thread's in flight
+  uint2 qv[kQLoads];
+#pragma unroll
+  for (int i = 0; i < kQLoads; ++i) {
+    const int r = (i * 256 + tid) / (D / 4), d = (i * 256 + tid) % (D / 4) * 4;
+    qv[i] = r < G ? *reinterpret_cast<const uint2*>(a.q + (static_cast<size_t>(r / gqa) * a.Hq + hkv * gqa + r % gqa) * D + d) : make_uint2(0u, 0u);
+  }
+#pragma unroll
+  for (int i = 0; i < kQLoads; ++i) {
+    const int r = (i * 256 + tid) / (D / 4), d = (i * 256 + tid) % (D / 4) * 4;
+    const __half2 h01 = __floats2half2_rn(BfLo(qv[i].x) * sm_scale, BfHi(qv[i].x) * sm_scale);
+    const __half2 h23 = __floats2half2_rn(BfLo(qv[i].y) * sm_scale, BfHi(qv[i].y) * sm_scale);
+    *reinterpret_cast<uint2*>(qs + r * S::kQ + d) = make_uint2(*reinterpret_cast<const uint32_t*>(&h01), *reinterpret_cast<const uint32_t*>(&h23));
+  }
+  for (int i = tid; i < 2 * S::kRows * S::kH; i += 256) Ph[i] = __float2half(0.f);      // (rows past the last one keep these)
+  if (tid < S::kRows) {
+    mrow[tid] = -INFINITY;
+    lrow[tid] = 0.f;
+    arow[tid] = 1.f;
+    qpos[tid] = tid < G ? a.positions[tid / gqa] : -1;
+  }
+  float acc[MT][4][4];
+#pragma unroll
+  for (int m = 0; m < MT; ++m)
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) acc[m][j][i] = 0.f;
+
+  for (int tile = 0; tile < ntiles; ++tile) {
+    const int buf = tile & 1;
+    __pipeline_wait_prior(0);
+    __syncthreads();                 // this tile's rows have landed; the previous tile is fully consumed by every thread
+    if (tile + 1 < ntiles) issue(tile + 1, buf ^ 1);
+    const int kp0 = (b0 + tile * 4) * kBlockTokens;
+    {                                // scores
+      const uint8_t* kr = Kt + buf * S::kKBytes + (8 * warp + g) * S::kK + 16 * c;
+      float sc[MT][4];
+#pragma unroll
+      for (int m = 0; m < MT; ++m) sc[m][0] = sc[m][1] = sc[m][2] = sc[m][3] = 0.f;
+#pragma unroll
+      for (int grp = 0; grp < D / 64; ++grp) {
+        const uint4 kv = *reinterpret_cast<const uint4*>(kr + grp * 64);
+        const uint32_t kw[4] = {kv.x, kv.y, kv.z, kv.w};
+#pragma unroll
+        for (int st = 0; st < 4; ++st) {
+          const uint32_t k01 = Fp8x2Bits(kw[st] & 0xFFFF), k23 = Fp8x2Bits(kw[st] >> 16);
+#pragma unroll
+          for (int m = 0; m < MT; ++m) {
+            const __half* q0 = qs + (16 * m + g) * S::kQ + grp * 64 + 16 * c + 4 * st;
+            const uint2 lo = *reinterpret_cast<const uint2*>(q0), hi = *reinterpret_cast<const uint2*>(q0 + 8 * S::kQ);
+            MmaF16(sc[m], lo.x, hi.x, lo.y, hi.y, k01, k23);
+          }
+        }
+      }
+#pragma unroll
+      for (int m = 0; m < MT; ++m)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int r = 16 * m + g + 8 * h, pos = qpos[r], kp = kp0 + 8 * warp + 2 * c;
+          auto seen = [&](int at) { return at <= pos && (a.window == 0 || at > pos - a.window); };
+          *reinterpret_cast<float2*>(P + r * S::kP + 8 * warp + 2 * c) =
+              make_float2(seen(kp) ? sc[m][2 * h] : -INFINITY, seen(kp + 1) ? sc[m][2 * h + 1] : -INFINITY);
+        }
+    }
+    __syncthreads();
+    // online softmax (log2 domain): one warp per query row, two keys per lane
+#pragma unroll 2
+    for (int r = warp; r < G; r += 8) {
+      const float s0 = P[r * S::kP + lane], s1 = P[r * S::kP + 32 + lane];
+      const float m_old = mrow[r];
+      const float mx = WarpMax(fmaxf(m_old, fmaxf(s0, s1)));
+      const float alpha = (mx == -INFINITY) ? 1.f : exp2f(m_old - mx);
+      const float p0 = (s0 == -INFINITY) ? 0.f : exp2f(s0 - mx + kProbScaleLog2), p1 = (s1 == -INFINITY) ? 0.f : exp2f(s1 - mx + kProbScaleLog2);
+      // key t = x + 4 i of a group of 16 is the fragment's column 2 x (+ 1: odd i; + 8: i >= 2)
+      const int i = (lane >> 2) & 3, at = (lane & 16) + 2 * (lane & 3) + (i & 1) + 8 * (i >> 1);
+      const __half h0 = __float2half_rn(p0), h1 = __float2half_rn(p1);
+      Ph[r * S::kH + at] = h0;
+      Ph[r * S::kH + 32 + at] = h1;
+      Pl[r * S::kH + at] = __float2half_rn(p0 - __half2float(h0));
+      Pl[r * S::kH + 32 + at] = __float2half_rn(p1 - __half2float(h1));
+      const float l = lrow[r] * alpha + WarpSum(p0 + p1);
+      __syncwarp();
+      if (lane == 0) {
+        mrow[r] = mx;
+        lrow[r] = l;
+        arow[r] = alpha;
+      }
+    }
+    __syncthreads();
+    if (32 * warp < D) {             // values
+#pragma unroll
+      for (int m = 0; m < MT; ++m) {
+        const float f0 = arow[16 * m + g], f1 = arow[16 * m + g + 8];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          acc[m][j][0] *= f0; acc[m][j][1] *= f0;
+          acc[m][j][2] *= f1; acc[m][j][3] *= f1;
+        }
+      }
+      const uint8_t* vr = Vt + buf * S::kVBytes + c * S::kV + 32 * warp + 4 * g;
+      const __half* pr = Ph + (lane & 15) * S::kH + (lane >> 4) * 8;
+#pragma unroll
+      for (int kk = 0; kk < 4; ++kk) {
+        uint32_t v[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) v[i] = *reinterpret_cast<const uint32_t*>(vr + (16 * kk + 4 * i) * S::kV);
+        // (v0 v1 | v2 v3) of columns 0 and 1, of columns 2 and 3
+        const uint32_t t[4] = {__byte_perm(v[0], v[1], 0x5140), __byte_perm(v[2], v[3], 0x5140), __byte_perm(v[0], v[1], 0x7362), __byte_perm(v[2], v[3], 0x7362)};
+        uint32_t b[4][2];
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+#pragma unroll
+          for (int h = 0; h < 2; ++h) b[j][h] = Fp8x2Bits(j & 1 ? t[(j >> 1) * 2 + h] >> 16 : t[(j >> 1) * 2 + h] & 0xFFFF);
+#pragma unroll
+        for (int m = 0; m < MT; ++m) {
+          uint32_t ph[4], pl[4];
+          LoadMatrix4(ph, pr + 16 * m * S::kH + 16 * kk);
+          LoadMatrix4(pl, pr + S::kRows * S::kH + 16 * m * S::kH + 16 * kk);
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            MmaF16(acc[m][j], pl[0], pl[1], pl[2], pl[3], b[j][0], b[j][1]);
+            MmaF16(acc[m][j], ph[0], ph[1], ph[2], ph[3], b[j][0], b[j][1]);
+          }
+        }
+      }
+    }
+  }
+  __pipeline_wait_prior(0);
+  __syncthreads();
+  const float vds = a.v_descale[hkv];
+  const size_t base = (static_cast<size_t>(split) * a.Hkv + hkv) * G;
+  if (32 * warp < D) {
+#pragma unroll
+    for (int m = 0; m < MT; ++m)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int r = 16 * m + g + 8 * h;
+        if (r >= G) continue;
+        // the fragment's column 2 c (+ 1) of n-tile j is column 4 (2 c (+ 1)) + j of the warp's 32
+        float4* dst = reinterpret_cast<float4*>(a.part_acc + (base + r) * D + 32 * warp + 8 * c);
+        dst[0] = make_float4(acc[m][0][2 * h] * vds, acc[m][1][2 * h] * vds, acc[m][2][2 * h] * vds, acc[m][3][2 * h] * vds);
+        dst[1] = make_float4(acc[m][0][2 * h + 1] * vds, acc[m][1][2 * h + 1] * vds, acc[m][2][2 * h + 1] * vds, acc[m][3][2 * h + 1] * vds);
+      }
+  }
+  if (tid < G) {
+    a.part_ml[(base + tid) * 2] = mrow[tid];
+    a.part_ml[(base + tid) * 2 + 1] = lrow[tid];
+  }
+}
+
+template <int D, int MT>
+int LaunchDecodeTc(const DecodeArgs& a, cudaStream_t s, int batch) {
+  auto kern = DecodeTcKernel<D, MT>;
+  const cudaError_t e = AllowAllSharedMemory(kern);
+  if (e != cudaSuccess) return static_cast<int>(e);
+  return LaunchPdl(kern, dim3(a.splits, a.Hkv, batch), dim3(256), TcShape<D, MT>::kSmem, s, a);
+}
+
+template <int D>
+int LaunchDecodeTcRows(const DecodeArgs& a, cudaStream_t s, int batch) {
+  const int G = a.Hq / a.Hkv * a.T;
+  if (G <= 16) return LaunchDecodeTc<D, 1>(a, s, batch);
+  if (G <= 32) return LaunchDecodeTc<D, 2>(a, s, batch);
+  if (G <= 48) return LaunchDecodeTc<D, 3>(a, s, batch);
+  return LaunchDecodeTc<D, 4>(a, s, batch);
+}
+
+// the window kernel of up to 64 rows per KV head
+template <int GMAX>
+int LaunchDecode(const DecodeArgs& a, cudaStream_t s, int batch = 1);
+int LaunchWindow(const DecodeArgs& a, cudaStream_t s, int batch) {
+  const int G = a.Hq / a.Hkv * a.T;
+  if (G > 64) return R4DXB_UNSUPPORTED;
+  // (16-byte copies of the cache and stores of the partial sums, 8-byte loads of q)
+  const bool aligned = ((reinterpret_cast<uintptr_t>(a.cache) | reinterpret_cast<uintptr_t>(a.part_acc)) & 15) == 0 && (reinterpret_cast<uintptr_t>(a.q) & 7) == 0;
+  if (aligned && a.D == 256) return LaunchDecodeTcRows<256>(a, s, batch);
+  if (aligned && a.D == 128) return LaunchDecodeTcRows<128>(a, s, batch);
+  if (aligned && a.D == 64) return LaunchDecodeTcRows<64>(a, s, batch);
+  if (G <= 8) return LaunchDecode<8>(a, s, batch);
+  if (G <= 16) return LaunchDecode<16>(a, s, batch);
+  if (G <= 32) return LaunchDecode<32>(a, s, batch);
+  return LaunchDecode<64>(a, s, batch);
+}
+
 // ---- one query token, at most 8 query heads per KV head: the shape of every decode step ----------------------
 // Split-KV like DecodeKernel, but every warp walks its own 16-token cache blocks from global memory to registers
 // with no block-wide barrier in the loop, so the eight warps of a CTA keep eight blocks (64 KiB per SM) in flight:
@@ -663,7 +942,7 @@ CombineKernel(const float* __restrict__ part_acc, const float* __restrict__ part
 }
 
 template <int GMAX>
-int LaunchDecode(const DecodeArgs& a, cudaStream_t s, int batch = 1) {
+int LaunchDecode(const DecodeArgs& a, cudaStream_t s, int batch) {
   const int D = a.D;
   const size_t smem = 2 * kTileTokens * (D + 16) + 2 * kTileTokens * D + static_cast<size_t>(GMAX) * D * 2 +
                       static_cast<size_t>(GMAX) * kTileTokens * 4 + GMAX * 4 * 4;
@@ -740,11 +1019,9 @@ int r4dxb_attn_decode(const void* q, const void* qg, const void* cache, const in
   int e;
   if (T == 1 && G <= 8 && g_decode_row && (D == 256 || D == 128 || D == 64)) {
     e = D == 256 ? LaunchDecodeRow<256>(a, s, 1) : (D == 128 ? LaunchDecodeRow<128>(a, s, 1) : LaunchDecodeRow<64>(a, s, 1));
-  } else if (G <= 8) e = LaunchDecode<8>(a, s);
-  else if (G <= 16) e = LaunchDecode<16>(a, s);
-  else if (G <= 32) e = LaunchDecode<32>(a, s);
-  else if (G <= 64) e = LaunchDecode<64>(a, s);
-  else return R4DXB_UNSUPPORTED;
+  } else {
+    e = LaunchWindow(a, s, 1);
+  }
   if (e) return e;
   return LaunchPdl(CombineKernel, dim3(G * ((D + 31) / 32), Hkv), dim3(kCombineThreads), 0, s, static_cast<const float*>(part_acc), static_cast<const float*>(part_ml),
                    static_cast<const __nv_bfloat16*>(qg), static_cast<__nv_bfloat16*>(out), T, Hq, Hkv, D, splits, gated, 0);
@@ -792,10 +1069,9 @@ int r4dxb_attn_decode_batch(const void* q, const void* qg, const void* cache, co
   int e;
   if (G <= 8 && g_decode_row && (D == 256 || D == 128 || D == 64)) {
     e = D == 256 ? LaunchDecodeRow<256>(a, s, B) : (D == 128 ? LaunchDecodeRow<128>(a, s, B) : LaunchDecodeRow<64>(a, s, B));
-  } else if (G <= 8) e = LaunchDecode<8>(a, s, B);
-  else if (G <= 16) e = LaunchDecode<16>(a, s, B);
-  else if (G <= 32) e = LaunchDecode<32>(a, s, B);
-  else e = LaunchDecode<64>(a, s, B);
+  } else {
+    e = LaunchWindow(a, s, B);
+  }
   if (e) return e;
   CombineKernel<<<dim3(G * ((D + 31) / 32), Hkv, B), kCombineThreads, 0, s>>>(part_acc, part_ml, static_cast<const __nv_bfloat16*>(qg),
                                               static_cast<__nv_bfloat16*>(out), 1, Hq, Hkv, D, splits, gated, 1);

@@ -1416,3 +1416,34 @@ def test_moe_combine_wide_and_narrow(K, T, H, shift):
     out = torch.empty(T, H, dtype=BF, device="cuda")
     K.moe_combine(y.cuda(), ids.cuda(), w.cuda(), None, None, x, out, T, H, k)
     assert ((out.double().cpu() - ref).abs() <= 2.0 ** -8 * ref.abs() + 1e-5 * ref.abs().max()).all()
+
+
+@pytest.mark.parametrize("D,Hq,Hkv,T,ctx,window,splits", [(256, 24, 4, 8, 4099, 0, 37), (256, 24, 4, 2, 9, 0, 37), (256, 12, 2, 7, 64, 0, 1), (256, 8, 1, 8, 65, 0, 2),
+                                                          (128, 32, 8, 4, 1000, 200, 19), (128, 4, 4, 8, 130, 0, 3), (64, 16, 4, 5, 333, 17, 5), (64, 16, 1, 4, 700, 0, 8)])
+def test_window_attention_on_the_tensor_cores_against_fp64(K, D, Hq, Hkv, T, ctx, window, splits):
+    """1 to 64 rows per KV head (remainders of 16), tiles and blocks that end inside, empty splits, sliding windows.  The merged partial
+    results against 64 bits on the fp16 rows that both use: fp32 sums of D products, fp32 exponents (2^-24 of a score of some 30) and
+    probabilities of 22 bits leave a few 1e-6; 1e-5 is allowed (fp16 sums of four products: 6e-4)."""
+    g = torch.Generator(device="cuda").manual_seed(ctx)
+    nblk, gqa = (ctx + 15) // 16 + 1, Hq // Hkv
+    G = gqa * T
+    cache = (torch.randn(nblk, Hkv, 2, 16, D, generator=g, device="cuda") * 2).to(torch.float8_e4m3fn).view(torch.uint8)
+    table = torch.randperm(nblk, device="cuda").to(torch.int32)
+    q = (torch.randn(T, Hq, D, generator=g, device="cuda") * 1.5).to(BF)
+    kds, vds = torch.full((Hkv,), 0.6, device="cuda"), torch.full((Hkv,), 0.3, device="cuda")
+    pos = torch.arange(ctx - T, ctx, dtype=torch.int32, device="cuda")
+    pa, pm = torch.full((splits * Hkv * G * D,), float("nan"), device="cuda"), torch.full((splits * Hkv * G * 2,), float("nan"), device="cuda")
+    out = torch.zeros(T, Hq * D, dtype=BF, device="cuda")
+    K.attn_decode(q, q, cache, table, pos, kds, vds, pa, pm, out, T, Hq, Hkv, D, splits, False, window)
+    acc, ml = pa.view(splits, Hkv, G, D).double(), pm.view(splits, Hkv, G, 2).double()
+    w = torch.exp2(ml[..., 0] - ml[..., 0].max(0).values)
+    o = (w[..., None] * acc).sum(0) / (w * ml[..., 1]).sum(0)[..., None]
+    kv = cache.view(torch.float8_e4m3fn).double()[table.long()]
+    k, v = (kv[:, :, i].permute(1, 0, 2, 3).reshape(Hkv, -1, D)[:, :ctx] for i in (0, 1))
+    scale = torch.rsqrt(torch.tensor(float(D), device="cuda")) * kds * 1.4426950408889634
+    qh = (q.float().view(T, Hkv, gqa, D) * scale[None, :, None, None]).half().double().permute(1, 0, 2, 3).reshape(Hkv, G, D)
+    at, row = torch.arange(ctx, device="cuda"), pos.repeat_interleave(gqa)[:, None]
+    s = (qh @ k.transpose(1, 2)).masked_fill(~((at <= row) & ((at > row - window) | (window == 0))), float("-inf"))
+    ref = torch.softmax(s * math.log(2), -1) @ (v * vds.double()[:, None, None])
+    assert (o - ref).norm() < 1e-5 * ref.norm()
+    assert ((out.view(T, Hkv, gqa, D).permute(1, 0, 2, 3).reshape(Hkv, G, D).double() - ref).abs() <= 2.0 ** -8 * ref.abs() + 1e-4 * ref.abs().max()).all()
