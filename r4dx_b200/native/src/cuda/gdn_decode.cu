@@ -13,6 +13,11 @@
 //
 // One CTA per value head (512 threads): warp w owns state rows w*D/16 .., a lane owns D/32
 // consecutive K columns, so a state row is one coalesced 128-lane... 32-lane vector load.
+//
+// What bounds it is the chain of waits, not the bytes (a head's state of 64 KB passes in 1 us): so each phase has all its loads in
+// flight at once (the conv inputs of all rows, the first a / b chunks of all rows, what the gates and the norm read), the rows share
+// the barriers, and the sums over a warp hand over half of their values at a time.  48 heads of 128, K = 5120, alone on the device:
+// 1 row 8.9 us (11.2 with one row after another), 4 rows 14.4 (23.5), 8 rows 21.9 (40.6); 16 sequences of one row 41.8 (47).
 #include "common.cuh"
 
 namespace r4dxb {
@@ -52,6 +57,35 @@ struct GdnArgs {
   int gate_act;                  // output gate of the norm: 0 silu(z), 1 sigmoid(z)
 };
 
+// The sums of R values over the warp: the lanes hand over half of the values at a time (R - 1 + log2(32 / R) exchanges instead
+// of 5 R) and end up with the sum of value `WarpScatterIndex`; WarpSums gives every lane all of them.
+template <int R, int M = 16>
+__device__ __forceinline__ float WarpScatterSum(const float (&v)[R]) {
+  if constexpr (R > 1) {
+    const bool up = threadIdx.x & M;
+    float half[R / 2];
+#pragma unroll
+    for (int i = 0; i < R / 2; ++i) {
+      const float give = up ? v[i] : v[i + R / 2], keep = up ? v[i + R / 2] : v[i];
+      half[i] = keep + __shfl_xor_sync(0xffffffffu, give, M);
+    }
+    return WarpScatterSum<R / 2, M / 2>(half);
+  } else {
+    float sum = v[0];
+#pragma unroll
+    for (int m = M; m >= 1; m >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, m);
+    return sum;
+  }
+}
+template <int R>
+__device__ __forceinline__ int WarpScatterIndex() { return (threadIdx.x & 31) / (32 / R); }
+template <int R>
+__device__ __forceinline__ void WarpSums(float (&v)[R]) {
+  const float sum = WarpScatterSum(v);
+#pragma unroll
+  for (int r = 0; r < R; ++r) v[r] = __shfl_sync(0xffffffffu, sum, r * (32 / R));
+}
+
 template <int D>
 __global__ void __launch_bounds__(kThreads) GdnDecodeKernel(GdnArgs a) {
   PdlEnter();
@@ -60,7 +94,7 @@ __global__ void __launch_bounds__(kThreads) GdnDecodeKernel(GdnArgs a) {
   __shared__ float sq[kMaxT][D], sk[kMaxT][D], sv[kMaxT][D], so[kMaxT][D];
   __shared__ float seg[kMaxT], sbeta[kMaxT];
   __shared__ float rk[kMaxT][D], ru[kMaxT][D], reg[kMaxT];
-  __shared__ float red[32], red2[32];
+  __shared__ float red[kThreads / 32], red2[kThreads / 32], red3[kThreads / 32];
   if (a.row_slot != nullptr) {
     const int b = blockIdx.y, slot = a.row_slot[b];
     a.mixed += static_cast<size_t>(b) * a.conv_dim;
@@ -97,6 +131,32 @@ __global__ void __launch_bounds__(kThreads) GdnDecodeKernel(GdnArgs a) {
     }
   }
 
+  // ---- the a / b projections: all rows at once, a share of the warps each (row after row, with four barriers each, took 2 us a
+  // row).  16 bytes a load where the rows allow it; the first of each is in flight over the conv phase, as is what the gates and
+  // the norm read.
+  constexpr int kWarps = kThreads / 32;
+  const int per_row = T == 1 ? kWarps : (T == 2 ? kWarps / 2 : (T <= 4 ? kWarps / 4 : kWarps / 8));         // warps of a row
+  const int t_ab = warp / per_row, mine = threadIdx.x - t_ab * per_row * 32, stride = per_row * 64;
+  const __nv_bfloat16* wa = a.ab_w + static_cast<size_t>(h) * a.K;
+  const __nv_bfloat16* wb = a.ab_w + static_cast<size_t>(a.H + h) * a.K;
+  const __nv_bfloat16* xr = a.x + static_cast<size_t>(t_ab) * a.K;
+  const uintptr_t bases = reinterpret_cast<uintptr_t>(a.x) | reinterpret_cast<uintptr_t>(a.ab_w) | reinterpret_cast<uintptr_t>(a.in_norm_w);
+  const bool wide = a.K % 8 == 0 && (bases & 15) == 0;
+  uint4 px = make_uint4(0, 0, 0, 0), pg = px, pa = px, pb = px;
+  if (a.ab_w != nullptr && wide && t_ab < T && mine * 8 < a.K) {
+    px = *reinterpret_cast<const uint4*>(xr + mine * 8);
+    pg = *reinterpret_cast<const uint4*>(a.in_norm_w + mine * 8);
+    pa = *reinterpret_cast<const uint4*>(wa + mine * 8);
+    pb = *reinterpret_cast<const uint4*>(wb + mine * 8);
+  }
+  const float dt_bias = a.dt_bias[h], A_log = a.A_log[h];
+  __nv_bfloat16 zv[CPL], nw[CPL];
+#pragma unroll
+  for (int c = 0; c < CPL; ++c) {
+    zv[c] = warp < T ? a.z[(static_cast<size_t>(warp) * a.H + h) * D + c * 32 + lane] : __nv_bfloat16();
+    nw[c] = warp < T ? a.norm_w[c * 32 + lane] : __nv_bfloat16();
+  }
+
   // ---- stage the previous log (before anything overwrites it) --------------------------------
   for (int i = threadIdx.x; i < nrep * D; i += kThreads) {
     const int r = i / D, c = i % D;
@@ -105,71 +165,104 @@ __global__ void __launch_bounds__(kThreads) GdnDecodeKernel(GdnArgs a) {
   }
   if (threadIdx.x < nrep) reg[threadIdx.x] = a.log_eg[threadIdx.x * a.H + h];
 
-  // ---- phase A: ring write + conv + SiLU for this head's q, k, v channels ---------------------
-  for (int i = threadIdx.x; i < T * 3 * D; i += kThreads) {
-    const int t = i / (3 * D), j = i % (3 * D);
+  // ---- phase A: ring write + conv + SiLU for this head's q, k, v channels: a thread per channel, the inputs of all rows in flight
+  // together (an element per thread and step waits for memory in every step: 1.1 us a row) ------------------------------------
+  for (int j = threadIdx.x; j < 3 * D; j += kThreads) {
     const int part = j / D, c = j % D;
     const int ch = part == 0 ? hk * D + c : (part == 1 ? key_dim + hk * D + c : 2 * key_dim + h * D + c);
-    const int pos = a.positions[t];
-    const __nv_bfloat16 xin = a.mixed[static_cast<size_t>(t) * a.conv_dim + ch];
-    a.ring[static_cast<size_t>(pos % kRing) * a.conv_dim + ch] = xin;
     // taps: weight index 3 multiplies the newest input
     const uint2 wv = *reinterpret_cast<const uint2*>(a.conv_w + static_cast<size_t>(ch) * 4);
     const float w0 = BfLo(wv.x), w1 = BfHi(wv.x), w2 = BfLo(wv.y), w3 = BfHi(wv.y);
-    float acc = w3 * __bfloat162float(xin);
-    // older inputs: rows of this call that precede t, else the ring
-    auto past = [&](int back) -> float {
-      const int p = pos - back;
-      if (p < 0) return 0.f;
-      if (t - back >= 0) return __bfloat162float(a.mixed[static_cast<size_t>(t - back) * a.conv_dim + ch]);
-      return __bfloat162float(a.ring[static_cast<size_t>(p % kRing) * a.conv_dim + ch]);
-    };
-    acc += w2 * past(1) + w1 * past(2) + w0 * past(3);
-    const float y = Silu(acc);
-    if (part == 0) sq[t][c] = y; else if (part == 1) sk[t][c] = y; else sv[t][c] = y;
+    __nv_bfloat16 in[kMaxT];
+#pragma unroll
+    for (int t = 0; t < kMaxT; ++t) in[t] = t < T ? a.mixed[static_cast<size_t>(t) * a.conv_dim + ch] : __nv_bfloat16();
+    // inputs older than the call's first row come from the ring; rows 0..2 reach that far back
+    float old[3][3];
+#pragma unroll
+    for (int t = 0; t < 3; ++t)
+#pragma unroll
+      for (int back = t + 1; back <= 3; ++back) {
+        const int p = t < T ? a.positions[t] - back : -1;
+        old[t][back - 1] = p < 0 ? 0.f : __bfloat162float(a.ring[static_cast<size_t>(p % kRing) * a.conv_dim + ch]);
+      }
+#pragma unroll
+    for (int t = 0; t < kMaxT; ++t) {
+      if (t >= T) break;
+      const int pos = a.positions[t];
+      a.ring[static_cast<size_t>(pos % kRing) * a.conv_dim + ch] = in[t];
+      auto past = [&](int back) -> float {
+        if (t - back < 0) return old[t < 3 ? t : 0][back - 1];
+        return pos - back < 0 ? 0.f : __bfloat162float(in[t - back < 0 ? 0 : t - back]);
+      };
+      const float y = Silu(w3 * __bfloat162float(in[t]) + (w2 * past(1) + w1 * past(2) + w0 * past(3)));
+      if (part == 0) sq[t][c] = y; else if (part == 1) sk[t][c] = y; else sv[t][c] = y;
+    }
   }
   if (a.ab_w != nullptr) {
-    // a[t, h] and b[t, h] = W rows . bf16(rmsnorm(x[t])): the same rounding points as the stand-alone kernel
-    const __nv_bfloat16* wa = a.ab_w + static_cast<size_t>(h) * a.K;
-    const __nv_bfloat16* wb = a.ab_w + static_cast<size_t>(a.H + h) * a.K;
-    for (int t = 0; t < T; ++t) {
-      const __nv_bfloat16* xr = a.x + static_cast<size_t>(t) * a.K;
-      float ss = 0.f;
-      for (int k = threadIdx.x * 2; k < a.K; k += kThreads * 2) {
+    float ss = 0.f;
+    if (t_ab < T && wide) {
+      auto squares = [&](uint4 b) {
+        const uint32_t bs[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) ss += BfLo(bs[i]) * BfLo(bs[i]) + BfHi(bs[i]) * BfHi(bs[i]);
+      };
+      squares(px);
+#pragma unroll 4
+      for (int k = mine * 8 + 4 * stride; k < a.K; k += 4 * stride) squares(*reinterpret_cast<const uint4*>(xr + k));
+    } else if (t_ab < T) {
+      for (int k = mine * 2; k < a.K; k += stride) {
         const uint32_t b = *reinterpret_cast<const uint32_t*>(xr + k);
         ss += BfLo(b) * BfLo(b) + BfHi(b) * BfHi(b);
       }
-      const float r = rsqrtf(BlockSum(ss, red) / a.K + a.in_eps);
-      float sa = 0.f, sb = 0.f;
-      for (int k = threadIdx.x * 2; k < a.K; k += kThreads * 2) {
-        const uint32_t b = *reinterpret_cast<const uint32_t*>(xr + k);
-        const uint32_t g = *reinterpret_cast<const uint32_t*>(a.in_norm_w + k);
-        const uint32_t hh = PackBf16(BfLo(b) * r * (1.f + BfLo(g)), BfHi(b) * r * (1.f + BfHi(g)));
-        const uint32_t va = *reinterpret_cast<const uint32_t*>(wa + k), vb = *reinterpret_cast<const uint32_t*>(wb + k);
-        sa += BfLo(va) * BfLo(hh) + BfHi(va) * BfHi(hh);
-        sb += BfLo(vb) * BfLo(hh) + BfHi(vb) * BfHi(hh);
-      }
-      // both dot products through one block reduction (two values per warp slot)
-      sa = WarpSum(sa);
-      sb = WarpSum(sb);
-      __syncthreads();
-      if (lane == 0) { red[warp] = sa; red2[warp] = sb; }
-      __syncthreads();
-      sa = WarpSum(lane < kThreads / 32 ? red[lane] : 0.f);
-      sb = WarpSum(lane < kThreads / 32 ? red2[lane] : 0.f);
-      if (threadIdx.x == 0) {
-        const float xs = sa + a.dt_bias[h];
+    }
+    ss = WarpSum(ss);
+    if (lane == 0) red3[warp] = ss;
+    __syncthreads();
+    ss = WarpSum(lane < per_row && t_ab < T ? red3[t_ab * per_row + lane] : 0.f);
+    const float r = rsqrtf(ss / a.K + a.in_eps);
+    float sa = 0.f, sb = 0.f;
+    auto dots = [&](uint32_t b, uint32_t g, uint32_t va, uint32_t vb) {
+      const uint32_t hh = PackBf16(BfLo(b) * r * (1.f + BfLo(g)), BfHi(b) * r * (1.f + BfHi(g)));
+      sa += BfLo(va) * BfLo(hh) + BfHi(va) * BfHi(hh);
+      sb += BfLo(vb) * BfLo(hh) + BfHi(vb) * BfHi(hh);
+    };
+    auto dots8 = [&](uint4 b, uint4 g, uint4 va, uint4 vb) {
+      dots(b.x, g.x, va.x, vb.x);
+      dots(b.y, g.y, va.y, vb.y);
+      dots(b.z, g.z, va.z, vb.z);
+      dots(b.w, g.w, va.w, vb.w);
+    };
+    if (t_ab < T && wide) {
+      dots8(px, pg, pa, pb);
+#pragma unroll 2
+      for (int k = mine * 8 + 4 * stride; k < a.K; k += 4 * stride)
+        dots8(*reinterpret_cast<const uint4*>(xr + k), *reinterpret_cast<const uint4*>(a.in_norm_w + k),
+              *reinterpret_cast<const uint4*>(wa + k), *reinterpret_cast<const uint4*>(wb + k));
+    } else if (t_ab < T) {
+      for (int k = mine * 2; k < a.K; k += stride)
+        dots(*reinterpret_cast<const uint32_t*>(xr + k), *reinterpret_cast<const uint32_t*>(a.in_norm_w + k),
+             *reinterpret_cast<const uint32_t*>(wa + k), *reinterpret_cast<const uint32_t*>(wb + k));
+    }
+    sa = WarpSum(sa);
+    sb = WarpSum(sb);
+    if (lane == 0) { red[warp] = sa; red2[warp] = sb; }
+    __syncthreads();
+    if (warp < T) {                          // warp t finishes row t
+      sa = WarpSum(lane < per_row ? red[warp * per_row + lane] : 0.f);
+      sb = WarpSum(lane < per_row ? red2[warp * per_row + lane] : 0.f);
+      if (lane == 0) {
+        const float xs = sa + dt_bias;
         const float sp = xs > 20.f ? xs : log1pf(__expf(xs));
-        seg[t] = __expf(-__expf(a.A_log[h]) * sp);
-        sbeta[t] = Sigmoid(sb);
+        seg[warp] = __expf(-__expf(A_log) * sp);
+        sbeta[warp] = Sigmoid(sb);
       }
     }
   } else if (threadIdx.x < T) {
     const int t = threadIdx.x;
     const float av = a.ab[static_cast<size_t>(t) * 2 * a.H + h], bv = a.ab[static_cast<size_t>(t) * 2 * a.H + a.H + h];
-    const float xs = av + a.dt_bias[h];
+    const float xs = av + dt_bias;
     const float sp = xs > 20.f ? xs : log1pf(__expf(xs));
-    seg[t] = __expf(-__expf(a.A_log[h]) * sp);
+    seg[t] = __expf(-__expf(A_log) * sp);
     sbeta[t] = Sigmoid(bv);
   }
   __syncthreads();
@@ -222,8 +315,7 @@ __global__ void __launch_bounds__(kThreads) GdnDecodeKernel(GdnArgs a) {
       for (int c = 0; c < CPL; ++c) s = fmaf(S[r][c] * eg, kc[c], s);
       d1[r] = s;
     }
-#pragma unroll
-    for (int r = 0; r < RPW; ++r) d1[r] = WarpSum(d1[r]);
+    WarpSums(d1);
     float d2[RPW];
 #pragma unroll
     for (int r = 0; r < RPW; ++r) {
@@ -238,11 +330,8 @@ __global__ void __launch_bounds__(kThreads) GdnDecodeKernel(GdnArgs a) {
       d2[r] = s;
       if (lane == 0) a.log_u[(static_cast<size_t>(t) * a.H + h) * D + v] = u;
     }
-#pragma unroll
-    for (int r = 0; r < RPW; ++r) {
-      d2[r] = WarpSum(d2[r]);
-      if (lane == 0) so[t][warp * RPW + r] = d2[r] * scale;
-    }
+    const float o = WarpScatterSum(d2);
+    if (lane % (32 / RPW) == 0) so[t][warp * RPW + WarpScatterIndex<RPW>()] = o * scale;
     if (warp == 0) {
 #pragma unroll
       for (int c = 0; c < CPL; ++c) a.log_k[(static_cast<size_t>(t) * a.H + h) * D + lane * CPL + c] = kc[c];
@@ -251,15 +340,22 @@ __global__ void __launch_bounds__(kThreads) GdnDecodeKernel(GdnArgs a) {
   }
   __syncthreads();
 
-  // ---- phase D: gated RMSNorm ------------------------------------------------------------------
-  for (int t = 0; t < T; ++t) {
-    const float o = threadIdx.x < D ? so[t][threadIdx.x] : 0.f;
-    const float ss = BlockSum(o * o, red);
-    if (threadIdx.x < D) {
-      const float r = rsqrtf(ss / D + a.eps);
-      const float zv = __bfloat162float(a.z[(static_cast<size_t>(t) * a.H + h) * D + threadIdx.x]);
-      a.out[(static_cast<size_t>(t) * a.H + h) * D + threadIdx.x] =
-          __float2bfloat16(o * r * __bfloat162float(a.norm_w[threadIdx.x]) * (a.gate_act ? Sigmoid(zv) : Silu(zv)));
+  // ---- phase D: gated RMSNorm, a warp per row --------------------------------------------------
+  if (warp < T) {
+    const int t = warp;
+    float o[CPL], ss = 0.f;
+#pragma unroll
+    for (int c = 0; c < CPL; ++c) {
+      o[c] = so[t][c * 32 + lane];
+      ss += o[c] * o[c];
+    }
+    const float r = rsqrtf(WarpSum(ss) / D + a.eps);
+#pragma unroll
+    for (int c = 0; c < CPL; ++c) {
+      const int v = c * 32 + lane;
+      const float z = __bfloat162float(zv[c]);
+      a.out[(static_cast<size_t>(t) * a.H + h) * D + v] =
+          __float2bfloat16(o[c] * r * __bfloat162float(nw[c]) * (a.gate_act ? Sigmoid(z) : Silu(z)));
     }
   }
 }

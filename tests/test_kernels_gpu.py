@@ -499,6 +499,37 @@ def test_gdn_decode_with_in_kernel_ab_projection(K, T):
     assert torch.allclose(outs[0], outs[1], atol=2e-2, rtol=2e-2)
 
 
+@pytest.mark.parametrize("T,Kd,shift", [(1, 1032, 0), (2, 4104, 0), (4, 8 * 33, 0), (5, 1026, 0), (7, 520, 2), (8, 8, 0), (8, 5120, 0)])
+def test_gdn_decode_ab_projection_at_odd_widths_and_bases(K, T, Kd, shift):
+    """Widths that end inside a 16-byte load or are no multiple of one, and rows off a 16-byte boundary: the logged decays are those of
+    the same projection in fp64, over the bf16 rounding points of the norm.  A bf16 flip of one normed value moves a sum of Kd products
+    by 2^-8 |h w| <= 2^-8 * 4 * 0.02 = 3e-4, and the decay by at most 1 / e of that (A s e^(-A s))."""
+    g = torch.Generator().manual_seed(T + Kd)
+    D, Hv, Hk = 128, 4, 2
+    conv_dim = 2 * Hk * D + Hv * D
+    x0, nw0, w0 = (torch.empty(n + 8, dtype=BF, device="cuda") for n in (T * Kd, Kd, 2 * Hv * Kd))
+    x, nw, ab_w = x0[shift:shift + T * Kd].view(T, Kd), nw0[shift:shift + Kd], w0[shift:shift + 2 * Hv * Kd].view(2 * Hv, Kd)
+    x.copy_(torch.randn(T, Kd, generator=g))
+    nw.copy_(torch.randn(Kd, generator=g) * 0.1)
+    ab_w.copy_((torch.randn(2 * Hv, Kd, generator=g) * 0.02).clamp(-0.02, 0.02))
+    mixed = (torch.randn(T, conv_dim, generator=g) * 0.5).to(BF).cuda()
+    z = torch.randn(T, Hv * D, generator=g).to(BF).cuda()
+    conv_w = torch.randn(conv_dim, 4, generator=g).to(BF).cuda()
+    A_log, dt_bias = torch.randn(Hv, generator=g) * 0.3, torch.randn(Hv, generator=g) * 0.3
+    ring, state = torch.zeros(16, conv_dim, dtype=BF, device="cuda"), torch.zeros(Hv, D, D, device="cuda")
+    log_u, log_k, log_eg = (torch.zeros(8, Hv, n, device="cuda") for n in (D, D, 1))
+    out = torch.empty(T, Hv * D, dtype=BF, device="cuda")
+    K.gdn_decode(mixed, z, torch.empty(0, device="cuda"), conv_w, A_log.cuda(), dt_bias.cuda(), torch.ones(D, dtype=BF, device="cuda"), ring,
+                 state, log_u, log_k, log_eg, torch.arange(5, 5 + T, dtype=torch.int32, device="cuda"),
+                 torch.zeros(1, dtype=torch.int32, device="cuda"), out, T, Hv, Hk, D, ab_w=ab_w, x=x, in_norm_w=nw, in_eps=1e-6)
+    xf = x.cpu().double()
+    hn = (xf * torch.rsqrt((xf * xf).mean(1, keepdim=True) + 1e-6) * (1 + nw.cpu().double())).to(BF).double()
+    a = hn @ ab_w[:Hv].cpu().double().T
+    want = torch.exp(-torch.exp(A_log.double()) * torch.nn.functional.softplus(a + dt_bias.double()))
+    assert torch.allclose(log_eg.view(-1)[:T * Hv].view(T, Hv).cpu().double(), want, atol=3e-4, rtol=0)
+    assert torch.isfinite(out).all()
+
+
 @pytest.mark.parametrize("D,Hv,Hk", [(128, 6, 2), (64, 4, 2)])
 def test_gdn_decode_matches_recurrence_with_rollback(K, D, Hv, Hk):
     """Rows are fed in windows; only an accepted prefix of each window is committed."""
