@@ -34,10 +34,22 @@ struct TrellisLane {
   }
 };
 
+// 0x6400 + the sum of the four bytes, on the unit of shifts and permutes
+__device__ __forceinline__ uint32_t TrellisByteSumAlu(uint32_t v) {
+  uint32_t r;
+  asm("vabsdiff4.u32.u32.u32.add %0, %1, %2, %3;" : "=r"(r) : "r"(v), "r"(0u), "r"(0x6400u));
+  return r;
+}
+
 // Two code values from two 16-bit states: fp16x2( (1024 + bytesum(s * M)) * scale + bias ).
+// The multiplies, the dot products of bytes and the fp16 multiply-adds share one unit (2 clocks an instruction), shifts and permutes
+// another.  With KB = 4 the states are so cheap to extract that the first is the busier one, so every second byte sum goes to the
+// second (a sum of absolute differences from zero, the same number): 54 -> 50 clocks per 256 weights and scheduler with fp16
+// multiply-adds behind it, 49 -> 47 with mma.sync, 45 -> 43 with stores to shared memory.  With 3 and 5 bits the units are level.
+template <int KB>
 __device__ __forceinline__ __half2 TrellisCode2(uint32_t s0, uint32_t s1) {
   const uint32_t h0 = __dp4a(s0 * R4DXB_TRELLIS_MUL, 0x01010101u, 0x6400u);
-  const uint32_t h1 = __dp4a(s1 * R4DXB_TRELLIS_MUL, 0x01010101u, 0x6400u);
+  const uint32_t h1 = KB == 4 ? TrellisByteSumAlu(s1 * R4DXB_TRELLIS_MUL) : __dp4a(s1 * R4DXB_TRELLIS_MUL, 0x01010101u, 0x6400u);
   const uint32_t packed = __byte_perm(h0, h1, 0x5410);
   const __half2 scale = __halves2half2(__ushort_as_half(R4DXB_TRELLIS_SCALE_F16), __ushort_as_half(R4DXB_TRELLIS_SCALE_F16));
   const __half2 bias = __halves2half2(__ushort_as_half(R4DXB_TRELLIS_BIAS_F16), __ushort_as_half(R4DXB_TRELLIS_BIAS_F16));
@@ -62,16 +74,16 @@ __device__ __forceinline__ void TrellisDecode8(uint32_t hi, uint32_t lo, __half2
     // whole bytes of some 32-bit word and one byte permute against a zero register extracts it
     // (11 instructions for 8 states instead of 15 shifts and masks).
     const uint32_t z = __funnelshift_r(lo, hi, 4), y = __funnelshift_r(lo, hi, 16), u = __funnelshift_r(lo, hi, 20);
-    w[3] = TrellisCode2(__byte_perm(z, 0u, 0x4410), __byte_perm(lo, 0u, 0x4410));     // shifts 4, 0
-    w[2] = TrellisCode2(__byte_perm(z, 0u, 0x4421), __byte_perm(lo, 0u, 0x4421));     // shifts 12, 8
-    w[1] = TrellisCode2(__byte_perm(u, 0u, 0x4410), __byte_perm(y, 0u, 0x4410));      // shifts 20, 16
-    w[0] = TrellisCode2(__byte_perm(u, 0u, 0x4421), __byte_perm(y, 0u, 0x4421));      // shifts 28, 24
+    w[3] = TrellisCode2<KB>(__byte_perm(z, 0u, 0x4410), __byte_perm(lo, 0u, 0x4410));     // shifts 4, 0
+    w[2] = TrellisCode2<KB>(__byte_perm(z, 0u, 0x4421), __byte_perm(lo, 0u, 0x4421));     // shifts 12, 8
+    w[1] = TrellisCode2<KB>(__byte_perm(u, 0u, 0x4410), __byte_perm(y, 0u, 0x4410));      // shifts 20, 16
+    w[0] = TrellisCode2<KB>(__byte_perm(u, 0u, 0x4421), __byte_perm(y, 0u, 0x4421));      // shifts 28, 24
     return;
   }
-  w[0] = TrellisCode2(TrellisStateFromWindow<KB, 0>(hi, lo), TrellisStateFromWindow<KB, 1>(hi, lo));
-  w[1] = TrellisCode2(TrellisStateFromWindow<KB, 2>(hi, lo), TrellisStateFromWindow<KB, 3>(hi, lo));
-  w[2] = TrellisCode2(TrellisStateFromWindow<KB, 4>(hi, lo), TrellisStateFromWindow<KB, 5>(hi, lo));
-  w[3] = TrellisCode2(TrellisStateFromWindow<KB, 6>(hi, lo), TrellisStateFromWindow<KB, 7>(hi, lo));
+  w[0] = TrellisCode2<KB>(TrellisStateFromWindow<KB, 0>(hi, lo), TrellisStateFromWindow<KB, 1>(hi, lo));
+  w[1] = TrellisCode2<KB>(TrellisStateFromWindow<KB, 2>(hi, lo), TrellisStateFromWindow<KB, 3>(hi, lo));
+  w[2] = TrellisCode2<KB>(TrellisStateFromWindow<KB, 4>(hi, lo), TrellisStateFromWindow<KB, 5>(hi, lo));
+  w[3] = TrellisCode2<KB>(TrellisStateFromWindow<KB, 6>(hi, lo), TrellisStateFromWindow<KB, 7>(hi, lo));
 }
 
 // The 16 states of one row of a tile (positions 16 r .. 16 r + 15) out of a 96-bit window x2:x1:x0 that ends with the row's

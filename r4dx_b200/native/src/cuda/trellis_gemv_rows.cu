@@ -211,7 +211,7 @@ __global__ void __launch_bounds__(kInWarps * 32) TrellisRowsInputKernel(RowsArgs
 // two code values of a row of a tile (positions J, J + 1) as an operand register
 template <int KB, int J>
 __device__ __forceinline__ uint32_t Code2(const uint32_t (&w)[3]) {
-  const __half2 q = TrellisCode2(TrellisRow<KB>::template State<J>(w[2], w[1], w[0]), TrellisRow<KB>::template State<J + 1>(w[2], w[1], w[0]));
+  const __half2 q = TrellisCode2<KB>(TrellisRow<KB>::template State<J>(w[2], w[1], w[0]), TrellisRow<KB>::template State<J + 1>(w[2], w[1], w[0]));
   return *reinterpret_cast<const uint32_t*>(&q);
 }
 
