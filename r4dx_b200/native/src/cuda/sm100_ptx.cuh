@@ -353,6 +353,15 @@ __device__ __forceinline__ void UmmaF16FromTmem(uint32_t tmem_d, uint32_t tmem_a
       ::"r"(tmem_d), "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
       : "memory");
 }
+// The same over a pair of CTAs (see UmmaF16Pair): A rows 0..127 from the first CTA's tensor memory, the others from the second's.
+__device__ __forceinline__ void UmmaF16PairFromTmem(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc,
+                                                    uint32_t accumulate) {
+  asm volatile(
+      "{ .reg .pred p; setp.ne.b32 p, %4, 0;\n"
+      "  tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p; }"
+      ::"r"(tmem_d), "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
 // 32 lanes x 8 consecutive 32-bit columns.
 __device__ __forceinline__ void TmemStore32x8(uint32_t taddr, const uint32_t (&r)[8]) {
   asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"

@@ -888,6 +888,38 @@ def test_attention_prefill(K, D, Hq, Hkv, T, ctx, impl):
     assert torch.allclose(out.float().cpu().view(T, Hq, D), o, atol=2e-2, rtol=3e-2)
 
 
+@pytest.mark.parametrize("D,Hq,Hkv,T,ctx,window,gated", [
+    (256, 2, 1, 1, 0, 0, True), (256, 3, 1, 129, 127, 0, True), (256, 3, 3, 128, 0, 0, False), (128, 4, 2, 127, 1, 0, True),
+    (128, 5, 5, 257, 300, 64, True), (256, 4, 2, 260, 500, 130, True), (128, 6, 2, 385, 0, 0, False), (256, 1, 1, 300, 1000, 0, True)])
+def test_attention_prefill_pairs_at_tile_edges(K, D, Hq, Hkv, T, ctx, window, gated):
+    """Two heads or two row tiles to a pair, an empty second tile, tiles of keys that end inside a page, windows that start inside a
+    tile, gate rows off a 16-byte boundary: against fp64 attention over the stored fp8 rows.  Q is rounded to fp16,
+    which moves a score below 5 by at most 5 * 2^-11, and so are the probabilities (2^-11): 6 * 2^-11 of the |v| <= 4 that are
+    averaged is 1.2e-2.  Outputs are rounded to bf16 (2^-9 of them)."""
+    K.set_attn_prefill_impl("tc")
+    g = torch.Generator().manual_seed(T + ctx)
+    total = ctx + T
+    pages = (total + 15) // 16
+    table = torch.randperm(pages, generator=g).to(torch.int32)
+    cache8 = torch.randn(pages, Hkv, 2, 16, D, generator=g).clamp(-4, 4).to(torch.float8_e4m3fn)
+    q = torch.randn(T, Hq, D, generator=g).to(BF)
+    flat = torch.empty(T * Hq * 2 * D + 2, dtype=BF, device="cuda")
+    qg = flat[2 * (T % 2):2 * (T % 2) + T * Hq * 2 * D].view(T, Hq, 2 * D)
+    qg.copy_(torch.randn(T, Hq, 2 * D, generator=g))
+    kd, vd = torch.rand(Hkv, generator=g) * 0.5 + 0.5, torch.rand(Hkv, generator=g) * 0.5 + 0.5
+    out = torch.full((T, Hq, D), float("nan"), dtype=BF, device="cuda")
+    K.attn_prefill(q.cuda(), qg, cache8.view(torch.uint8).cuda(), table.cuda(), kd.cuda(), vd.cuda(), out, T, Hq, Hkv, D, ctx, gated, window)
+    rows = cache8.double()[table.long()].permute(2, 1, 0, 3, 4).reshape(2, Hkv, pages * 16, D)[:, :, :total]
+    k, v = (rows[i].repeat_interleave(Hq // Hkv, 0) * s.double().repeat_interleave(Hq // Hkv)[:, None, None] for i, s in ((0, kd), (1, vd)))
+    sc = torch.einsum("thd,hkd->htk", q.double(), k) / D ** 0.5
+    pos, kp = torch.arange(ctx, total)[:, None], torch.arange(total)[None]
+    sc = sc.masked_fill((kp > pos) | ((kp <= pos - window) if window else torch.zeros_like(kp > pos)), float("-inf"))
+    want = torch.einsum("htk,hkd->thd", sc.softmax(-1), v)
+    if gated:
+        want = want * torch.sigmoid(qg.cpu()[..., D:].double())
+    assert torch.allclose(out.cpu().double(), want, atol=2e-2, rtol=2 ** -8)
+
+
 @pytest.mark.parametrize("T", [1, 3, 8])
 def test_trellis_gemv_fused_prologues_equal_the_unfused_chain(K, T):
     """RMSNorm / SwiGLU folded into the GEMV prologue give the same bits as the separate kernels."""
