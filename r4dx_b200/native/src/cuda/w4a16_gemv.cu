@@ -328,7 +328,7 @@ int r4dxb_w4a16_gemv(const void* wq, const void* wsz, const void* x, void* y, in
                      int out_f32, void* stream) {
   if (T < 1 || T > 8 || K % 32 || (group != 32 && group != 64 && group != 128) || K % group) return R4DXB_BAD_ARG;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  // whole tiles and chunks stream through mma.sync (w4a16_mma.cu: 172 us for a 248320 x 5120 head at 1..8 rows, this file's
+  // whole tiles and chunks stream through mma.sync (w4a16_mma.cu: 153 us for a 248320 x 5120 head at 1..8 rows, this file's
   // kernel 218 us at one row and 2414 us at eight); the kernel here takes what is left over
   if (W4MmaCovers(wq, x, T, N, K, group)) return W4Mma(wq, wsz, x, y, T, N, K, group, out_f32, s);
   if (T == 1) return LaunchW4<1>(wq, wsz, x, y, T, N, K, group, out_f32, s);

@@ -9,12 +9,15 @@
 // 109 us.  Here m16n8k16 takes 16 weight rows times 8 rows of x per instruction, so the cost hardly depends on T:
 // (n - zero) is exact in fp16, products and sums are fp32, and the group's scale multiplies the group sum in fp32.
 //
-// Layout: a warp owns 16 weight rows at a time and keeps the next four groups' words of them in flight in registers, loaded
-// straight from global memory: lane c of a quad takes words c * G / 32 .. of each group, so a quad's loads are whole sectors
-// and all columns of an MMA share one group.  Sixteen warps per SM hold about 32 KB in flight; nothing synchronises across
-// warps after the rows of x are staged.  (A ring of bulk copies into shared memory per warp, 16 copies of 256 bytes a stage,
-// took 262 us at 248320 x 5120: the copy engine, not the math, set the pace.)  x is staged in the nibble order
-// 0,4,1,5,2,6,3,7, so the 16 bytes of x behind one word of weights are one shared-memory load.
+// Layout: a warp owns 16 weight rows at a time and keeps the next chunks' words of them (four groups each) in flight in registers,
+// loaded straight from global memory: lane c of a quad takes words c * G / 32 .. of each group, so a quad's loads are whole
+// sectors and all columns of an MMA share one group.  A ring slot is refilled group by group as its words are widened, through
+// pointers that move along: with the words copied out first, and zeros put in place of absent rows of x, the kernel issued 49
+// instructions per 512 weights and scheduler, 71 % of its slots, for 166 us at 1 row and 234 at 16; now 153 and 208.  What is left
+// is the L1 (89 %): a load of 32-byte sectors from eight rows looks up eight lines.  Nothing synchronises across warps after the
+// rows of x are staged.  (A ring of bulk copies into shared memory per warp, 16 copies of 256 bytes a stage, took 262 us at
+// 248320 x 5120: the copy engine, not the math, set the pace.)  x is staged in the nibble order 0,4,1,5,2,6,3,7, so the 16 bytes of
+// x behind one word of weights are one shared-memory load.
 #include "common.cuh"
 
 namespace r4dxb {
@@ -56,12 +59,16 @@ __device__ __forceinline__ void LoadStream(const uint32_t* p, uint32_t (&o)[V]) 
   }
 }
 
+// chunks in flight per warp: what 128 registers allow
+template <int NT, int G>
+constexpr int Chunks() { return G == 32 ? 4 : (G == 64 ? 3 : (NT == 1 ? 2 : 1)); }
+
 template <int NT, int G>
 __global__ void __launch_bounds__(kW4Threads, 1)
 W4MmaKernel(const uint32_t* __restrict__ wq, const uint32_t* __restrict__ wsz, const __nv_bfloat16* __restrict__ x,
             void* __restrict__ y, int T, int N, int K, int out_f32, int slices) {
   constexpr int V = G / 32;                        // words a lane takes of a row's group
-  constexpr int D = NT == 1 && G == 64 ? 2 : 1;    // chunks in flight per warp (what the registers allow)
+  constexpr int D = Chunks<NT, G>();               // chunks in flight per warp
   extern __shared__ __align__(128) unsigned char xs[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, c = lane & 3;
   const int xstride = K * 2 + 16;                  // bytes: the eight rows of a fragment start 16 bytes apart modulo the banks
@@ -71,24 +78,35 @@ W4MmaKernel(const uint32_t* __restrict__ wq, const uint32_t* __restrict__ wsz, c
   const int step = gridDim.x * (kWarps / slices);
   int tile = blockIdx.x + gridDim.x * (warp / slices), chunk = c_lo;
   uint32_t w0[D][kChunk][V], w1[D][kChunk][V], sz[D][2];
-  int load_tile = tile, load_chunk = c_lo;                     // the next chunk to load
-  auto load = [&](uint32_t (&w0)[kChunk][V], uint32_t (&w1)[kChunk][V], uint32_t (&sz)[2]) {
+  // the next chunk to load; a ring slot is refilled group by group as its words are widened
+  int load_tile = tile, load_chunk = c_lo;
+  const size_t row8 = static_cast<size_t>(8) * (K / 8);
+  const uint32_t* lp = wq + (static_cast<size_t>(tile) * 16 + g) * (K / 8) + c_lo * (kChunk * G / 8) + c * V;
+  const uint32_t* ls = wsz + (static_cast<size_t>(tile) * 16 + g) * groups + c_lo * kChunk + c;
+  auto load_group = [&](int i, uint32_t (&o0)[V], uint32_t (&o1)[V]) {
     if (load_tile >= tiles) return;
-    const int tl = load_tile, ch = load_chunk;
-    if (++load_chunk == c_hi) { load_chunk = c_lo; load_tile += step; }
-    const uint32_t* p0 = wq + (static_cast<size_t>(tl) * 16 + g) * (K / 8) + ch * (kChunk * G / 8) + c * V;
-    const uint32_t* p1 = p0 + static_cast<size_t>(8) * (K / 8);
-#pragma unroll
-    for (int i = 0; i < kChunk; ++i) {
-      LoadStream<V>(p0 + i * (G / 8), w0[i]);
-      LoadStream<V>(p1 + i * (G / 8), w1[i]);
+    LoadStream<V>(lp + i * (G / 8), o0);
+    LoadStream<V>(lp + row8 + i * (G / 8), o1);
+  };
+  auto load_scales = [&](uint32_t (&o)[2]) {       // and on to the next chunk
+    if (load_tile >= tiles) return;
+    o[0] = __ldg(ls);
+    o[1] = __ldg(ls + static_cast<size_t>(8) * groups);
+    lp += kChunk * G / 8;
+    ls += kChunk;
+    if (++load_chunk == c_hi) {
+      load_chunk = c_lo;
+      load_tile += step;
+      lp = wq + (static_cast<size_t>(load_tile) * 16 + g) * (K / 8) + c_lo * (kChunk * G / 8) + c * V;
+      ls = wsz + (static_cast<size_t>(load_tile) * 16 + g) * groups + c_lo * kChunk + c;
     }
-    const uint32_t* ps = wsz + (static_cast<size_t>(tl) * 16 + g) * groups + ch * kChunk + c;
-    sz[0] = __ldg(ps);
-    sz[1] = __ldg(ps + static_cast<size_t>(8) * groups);
   };
 #pragma unroll
-  for (int d = 0; d < D; ++d) load(w0[d], w1[d], sz[d]);
+  for (int d = 0; d < D; ++d) {
+#pragma unroll
+    for (int i = 0; i < kChunk; ++i) load_group(i, w0[d][i], w1[d][i]);
+    load_scales(sz[d]);
+  }
 
   // rows of x, fp16, in nibble order, while the first words are on their way
   for (int i = threadIdx.x; i < T * (K / 8); i += kW4Threads) {
@@ -122,65 +140,68 @@ W4MmaKernel(const uint32_t* __restrict__ wq, const uint32_t* __restrict__ wsz, c
         }
       }
   };
-  while (tile < tiles) {
-    // (the words of this chunk, then the loads of the next one, then the products)
-    uint32_t a0[kChunk][V], a1[kChunk][V];
-    const uint32_t cs0 = sz[0][0], cs1 = sz[0][1];
+  // rows past T take the last one's x: their columns of the product are never stored
+  const unsigned char* xrow[NT];
 #pragma unroll
-    for (int i = 0; i < kChunk; ++i)
+  for (int nt = 0; nt < NT; ++nt) xrow[nt] = xs + static_cast<size_t>(min(nt * 8 + g, T - 1)) * xstride + c * (V * 16);
+  bool live = tile < tiles;
+  while (live) {
 #pragma unroll
-      for (int v = 0; v < V; ++v) {
-        a0[i][v] = w0[0][i][v];
-        a1[i][v] = w1[0][i][v];
-        if constexpr (D == 2) { w0[0][i][v] = w0[1][i][v]; w1[0][i][v] = w1[1][i][v]; }
-      }
-    if constexpr (D == 2) { sz[0][0] = sz[1][0]; sz[0][1] = sz[1][1]; }
-    load(w0[D - 1], w1[D - 1], sz[D - 1]);
-    const unsigned char* xp = xs + static_cast<size_t>(g) * xstride + static_cast<size_t>(chunk) * (kChunk * G * 2) + c * (V * 16);
+    for (int d = 0; d < D; ++d) {
+      if (!live) break;
+      const unsigned char* xp[NT];
 #pragma unroll
-    for (int gi = 0; gi < kChunk; ++gi) {
-      float acc[NT][4];
+      for (int nt = 0; nt < NT; ++nt) xp[nt] = xrow[nt] + chunk * (kChunk * G * 2);
 #pragma unroll
-      for (int nt = 0; nt < NT; ++nt)
+      for (int gi = 0; gi < kChunk; ++gi) {
+        float acc[NT][4];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) acc[nt][j] = 0.f;
-      const uint32_t s0 = __shfl_sync(0xffffffffu, cs0, (lane & ~3) | gi), s1 = __shfl_sync(0xffffffffu, cs1, (lane & ~3) | gi);
-      const uint32_t z0 = __byte_perm(s0, 0u, 0x3232), z1 = __byte_perm(s1, 0u, 0x3232);
-      const __half2 k960 = __float2half2_rn(960.f);
-      const __half2 nz0 = *reinterpret_cast<const __half2*>(&z0), nz1 = *reinterpret_cast<const __half2*>(&z1);
-      const __half2 nzs0 = __hadd2(nz0, k960), nzs1 = __hadd2(nz1, k960);       // -(64 + zero)
+        for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
-      for (int v = 0; v < V; ++v) {
-        uint32_t a[4], b[4];
-        Widen(a0[gi][v], nz0, nzs0, a);
-        Widen(a1[gi][v], nz1, nzs1, b);
+          for (int j = 0; j < 4; ++j) acc[nt][j] = 0.f;
+        const uint32_t s0 = __shfl_sync(0xffffffffu, sz[d][0], (lane & ~3) | gi), s1 = __shfl_sync(0xffffffffu, sz[d][1], (lane & ~3) | gi);
+        const uint32_t z0 = __byte_perm(s0, 0u, 0x3232), z1 = __byte_perm(s1, 0u, 0x3232);
+        const __half2 k960 = __float2half2_rn(960.f);
+        const __half2 nz0 = *reinterpret_cast<const __half2*>(&z0), nz1 = *reinterpret_cast<const __half2*>(&z1);
+        const __half2 nzs0 = __hadd2(nz0, k960), nzs1 = __hadd2(nz1, k960);       // -(64 + zero)
+#pragma unroll
+        for (int v = 0; v < V; ++v) {
+          uint32_t a[4], b[4];
+          Widen(w0[d][gi][v], nz0, nzs0, a);
+          Widen(w1[d][gi][v], nz1, nzs1, b);
+#pragma unroll
+          for (int nt = 0; nt < NT; ++nt) {
+            const uint4 xv = *reinterpret_cast<const uint4*>(xp[nt] + gi * (G * 2) + v * 16);
+            MmaF16(acc[nt], a[0], b[0], a[1], b[1], xv.x, xv.y);
+            MmaF16(acc[nt], a[2], b[2], a[3], b[3], xv.z, xv.w);
+          }
+        }
+        load_group(gi, w0[d][gi], w1[d][gi]);
+        const float f0 = __half2float(__ushort_as_half(static_cast<unsigned short>(s0 & 0xFFFFu)));
+        const float f1 = __half2float(__ushort_as_half(static_cast<unsigned short>(s1 & 0xFFFFu)));
 #pragma unroll
         for (int nt = 0; nt < NT; ++nt) {
-          uint4 xv = make_uint4(0u, 0u, 0u, 0u);
-          if (nt * 8 + g < T) xv = *reinterpret_cast<const uint4*>(xp + static_cast<size_t>(nt * 8) * xstride + gi * (G * 2) + v * 16);
-          MmaF16(acc[nt], a[0], b[0], a[1], b[1], xv.x, xv.y);
-          MmaF16(acc[nt], a[2], b[2], a[3], b[3], xv.z, xv.w);
+          tot[nt][0] = fmaf(acc[nt][0], f0, tot[nt][0]);
+          tot[nt][1] = fmaf(acc[nt][1], f0, tot[nt][1]);
+          tot[nt][2] = fmaf(acc[nt][2], f1, tot[nt][2]);
+          tot[nt][3] = fmaf(acc[nt][3], f1, tot[nt][3]);
         }
       }
-      const float f0 = __half2float(__ushort_as_half(static_cast<unsigned short>(s0 & 0xFFFFu)));
-      const float f1 = __half2float(__ushort_as_half(static_cast<unsigned short>(s1 & 0xFFFFu)));
+      load_scales(sz[d]);
+      if (++chunk == c_hi) {
+        if (slices > 1) {
+          live = false;
+          break;
+        }
+        store(tile, tot);
 #pragma unroll
-      for (int nt = 0; nt < NT; ++nt) {
-        tot[nt][0] = fmaf(acc[nt][0], f0, tot[nt][0]);
-        tot[nt][1] = fmaf(acc[nt][1], f0, tot[nt][1]);
-        tot[nt][2] = fmaf(acc[nt][2], f1, tot[nt][2]);
-        tot[nt][3] = fmaf(acc[nt][3], f1, tot[nt][3]);
+        for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+          for (int j = 0; j < 4; ++j) tot[nt][j] = 0.f;
+        chunk = c_lo;
+        tile += step;
+        live = tile < tiles;
       }
-    }
-    if (++chunk == c_hi) {
-      if (slices > 1) break;
-      store(tile, tot);
-#pragma unroll
-      for (int nt = 0; nt < NT; ++nt)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) tot[nt][j] = 0.f;
-      chunk = c_lo;
-      tile += step;
     }
   }
   if (slices > 1) {
