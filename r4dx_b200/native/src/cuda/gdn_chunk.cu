@@ -10,7 +10,10 @@
 //           solve for U~ = (I + A)^-1 beta V and W = (I + A)^-1 beta gamma K by forward substitution,
 //           one right-hand-side column per thread with the 64 unknowns in registers.  The solve is right-looking (a
 //           solved unknown is subtracted from all later ones at once): the sums are independent, where adding up
-//           unknown i's terms when its turn comes is a chain of i multiply-adds behind a global load;
+//           unknown i's terms when its turn comes is a chain of i multiply-adds behind a global load.  What bounds it is the
+//           fp32 multiply-adds of the two products and the solve (packed in pairs: 27k of a CTA's 41k clocks, two CTAs to an SM)
+//           and the waits for the rows between them: 601 -> 468 us for 8192 tokens of 48 heads with pairs and with the rows
+//           of q and k copied asynchronously (three CTAs to an SM, in 80 registers with spills: 628);
 //   phase B (grid heads x 2 or 4 row blocks of the state, sequential over chunks): U = U~ - W S0^T,
 //           O, and the state update as TF32 tensor-core products (mma.sync m16n8k8, fp32
 //           accumulate) out of shared memory; W, Q, P and K have a cp.async slot each that is refilled for the
@@ -24,6 +27,7 @@
 #include <cuda_pipeline.h>
 
 #include "common.cuh"
+#include "sm100_ptx.cuh"
 
 namespace r4dxb {
 namespace {
@@ -48,11 +52,10 @@ __device__ __forceinline__ uint32_t Tf32(float x) {
   return r;
 }
 
-__device__ __forceinline__ float Dot4(const float4& a, const float4& b, float acc) {
-  acc = fmaf(a.x, b.x, acc);
-  acc = fmaf(a.y, b.y, acc);
-  acc = fmaf(a.z, b.z, acc);
-  return fmaf(a.w, b.w, acc);
+// two products and two sums an instruction, the even and the odd columns apart
+__device__ __forceinline__ float2 Dot4(const float4& a, const float4& b, float2 acc) {
+  acc = ptx::Fma2(make_float2(a.x, a.y), make_float2(b.x, b.y), acc);
+  return ptx::Fma2(make_float2(a.z, a.w), make_float2(b.z, b.w), acc);
 }
 
 // grid (chunks, H), 256 threads
@@ -67,17 +70,19 @@ __global__ void __launch_bounds__(256) GdnChunkPrepKernel(const float* __restric
   const int t0 = c * kC, tid = threadIdx.x;
   const size_t ch = static_cast<size_t>(c) * H + h;
 
+  // all rows in flight at once, zeros past the last token (through registers, two loads a step, this was 10k clocks of 41k a CTA)
+#pragma unroll
   for (int i = tid; i < kC * kD / 4; i += 256) {
     const int row = i / (kD / 4), off = (i % (kD / 4)) * 4;
-    const int t = t0 + row;
-    float4 kv = make_float4(0.f, 0.f, 0.f, 0.f), qv = kv;
-    if (t < T) {
-      kv = *reinterpret_cast<const float4*>(k + (static_cast<size_t>(t) * Hk + hk) * kD + off);
-      qv = *reinterpret_cast<const float4*>(q + (static_cast<size_t>(t) * Hk + hk) * kD + off);
-    }
-    *reinterpret_cast<float4*>(&sm.ks[row][off]) = kv;
-    *reinterpret_cast<float4*>(&sm.qs[row][off]) = qv;
+    const size_t at = (static_cast<size_t>(min(t0 + row, T - 1)) * Hk + hk) * kD + off;
+    const size_t zeros = t0 + row < T ? 0 : 16;
+    __pipeline_memcpy_async(&sm.ks[row][off], k + at, 16, zeros);
+    __pipeline_memcpy_async(&sm.qs[row][off], q + at, 16, zeros);
   }
+  __pipeline_commit();
+  // the right-hand sides are read after the products: a line of v per thread on its way to L2 until then
+  if (t0 + tid / 4 < T)
+    asm volatile("prefetch.global.L2 [%0];" ::"l"(v + (static_cast<size_t>(t0 + tid / 4) * H + h) * kD + tid % 4 * 32));
   if (tid < kC) {
     const int t = t0 + tid;
     // rows past the end are identity steps: decay 1, beta 0
@@ -103,17 +108,18 @@ __global__ void __launch_bounds__(256) GdnChunkPrepKernel(const float* __restric
     sm.G[tid] = sum;
     sm.BG[tid] = sm.B[tid] * expf(sum);
   }
+  __pipeline_wait_prior(0);
   __syncthreads();
   if (tid < kC) ws_g[ch * kC + tid] = sm.G[tid];
 
   // ---- k.k and q.k for the lower triangle: thread (ty, tx) owns rows ty + 16 rr, columns tx + 16 cc ----
   {
     const int ty = tid >> 4, tx = tid & 15;
-    float kk[4][4], qk[4][4];
+    float2 kk[4][4], qk[4][4];
 #pragma unroll
     for (int rr = 0; rr < 4; ++rr)
 #pragma unroll
-      for (int cc = 0; cc < 4; ++cc) kk[rr][cc] = qk[rr][cc] = 0.f;
+      for (int cc = 0; cc < 4; ++cc) kk[rr][cc] = qk[rr][cc] = make_float2(0.f, 0.f);
     for (int kq = 0; kq < kD; kq += 4) {
       float4 kr[4], qr[4], kc[4];
 #pragma unroll
@@ -137,8 +143,8 @@ __global__ void __launch_bounds__(256) GdnChunkPrepKernel(const float* __restric
       for (int cc = 0; cc < 4; ++cc) {
         const int i = ty + 16 * rr, j = tx + 16 * cc;
         const float decay = j <= i ? expf(sm.G[i] - sm.G[j]) : 0.f;
-        if (j < i) sm.At[j][i] = -(sm.B[i] * decay * kk[rr][cc]);
-        ws_p[(ch * kC + i) * kC + j] = __uint_as_float(Tf32(decay * qk[rr][cc]));     // (as phase B's product takes it)
+        if (j < i) sm.At[j][i] = -(sm.B[i] * decay * (kk[rr][cc].x + kk[rr][cc].y));
+        ws_p[(ch * kC + i) * kC + j] = __uint_as_float(Tf32(decay * (qk[rr][cc].x + qk[rr][cc].y)));     // (as phase B's product takes it)
       }
   }
   __syncthreads();
@@ -148,29 +154,32 @@ __global__ void __launch_bounds__(256) GdnChunkPrepKernel(const float* __restric
     const bool is_u = tid < kD;
     const int col = is_u ? tid : tid - kD;
     float* dst = (is_u ? ws_ut : ws_w) + ch * kC * kD + col;
-    float x[kC];
+    float2 x[kC / 2];                        // unknowns 2 p and 2 p + 1
+    auto at = [&](int i) -> float& { return i & 1 ? x[i >> 1].y : x[i >> 1].x; };
     if (is_u) {
       const float* src = v + (static_cast<size_t>(t0) * H + h) * kD + col;
 #pragma unroll
-      for (int i = 0; i < kC; ++i) x[i] = t0 + i < T ? src[static_cast<size_t>(i) * H * kD] : 0.f;
+      for (int i = 0; i < kC; ++i) at(i) = t0 + i < T ? src[static_cast<size_t>(i) * H * kD] : 0.f;
 #pragma unroll
-      for (int i = 0; i < kC; ++i) x[i] *= sm.B[i];
+      for (int i = 0; i < kC; ++i) at(i) *= sm.B[i];
     } else {
 #pragma unroll
-      for (int i = 0; i < kC; ++i) x[i] = sm.BG[i] * sm.ks[i][col];
+      for (int i = 0; i < kC; ++i) at(i) = sm.BG[i] * sm.ks[i][col];
     }
 #pragma unroll
     for (int j = 0; j < kC; ++j) {
+      const float xj = at(j);
+      const float2 xj2 = make_float2(xj, xj);
 #pragma unroll
       for (int i4 = ((j + 1) / 4) * 4; i4 < kC; i4 += 4) {
         const float4 a = *reinterpret_cast<const float4*>(&sm.At[j][i4]);
-        if (i4 > j) x[i4] = fmaf(a.x, x[j], x[i4]);
-        if (i4 + 1 > j) x[i4 + 1] = fmaf(a.y, x[j], x[i4 + 1]);
-        if (i4 + 2 > j) x[i4 + 2] = fmaf(a.z, x[j], x[i4 + 2]);
-        if (i4 + 3 > j) x[i4 + 3] = fmaf(a.w, x[j], x[i4 + 3]);
+        if (i4 > j) x[i4 / 2] = ptx::Fma2(make_float2(a.x, a.y), xj2, x[i4 / 2]);
+        else if (i4 + 1 > j) x[i4 / 2].y = fmaf(a.y, xj, x[i4 / 2].y);
+        if (i4 + 2 > j) x[i4 / 2 + 1] = ptx::Fma2(make_float2(a.z, a.w), xj2, x[i4 / 2 + 1]);
+        else if (i4 + 3 > j) x[i4 / 2 + 1].y = fmaf(a.w, xj, x[i4 / 2 + 1].y);
       }
       // W is an operand of phase B's tensor-core products only: rounded here instead of at every read
-      dst[static_cast<size_t>(j) * kD] = is_u ? x[j] : __uint_as_float(Tf32(x[j]));
+      dst[static_cast<size_t>(j) * kD] = is_u ? xj : __uint_as_float(Tf32(xj));
     }
   }
 }
