@@ -167,8 +167,10 @@ class MoeBlock:
                                    P, d.E, d.N, d.K, d.kb, self.xh_pairs, tile_rows=8)
             return
         avg = max(1, P // experts)
-        # the weights of an expert are decoded once per token tile, so a tile should hold all of an expert's rows
-        tn = 16 if avg <= 12 else (32 if avg <= 24 else (64 if avg <= 48 else (128 if avg <= 100 else 256)))
+        # the weights of an expert are decoded once per token tile, so a tile should hold all of an expert's rows, with room for
+        # uneven routing.  Between 48 and 80 rows per expert a tile of 96 carries less padding than one of 128 (us a block of 512
+        # experts: 1006 / 1033 at 51, 1071 / 1129 at 64, 1204 / 1219 at 80); above, too many experts need a second one (1430 / 1283 at 92).
+        tn = 16 if avg <= 12 else (32 if avg <= 24 else (64 if avg <= 48 else (96 if avg <= 80 else (128 if avg <= 100 else 256))))
         K.moe_tiles(self.offsets, self.e_count, tn, self.tiles, self.ntiles)
         xh = self.xh_pairs.view(-1)[:P * g.K].view(P, g.K)
         K.trellis_input_grouped(h, g.suh, xh, self.offsets, self.perm, P, self.k, 0)

@@ -560,6 +560,7 @@ int LaunchGrouped(const void* xh, const ProductArgs& a, int tn, int decode_warps
       case 16: return Launch<KB, 16, 8, false, true>(xh, a, 1, s);
       case 32: return Launch<KB, 32, 8, false, true>(xh, a, 1, s);
       case 64: return Launch<KB, 64, 8, false, true>(xh, a, 1, s);
+      case 96: return Launch<KB, 96, 8, false, true>(xh, a, 1, s);
       case 128: return Launch<KB, 128, 8, false, true>(xh, a, 1, s);
       default: return R4DXB_BAD_ARG;
     }
@@ -568,6 +569,7 @@ int LaunchGrouped(const void* xh, const ProductArgs& a, int tn, int decode_warps
     case 16: return Launch<KB, 16, 16, false, true>(xh, a, 1, s);
     case 32: return Launch<KB, 32, 16, false, true>(xh, a, 1, s);
     case 64: return Launch<KB, 64, 16, false, true>(xh, a, 1, s);
+    case 96: return Launch<KB, 96, 16, false, true>(xh, a, 1, s);
     case 128: return Launch<KB, 128, 16, false, true>(xh, a, 1, s);
     case 256: return Launch<KB, 256, 16, false, true>(xh, a, 1, s);
     default: return R4DXB_BAD_ARG;

@@ -1118,6 +1118,35 @@ def test_grouped_expert_gemm_matches_the_per_pair_reference(K, kb, tn, T):
     assert checked > T
 
 
+@pytest.mark.parametrize("kb,rows,warps", [(3, 95, 0), (4, 96, 0), (5, 97, 0), (4, 193, 16)])
+def test_grouped_expert_gemm_in_tiles_of_96(K, kb, rows, warps):
+    """A tile one row short, full, and with a remainder: a row's sums do not depend on the tile it lies in, so the results are those of
+    tiles of 64 to the bit; rows of other experts are left alone."""
+    from r4dx_b200 import native
+    from r4dx_b200.models.moe import ExpertStack
+    from r4dx_b200.quant import trellis
+    E, N, Kd = 3, 256, 512
+    st = ExpertStack.from_list([trellis.random_weight(N, Kd, kb, seed=e, sigma=0.06).to("cuda") for e in range(E)])
+    off = torch.tensor([0, rows, rows, rows + 40], dtype=torch.int32, device="cuda")       # the second expert has none
+    P = rows + 40
+    g = torch.Generator().manual_seed(rows)
+    perm = torch.randperm(P, generator=g).to(torch.int32).cuda()
+    xh = torch.randn(P, Kd, generator=g).half().cuda()
+    outs = []
+    try:
+        for tn in (96, 64):
+            native.cuda().r4dxb_set_gemm_decode_warps(warps if tn == 96 else 0)
+            tiles, nt = torch.zeros(2 * (P // 64 + E), dtype=torch.int32, device="cuda"), torch.zeros(1, dtype=torch.int32, device="cuda")
+            K.moe_tiles(off, E, tn, tiles, nt)
+            y = torch.full((P + 1, N), float("nan"), dtype=BF, device="cuda")
+            K.trellis_gemm_grouped(st.words, st.svh, xh, y, off, perm, tiles, nt, P, E, N, Kd, kb, tn)
+            outs.append(y)
+        K.check_gemm_status(y.device)
+    finally:
+        native.cuda().r4dxb_set_gemm_decode_warps(0)
+    assert torch.equal(outs[0][:P], outs[1][:P]) and bool(outs[0][P].isnan().all())
+
+
 def test_topk_lse_summary_and_device_rep_penalty(K):
     from r4dx_b200.runtime.sampler import SampleParams, sample_canonical, sample_from_summary
     g = torch.Generator().manual_seed(12)
