@@ -102,11 +102,11 @@ def main() -> None:
                 x = torch.randn(Tg, Kd, device=dev).to(BF)
                 xh = K.trellis_input(x, w.suh)
                 y = torch.empty(Tg, N, dtype=BF, device=dev)
-                tn = a.tn or K.pick_token_tile(Tg, N)
-                us = timed(lambda: K.trellis_gemm(w, xh, out=y, tn=tn), a.iters, flush)
+                tn, ks = (a.tn, 1) if a.tn else K.pick_product(Tg, N, Kd)
+                us = timed(lambda: K.trellis_gemm(w, xh, out=y, tn=tn, ksplit=ks), a.iters, flush)
                 K.check_gemm_status(dev)
                 tf = 2.0 * N * Kd * Tg / us / 1e6
-                print(f"trellis_gemm {name:12s} N={N:6d} K={Kd:6d} kb={kb} T={Tg} tn={tn}: {us:9.1f} us  "
+                print(f"trellis_gemm {name:12s} N={N:6d} K={Kd:6d} kb={kb} T={Tg} tn={tn} split={ks}: {us:9.1f} us  "
                       f"{tf:7.1f} TFLOP/s  {tf / tf_peak:5.2f} of measured cuBLAS bf16")
                 if a.f8:
                     xq, sc = K.quantize_rows_e4m3(xh)

@@ -5,7 +5,7 @@
 For every linear shape of the 27B hybrid geometry, at every requested tensor-parallel degree's shard shape, the tool
 times the weight-streaming kernel at each cluster split (1 / 2 / 4 / 8) and the tcgen05 GEMM at each token tile
 (128 / 256 / 512), cold (a buffer larger than L2 is rewritten between launches), and writes the winners to
-``r4dx_b200/ops/tuning_table.json``.  ``ops/kernels.py:pick_ksplit`` / ``pick_token_tile`` look a shape up there first
+``r4dx_b200/ops/tuning_table.json``.  ``ops/kernels.py:pick_ksplit`` / ``pick_product`` look a shape up there first
 and fall back to their heuristics for shapes the table does not hold.  An entry is only written when its winner beats the
 heuristic's choice by more than ``--min-gain`` (default 5 %): the table records measured exceptions, not noise.
 
@@ -81,10 +81,13 @@ def main() -> None:
                 x = torch.randn(T, Kd, device=dev).to(BF)
                 xh = K.trellis_input(x, w.suh)
                 y = torch.empty(T, N, dtype=BF, device=dev)
-                base = K.pick_token_tile(T, N)
+                base, base_split = K.pick_product(T, N, Kd)
                 res = {}
-                for tn in (128, 256, 512):
-                    if tn > max(128, T):
+                for tn in (128, 192, 256, 384, 512):
+                    if tn > max(128, T) and tn != base:
+                        continue
+                    if tn == base:           # (with the split that goes with it; a table entry stands for an unsplit product)
+                        res[tn] = timed(lambda: K.trellis_gemm(w, xh, out=y, tn=tn, ksplit=base_split), max(4, a.iters // 2), flush)
                         continue
                     res[tn] = timed(lambda: K.trellis_gemm(w, xh, out=y, tn=tn), max(4, a.iters // 2), flush)
                 K.check_gemm_status(dev)
