@@ -23,6 +23,58 @@ __global__ void EmbedGatherKernel(const int* __restrict__ ids, const uint4* __re
 }
 
 // mode bit 0: weight is zero-centred (multiply by 1 + w); bit 1: no weight.
+// A row of a few kilobytes is a chain of memory latencies, so rows of up to kRegColumns columns have all their loads in flight at once
+// and stay in registers; longer ones pass through shared memory, 512 columns a step.  The sums are the same in both.  5120 columns,
+// 1 / 16 / 333 / 8192 rows: 2.6 / 2.8 / 3.8 / 44 us (5.1 / 5.1 / 5.6 / 59 through shared memory).
+constexpr int kRegPairs = 16;
+constexpr int kRegColumns = kRegPairs * 2 * kRowThreads;
+
+template <bool kAdd>
+__global__ void __launch_bounds__(kRowThreads) RmsNormRowKernel(__nv_bfloat16* __restrict__ res, const __nv_bfloat16* __restrict__ delta,
+                                                                const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ out,
+                                                                int H, float eps, int mode) {
+  __shared__ float red[32];
+  const size_t base = static_cast<size_t>(blockIdx.x) * H;
+  uint32_t v[kRegPairs], d[kAdd ? kRegPairs : 1], g[kRegPairs];
+#pragma unroll
+  for (int k = 0; k < kRegPairs; ++k) {
+    const int i = (k * kRowThreads + threadIdx.x) * 2;
+    if (i < H) {
+      v[k] = *reinterpret_cast<const uint32_t*>(res + base + i);
+      if constexpr (kAdd) d[k] = *reinterpret_cast<const uint32_t*>(delta + base + i);
+      if (!(mode & 2)) g[k] = *reinterpret_cast<const uint32_t*>(w + i);
+    }
+  }
+  float ss = 0.0f;
+#pragma unroll
+  for (int k = 0; k < kRegPairs; ++k) {
+    const int i = (k * kRowThreads + threadIdx.x) * 2;
+    if (i < H) {
+      if constexpr (kAdd) {                  // the residual stream is bf16: round, then normalise what is stored
+        v[k] = PackBf16(BfLo(v[k]) + BfLo(d[k]), BfHi(v[k]) + BfHi(d[k]));
+        *reinterpret_cast<uint32_t*>(res + base + i) = v[k];
+      }
+      const float a = BfLo(v[k]), b = BfHi(v[k]);
+      ss += a * a + b * b;
+    }
+  }
+  ss = BlockSum(ss, red);
+  const float r = rsqrtf(ss / H + eps);
+#pragma unroll
+  for (int k = 0; k < kRegPairs; ++k) {
+    const int i = (k * kRowThreads + threadIdx.x) * 2;
+    if (i < H) {
+      float wa = 1.0f, wb = 1.0f;
+      if (!(mode & 2)) {
+        wa = BfLo(g[k]);
+        wb = BfHi(g[k]);
+        if (mode & 1) { wa += 1.0f; wb += 1.0f; }
+      }
+      *reinterpret_cast<uint32_t*>(out + base + i) = PackBf16(BfLo(v[k]) * r * wa, BfHi(v[k]) * r * wb);
+    }
+  }
+}
+
 template <bool kAdd>
 __global__ void RmsNormKernel(__nv_bfloat16* __restrict__ res, const __nv_bfloat16* __restrict__ delta,
                               const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ out, int H,
@@ -157,6 +209,18 @@ __global__ void SpecAcceptKernel(const int* __restrict__ next_ids, const int* __
 
 using namespace r4dxb;
 
+template <bool kAdd>
+static int RmsNormRows(void* res, const void* delta, const void* w, void* out, int T, int H, float eps, int mode, void* stream) {
+  const cudaStream_t s = static_cast<cudaStream_t>(stream);
+  __nv_bfloat16* r = static_cast<__nv_bfloat16*>(res);
+  const __nv_bfloat16* d = static_cast<const __nv_bfloat16*>(delta);
+  const __nv_bfloat16* g = static_cast<const __nv_bfloat16*>(w);
+  __nv_bfloat16* o = static_cast<__nv_bfloat16*>(out);
+  if (H <= kRegColumns) RmsNormRowKernel<kAdd><<<T, kRowThreads, 0, s>>>(r, d, g, o, H, eps, mode);
+  else RmsNormKernel<kAdd><<<T, kRowThreads, H * sizeof(float), s>>>(r, d, g, o, H, eps, mode);
+  return FinishLaunch();
+}
+
 extern "C" {
 
 unsigned long long r4dxb_launch_count() { return g_launch_count; }
@@ -177,19 +241,13 @@ int r4dxb_embed_gather_bf16(const int* ids, const void* table, void* out, int T,
 
 int r4dxb_rmsnorm_bf16(const void* x, const void* w, void* out, int T, int H, float eps, int mode, void* stream) {
   if (H % 2 || T <= 0) return R4DXB_BAD_ARG;
-  RmsNormKernel<false><<<T, kRowThreads, H * sizeof(float), static_cast<cudaStream_t>(stream)>>>(
-      const_cast<__nv_bfloat16*>(static_cast<const __nv_bfloat16*>(x)), nullptr,
-      static_cast<const __nv_bfloat16*>(w), static_cast<__nv_bfloat16*>(out), H, eps, mode);
-  return FinishLaunch();
+  return RmsNormRows<false>(const_cast<void*>(x), nullptr, w, out, T, H, eps, mode, stream);
 }
 
 int r4dxb_add_rmsnorm_bf16(void* res, const void* delta, const void* w, void* out, int T, int H, float eps, int mode,
                            void* stream) {
   if (H % 2 || T <= 0) return R4DXB_BAD_ARG;
-  RmsNormKernel<true><<<T, kRowThreads, H * sizeof(float), static_cast<cudaStream_t>(stream)>>>(
-      static_cast<__nv_bfloat16*>(res), static_cast<const __nv_bfloat16*>(delta),
-      static_cast<const __nv_bfloat16*>(w), static_cast<__nv_bfloat16*>(out), H, eps, mode);
-  return FinishLaunch();
+  return RmsNormRows<true>(res, delta, w, out, T, H, eps, mode, stream);
 }
 
 int r4dxb_norm_add_bf16(void* res, const void* delta, const void* w, int T, int H, float eps, void* stream) {

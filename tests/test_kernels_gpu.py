@@ -444,6 +444,21 @@ def test_linear_tc_dense_matches_fp32_reference(K, dtype, T, N, Kd):
         assert torch.allclose(ya.cpu(), fn(ref), atol=3e-2, rtol=1e-2)
 
 
+@pytest.mark.parametrize("H", [2, 510, 514, 8190, 8192, 8194])
+@pytest.mark.parametrize("add", [False, True])
+def test_rmsnorm_at_the_edges_of_its_register_rows(K, H, add):
+    """Rows below, at and past what the threads keep in registers, ragged against the 512 columns of a step: one bf16 rounding of the fp64
+    norm (2^-8 of the value allows a flip beside a tie), the residual rows rounded once."""
+    g = torch.Generator().manual_seed(H)
+    x, d, w = torch.randn(3, H, generator=g).to(BF), torch.randn(3, H, generator=g).to(BF), (torch.randn(H, generator=g) * 0.1).to(BF)
+    r = x.cuda()
+    out = K.add_rmsnorm(r, d.cuda(), w.cuda()) if add else K.rmsnorm(r, w.cuda())
+    ref = (x.float() + d.float()).to(BF) if add else x
+    assert torch.equal(r.cpu(), ref)
+    want = ref.double() * torch.rsqrt((ref.double() ** 2).mean(1, keepdim=True) + 1e-6) * (1 + w.double())
+    assert torch.allclose(out.cpu().double(), want, rtol=2 ** -8, atol=1e-6)
+
+
 def test_argmax_ties_take_lowest_id(K):
     lg = torch.zeros(2, 5000, device="cuda")
     lg[0, 4000] = 1.0
