@@ -127,6 +127,7 @@ class StepBuffers:
     ids: torch.Tensor
     positions: torch.Tensor
     n_replay: torch.Tensor
+    status_and_ids: torch.Tensor     # the GEMM status word as of the latest argmax, then `next_ids`: one read-back brings both
     next_ids: torch.Tensor
     next_vals: torch.Tensor
     x: torch.Tensor
@@ -225,9 +226,10 @@ class HybridModel:
         R = MAX_ROWS
         V = cfg.vocab_shard_size
         e = lambda *s, dtype=BF: torch.zeros(*s, dtype=dtype, device=dev)
+        status_and_ids = e(1 + R, dtype=torch.int32)
         self.buf = StepBuffers(
             ids=e(R, dtype=torch.int32), positions=e(R, dtype=torch.int32), n_replay=e(1, dtype=torch.int32),
-            next_ids=e(R, dtype=torch.int32), next_vals=e(R, dtype=torch.float32),
+            status_and_ids=status_and_ids, next_ids=status_and_ids[1:], next_vals=e(R, dtype=torch.float32),
             x=e(R, H), h=e(R, H), mixed=e(R, max(cfg.conv_dim, 3 * H if cfg.has_conv_layers else 0)), z=e(R, cfg.value_dim),
             ab=e(R, 2 * Hv, dtype=torch.float32), core=e(R, max(cfg.value_dim, cfg.q_dim, H if cfg.has_conv_layers else 0)),
             qg=e(R, cfg.q_proj_dim), k=e(R, cfg.kv_dim), v=e(R, cfg.kv_dim), q=e(R, cfg.q_dim),
@@ -466,9 +468,14 @@ class HybridModel:
         if want_logits and self.layer_end == cfg.num_hidden_layers:
             K.rmsnorm(b.x[:T], w["text.final_norm"], cfg.rms_norm_eps, out=b.h[:T])
             self.lin["lm_head"](b.h[:T], out=b.logits[:T])
-            K.argmax_rows(b.logits[:T], cfg.vocab_shard_begin, b.next_ids[:T], b.next_vals[:T], b.argmax_scratch)
-            if self.comm is not None and self.comm.world > 1:
-                self.comm.merge_argmax(b.next_ids[:T], b.next_vals[:T])
+            self._pick(T)
+
+    def _pick(self, T: int) -> None:
+        """``buf.next_ids[:T]`` out of the logits rows, with the status word of the products behind them in front."""
+        b = self.buf
+        K.argmax_rows(b.logits[:T], self.cfg.vocab_shard_begin, b.next_ids[:T], b.next_vals[:T], b.argmax_scratch, b.status_and_ids[:1])
+        if self.comm is not None and self.comm.world > 1:
+            self.comm.merge_argmax(b.next_ids[:T], b.next_vals[:T])
 
     # ---- feature capture for drafters that condition on intermediate residuals ----------------------
     capture_layers: tuple = ()
@@ -507,20 +514,20 @@ class HybridModel:
 
     def check_healthy(self, rows: int = 1) -> None:
         """Raises if a bounded device wait ran out since the last check: a timed-out collective leaves an un-reduced partial
-        in the residual stream, so a token read after it must not be trusted (one small device-to-host read per call).
-        ``rows``: the row count of the call being checked (from ``K.ROWS_MIN_ROWS`` rows its products may have run on the
-        mma.sync or tensor-memory weight-streaming kernel, whose waits report through the GEMM status word; a one-row step does not
-        read it: a wait that ran out there leaves NaN in its logits, and the word set for the next call that reads it)."""
+        in the residual stream and a timed-out product NaN, from which a plausible first token id is picked, so a token read after it
+        must not be trusted (one small device-to-host read per call).  ``rows`` (the row count of the call being checked) makes no
+        difference: products of every row count have kernels whose waits report through the GEMM status word."""
         if self.comm is not None and self.comm.world > 1:
             self.comm.check_healthy()
-        if K.GEMV_IMPL == "mma" or (K.GEMV_IMPL == "auto" and rows >= K.ROWS_MIN_ROWS):
-            K.check_gemm_status(self.device)
+        K.check_gemm_status(self.device)
 
     def _read_token(self, idx: int) -> int:
         self.last_row = idx              # the logits row this token was picked from (samplers read it)
-        tok = int(self.buf.next_ids[idx].item())
-        self.check_healthy()
-        return tok
+        words = self.buf.status_and_ids[:idx + 2].tolist()
+        if self.comm is not None and self.comm.world > 1:
+            self.comm.check_healthy()
+        K.check_gemm_status(self.device, words[0])
+        return words[-1]
 
     def prefill_small(self, ids: torch.Tensor) -> int:
         """Feeds a prompt through the small-batch path (MAX_ROWS rows per call); returns the greedy next token."""
@@ -642,9 +649,7 @@ class HybridModel:
             b = self.buf
             K.rmsnorm(x[T - 1:T], w["text.final_norm"], cfg.rms_norm_eps, out=b.h[:1])
             self.lin["lm_head"](b.h[:1], out=b.logits[:1])
-            K.argmax_rows(b.logits[:1], cfg.vocab_shard_begin, b.next_ids[:1], b.next_vals[:1], b.argmax_scratch)
-            if self.comm is not None and self.comm.world > 1:
-                self.comm.merge_argmax(b.next_ids[:1], b.next_vals[:1])
+            self._pick(1)
         self.pos += T
         self.pending_rows = 0
 
@@ -869,6 +874,7 @@ class HybridModel:
             raise ValueError("context overflow")
         self.buf.n_replay.fill_(self.pending_rows)
         self._run_rows(T)
+        self.check_healthy(T)
         self._window_rows = T
         return self.buf.logits[:T]
 
@@ -899,6 +905,7 @@ class HybridModel:
     def decode_step_logits(self, token: int) -> torch.Tensor:
         """Eager single step returning this rank's fp32 logits row (sampling path)."""
         self.feed(torch.tensor([token], dtype=torch.int32))
+        self.check_healthy()
         return self.buf.logits[0]
 
     # ---- graph decode ---------------------------------------------------------------------------

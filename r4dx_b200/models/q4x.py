@@ -217,7 +217,7 @@ class Qwen4ExpModel(HybridModel):
         if want_logits:
             self._gate("text.hc_final.", T, inject=False)
             self.lin["lm_head"](b.x[:T], out=b.logits[:T])
-            K.argmax_rows(b.logits[:T], 0, b.next_ids[:T], b.next_vals[:T], b.argmax_scratch)
+            self._pick(T)
 
     def feed(self, ids: torch.Tensor, want_logits: bool = True, accepted: Optional[int] = None) -> None:
         if accepted is not None and accepted != ids.numel():
@@ -383,7 +383,7 @@ class Qwen4ExpModel(HybridModel):
             self.hx[:1].copy_(hx[T - 1:T])
             self._gate("text.hc_final.", 1, inject=False)
             self.lin["lm_head"](b.x[:1], out=b.logits[:1])
-            K.argmax_rows(b.logits[:1], 0, b.next_ids[:1], b.next_vals[:1], b.argmax_scratch)
+            self._pick(1)
         self.pos += T
         self.pending_rows = 0
 

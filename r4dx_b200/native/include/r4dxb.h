@@ -74,6 +74,9 @@ int r4dxb_bf16_gemv_norm(const void* W, const void* x, const void* norm_w, float
  * scratch: 2 * T * 256 * 4 bytes */
 int r4dxb_argmax_rows(const void* logits, int is_f32, int T, int V, int id_offset, int* out_ids, float* out_vals,
                       void* scratch, void* stream);
+/* The same; *out_status = *status, the word that a bounded wait of the products before it sets (both null: no copy). */
+int r4dxb_argmax_rows_status(const void* logits, int is_f32, int T, int V, int id_offset, int* out_ids, float* out_vals,
+                             void* scratch, const int* status, int* out_status, void* stream);
 
 /* row summary for exact host sampling: top-K (K <= 64) raw logits + ids (canonical order) and the log-sum-exp
  * of logits / temperature.  scratch: T * 128 * (2K + 2) * 4 bytes */

@@ -274,11 +274,14 @@ __global__ void ArgmaxPartial(const void* __restrict__ logits, int V, float* __r
   }
 }
 
+// `status` (null: none): the device word that a bounded wait of a product sets; copied to `out_status`, so that one read-back brings a
+// step's tokens and whether they may be used (a second copy of four bytes after each token would be about 2 us of the stream).
 __global__ void ArgmaxFinal(const float* __restrict__ pv, const int* __restrict__ pi, int id_offset,
-                            int* __restrict__ out_ids, float* __restrict__ out_vals) {
+                            int* __restrict__ out_ids, float* __restrict__ out_vals, const int* status, int* out_status) {
   __shared__ float sv[8];
   __shared__ int si[8];
   const int t = blockIdx.x;
+  if (t == 0 && threadIdx.x == 32 && status != nullptr) *out_status = *status;
   float bv = pv[t * kArgParts + threadIdx.x];
   int bi = pi[t * kArgParts + threadIdx.x];
 #pragma unroll
@@ -381,7 +384,12 @@ int r4dxb_bf16_gemv_norm(const void* W, const void* x, const void* norm_w, float
 
 int r4dxb_argmax_rows(const void* logits, int is_f32, int T, int V, int id_offset, int* out_ids, float* out_vals,
                       void* scratch, void* stream) {
-  if (T < 1 || V < 1) return R4DXB_BAD_ARG;
+  return r4dxb_argmax_rows_status(logits, is_f32, T, V, id_offset, out_ids, out_vals, scratch, nullptr, nullptr, stream);
+}
+
+int r4dxb_argmax_rows_status(const void* logits, int is_f32, int T, int V, int id_offset, int* out_ids, float* out_vals,
+                             void* scratch, const int* status, int* out_status, void* stream) {
+  if (T < 1 || V < 1 || (status != nullptr && out_status == nullptr)) return R4DXB_BAD_ARG;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   float* pv = static_cast<float*>(scratch);
   int* pi = reinterpret_cast<int*>(pv + static_cast<size_t>(T) * kArgParts);
@@ -390,7 +398,7 @@ int r4dxb_argmax_rows(const void* logits, int is_f32, int T, int V, int id_offse
   else ArgmaxPartial<false><<<grid, 256, 0, s>>>(logits, V, pv, pi);
   int e = FinishLaunch();
   if (e) return e;
-  ArgmaxFinal<<<T, kArgParts, 0, s>>>(pv, pi, id_offset, out_ids, out_vals);
+  ArgmaxFinal<<<T, kArgParts, 0, s>>>(pv, pi, id_offset, out_ids, out_vals, status, out_status);
   return FinishLaunch();
 }
 
@@ -453,6 +461,6 @@ extern "C" int r4dxb_argmax_rows_static(const void* logits, int is_f32, int T, i
   else ArgmaxPartial<false><<<grid, 256, 0, s>>>(logits, V, pv, pi);
   int err = FinishLaunch();
   if (err) return err;
-  ArgmaxFinal<<<T, kArgParts, 0, s>>>(pv, pi, id_offset, out_ids, out_vals);
+  ArgmaxFinal<<<T, kArgParts, 0, s>>>(pv, pi, id_offset, out_ids, out_vals, nullptr, nullptr);
   return FinishLaunch();
 }

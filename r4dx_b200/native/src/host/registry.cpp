@@ -155,6 +155,8 @@ const R4dxbKernelInfo kKernels[] = {
      "", "bf16", "simt", c22, 2},
     {"argmax_rows", "sampling", "row_argmax", "two-stage argmax with an id offset; lowest id wins ties",
      "", "fp32 or bf16 logits", "simt", nullptr, 0},
+    {"argmax_rows_status", "sampling", "row_argmax_with_status", "the same, and the products' status word beside the ids",
+     "", "fp32 or bf16 logits", "simt", nullptr, 0},
     {"argmax_rows_static", "sampling", "row_argmax", "the same with its partials in a fixed device array (no caller scratch)",
      "rows <= 64", "fp32 or bf16 logits", "simt", c24, 1},
     {"topk_lse", "sampling", "topk_and_logsumexp", "top-k values / ids in canonical order and the row's log-sum-exp",

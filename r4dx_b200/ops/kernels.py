@@ -38,6 +38,7 @@ register_cuda_sig("r4dxb_w4a16_rows", _I, [_P, _P, _P, _P, _I, _I, _I, _I, _I, _
 register_cuda_sig("r4dxb_bf16_gemv", _I, [_P, _P, _P, _I, _I, _I, _P])
 register_cuda_sig("r4dxb_bf16_gemv_norm", _I, [_P, _P, _P, _F, _P, _I, _I, _I, _P])
 register_cuda_sig("r4dxb_argmax_rows", _I, [_P, _I, _I, _I, _I, _P, _P, _P, _P])
+register_cuda_sig("r4dxb_argmax_rows_status", _I, [_P, _I, _I, _I, _I, _P, _P, _P, _P, _P, _P])
 register_cuda_sig("r4dxb_gdn_decode", _I, [_P] * 15 + [_I, _I, _I, _I, _F, _P])
 register_cuda_sig("r4dxb_attn_precore", _I, [_P] * 11 + [_I, _I, _I, _I, _I, _F, _F, _I, _P])
 register_cuda_sig("r4dxb_attn_decode", _I, [_P] * 10 + [_I, _I, _I, _I, _I, _I, _P])
@@ -260,8 +261,9 @@ def gemm_status(device) -> torch.Tensor:
     return _STATUS[key]
 
 
-def check_gemm_status(device) -> None:
-    code = int(gemm_status(device).item())
+def check_gemm_status(device, code: Optional[int] = None) -> None:
+    """Raises if the word is set, and clears it; ``code``: its value where the caller has read it already."""
+    code = int(gemm_status(device).item()) if code is None else code
     if code:
         gemm_status(device).zero_()
         raise KernelError(f"a tensor-core product gave up in a bounded wait (role code {code})")
@@ -419,7 +421,9 @@ def bf16_gemv_norm(W: torch.Tensor, x: torch.Tensor, norm_w: torch.Tensor, eps: 
 
 
 def argmax_rows(logits: torch.Tensor, id_offset: int = 0, out_ids: Optional[torch.Tensor] = None,
-                out_vals: Optional[torch.Tensor] = None, scratch: Optional[torch.Tensor] = None):
+                out_vals: Optional[torch.Tensor] = None, scratch: Optional[torch.Tensor] = None,
+                out_status: Optional[torch.Tensor] = None):
+    """Ids (ties to the lowest) and values of the rows' maxima; ``out_status`` ([1] int32) receives the GEMM status word."""
     T, V = logits.shape
     is_f32 = logits.dtype == torch.float32
     if not is_f32:
@@ -428,8 +432,10 @@ def argmax_rows(logits: torch.Tensor, id_offset: int = 0, out_ids: Optional[torc
     out_ids = out_ids if out_ids is not None else torch.empty(T, dtype=torch.int32, device=dev)
     out_vals = out_vals if out_vals is not None else torch.empty(T, dtype=torch.float32, device=dev)
     scratch = scratch if scratch is not None else torch.empty(2 * T * 256, dtype=torch.float32, device=dev)
-    _check(_lib().r4dxb_argmax_rows(_p(logits), 1 if is_f32 else 0, T, V, id_offset, _p(out_ids), _p(out_vals),
-                                    _p(scratch), _stream()), "argmax_rows")
+    args = (_p(logits), 1 if is_f32 else 0, T, V, id_offset, _p(out_ids), _p(out_vals), _p(scratch))
+    rc = (_lib().r4dxb_argmax_rows(*args, _stream()) if out_status is None else
+          _lib().r4dxb_argmax_rows_status(*args, _p(gemm_status(dev)), _p(out_status), _stream()))
+    _check(rc, "argmax_rows")
     return out_ids, out_vals
 
 

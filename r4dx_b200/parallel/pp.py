@@ -104,6 +104,7 @@ class PipelinePrefill:
         if self.rank == 1:
             tok.copy_(st.buf.next_ids[:1])
         dist.broadcast(tok, src=1, group=self.group)
+        st.check_healthy()
         return int(tok.item())
 
 
@@ -134,6 +135,7 @@ class LayerSplitDecode:
         st.pending_rows = T
         st.pos += T
         dist.broadcast(self.tok, src=1, group=self.group)
+        st.check_healthy()
         return int(self.tok.item())
 
 

@@ -57,10 +57,31 @@ def test_rows_kernel_reports_a_wait_that_ran_out(lib, large, monkeypatch):
     read = []
     monkeypatch.setattr(K, "check_gemm_status", read.append)
     m = SimpleNamespace(comm=None, device="cpu")
-    HybridModel.check_healthy(m, 1)
-    assert not read
-    HybridModel.check_healthy(m, K.ROWS_MIN_ROWS)
-    assert read == ["cpu"]
+    for rows in (1, K.ROWS_MIN_ROWS):
+        HybridModel.check_healthy(m, rows)
+    assert read == ["cpu"] * 2
+
+
+def test_one_row_of_large_weights_reports_a_wait_that_ran_out(lib):
+    """The one-row launch is given the status word, the argmax puts the word before the ids, and the token is not handed out."""
+    big = trellis.random_weight(8192, 4096, 4, seed=1)
+    word = K.gemm_status("cpu").data_ptr()
+    K.trellis_gemv(big, torch.zeros(1, 4096, dtype=BF))
+    buf = torch.zeros(9, dtype=torch.int32)
+    m = SimpleNamespace(comm=None, device="cpu", cfg=SimpleNamespace(vocab_shard_begin=0),
+                        buf=SimpleNamespace(logits=torch.zeros(8, 16), status_and_ids=buf, next_ids=buf[1:], next_vals=torch.zeros(8),
+                                            argmax_scratch=torch.zeros(2 * 8 * 256)))
+    HybridModel._pick(m, 1)
+    (rows, a), (argmax, b) = lib.calls
+    assert rows == "r4dxb_trellis_gemv_rows" and _address(a[-2]) == word
+    assert argmax == "r4dxb_argmax_rows_status" and b[-3:-1] == (word, buf.data_ptr()) and b[5] == buf.data_ptr() + 4
+    buf[:3] = torch.tensor([0, 7, 9])
+    assert HybridModel._read_token(m, 0) == 7 and HybridModel._read_token(m, 1) == 9
+    buf[0] = 702
+    K.gemm_status("cpu").fill_(702)
+    with pytest.raises(K.KernelError, match="702"):
+        HybridModel._read_token(m, 0)
+    assert int(K.gemm_status("cpu")) == 0           # reported once
 
 
 @pytest.mark.parametrize("T,entry", [(1, "r4dxb_trellis_gemv_ex"), (2, "r4dxb_trellis_gemv_ex"), (8, "r4dxb_trellis_gemv_mma")])

@@ -645,3 +645,30 @@ def test_captured_moe_block_runs_its_shared_expert_beside_the_routed_ones(T):
         z = x.clone()
         blk.forward(h, z, T)
         assert torch.equal(y, z)
+
+
+def test_every_call_that_hands_out_tokens_or_logits_reads_the_status_word():
+    """A bounded wait that ran out in a product (the word is set by hand here) ends the call with an error, whatever its row count, and the
+    calls after it run again."""
+    from r4dx_b200.ops import kernels as K
+    from r4dx_b200.runtime.engine import GreedySession
+    from r4dx_b200.runtime.text_model import LocalTextModel
+    from r4dx_b200.config import small_hybrid_config
+    from r4dx_b200.models.hybrid import HybridModel
+    from r4dx_b200.quant.weights import synthetic_weight_set
+    cfg = small_hybrid_config(4)
+    m = HybridModel(cfg, synthetic_weight_set(cfg, device="cuda", seed=0), max_ctx=256)
+    tok = m.prefill(torch.arange(40, dtype=torch.int32))
+    s = GreedySession(m)
+    s.begin(tok)
+    t = LocalTextModel(m)
+    calls = {"session": lambda: s.step(5), "greedy": lambda: m.decode_step_greedy(5), "logits": lambda: m.decode_step_logits(5),
+             "model": lambda: t.decode_step_greedy(5), "sampled": lambda: t.decode_step(5), "window": lambda: m.verify_window(5, [6, 7]),
+             "window logits": lambda: m.window_logits(5, [6, 7]), "prompt": lambda: m.prefill(torch.arange(20, dtype=torch.int32)),
+             "generation": lambda: m.generate_greedy(torch.arange(20, dtype=torch.int32), 3)}
+    for name, call in calls.items():
+        K.gemm_status("cuda").fill_(702)
+        with pytest.raises(K.KernelError, match="702"):
+            call()
+        assert int(K.gemm_status("cuda")) == 0, name
+        call()
