@@ -26,10 +26,13 @@ constexpr int kMaxK = 16;
 // One warp routes one row.  The row's selection values live in registers (E <= 1024: 32 per lane) and a lane remembers its taken
 // entries in a bit mask.  Every lane keeps its best entry; a round is two reductions over the lanes, and only the lane that loses
 // its entry looks for the next one.  (With a search of all lanes and ten shuffles a round, 4096 rows of 512 experts took 30 us, now 18.)
+// A NaN (what a wait that ran out leaves in a row) ranks with minus infinity, so that every row gets k experts that exist; the softmax
+// weights of such a row are NaN, and so is the sigmoid weight of a NaN that is picked.
 __device__ __forceinline__ void RouteRow(const float* __restrict__ row, const float* __restrict__ bias, int E, int k, int renorm,
                                          int mode, float scale, int lane, int* __restrict__ ids, float* __restrict__ weights) {
   float v[32];
   float mx = -INFINITY, z = 0.f;
+  bool nan = false;
 #pragma unroll
   for (int s = 0; s < 32; ++s) v[s] = -INFINITY;
 #pragma unroll
@@ -38,7 +41,11 @@ __device__ __forceinline__ void RouteRow(const float* __restrict__ row, const fl
 #pragma unroll
     for (int s = s0; s < s0 + 8; ++s) {
       const int e = lane + 32 * s;
-      if (e < E) v[s] = mode == 0 ? row[e] : 1.0f / (1.0f + expf(-row[e])) + (bias ? bias[e] : 0.f);
+      if (e < E) {
+        const float x = mode == 0 ? row[e] : 1.0f / (1.0f + expf(-row[e])) + (bias ? bias[e] : 0.f);
+        nan |= x != x;
+        v[s] = fmaxf(x, -INFINITY);          // (a NaN gives the other operand)
+      }
       mx = fmaxf(mx, v[s]);
     }
   }
@@ -51,6 +58,7 @@ __device__ __forceinline__ void RouteRow(const float* __restrict__ row, const fl
       for (int s = s0; s < s0 + 8; ++s) z += (lane + 32 * s < E) ? __expf(v[s] - mx) : 0.f;
     }
     z = WarpSum(z);
+    if (__any_sync(0xffffffffu, nan)) z = __int_as_float(0x7FC00000);
   }
   float wsum = 0.f;
   uint32_t taken = 0;              // bit s: this lane's entry lane + 32 s is already picked

@@ -1554,3 +1554,36 @@ def test_window_attention_on_the_tensor_cores_against_fp64(K, D, Hq, Hkv, T, ctx
     ref = torch.softmax(s * math.log(2), -1) @ (v * vds.double()[:, None, None])
     assert (o - ref).norm() < 1e-5 * ref.norm()
     assert ((out.view(T, Hkv, gqa, D).permute(1, 0, 2, 3).reshape(Hkv, G, D).double() - ref).abs() <= 2.0 ** -8 * ref.abs() + 1e-4 * ref.abs().max()).all()
+
+
+@pytest.mark.parametrize("sigmoid", [False, True])
+@pytest.mark.parametrize("E,k,T", [(16, 4, 6), (64, 16, 8), (257, 10, 40), (1024, 16, 6)])
+def test_router_gives_rows_with_nan_experts_that_exist(K, E, k, T, sigmoid):
+    """Rows of NaN, with one value fewer than they pick, with one NaN, and with NaN beside minus infinity: the ids are those of a sort
+    in which a NaN is minus infinity (distinct, below E), the weights of the picks say that the row is no good, other rows are as without them."""
+    g = torch.Generator().manual_seed(E + T)
+    logits = torch.randn(T, E, generator=g)
+    clean = logits.clone()
+    nan = float("nan")
+    logits[0] = nan
+    logits[1, torch.randperm(E, generator=g)[:E - k + 1]] = nan
+    logits[2, E - 1] = nan
+    logits[3, :E // 2], logits[3, E // 2:] = float("-inf"), nan
+    bias = torch.rand(E, generator=g) if sigmoid else None
+    value = torch.sigmoid(logits) + bias if sigmoid else logits
+    order = torch.sort(torch.where(value.isnan(), float("-inf"), value), dim=-1, descending=True, stable=True).indices[:, :k].to(torch.int32)
+    ids, w = torch.empty(T, k, dtype=torch.int32, device="cuda"), torch.empty(T, k, device="cuda")
+    ids0, w0 = torch.empty_like(ids), torch.empty_like(w)
+    route = lambda lg, i, x: (K.moe_router_sigmoid(lg.cuda(), bias.cuda(), k, True, 2.0, i, x) if sigmoid else K.moe_router(lg.cuda(), k, True, i, x))
+    route(logits, ids, w)
+    route(clean, ids0, w0)
+    assert torch.equal(ids[4:], ids0[4:]) and torch.equal(w[4:], w0[4:])
+    # (sigmoid: values that tie within the rounding of the exponential are left to the comparison with the clean rows above)
+    assert torch.equal(ids[:2].cpu(), order[:2]) and torch.equal(ids[3].cpu(), order[3]) and (sigmoid or torch.equal(ids[2].cpu(), order[2]))
+    # (the sigmoids of minus infinity are zeros)
+    assert bool(w[:2].isnan().all()) and all(bool(w[r].isnan().all()) == (not sigmoid) for r in (2, 3))
+    if T <= 8:
+        off, pm = torch.zeros(E + 1, dtype=torch.int32, device="cuda"), torch.full((T * k,), -1, dtype=torch.int32, device="cuda")
+        ids2, w2 = torch.empty_like(ids), torch.empty_like(w)
+        K.moe_route_plan(logits.cuda(), bias.cuda() if sigmoid else None, k, True, sigmoid, 2.0 if sigmoid else 1.0, ids2, w2, 0, E, off, pm)
+        assert torch.equal(ids2, ids) and int(off[-1]) == T * k and torch.equal(pm.sort().values.cpu(), torch.arange(T * k, dtype=torch.int32))
