@@ -211,8 +211,11 @@ class BatchModel:
         else:
             logits = torch.empty(B, V, dtype=torch.float32, device=dev)
             b.lin["lm_head"](h, out=logits)
-        nxt, _ = K.argmax_rows(logits, cfg.vocab_shard_begin)
+        words = torch.empty(1 + B, dtype=torch.int32, device=dev)          # the products' status word, then the ids
+        K.argmax_rows(logits, cfg.vocab_shard_begin, words[1:], out_status=words[:1])
+        self.last_logits = logits
+        status, *nxt = words.tolist()
+        K.check_gemm_status(dev, status)         # (a wait that ran out left rows that no product wrote)
         for s in slots:
             self.pos[s] += 1
-        self.last_logits = logits
-        return nxt.tolist()
+        return nxt

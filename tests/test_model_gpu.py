@@ -672,3 +672,19 @@ def test_every_call_that_hands_out_tokens_or_logits_reads_the_status_word():
             call()
         assert int(K.gemm_status("cuda")) == 0, name
         call()
+
+
+@pytest.mark.parametrize("B", [1, 3, 12])
+def test_a_batched_step_reads_the_status_word(B):
+    """One-row products, the weight-streaming kernels and the GEMM, whichever a step of B sequences takes, all report there."""
+    from r4dx_b200.models.batch import BatchModel
+    from r4dx_b200.ops import kernels as K
+    from r4dx_b200.quant.weights import synthetic_weight_set
+    cfg = tiny_hybrid_config()
+    m = BatchModel(cfg, synthetic_weight_set(cfg, device="cuda", seed=0), slots=B, slot_ctx=64)
+    toks = [m.import_slot(j, list(range(3 + j))) for j in range(B)]
+    K.gemm_status("cuda").fill_(702)
+    with pytest.raises(K.KernelError, match="702"):
+        m.decode_batch(list(range(B)), toks)
+    assert int(K.gemm_status("cuda")) == 0
+    assert len(m.decode_batch(list(range(B)), toks)) == B
