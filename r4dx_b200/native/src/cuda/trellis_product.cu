@@ -423,7 +423,8 @@ TrellisProductKernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_co
     } else {
       // Two buffers a group where they fit: a warp loads its next columns while others finish theirs.  Wide tiles: the rounded rows
       // of a token replace its sums and leave as one bulk copy of 256 bytes (stores of a lane's rows, 32 bytes of eight tokens
-      // each, took half of the epilogue: 27k of 115k clocks a tile at 512 tokens).
+      // each, took half of the epilogue: 27k of 115k clocks a tile at 512 tokens).  A warp whose wait ran out writes NaN: into the
+      // buffer for the others, and by plain stores into its tokens' rows.
       constexpr int kBuffers = 2 * S::kEpiGroups <= S::kRings ? 2 : 1;
       const bool bulk = S::kWide && a.rs.world == 0 && (reinterpret_cast<uintptr_t>(a.y) & 15) == 0;
       int buf = 0;
@@ -435,14 +436,19 @@ TrellisProductKernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_co
           ptx::TmemLoadWait();
 #pragma unroll
           for (int c = 0; c < CW; ++c) epi[c * S::kEpiStride + q * 32 + lane] = __uint_as_float(v[c]);
+        } else {
+          for (int c = 0; c < CW; ++c) epi[c * S::kEpiStride + q * 32 + lane] = __int_as_float(0x7FC00000);
         }
         if (kBuffers == 2 && bulk) ptx::BulkStoreWaitRead();      // (the copies out of the other buffer, before anyone writes there)
         asm volatile("bar.sync %0, 128;" ::"r"(1 + grp) : "memory");
         const int c_end = min(c0 + CW, tile_end);
         auto load = [&](int ct, int row) { return *reinterpret_cast<const float4*>(epi + (ct - c0) * S::kEpiStride + row); };
-        if (bulk) {
+        if (!ok) {
+          for (int c = c0 + q * kTokens; c < c_end; c += 4 * kTokens)
+            for (int i = 0; i < min(kTokens, c_end - c); ++i) to_row(t0 + c + i, lane * 4, make_uint2(0x7FC07FC0u, 0x7FC07FC0u));
+        } else if (bulk) {
           const int c = c0 + q * kTokens;
-          if (ok && c < c_end) {
+          if (c < c_end) {
             finish(c, c_end, load, [&](int t, int r, uint2 v) {
               *reinterpret_cast<uint2*>(reinterpret_cast<__nv_bfloat16*>(epi + (t - t0 - c0) * S::kEpiStride) + r) = v;
             });
@@ -454,7 +460,7 @@ TrellisProductKernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_co
             }
             if (kBuffers == 1) ptx::BulkStoreWaitRead();
           }
-        } else if (ok) {
+        } else {
           for (int c = c0 + q * kTokens; c < c_end; c += 4 * kTokens) finish(c, c_end, load, to_row);
         }
         if (kBuffers == 1) asm volatile("bar.sync %0, 128;" ::"r"(1 + grp) : "memory");
