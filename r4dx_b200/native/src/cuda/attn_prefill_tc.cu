@@ -500,11 +500,12 @@ __global__ void __launch_bounds__(kThreads, 1) AttnPrefillTcKernel(TcArgs a) {
 template <int D>
 int LaunchTc(const TcArgs& a, cudaStream_t s) {
   constexpr int NS = D / 64;
-  // at least half of an SM's shared memory: two pairs that each held the tensor memory of one SM and waited for the other's
-  // would wait for good, so no two CTAs may meet on an SM
+  // All of an SM's shared memory, so that no other CTA shares the SM.  A pair takes the whole tensor memory of two SMs and the first
+  // CTA waits for the second; were one of them held up by columns of another kernel's CTA (on another stream) whose cluster in turn
+  // waits for a CTA that the other one holds up, both would wait for good.
   constexpr size_t kSmem = NS * kQRows * 128 + 2 * NS * kHalfTile * 128 + 2 * D * 128 + sizeof(Control) + 1024;
-  constexpr size_t kAlone = 116 * 1024;
-  constexpr size_t smem = kSmem > kAlone ? kSmem : kAlone;
+  constexpr size_t smem = 227 * 1024, kReserved = 1024, kPerSm = 228 * 1024;
+  static_assert(kSmem <= smem && smem + 2 * kReserved > kPerSm, "fits, and nothing fits beside it");
   auto kern = AttnPrefillTcKernel<D>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
   if (e != cudaSuccess) return static_cast<int>(e);
