@@ -500,12 +500,10 @@ __global__ void __launch_bounds__(kThreads, 1) AttnPrefillTcKernel(TcArgs a) {
 template <int D>
 int LaunchTc(const TcArgs& a, cudaStream_t s) {
   constexpr int NS = D / 64;
-  // All of an SM's shared memory, so that no other CTA shares the SM.  A pair takes the whole tensor memory of two SMs and the first
-  // CTA waits for the second; were one of them held up by columns of another kernel's CTA (on another stream) whose cluster in turn
-  // waits for a CTA that the other one holds up, both would wait for good.
+  // kClusterAlone: so much of an SM's shared memory that no other CTA shares the SM whose cluster may wait with tensor memory in its
+  // hands (sm100_ptx.cuh).  More would cost L1: 8192 rows of 32 heads of 128 columns take 808 us with 116 KB, 821 with 156, 878 with 227.
   constexpr size_t kSmem = NS * kQRows * 128 + 2 * NS * kHalfTile * 128 + 2 * D * 128 + sizeof(Control) + 1024;
-  constexpr size_t smem = 227 * 1024, kReserved = 1024, kPerSm = 228 * 1024;
-  static_assert(kSmem <= smem && smem + 2 * kReserved > kPerSm, "fits, and nothing fits beside it");
+  constexpr size_t smem = kSmem > ptx::kClusterAlone ? kSmem : ptx::kClusterAlone;
   auto kern = AttnPrefillTcKernel<D>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
   if (e != cudaSuccess) return static_cast<int>(e);

@@ -203,6 +203,16 @@ __device__ __forceinline__ void BulkStoreWaitRead() { asm volatile("cp.async.bul
 __device__ __forceinline__ void BulkStoreWait() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 
 // ---- tensor memory ------------------------------------------------------------------------------------
+// CTAs of a cluster that hold tensor memory while they wait for each other can lock up: one waits for columns that a CTA of another
+// such cluster (of a launch on another stream) holds, whose partner waits for columns that the first one's partner holds.  Shared
+// memory keeps them apart: an SM has 228 KB, 1 KB of it reserved per CTA.
+//   prefill attention, pairs: kClusterAlone or more (all tensor memory)
+//   trellis product, pairs and splits: kProductAlone or more
+//   plain linears with a split of K: kClusterShared or more, so two at most on an SM, and none beside the others
+// (The waits of the weight-streaming kernel of trellis_gemv_mma.cu for its cluster are bounded: beside it a launch may be late, never stuck.)
+constexpr size_t kClusterAlone = 116 * 1024, kProductAlone = 176 * 1024, kClusterShared = 112 * 1024;
+static_assert(kClusterAlone + kClusterShared + 2 * 1024 > 228 * 1024 && 2 * (kClusterShared + 1024) <= 228 * 1024 &&
+              kClusterAlone <= kProductAlone, "none of the first two kinds meets one of the three");
 // Whole-warp calls (.sync.aligned).  Columns: power of two, 32..512.
 __device__ __forceinline__ void TmemAlloc(uint32_t* smem_result, uint32_t columns) {
   asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(SmemAddr(smem_result)), "r"(columns)

@@ -676,17 +676,17 @@ int LaunchGemm(const void* wsrc, const void* svh, const void* xh, void* y, const
     if (ra) return ra;
   }
   auto kern = TrellisGemmKernel<KB, TN, DW, MODE>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, S::kTotal);
+  cudaError_t e = AllowAllSharedMemory(kern);
   if (e != cudaSuccess) return static_cast<int>(e);
   if (ksplit > 1 && !S::kSplits) return R4DXB_BAD_ARG;
-  // The CTAs of a split hold tensor memory while they wait for each other.  By their shared memory at most three of them meet on an SM
-  // (three of up to 32 columns, two of 64, one of more), and no CTA of a paired or split trellis product or of prefill attention, which
-  // wait in the same way, has room beside one: none waits for columns that a waiting one holds.
-  static_assert(!S::kSplits || S::kTotal * (TN <= 32 ? 4 : (TN <= 64 ? 3 : 2)) > 228 * 1024, "tensor memory of a split");
+  // (clusters that wait with tensor memory in hand: see kClusterShared; two CTAs of a split then meet on an SM, with 64 columns each)
+  constexpr int kSplitSmem = S::kTotal > static_cast<int>(ptx::kClusterShared) ? S::kTotal : static_cast<int>(ptx::kClusterShared);
+  static_assert(!S::kSplits || TN <= 64 || 2 * (S::kTotal + 1024) > 228 * 1024, "two CTAs' columns fit into tensor memory");
+  const int smem = ksplit > 1 ? kSplitSmem : S::kTotal;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((N + 127) / 128, (T + TN - 1) / TN, ksplit);
   cfg.blockDim = dim3((DW + 3) * 32, 1, 1);
-  cfg.dynamicSmemBytes = S::kTotal;
+  cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeClusterDimension;

@@ -25,11 +25,6 @@
 //
 // Split of K (ksplit CTAs of a cluster): for few tokens and short N, where row blocks alone leave SMs idle.  Sums meet over
 // distributed shared memory in rank order.
-//
-// CTAs of a pair or a split hold tensor memory while they wait for each other, so a kernel on another stream whose CTAs do the same
-// must not hold columns that one of them lacks.  Such instances have sixteen decode warps and 176 KB of shared memory or more (Launch
-// checks it): beside one an SM has no room for a K-split plain linear (73 KB at least) or for prefill attention (all of it).  The
-// tensor-memory weight-streaming kernel may fit, but its waits for its cluster are bounded.
 // (The reference engine's counterparts are WMMA kernels whose decoded fragments are shared through LDS, reference:
 // third_party/libr4d/r4d_gemm_trellis_nt_m256.hip:1-60; nothing is shared with them.)
 #include "sm100_ptx.cuh"
@@ -510,7 +505,7 @@ TrellisProductKernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_co
 template <int KB, int TN, int DW, bool kPair, bool kGrouped>
 int Launch(const void* xh, const ProductArgs& a, int ksplit, cudaStream_t stream) {
   using S = Shape<KB, TN, DW, kPair>;
-  static_assert(DW == 8 || kGrouped || S::kTotal >= 176 * 1024, "CTAs that wait for each other share no SM with others that do");
+  static_assert(DW == 8 || kGrouped || S::kTotal >= ptx::kProductAlone, "CTAs of a cluster wait for each other with tensor memory in hand");
   CUtensorMap tmap;
   const int rc = MakeTensorMap2D16(&tmap, xh, static_cast<uint64_t>(a.T), static_cast<uint64_t>(a.K), S::kXRows, kSlabK, false);
   if (rc) return rc;
