@@ -523,11 +523,15 @@ class HybridModel:
 
     def _read_token(self, idx: int) -> int:
         self.last_row = idx              # the logits row this token was picked from (samplers read it)
-        words = self.buf.status_and_ids[:idx + 2].tolist()
+        if idx == 0:                     # (a step's token: word and id as one number, 3 us less on the host than a list of two)
+            pair = self.buf.status_and_ids[:2].view(torch.int64).item()
+            status, tok = pair & 0xFFFFFFFF, pair >> 32
+        else:
+            status, *_, tok = self.buf.status_and_ids[:idx + 2].tolist()
         if self.comm is not None and self.comm.world > 1:
             self.comm.check_healthy()
-        K.check_gemm_status(self.device, words[0])
-        return words[-1]
+        K.check_gemm_status(self.device, status)
+        return tok
 
     def prefill_small(self, ids: torch.Tensor) -> int:
         """Feeds a prompt through the small-batch path (MAX_ROWS rows per call); returns the greedy next token."""
