@@ -527,7 +527,7 @@ _SLAB_US_PAIR = {256: 0.46, 384: 0.62, 512: 0.74}
 _CLUSTER_SLOTS = {1: 148, 2: 148, 3: 144, 4: 136, 6: 126, 8: 112}
 
 
-@functools.lru_cache(maxsize=None)
+@functools.lru_cache(maxsize=4096)           # (a server sees ever new prompt lengths)
 def pick_product(T: int, N: int, K: int) -> tuple:
     """(token tile, split of K) of the trellis product: the fewest us by waves of CTAs, each with a fixed part (start, first loads,
     epilogue) and its share of K.  Short N and few tokens leave SMs idle without a split: 5120 x 17408 at 16 tokens 98 us with one
@@ -649,7 +649,7 @@ def _w4a16_rows(W: W4Weight, x: torch.Tensor, out_f32: bool, out: Optional[torch
     return y
 
 
-@functools.lru_cache(maxsize=None)
+@functools.lru_cache(maxsize=4096)
 def pick_plain(T: int, N: int, K: int) -> tuple:
     """(token tile, split of K) of a plain linear.  Where row blocks and tiles leave most SMs idle - a router, the a / b projections -
     narrower tiles and CTAs that share K: 96 x 5120 at 333 / 8192 rows 49 / 104 us with 256- and 512-row tiles, 12 / 33 so; 512 x

@@ -148,3 +148,4 @@ def test_products_get_a_tile_and_a_split_that_the_kernel_has():
                 tp, kp = K.pick_plain(T, N, Kd)
                 assert tp in (16, 32, 64, 128, 256, 512) and 1 <= kp <= (Kd + 63) // 64 and (kp == 1 or tp <= 256)
     assert K.pick_plain(4096, 4096, 4096) == (K.pick_token_tile(4096, 4096), 1)
+    assert K.pick_product.cache_info().maxsize and K.pick_plain.cache_info().maxsize          # (bounded: one entry per prompt length)
