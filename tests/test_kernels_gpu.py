@@ -177,8 +177,9 @@ def test_trellis_rows_kernel_multiplies_the_formats_values(K, kb, T, N, Kd, spli
     assert ((y - ref).abs() <= 2.0 ** -8 * ref.abs() + 2e-5 * ref.pow(2).mean().sqrt()).all()
 
 
-def test_one_row_products_of_large_weights_have_the_bits_of_the_cuda_core_kernel(K):
-    """Whatever the size: the rounding of a one-row step decides the logits of all later ones."""
+def test_one_row_products_below_the_one_row_line_have_the_bits_of_the_cuda_core_kernel(K):
+    """Weights that two rows would take to the rows kernel, below those from which one row takes its other form: that one rounds alike but
+    for the order of its fp32 sums (test_one_row_on_the_rows_kernel_rounds_as_the_cuda_core_kernel)."""
     from r4dx_b200.quant import trellis
     N, Kd = 4096, 2048
     ws = [trellis.random_weight(N, Kd, 4, seed=i, sigma=0.02, device="cuda") for i in range(3)]
@@ -193,7 +194,7 @@ def test_one_row_products_of_large_weights_have_the_bits_of_the_cuda_core_kernel
         return outs + [K.trellis_gemv(ws[0], x), K.trellis_gemv(ws[0], x, residual=res), K.trellis_gemv(ws[0], gu, prologue=K.PRO_SILU_MUL),
                        K.trellis_gemv(ws[0], gu, prologue=K.PRO_GELU_MUL)]
 
-    assert K.GEMV_IMPL == "auto" and N * Kd >= K.ROWS_MIN_WEIGHTS
+    assert K.GEMV_IMPL == "auto" and N * Kd >= K.ROWS_MIN_WEIGHTS and len(ws) * N * Kd < K.ONE_ROW_MIN_WEIGHTS
     auto = calls()
     K.set_gemv_impl("simt")
     try:
@@ -1587,3 +1588,39 @@ def test_router_gives_rows_with_nan_experts_that_exist(K, E, k, T, sigmoid):
         ids2, w2 = torch.empty_like(ids), torch.empty_like(w)
         K.moe_route_plan(logits.cuda(), bias.cuda() if sigmoid else None, k, True, sigmoid, 2.0 if sigmoid else 1.0, ids2, w2, 0, E, off, pm)
         assert torch.equal(ids2, ids) and int(off[-1]) == T * k and torch.equal(pm.sort().values.cpu(), torch.arange(T * k, dtype=torch.int32))
+
+
+@pytest.mark.parametrize("D,Hq,Hkv,splits,gated", [(256, 16, 1, 3, True), (128, 36, 2, 16, False), (64, 48, 1, 5, True), (128, 64, 1, 1, True)])
+def test_batched_attention_of_many_heads_per_kv_head(K, D, Hq, Hkv, splits, gated):
+    """More than eight query heads per KV head take the window kernel, here with a slot per row: slots out of order, one unused, contexts
+    that end in other splits.  Every row has the bits of its own call, and is right against fp64 attention over the stored fp8 rows within
+    the bf16 rounding of the result (2^-9) and the fp16 rounding of q (2^-11 of a score below 8, so 4e-3 of the |v| that are averaged)."""
+    from r4dx_b200.models import batch  # noqa: F401  (declares the entry point)
+    g = torch.Generator(device="cuda").manual_seed(D + Hq)
+    ctxs, slots = [1, 700, 64, 129, 16], [3, 0, 5, 1, 4]
+    B, nblk = len(ctxs), 45
+    cache = (torch.randn(6 * nblk, Hkv, 2, 16, D, generator=g, device="cuda") * 1.5).to(torch.float8_e4m3fn).view(torch.uint8)
+    tables = torch.randperm(6 * nblk, generator=g, device="cuda").to(torch.int32).view(6, nblk)
+    q = torch.randn(B, Hq, D, generator=g, device="cuda").to(BF)
+    qg = torch.randn(B, Hq, 2 * D, generator=g, device="cuda").to(BF)
+    kds, vds = torch.rand(Hkv, generator=g, device="cuda") + 0.5, torch.rand(Hkv, generator=g, device="cuda") + 0.5
+    pos = torch.tensor([c - 1 for c in ctxs], dtype=torch.int32, device="cuda")
+    row_slot = torch.tensor(slots, dtype=torch.int32, device="cuda")
+    G = Hq // Hkv
+    assert G > 8
+    part = lambda n: (torch.full((n * splits * Hkv * G * D,), float("nan"), device="cuda"), torch.full((n * splits * Hkv * G * 2,), float("nan"), device="cuda"))
+    (pa, pm), out = part(B), torch.zeros(B, Hq * D, dtype=BF, device="cuda")
+    K._check(K._lib().r4dxb_attn_decode_batch(K._p(q), K._p(qg), K._p(cache), K._p(tables), K._p(row_slot), nblk, K._p(pos), K._p(kds), K._p(vds),
+                                              K._p(pa), K._p(pm), K._p(out), B, Hq, Hkv, D, splits, 1 if gated else 0, K._stream()), "attn_decode_batch")
+    for b, (c, s) in enumerate(zip(ctxs, slots)):
+        (pa1, pm1), one = part(1), torch.zeros(1, Hq * D, dtype=BF, device="cuda")
+        K.attn_decode(q[b:b + 1], qg[b:b + 1], cache, tables[s], pos[b:b + 1], kds, vds, pa1, pm1, one, 1, Hq, Hkv, D, splits, gated)
+        assert torch.equal(out[b], one[0])
+        kv = cache.view(torch.float8_e4m3fn).double()[tables[s].long()]
+        k, v = (kv[:, :, i].permute(1, 0, 2, 3).reshape(Hkv, -1, D)[:, :c] * d.double()[:, None, None] for i, d in ((0, kds), (1, vds)))
+        p = torch.softmax(q[b].double().view(Hkv, G, D) @ k.transpose(1, 2) / D ** 0.5, -1)
+        ref, bound = p @ v, p @ v.abs()
+        if gated:
+            sg = torch.sigmoid(qg[b, :, D:].double()).view(Hkv, G, D)
+            ref, bound = ref * sg, bound * sg
+        assert ((out[b].double().view(Hkv, G, D) - ref).abs() <= 2.0 ** -9 * ref.abs() + 8e-3 * bound + 1e-6).all()

@@ -350,6 +350,45 @@ def test_windows_of_large_weights_replay_as_they_run():
     assert not torch.equal(simt, eager) and (simt - eager).norm() < 0.022 * eager.norm()
 
 
+def test_one_row_steps_of_large_weights_replay_as_they_run():
+    """The same for a token step, whose products above the one-row line take the one-row form of the rows kernel: gate_up and down here."""
+    import dataclasses
+    from r4dx_b200.config import small_hybrid_config
+    from r4dx_b200.models.hybrid import HybridModel
+    from r4dx_b200.ops import kernels as K
+    from r4dx_b200.quant.weights import synthetic_weight_set
+    cfg = dataclasses.replace(small_hybrid_config(4), hidden_size=4096, intermediate_size=8192)
+    w = synthetic_weight_set(cfg, device="cuda", seed=3)
+    prompt = torch.randint(0, cfg.vocab_size, (70,), generator=torch.Generator().manual_seed(0), dtype=torch.int32)
+
+    def steps(graph):
+        m = HybridModel(cfg, w, max_ctx=256, device="cuda")
+        m.prefill(prompt)
+        if graph:
+            m.enable_graphs((1,))
+            m.decode_begin(5)
+        logits = []
+        for i in range(4):
+            if graph:
+                m.buf.ids[:1].fill_(5 + i)
+                m.decode_step_graph()
+                logits.append(m.buf.logits[0].clone())
+            else:
+                logits.append(m.decode_step_logits(5 + i).clone())
+        return torch.stack(logits), [m.gdn_state[i].clone() for i in sorted(m.gdn_state)]
+
+    assert K.GEMV_IMPL == "auto" and K.rows_split(2 * cfg.intermediate_size, cfg.hidden_size, 1) and K.rows_split(cfg.hidden_size, cfg.intermediate_size, 1)
+    eager, eager_state = steps(False)
+    replayed, replayed_state = steps(True)
+    assert torch.equal(eager, replayed) and all(torch.equal(a, b) for a, b in zip(eager_state, replayed_state))
+    K.set_gemv_impl("simt")
+    try:
+        simt, _ = steps(False)
+    finally:
+        K.set_gemv_impl("auto")
+    assert (simt - eager).norm() < 0.022 * eager.norm()
+
+
 def test_batched_decode_matches_independent_sequences(tiny):
     from r4dx_b200.models.batch import BatchModel
     from r4dx_b200.models.hybrid import HybridModel

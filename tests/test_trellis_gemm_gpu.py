@@ -101,6 +101,35 @@ def test_trellis_product_writes_rows_that_are_not_16_byte_aligned(K):
     assert not buf[:4].any() and not buf[4 + 300 * 256:].any()
 
 
+@pytest.mark.parametrize("world,T,N,tn", [(2, 300, 256, 256), (2, 513, 384, 256), (3, 100, 128, 128), (4, 1025, 512, 512), (8, 20, 256, 32), (3, 7, 128, 16)])
+def test_reduce_scatter_epilogue_deals_out_rows_and_counts(K, world, T, N, tn):
+    """Every rank's product with its receive buffers and counters in this GPU's memory, one launch after the other (none waits for
+    another): partial rows have the bits of the product alone and lie with their owner, in their source's part; an owner's counter has
+    one arrival per CTA and rank whose tile touches its rows.  Pairs of CTAs and single ones, owners without a full share of rows."""
+    import ctypes
+    from r4dx_b200.parallel import tp_fused  # noqa: F401  (declares the entry point)
+    from r4dx_b200.quant import trellis
+    tw = trellis.random_weight(N, 512, 4, seed=T, sigma=0.02).to("cuda")
+    rpr = (T + world - 1) // world
+    recv = [torch.full((world, rpr, N), float("nan"), dtype=BF, device="cuda") for _ in range(world)]
+    cnt = [torch.zeros(1, dtype=torch.int32, device="cuda") for _ in range(world)]
+    tab = lambda ts: (ctypes.c_void_p * world)(*[t.data_ptr() for t in ts])
+    g = torch.Generator().manual_seed(world)
+    alone = []
+    for rank in range(world):
+        xh = torch.randn(T, 512, generator=g).half().cuda()
+        K._check(K._lib().r4dxb_trellis_gemm_rs(K._p(tw.words), K._p(tw.svh), K._p(xh), T, N, 512, 4, tn, K._p(K.gemm_status("cuda")), tab(recv),
+                                                tab(cnt), world, rank, rpr, K._stream()), "trellis_gemm_rs")
+        alone.append(K.trellis_gemm(tw, xh, tn=tn))
+    K.check_gemm_status("cuda")
+    for owner in range(world):
+        lo, hi = min(T, owner * rpr), min(T, (owner + 1) * rpr)
+        for rank in range(world):
+            assert torch.equal(recv[owner][rank, :hi - lo], alone[rank][lo:hi]) and bool(recv[owner][rank, hi - lo:].isnan().all())
+        tiles = (hi - 1) // tn - lo // tn + 1 if hi > lo else 0
+        assert int(cnt[owner]) == world * (N // 128) * tiles
+
+
 @pytest.mark.parametrize("N,Kd,T,tn,ksplit", [(96, 5120, 333, 16, 8), (100, 72, 40, 32, 2), (512, 2048, 65, 64, 3), (1000, 200, 257, 256, 4)])
 def test_plain_linear_with_a_split_of_k(K, N, Kd, T, tn, ksplit):
     """fp32 results of bf16 operands with K shared by a cluster (ragged last slab, remainders of tokens and outputs): sums of K
