@@ -90,6 +90,24 @@ def test_trellis_product_tiles_pairs_and_splits(K, kb, T, tn, ksplit, N):
     assert ((z.double() - ref - res.double()).norm() / (ref + res.double()).norm()).item() < 2 ** -8
 
 
+@pytest.mark.parametrize("kb", [3, 4, 5])
+@pytest.mark.parametrize("T", [9, 16, 31, 64])
+def test_trellis_product_of_more_row_blocks_than_sms(K, kb, T):
+    """150 row blocks of few tokens (eight decode warps, two CTAs to an SM) have the bits of the same blocks a few at a time (sixteen)."""
+    from r4dx_b200.quant import trellis
+    N, Kd, part = 150 * 128, 384, 50 * 128
+    tw = trellis.random_weight(N, Kd, kb, seed=kb, sigma=0.02).to("cuda")
+    xh = torch.randn(T, Kd, generator=torch.Generator().manual_seed(T)).half().cuda()
+    tn = 16 if T <= 16 else (32 if T <= 32 else 64)
+    y = K.trellis_gemm(tw, xh, tn=tn, ksplit=1)
+    per = tw.words.numel() // 3
+    for i in range(3):
+        w = trellis.TrellisWeight(tw.words[i * per:(i + 1) * per], tw.suh, tw.svh[i * part:(i + 1) * part], part, Kd, kb)
+        assert torch.equal(y[:, i * part:(i + 1) * part], K.trellis_gemm(w, xh, tn=tn, ksplit=1))
+    ref = R.fwht(xh[:2].double().cpu() @ trellis.decode_codes(tw).double().T) * tw.svh.double().cpu()
+    assert ((y[:2].double().cpu() - ref).norm() / ref.norm()).item() < 2 ** -8
+
+
 def test_trellis_product_writes_rows_that_are_not_16_byte_aligned(K):
     """An output whose base is 8-byte aligned only takes the lane stores instead of the bulk copies."""
     from r4dx_b200.quant import trellis
