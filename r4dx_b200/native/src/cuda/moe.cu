@@ -26,13 +26,12 @@ constexpr int kMaxK = 16;
 // One warp routes one row.  The row's selection values live in registers (E <= 1024: 32 per lane) and a lane remembers its taken
 // entries in a bit mask.  Every lane keeps its best entry; a round is two reductions over the lanes, and only the lane that loses
 // its entry looks for the next one.  (With a search of all lanes and ten shuffles a round, 4096 rows of 512 experts took 30 us, now 18.)
-// A NaN (what a wait that ran out leaves in a row) ranks with minus infinity, so that every row gets k experts that exist; the softmax
-// weights of such a row are NaN, and so is the sigmoid weight of a NaN that is picked.
+// A NaN (what a wait that ran out leaves in a row) ranks last, so that every row gets k experts that exist; the softmax weights of
+// such a row are NaN, and so is the sigmoid weight of a NaN that is picked.
 __device__ __forceinline__ void RouteRow(const float* __restrict__ row, const float* __restrict__ bias, int E, int k, int renorm,
                                          int mode, float scale, int lane, int* __restrict__ ids, float* __restrict__ weights) {
   float v[32];
   float mx = -INFINITY, z = 0.f;
-  bool nan = false;
 #pragma unroll
   for (int s = 0; s < 32; ++s) v[s] = -INFINITY;
 #pragma unroll
@@ -41,11 +40,7 @@ __device__ __forceinline__ void RouteRow(const float* __restrict__ row, const fl
 #pragma unroll
     for (int s = s0; s < s0 + 8; ++s) {
       const int e = lane + 32 * s;
-      if (e < E) {
-        const float x = mode == 0 ? row[e] : 1.0f / (1.0f + expf(-row[e])) + (bias ? bias[e] : 0.f);
-        nan |= x != x;
-        v[s] = fmaxf(x, -INFINITY);          // (a NaN gives the other operand)
-      }
+      if (e < E) v[s] = mode == 0 ? row[e] : 1.0f / (1.0f + expf(-row[e])) + (bias ? bias[e] : 0.f);
       mx = fmaxf(mx, v[s]);
     }
   }
@@ -58,7 +53,6 @@ __device__ __forceinline__ void RouteRow(const float* __restrict__ row, const fl
       for (int s = s0; s < s0 + 8; ++s) z += (lane + 32 * s < E) ? __expf(v[s] - mx) : 0.f;
     }
     z = WarpSum(z);
-    if (__any_sync(0xffffffffu, nan)) z = __int_as_float(0x7FC00000);
   }
   float wsum = 0.f;
   uint32_t taken = 0;              // bit s: this lane's entry lane + 32 s is already picked
@@ -84,8 +78,15 @@ __device__ __forceinline__ void RouteRow(const float* __restrict__ row, const fl
     // (values as integers of the same order; adding zero makes the two zeros one)
     const uint32_t bits = __float_as_uint(lv + 0.0f), key = bits ^ ((bits >> 31) ? 0xFFFFFFFFu : 0x80000000u);
     const uint32_t top = __reduce_max_sync(0xffffffffu, key);
-    const int bi = static_cast<int>(__reduce_min_sync(0xffffffffu, key == top ? static_cast<uint32_t>(li) : 0x7fffffffu));
-    const float bv = __shfl_sync(0xffffffffu, lv, bi & 31);
+    int bi = static_cast<int>(__reduce_min_sync(0xffffffffu, key == top ? static_cast<uint32_t>(li) : 0x7fffffffu));
+    float bv = __shfl_sync(0xffffffffu, lv, bi & 31);
+    if (bi >= E) {                 // (no lane has a number left: the lowest id that is not taken)
+      int next = 0x7fffffff;
+      for (int s = 31; s >= 0; --s)
+        if (lane + 32 * s < E && !((taken >> s) & 1u)) next = lane + 32 * s;
+      bi = static_cast<int>(__reduce_min_sync(0xffffffffu, static_cast<uint32_t>(next)));
+      bv = __int_as_float(0x7FC00000);
+    }
     if ((bi & 31) == lane) {
       taken |= 1u << (bi >> 5);
       look();

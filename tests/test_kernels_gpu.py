@@ -1561,7 +1561,7 @@ def test_window_attention_on_the_tensor_cores_against_fp64(K, D, Hq, Hkv, T, ctx
 @pytest.mark.parametrize("E,k,T", [(16, 4, 6), (64, 16, 8), (257, 10, 40), (1024, 16, 6)])
 def test_router_gives_rows_with_nan_experts_that_exist(K, E, k, T, sigmoid):
     """Rows of NaN, with one value fewer than they pick, with one NaN, and with NaN beside minus infinity: the ids are those of a sort
-    in which a NaN is minus infinity (distinct, below E), the weights of the picks say that the row is no good, other rows are as without them."""
+    in which a NaN comes last (distinct, below E), the weights of the picks say that the row is no good, other rows are as without them."""
     g = torch.Generator().manual_seed(E + T)
     logits = torch.randn(T, E, generator=g)
     clean = logits.clone()
