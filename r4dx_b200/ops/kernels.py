@@ -235,18 +235,37 @@ ROWS_MIN_WEIGHTS = 1 << 23
 ROWS_MIN_WORK = 3 << 24
 
 # Rows from which a launch takes the rows kernel's mma.sync form, and weights from which one row takes its other form, which rounds as
-# the CUDA-core kernel does (fp16 sums of 32 products, whose error decides the logits of all later steps) and transforms the row once
-# per launch instead of once per CTA.  us of a step of the 27B geometry (8 layers, 8192 tokens of context), one-row products on the
-# CUDA cores / on the rows kernel from 64M / from 28M weights: 1425 / 1279 / 1241.  Smaller ones stay: 8192 x 2048 14.3 and 15.4 us.
+# the CUDA-core kernel does (fp16 sums of 16 products, whose error decides the logits of all later steps) and transforms the row once
+# per launch instead of once per CTA.  us of a captured step of the 27B geometry (8 layers, 8192 tokens of context), one-row products on
+# the CUDA cores / on the rows kernel from 64M / from 29M weights: 1282 / 1150 / 1120.  Launches of fewer weights keep the bits they had,
+# which a test compares; for them the rows kernel alone is slower (8192 x 2048 13.9 and 15.3 us), though a step of a small model, whose
+# next product waits for the transform in every CTA, would gain (16 steps of four layers of width 1024: 2914 -> 2692 us).
 ROWS_MIN_ROWS = 2
 ONE_ROW_MIN_WEIGHTS = 7 << 22
+# CTAs that run at a time with one to an SM, by cluster size: 48 clusters of three take two waves, and so on
+_ROWS_SLOTS = {1: 148, 2: 148, 3: 138, 4: 132, 5: 140, 6: 118}
+ONE_ROW_MIN_FILL = 0.67
+
+
+def one_row_split(N: int, K: int) -> Optional[int]:
+    """Split of the rows kernel for one row, None where the CUDA-core kernel serves it: few weights, or a grid whose last wave leaves the
+    SMs idle - the share of their time that the K blocks need, three blocks' time a CTA for the rest, is below 0.67.  us at one row and 4
+    bits with L2 flushed, rows kernel / CUDA-core kernel, by that share: 6144 x 5120 0.59 19.2 / 17.3, 12288 x 5120 0.665 27.6 / 25.5,
+    5120 x 6144 0.68 18.1 / 19.0, 14336 x 5120 0.70 27.6 / 32.2, 5120 x 17408 0.75 31.8 / 37.4, 34816 x 5120 0.86 46.2 / 53.0.  Up to 18 row
+    blocks the CUDA-core kernel, which splits K by eight at most, has less than a CTA per SM (2048 x 17408 21.5 / 31.4)."""
+    rows, blocks = N // 128, K // 128
+    if N * K < ONE_ROW_MIN_WEIGHTS:
+        return None
+    cost = {c: -(-rows * c // slots) * (-(-blocks // c) + 3) for c, slots in _ROWS_SLOTS.items() if c <= blocks}
+    best = min(cost, key=cost.get)
+    return best if rows * 8 < 148 or rows * blocks >= ONE_ROW_MIN_FILL * 148 * cost[best] else None
 
 
 @functools.lru_cache(maxsize=None)
 def rows_split(N: int, K: int, T: int) -> Optional[int]:
     """Split of the rows kernel for T rows of a launch of N outputs, None where one of the other kernels serves it."""
     if T < ROWS_MIN_ROWS:
-        return pick_split(N, K) if N * K >= ONE_ROW_MIN_WEIGHTS else None
+        return one_row_split(N, K)
     return pick_split(N, K) if N * K >= ROWS_MIN_WEIGHTS and T * N * K >= ROWS_MIN_WORK else None
 
 

@@ -135,6 +135,21 @@ def test_a_streamed_head_that_writes_over_its_rows_takes_the_gemm(lib):
     assert [n for n, _ in lib.calls] == ["r4dxb_w4a16_rows"]
 
 
+def test_one_row_takes_the_rows_kernel_only_where_its_grid_fills_the_sms():
+    """The 27B launches (o, down, q / k / v, qkv / z, gate / up) do, with the splits they were measured with; launches of as many weights
+    whose clusters need a nearly empty wave more, which took 1.1 to 1.5 times as long there, do not, and no small one does."""
+    from r4dx_b200.ops import kernels as K
+    for N, Kd, split in ((5120, 6144, 3), (5120, 17408, 3), (14336, 5120, 1), (16384, 5120, 1), (34816, 5120, 1), (8192, 5120, 2), (4096, 11008, 4),
+                         (2048, 17408, 6)):
+        assert K.rows_split(N, Kd, 1) == split
+    for N, Kd in ((6144, 5120), (6144, 8192), (10240, 5120), (12288, 4096), (12288, 5120), (20480, 2048), (24576, 2048), (8192, 2048), (4096, 4096)):
+        assert K.rows_split(N, Kd, 1) is None
+    for N in range(128, 40000, 128 * 5):
+        for Kd in (128, 640, 5120, 17408, 28672):
+            s = K.rows_split(N, Kd, 1)
+            assert s is None or (1 <= s <= min(6, Kd // 128) and N * Kd >= K.ONE_ROW_MIN_WEIGHTS)
+
+
 def test_products_get_a_tile_and_a_split_that_the_kernel_has():
     """Token tile and split of K by shape: a tile of the kernel, at most eight CTAs in a cluster (a pair counts twice), at least 128
     columns of K for each; a plain linear that fills the chip keeps its tile and is not split."""
