@@ -23,13 +23,14 @@ __global__ void EmbedGatherKernel(const int* __restrict__ ids, const uint4* __re
 }
 
 // mode bit 0: weight is zero-centred (multiply by 1 + w); bit 1: no weight.
-// A row of a few kilobytes is a chain of memory latencies, so rows of up to kRegColumns columns have all their loads in flight at once
-// and stay in registers; longer ones pass through shared memory, 512 columns a step.  The sums are the same in both.  5120 columns,
-// 1 / 16 / 333 / 8192 rows: 2.6 / 2.8 / 3.8 / 44 us (5.1 / 5.1 / 5.6 / 59 through shared memory).
-constexpr int kRegPairs = 16;
-constexpr int kRegColumns = kRegPairs * 2 * kRowThreads;
+// A row of a few kilobytes is a chain of memory latencies, so rows of up to 8192 columns have all their loads in flight at once and stay
+// in registers, in an instance with the least power of two of column pairs a thread that holds them (with sixteen for every row, 8192
+// rows of 1024 / 2048 columns took 29 / 31 us); longer ones pass through shared memory, 512 columns a step.  The sums are the same in
+// both.  us at 1 / 333 / 8192 rows (through shared memory): 512 columns 1.9 / 2.1 / 8.9 (2.1 / 2.2 / 9.9), 2048 2.0 / 2.6 / 15.2
+// (3.0 / 3.5 / 18.4), 5120 3.0 / 3.8 / 43.6 (5.3 / 5.7 / 58.9), 8192 3.2 / 4.5 / 52 (7.3 / 7.9 / 121).
+constexpr int kPairColumns = 2 * kRowThreads;
 
-template <bool kAdd>
+template <bool kAdd, int kRegPairs>
 __global__ void __launch_bounds__(kRowThreads) RmsNormRowKernel(__nv_bfloat16* __restrict__ res, const __nv_bfloat16* __restrict__ delta,
                                                                 const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ out,
                                                                 int H, float eps, int mode) {
@@ -216,7 +217,11 @@ static int RmsNormRows(void* res, const void* delta, const void* w, void* out, i
   const __nv_bfloat16* d = static_cast<const __nv_bfloat16*>(delta);
   const __nv_bfloat16* g = static_cast<const __nv_bfloat16*>(w);
   __nv_bfloat16* o = static_cast<__nv_bfloat16*>(out);
-  if (H <= kRegColumns) RmsNormRowKernel<kAdd><<<T, kRowThreads, 0, s>>>(r, d, g, o, H, eps, mode);
+  if (H <= kPairColumns) RmsNormRowKernel<kAdd, 1><<<T, kRowThreads, 0, s>>>(r, d, g, o, H, eps, mode);
+  else if (H <= 2 * kPairColumns) RmsNormRowKernel<kAdd, 2><<<T, kRowThreads, 0, s>>>(r, d, g, o, H, eps, mode);
+  else if (H <= 4 * kPairColumns) RmsNormRowKernel<kAdd, 4><<<T, kRowThreads, 0, s>>>(r, d, g, o, H, eps, mode);
+  else if (H <= 8 * kPairColumns) RmsNormRowKernel<kAdd, 8><<<T, kRowThreads, 0, s>>>(r, d, g, o, H, eps, mode);
+  else if (H <= 16 * kPairColumns) RmsNormRowKernel<kAdd, 16><<<T, kRowThreads, 0, s>>>(r, d, g, o, H, eps, mode);
   else RmsNormKernel<kAdd><<<T, kRowThreads, H * sizeof(float), s>>>(r, d, g, o, H, eps, mode);
   return FinishLaunch();
 }

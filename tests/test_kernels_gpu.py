@@ -445,7 +445,7 @@ def test_linear_tc_dense_matches_fp32_reference(K, dtype, T, N, Kd):
         assert torch.allclose(ya.cpu(), fn(ref), atol=3e-2, rtol=1e-2)
 
 
-@pytest.mark.parametrize("H", [2, 510, 514, 8190, 8192, 8194])
+@pytest.mark.parametrize("H", [2, 510, 512, 514, 1024, 1026, 2048, 2050, 4096, 4098, 8190, 8192, 8194])
 @pytest.mark.parametrize("add", [False, True])
 def test_rmsnorm_at_the_edges_of_its_register_rows(K, H, add):
     """Rows below, at and past what the threads keep in registers, ragged against the 512 columns of a step: one bf16 rounding of the fp64
