@@ -421,8 +421,9 @@ TrellisGemmKernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
           for (int c = 0; c < CW; ++c) epi[c * S::kEpiStride + q * 32 + lane] = nan;
         }
         asm volatile("bar.sync %0, 128;" ::"r"(1 + grp) : "memory");
-        for (int c = q; c < CW; c += 4) {
-          const int t = t0 + c0 + c;
+#pragma unroll
+        for (int i = 0; i < CW / 4; ++i) {
+          const int c = q + 4 * i, t = t0 + c0 + c;
           if (t < T) {
             const float4 p = *reinterpret_cast<const float4*>(epi + c * S::kEpiStride + lane * 4);
             float f[4] = {ok ? p.x : nan, ok ? p.y : nan, ok ? p.z : nan, ok ? p.w : nan};
