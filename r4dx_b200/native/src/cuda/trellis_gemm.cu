@@ -409,16 +409,25 @@ TrellisGemmKernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
         finish(t0 + c, f);
       }
       ptx::ClusterSync();
-    } else {
+    } else if (!ok) {
+      // a wait ran out: NaN into the group's buffer for the warps that do not know of it, and into the rows of this warp's tokens
       const float nan = __int_as_float(0x7FC00000);
       for (int c0 = grp * 32; c0 < TN; c0 += kGroups * 32) {
-        if (ok) {
+        for (int c = 0; c < CW; ++c) epi[c * S::kEpiStride + q * 32 + lane] = nan;
+        asm volatile("bar.sync %0, 128;" ::"r"(1 + grp) : "memory");
+        for (int t = t0 + c0 + q; t < min(t0 + c0 + CW, T); t += 4) {
+          float f[4] = {nan, nan, nan, nan};
+          finish(t, f);
+        }
+        asm volatile("bar.sync %0, 128;" ::"r"(1 + grp) : "memory");
+      }
+    } else {
+      for (int c0 = grp * 32; c0 < TN; c0 += kGroups * 32) {
+        {
           uint32_t v[CW];
           load_columns(c0, v);
 #pragma unroll
           for (int c = 0; c < CW; ++c) epi[c * S::kEpiStride + q * 32 + lane] = __uint_as_float(v[c]);
-        } else {                             // (a wait that ran out shows as NaN)
-          for (int c = 0; c < CW; ++c) epi[c * S::kEpiStride + q * 32 + lane] = nan;
         }
         asm volatile("bar.sync %0, 128;" ::"r"(1 + grp) : "memory");
 #pragma unroll
@@ -426,7 +435,7 @@ TrellisGemmKernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
           const int c = q + 4 * i, t = t0 + c0 + c;
           if (t < T) {
             const float4 p = *reinterpret_cast<const float4*>(epi + c * S::kEpiStride + lane * 4);
-            float f[4] = {ok ? p.x : nan, ok ? p.y : nan, ok ? p.z : nan, ok ? p.w : nan};
+            float f[4] = {p.x, p.y, p.z, p.w};
             finish(t, f);
           }
         }

@@ -392,6 +392,7 @@ TrellisProductKernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_co
       }
     };
     const int tile_end = min(TN, t_end - t0);            // tokens of this tile
+    constexpr int kBuffers = 2 * S::kEpiGroups <= S::kRings ? 2 : 1;
     if (DW == 16 && ksplit > 1) {
       // K was split: the CTAs of the cluster lay their sums side by side in shared memory, a chunk of token columns at a time, and
       // each finishes its share of the tokens, adding up over distributed shared memory in rank order
@@ -420,33 +421,36 @@ TrellisProductKernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_co
           }, to_row);
         ptx::ClusterSync();
       }
+    } else if (!ok) {
+      // a wait ran out: NaN into the group's buffers for the warps that do not know of it, and into the rows of this warp's tokens
+      for (int c0 = grp * 32, buf = 0; c0 < tile_end; c0 += kGroups * 32, buf ^= kBuffers - 1) {
+        float* epi = reinterpret_cast<float*>(smem + (grp * kBuffers + buf) * S::kEpiBytes);
+        for (int c = 0; c < CW; ++c) epi[c * S::kEpiStride + q * 32 + lane] = __int_as_float(0x7FC00000);
+        asm volatile("bar.sync %0, 128;" ::"r"(1 + grp) : "memory");
+        for (int c = c0 + q * kTokens; c < min(c0 + CW, tile_end); c += 4 * kTokens)
+          for (int i = 0; i < min(kTokens, tile_end - c); ++i) to_row(t0 + c + i, lane * 4, make_uint2(0x7FC07FC0u, 0x7FC07FC0u));
+        if (kBuffers == 1) asm volatile("bar.sync %0, 128;" ::"r"(1 + grp) : "memory");
+      }
     } else {
       // Two buffers a group where they fit: a warp loads its next columns while others finish theirs.  Wide tiles: the rounded rows
       // of a token replace its sums and leave as one bulk copy of 256 bytes (stores of a lane's rows, 32 bytes of eight tokens
-      // each, took half of the epilogue: 27k of 115k clocks a tile at 512 tokens).  A warp whose wait ran out writes NaN: into the
-      // buffer for the others, and by plain stores into its tokens' rows.
-      constexpr int kBuffers = 2 * S::kEpiGroups <= S::kRings ? 2 : 1;
+      // each, took half of the epilogue: 27k of 115k clocks a tile at 512 tokens).
       const bool bulk = S::kWide && a.rs.world == 0 && (reinterpret_cast<uintptr_t>(a.y) & 15) == 0;
       int buf = 0;
       for (int c0 = grp * 32; c0 < tile_end; c0 += kGroups * 32, buf ^= kBuffers - 1) {
         float* epi = reinterpret_cast<float*>(smem + (grp * kBuffers + buf) * S::kEpiBytes);
-        if (ok) {
+        {
           uint32_t v[CW];
           TmemLoadColumns<CW>(tmem_lane + c0, v);
           ptx::TmemLoadWait();
 #pragma unroll
           for (int c = 0; c < CW; ++c) epi[c * S::kEpiStride + q * 32 + lane] = __uint_as_float(v[c]);
-        } else {
-          for (int c = 0; c < CW; ++c) epi[c * S::kEpiStride + q * 32 + lane] = __int_as_float(0x7FC00000);
         }
         if (kBuffers == 2 && bulk) ptx::BulkStoreWaitRead();      // (the copies out of the other buffer, before anyone writes there)
         asm volatile("bar.sync %0, 128;" ::"r"(1 + grp) : "memory");
         const int c_end = min(c0 + CW, tile_end);
         auto load = [&](int ct, int row) { return *reinterpret_cast<const float4*>(epi + (ct - c0) * S::kEpiStride + row); };
-        if (!ok) {
-          for (int c = c0 + q * kTokens; c < c_end; c += 4 * kTokens)
-            for (int i = 0; i < min(kTokens, c_end - c); ++i) to_row(t0 + c + i, lane * 4, make_uint2(0x7FC07FC0u, 0x7FC07FC0u));
-        } else if (bulk) {
+        if (bulk) {
           const int c = c0 + q * kTokens;
           if (c < c_end) {
             finish(c, c_end, load, [&](int t, int r, uint2 v) {
