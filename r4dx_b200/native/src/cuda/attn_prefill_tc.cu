@@ -501,7 +501,7 @@ template <int D>
 int LaunchTc(const TcArgs& a, cudaStream_t s) {
   constexpr int NS = D / 64;
   // kClusterAlone: so much of an SM's shared memory that no other CTA shares the SM whose cluster may wait with tensor memory in its
-  // hands (sm100_ptx.cuh).  More would cost L1: 8192 rows of 32 heads of 128 columns take 808 us with 116 KB, 821 with 156, 878 with 227.
+  // hands (sm100_ptx.cuh).  More would cost L1: 8192 rows of 32 heads of 128 columns take 808 us with 131 KB, 821 with 156, 878 with 227.
   constexpr size_t kSmem = NS * kQRows * 128 + 2 * NS * kHalfTile * 128 + 2 * D * 128 + sizeof(Control) + 1024;
   constexpr size_t smem = kSmem > ptx::kClusterAlone ? kSmem : ptx::kClusterAlone;
   auto kern = AttnPrefillTcKernel<D>;

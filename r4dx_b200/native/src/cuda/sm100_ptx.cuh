@@ -209,8 +209,10 @@ __device__ __forceinline__ void BulkStoreWait() { asm volatile("cp.async.bulk.wa
 //   prefill attention, pairs: kClusterAlone or more (all tensor memory)
 //   trellis product, pairs and splits: kProductAlone or more
 //   plain linears with a split of K: kClusterShared or more, so two at most on an SM, and none beside the others
+// The sizes are the last ones below a step of the split of 228 KB between shared memory and L1 (132 and, for two CTAs, 196 KB): with
+// 112 KB a w4a16 linear of 5120 x 17408, whose weights are read through the L1, took 72 us at 64 rows where it takes 67.
 // (The waits of the weight-streaming kernel of trellis_gemv_mma.cu for its cluster are bounded: beside it a launch may be late, never stuck.)
-constexpr size_t kClusterAlone = 116 * 1024, kProductAlone = 176 * 1024, kClusterShared = 112 * 1024;
+constexpr size_t kClusterAlone = 131 * 1024, kProductAlone = 176 * 1024, kClusterShared = 96 * 1024;
 static_assert(kClusterAlone + kClusterShared + 2 * 1024 > 228 * 1024 && 2 * (kClusterShared + 1024) <= 228 * 1024 &&
               kClusterAlone <= kProductAlone, "none of the first two kinds meets one of the three");
 // Whole-warp calls (.sync.aligned).  Columns: power of two, 32..512.

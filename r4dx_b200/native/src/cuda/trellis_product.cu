@@ -111,6 +111,17 @@ __device__ __forceinline__ void TmemLoadColumns(uint32_t taddr, uint32_t (&v)[CW
   else ptx::TmemLoad32x16(taddr, v);
 }
 
+// Where the outputs of token t of row block nb go.
+template <bool kGrouped>
+__device__ __forceinline__ __nv_bfloat16* OutRow(const ProductArgs& a, int t, int nb) {
+  if constexpr (kGrouped) return a.y + static_cast<size_t>(__ldg(a.g.perm + t)) * a.N + nb * 128;
+  if (a.rs.world > 0) {
+    const int owner = t / a.rs.rows_per_rank, tl = t - owner * a.rs.rows_per_rank;
+    return a.rs.recv[owner] + (static_cast<size_t>(a.rs.rank) * a.rs.rows_per_rank + tl) * a.N + nb * 128;
+  }
+  return a.y + static_cast<size_t>(t) * a.N + nb * 128;
+}
+
 template <int KB, int TN, int DW, bool kPair, bool kGrouped>
 __global__ void __launch_bounds__((DW + 3) * 32, DW == 8 ? 2 : 1)
 TrellisProductKernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ ProductArgs a) {
@@ -316,15 +327,7 @@ TrellisProductKernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_co
     constexpr int CW = TN < 32 ? 16 : 32;    // columns per TMEM load
     const int q = warp & 3, grp = warp >> 2;
     const uint32_t tmem_lane = tmem_base + (static_cast<uint32_t>(q * 32) << 16);
-    // where the outputs of token t of this CTA's row block go
-    auto out_row = [&](int t) -> __nv_bfloat16* {
-      if constexpr (kGrouped) return a.y + static_cast<size_t>(__ldg(a.g.perm + t)) * N + nb * 128;
-      if (a.rs.world > 0) {
-        const int owner = t / a.rs.rows_per_rank, tl = t - owner * a.rs.rows_per_rank;
-        return a.rs.recv[owner] + (static_cast<size_t>(a.rs.rank) * a.rs.rows_per_rank + tl) * N + nb * 128;
-      }
-      return a.y + static_cast<size_t>(t) * N + nb * 128;
-    };
+    auto out_row = [&](int t) { return OutRow<kGrouped>(a, t, nb); };
     auto to_row = [&](int t, int r, uint2 v) { *reinterpret_cast<uint2*>(out_row(t) + r) = v; };
     // four outputs (rows r ..) of token t: residual and rounding
     auto round4 = [&](int t, int r, float o0, float o1, float o2, float o3) {
@@ -392,7 +395,6 @@ TrellisProductKernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_co
       }
     };
     const int tile_end = min(TN, t_end - t0);            // tokens of this tile
-    constexpr int kBuffers = 2 * S::kEpiGroups <= S::kRings ? 2 : 1;
     if (DW == 16 && ksplit > 1) {
       // K was split: the CTAs of the cluster lay their sums side by side in shared memory, a chunk of token columns at a time, and
       // each finishes its share of the tokens, adding up over distributed shared memory in rank order
@@ -421,25 +423,16 @@ TrellisProductKernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_co
           }, to_row);
         ptx::ClusterSync();
       }
-    } else if (!ok) {
-      // a wait ran out: NaN into the group's buffers for the warps that do not know of it, and into the rows of this warp's tokens
-      for (int c0 = grp * 32, buf = 0; c0 < tile_end; c0 += kGroups * 32, buf ^= kBuffers - 1) {
-        float* epi = reinterpret_cast<float*>(smem + (grp * kBuffers + buf) * S::kEpiBytes);
-        for (int c = 0; c < CW; ++c) epi[c * S::kEpiStride + q * 32 + lane] = __int_as_float(0x7FC00000);
-        asm volatile("bar.sync %0, 128;" ::"r"(1 + grp) : "memory");
-        for (int c = c0 + q * kTokens; c < min(c0 + CW, tile_end); c += 4 * kTokens)
-          for (int i = 0; i < min(kTokens, tile_end - c); ++i) to_row(t0 + c + i, lane * 4, make_uint2(0x7FC07FC0u, 0x7FC07FC0u));
-        if (kBuffers == 1) asm volatile("bar.sync %0, 128;" ::"r"(1 + grp) : "memory");
-      }
     } else {
       // Two buffers a group where they fit: a warp loads its next columns while others finish theirs.  Wide tiles: the rounded rows
       // of a token replace its sums and leave as one bulk copy of 256 bytes (stores of a lane's rows, 32 bytes of eight tokens
       // each, took half of the epilogue: 27k of 115k clocks a tile at 512 tokens).
+      constexpr int kBuffers = 2 * S::kEpiGroups <= S::kRings ? 2 : 1;
       const bool bulk = S::kWide && a.rs.world == 0 && (reinterpret_cast<uintptr_t>(a.y) & 15) == 0;
       int buf = 0;
       for (int c0 = grp * 32; c0 < tile_end; c0 += kGroups * 32, buf ^= kBuffers - 1) {
         float* epi = reinterpret_cast<float*>(smem + (grp * kBuffers + buf) * S::kEpiBytes);
-        {
+        if (ok) {
           uint32_t v[CW];
           TmemLoadColumns<CW>(tmem_lane + c0, v);
           ptx::TmemLoadWait();
@@ -452,7 +445,7 @@ TrellisProductKernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_co
         auto load = [&](int ct, int row) { return *reinterpret_cast<const float4*>(epi + (ct - c0) * S::kEpiStride + row); };
         if (bulk) {
           const int c = c0 + q * kTokens;
-          if (c < c_end) {
+          if (ok && c < c_end) {
             finish(c, c_end, load, [&](int t, int r, uint2 v) {
               *reinterpret_cast<uint2*>(reinterpret_cast<__nv_bfloat16*>(epi + (t - t0 - c0) * S::kEpiStride) + r) = v;
             });
@@ -464,7 +457,7 @@ TrellisProductKernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_co
             }
             if (kBuffers == 1) ptx::BulkStoreWaitRead();
           }
-        } else {
+        } else if (ok) {
           for (int c = c0 + q * kTokens; c < c_end; c += 4 * kTokens) finish(c, c_end, load, to_row);
         }
         if (kBuffers == 1) asm volatile("bar.sync %0, 128;" ::"r"(1 + grp) : "memory");
@@ -495,6 +488,9 @@ TrellisProductKernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_co
   ptx::TcFenceBefore();
   __syncthreads();
   if (*abort_flag != 0) {
+    // a wait ran out: NaN instead of what the rows held before
+    for (int t = t0 + warp; t < min(t0 + TN, t_end); t += DW + 3)
+      *reinterpret_cast<uint2*>(OutRow<kGrouped>(a, t, nb) + lane * 4) = make_uint2(0x7FC07FC0u, 0x7FC07FC0u);
     // give copies that may still be in flight time to land before the shared memory goes away
     for (int i = 0; i < 64; ++i) __nanosleep(1000);
     if (threadIdx.x == 0) atomicExch(a.status, *abort_flag);

@@ -671,8 +671,9 @@ def _w4a16_rows(W: W4Weight, x: torch.Tensor, out_f32: bool, out: Optional[torch
 @functools.lru_cache(maxsize=4096)
 def pick_plain(T: int, N: int, K: int) -> tuple:
     """(token tile, split of K) of a plain linear.  Where row blocks and tiles leave most SMs idle - a router, the a / b projections -
-    narrower tiles and CTAs that share K: 96 x 5120 at 333 / 8192 rows 49 / 104 us with 256- and 512-row tiles, 12 / 33 so; 512 x
-    2048 at 64 rows 18 and 10."""
+    narrower tiles and CTAs that share K, the fewest us by waves of the clusters that fit the chip: 96 x 5120 at 333 / 8192 rows 37 / 85 us
+    with 256- and 512-row tiles, 7 / 18 so; 512 x 2048 at 64 / 1000 rows 15.4 / 17.0 and 6.5 / 9.6 (with eight CTAs to a cluster, as if 128
+    of them ran at a time and not 112, 1000 rows took 20.5); 4304 x 1152 at 64 rows 10.8 and 8.0 (13.1)."""
     blocks, slabs = (N + 127) // 128, (K + 63) // 64
     tn = pick_token_tile(T, N)
     if blocks * ((T + tn - 1) // tn) >= 74:
@@ -681,12 +682,12 @@ def pick_plain(T: int, N: int, K: int) -> tuple:
     for t, c in ((16, 0.25), (32, 0.26), (64, 0.28), (128, 0.33), (256, 0.50)):
         if t > 16 and t >= 2 * T:
             continue
-        slots = 296 if t <= 64 else 148      # (narrow tiles: two CTAs share an SM)
         for ks in (1, 2, 4, 8):
             if slabs < ks:
                 break
+            slots = _CLUSTER_SLOTS[ks] * (2 if t <= 64 else 1)         # (narrow tiles: two CTAs share an SM)
             ctas = blocks * ((T + t - 1) // t) * ks
-            cost = (ctas + slots - 1) // slots * (6 + (slabs + ks - 1) // ks * c) + (3 if ks > 1 else 0)
+            cost = (ctas + slots - 1) // slots * (6 + 0.005 * min(t, T) + (slabs + ks - 1) // ks * c) + (3 if ks > 1 else 0)
             if best_cost is None or cost < best_cost - 1e-9:
                 best, best_cost = (t, ks), cost
     return best

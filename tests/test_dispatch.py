@@ -163,4 +163,7 @@ def test_products_get_a_tile_and_a_split_that_the_kernel_has():
                 tp, kp = K.pick_plain(T, N, Kd)
                 assert tp in (16, 32, 64, 128, 256, 512) and 1 <= kp <= (Kd + 63) // 64 and (kp == 1 or tp <= 256)
     assert K.pick_plain(4096, 4096, 4096) == (K.pick_token_tile(4096, 4096), 1)
+    for N, Kd, T in ((512, 2048, 1000), (512, 2560, 1000), (4304, 1152, 64), (2048, 2048, 256), (96, 5120, 4096)):
+        tp, kp = K.pick_plain(T, N, Kd)          # (one wave of the clusters that fit the chip; these had two)
+        assert (N + 127) // 128 * ((T + tp - 1) // tp) * kp <= K._CLUSTER_SLOTS[kp] * (2 if tp <= 64 else 1)
     assert K.pick_product.cache_info().maxsize and K.pick_plain.cache_info().maxsize          # (bounded: one entry per prompt length)
