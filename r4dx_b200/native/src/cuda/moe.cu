@@ -181,7 +181,7 @@ MoeRoutePlanKernel(const float* __restrict__ logits, const float* __restrict__ b
 }
 
 // Single CTA: counting sort of the T*k pairs by expert (stable in pair order), a pair per thread; the warps place theirs one after
-// the other.  (640 pairs of 512 experts: 28.8 -> 5.8 us; one thread did it.)
+// the other.  (640 pairs of 512 experts: 28.8 -> 5.8 us; one thread did it.)  Few pairs and experts take a smaller CTA.
 constexpr int kPlanThreads = 1024;
 __global__ void __launch_bounds__(kPlanThreads) MoePlanKernel(const int* __restrict__ ids, int npairs, int E, int e_begin, int e_count,
                               int* __restrict__ offsets, int* __restrict__ perm) {
@@ -202,10 +202,10 @@ __global__ void __launch_bounds__(kPlanThreads) MoePlanKernel(const int* __restr
   BlockInclusiveScan(cnt, e_count + 1, warp_sums);
   for (int e = threadIdx.x; e <= e_count; e += blockDim.x) offsets[e] = cnt[e];
   __syncthreads();
-  for (int base = 0; base < npairs; base += kPlanThreads) {
+  for (int base = 0; base < npairs; base += blockDim.x) {
     const int p = base + threadIdx.x, e = expert_of(p);
     const unsigned same = SameExpert(e, 32 - __clz(e_count - 1));
-    for (int w = 0; w < (min(npairs - base, kPlanThreads) + 31) / 32; ++w) {
+    for (int w = 0; w < (min(npairs - base, static_cast<int>(blockDim.x)) + 31) / 32; ++w) {
       if (warp == w && e >= 0) perm[cnt[e] + __popc(same & ((1u << lane) - 1u))] = p;
       __syncwarp();
       if (warp == w && e >= 0 && lane == __ffs(same) - 1) cnt[e] += __popc(same);
@@ -246,7 +246,7 @@ MoePlanParallelKernel(const int* __restrict__ ids, int npairs, int e_begin, int 
     request(base);
 #pragma unroll
     for (int i = 0; i < kPlanAhead; ++i)
-      if (next[i] >= 0) atomicAdd(&mine[next[i]], 1);
+      if (base + 32 * i < p1 && next[i] >= 0) atomicAdd(&mine[next[i]], 1);
   }
   __syncthreads();
   // per expert: total, then each warp's first slot
@@ -272,6 +272,7 @@ MoePlanParallelKernel(const int* __restrict__ ids, int npairs, int e_begin, int 
     request(base);
 #pragma unroll
     for (int i = 0; i < kPlanAhead; ++i) {
+      if (base + 32 * i >= p1) break;
       const int e = next[i];
       const unsigned same = SameExpert(e, 32 - __clz(e_count - 1));
       if (e >= 0) perm[mine[e] + __popc(same & ((1u << lane) - 1u))] = base + 32 * i + lane;
@@ -380,7 +381,8 @@ int r4dxb_moe_plan(const int* ids, int npairs, int E, int e_begin, int e_count, 
     MoePlanParallelKernel<<<1, kPlanWarps * 32, big, static_cast<cudaStream_t>(stream)>>>(ids, npairs, e_begin, e_count, offsets, perm);
     return FinishLaunch();
   }
-  MoePlanKernel<<<1, kPlanThreads, (e_count + 1) * sizeof(int), static_cast<cudaStream_t>(stream)>>>(ids, npairs, E, e_begin, e_count,
+  const int threads = npairs <= 128 && e_count <= 128 ? 128 : kPlanThreads;
+  MoePlanKernel<<<1, threads, (e_count + 1) * sizeof(int), static_cast<cudaStream_t>(stream)>>>(ids, npairs, E, e_begin, e_count,
                                                                                              offsets, perm);
   return FinishLaunch();
 }

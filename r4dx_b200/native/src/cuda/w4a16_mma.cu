@@ -60,15 +60,19 @@ __device__ __forceinline__ void LoadStream(const uint32_t* p, uint32_t (&o)[V]) 
 }
 
 // chunks in flight per warp: what 128 registers allow
-template <int NT, int G>
-constexpr int Chunks() { return G == 32 ? 4 : (G == 64 ? 3 : (NT == 1 ? 2 : 1)); }
+template <int NT, int G, bool kRagged>
+constexpr int Chunks() { return G == 32 ? 4 : (G == 64 ? (kRagged ? 2 : 3) : (NT == 1 ? 2 : 1)); }
 
-template <int NT, int G>
+// kRagged: zeros in place of the absent rows of the second eight, not loaded.  The rows of x then come out of the L1, which bounds the
+// kernel, as often as there are rows: us of a 248320 x 5120 head, groups of 128, at 9 / 12 / 14 rows 187 / 189 / 204, without it 216 /
+// 214 / 211 (groups of 32: 303 / 331 / 367 and 326 / 345 / 357; of 64, where it leaves two chunks in flight: 128256 x 4096 90 / 92 / 95
+// and 94 / 94 / 95); the test costs more than it saves from there on.
+template <int NT, int G, bool kRagged>
 __global__ void __launch_bounds__(kW4Threads, 1)
 W4MmaKernel(const uint32_t* __restrict__ wq, const uint32_t* __restrict__ wsz, const __nv_bfloat16* __restrict__ x,
             void* __restrict__ y, int T, int N, int K, int out_f32, int slices) {
   constexpr int V = G / 32;                        // words a lane takes of a row's group
-  constexpr int D = Chunks<NT, G>();               // chunks in flight per warp
+  constexpr int D = Chunks<NT, G, kRagged>();               // chunks in flight per warp
   extern __shared__ __align__(128) unsigned char xs[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, c = lane & 3;
   const int xstride = K * 2 + 16;                  // bytes: the eight rows of a fragment start 16 bytes apart modulo the banks
@@ -140,10 +144,11 @@ W4MmaKernel(const uint32_t* __restrict__ wq, const uint32_t* __restrict__ wsz, c
         }
       }
   };
-  // rows past T take the last one's x: their columns of the product are never stored
+  // rows past T take the last one's x (kRagged: zeros): their columns of the product are never stored
   const unsigned char* xrow[NT];
 #pragma unroll
   for (int nt = 0; nt < NT; ++nt) xrow[nt] = xs + static_cast<size_t>(min(nt * 8 + g, T - 1)) * xstride + c * (V * 16);
+  const bool present = !kRagged || (NT - 1) * 8 + g < T;
   bool live = tile < tiles;
   while (live) {
 #pragma unroll
@@ -171,7 +176,8 @@ W4MmaKernel(const uint32_t* __restrict__ wq, const uint32_t* __restrict__ wsz, c
           Widen(w1[d][gi][v], nz1, nzs1, b);
 #pragma unroll
           for (int nt = 0; nt < NT; ++nt) {
-            const uint4 xv = *reinterpret_cast<const uint4*>(xp[nt] + gi * (G * 2) + v * 16);
+            uint4 xv = make_uint4(0u, 0u, 0u, 0u);
+            if (!kRagged || nt < NT - 1 || present) xv = *reinterpret_cast<const uint4*>(xp[nt] + gi * (G * 2) + v * 16);
             MmaF16(acc[nt], a[0], b[0], a[1], b[1], xv.x, xv.y);
             MmaF16(acc[nt], a[2], b[2], a[3], b[3], xv.z, xv.w);
           }
@@ -223,7 +229,7 @@ W4MmaKernel(const uint32_t* __restrict__ wq, const uint32_t* __restrict__ wsz, c
   }
 }
 
-template <int NT, int G>
+template <int NT, int G, bool kRagged = false>
 int LaunchW4Mma(const void* wq, const void* wsz, const void* x, void* y, int T, int N, int K, int out_f32, cudaStream_t stream) {
   const size_t xbytes = (static_cast<size_t>(T) * (K * 2 + 16) + 15) & ~static_cast<size_t>(15), red = static_cast<size_t>(kWarps) * NT * 512;
   const int tiles = N / 16, grid = min(148, tiles);                 // one CTA per SM, a warp walks its 16-row tiles
@@ -234,7 +240,7 @@ int LaunchW4Mma(const void* wq, const void* wsz, const void* x, void* y, int T, 
          xbytes + red <= 227 * 1024)
     slices *= 2;
   const size_t smem = xbytes + (slices > 1 ? red : 0);
-  auto kern = W4MmaKernel<NT, G>;
+  auto kern = W4MmaKernel<NT, G, kRagged>;
   const cudaError_t e = AllowAllSharedMemory(kern);
   if (e != cudaSuccess) return static_cast<int>(e);
   kern<<<grid, kW4Threads, smem, stream>>>(static_cast<const uint32_t*>(wq), static_cast<const uint32_t*>(wsz),
@@ -245,6 +251,7 @@ int LaunchW4Mma(const void* wq, const void* wsz, const void* x, void* y, int T, 
 template <int G>
 int LaunchW4MmaT(const void* wq, const void* wsz, const void* x, void* y, int T, int N, int K, int out_f32, cudaStream_t s) {
   if (T <= 8) return LaunchW4Mma<1, G>(wq, wsz, x, y, T, N, K, out_f32, s);
+  if (T <= (G == 128 ? 14 : 12)) return LaunchW4Mma<2, G, true>(wq, wsz, x, y, T, N, K, out_f32, s);
   return LaunchW4Mma<2, G>(wq, wsz, x, y, T, N, K, out_f32, s);
 }
 

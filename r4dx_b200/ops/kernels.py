@@ -687,7 +687,7 @@ def pick_plain(T: int, N: int, K: int) -> tuple:
                 break
             slots = _CLUSTER_SLOTS[ks] * (2 if t <= 64 else 1)         # (narrow tiles: two CTAs share an SM)
             ctas = blocks * ((T + t - 1) // t) * ks
-            cost = (ctas + slots - 1) // slots * (6 + 0.005 * min(t, T) + (slabs + ks - 1) // ks * c) + (3 if ks > 1 else 0)
+            cost = (ctas + slots - 1) // slots * (6 + 0.002 * min(t, T) + (slabs + ks - 1) // ks * c) + (3 if ks > 1 else 0)
             if best_cost is None or cost < best_cost - 1e-9:
                 best, best_cost = (t, ks), cost
     return best

@@ -302,8 +302,8 @@ def test_w4a16_gemv_and_argmax(K, T):
     assert torch.equal(ids.cpu().long(), y.cpu().argmax(-1) + 7)
 
 
-@pytest.mark.parametrize("T", [1, 3, 8, 9, 16])
-@pytest.mark.parametrize("N,Kd,group", [(16, 128, 32), (48, 512, 64), (1040, 512, 128), (2384, 1280, 64), (40000, 1024, 128)])
+@pytest.mark.parametrize("T", [1, 3, 8, 9, 12, 13, 14, 15, 16])
+@pytest.mark.parametrize("N,Kd,group", [(16, 128, 32), (1040, 1024, 32), (48, 512, 64), (1040, 512, 128), (2384, 1280, 64), (40000, 1024, 128)])
 def test_w4a16_streaming_rows_match_fp64(K, T, N, Kd, group):
     """Every shape class of the mma.sync streaming kernel (K split over 1..16 warps, one or many tiles per warp, both output
     types).  (n - zero) * x is exact in fp32 (5 + 11 bits) and each sum of K terms rounds at most once per term, so the error
@@ -1481,7 +1481,7 @@ def test_one_row_on_the_rows_kernel_rounds_as_the_cuda_core_kernel(K, kb, N, Kd,
         assert ((y - ref).abs() <= 2.0 ** -7 * ref.abs() + 2.0 ** -14 * ref.abs().max()).all()
 
 
-@pytest.mark.parametrize("E,k,T", [(16, 4, 3), (33, 16, 8), (257, 10, 40), (512, 10, 102), (1000, 8, 129), (1024, 16, 64), (512, 10, 700)])
+@pytest.mark.parametrize("E,k,T", [(16, 4, 3), (33, 16, 8), (128, 8, 16), (129, 8, 16), (128, 8, 17), (64, 4, 257), (512, 10, 103), (257, 10, 40), (512, 10, 102), (1000, 8, 129), (1024, 16, 64), (512, 10, 700)])
 def test_router_and_plan_at_the_edges_of_their_groups(K, E, k, T):
     """Ties, both zeros and minus infinity among the logits (larger value first, then the lower id), experts in groups of 256 and pairs on
     both sides of 1024, against a sort on the host."""
