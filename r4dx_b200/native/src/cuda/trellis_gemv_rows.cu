@@ -10,15 +10,15 @@
 // form and the tcgen05 product have 2.0e-4.)
 //
 // What bounds it: instructions.  Per 256 weights a warp issues 8 extractions, 8 multiplies, 8 byte sums, 4 permutes, 4 multiply-adds
-// and one MMA, 41 clocks of a scheduler by themselves.  us at 2 / 4 / 8 rows, 4 bits, against the CUDA-core kernel
-// (trellis_gemv.cu): 34816 x 5120 52 / 52 / 54 (66 / 82 / 121), 5120 x 17408 34 / 36 / 34 (45 / 68 / 98), 16384 x 5120
-// 32 / 32 / 30 (39 / 47 / 71), 5120 x 6144 20 / 19 / 19 (23 / 27 / 39).  (The 8-bit form took 44 / 44 / 56, 32 / 32 / 36.)
+// and one MMA, 41 clocks of a scheduler by themselves.  us at 2 / 4 / 8 rows, 4 bits, L2 flushed, against the CUDA-core kernel
+// (trellis_gemv.cu): 34816 x 5120 50 / 50 / 54 (64 / 80 / 118), 5120 x 17408 34 / 34 / 35 (44 / 67 / 98), 16384 x 5120
+// 30 / 30 / 30 (40 / 47 / 69), 5120 x 6144 19 / 19 / 19 (22 / 26 / 39).  (The 8-bit form took 44 / 44 / 56, 32 / 32 / 36.)
 //
 // One row: no MMA but fp16 multiply-adds in the order of the CUDA-core kernel, whose rounding it keeps (up to 3 of 34816 outputs
 // differ, by one bf16 step: the fp32 sums are added up in another order).  Multiplies, byte sums and fp16 multiply-adds share a pipe,
-// 24 of them per 256 weights at two clocks: 48 of the 60 clocks it takes.  us at one row, 4 / 5 bits (CUDA-core kernel): 34816 x 5120
-// 50 / 54 (57 / 64), 5120 x 17408 34 / 36 (39 / 43), 16384 x 5120 30 / 32 (34 / 39), 5120 x 6144 20 / 20 (18 / 21, but inside a
-// step the next product no longer waits for a transform in every CTA).
+// 24 of them per 256 weights at two clocks, with 4 bits 20 of them (every second byte sum runs elsewhere): 40 of the 50 clocks that the
+// loop takes.  us at one row, 4 / 5 bits, L2 flushed (CUDA-core kernel): 34816 x 5120 46 / 54 (53 / 62), 5120 x 17408 32 / 36 (37 / 43),
+// 16384 x 5120 28 / 32 (32 / 38), 5120 x 6144 18 / 19.5 (19 / 21).  ops/kernels.py:one_row_split says where it serves.
 //
 // Grouped mode (mixture-of-experts blocks with a few rows per expert): a CTA serves one 128-row block of one tile of the routing
 // plan, up to eight rows of one expert; the rows are those of the planned pairs in expert order.  A block of 512

@@ -295,7 +295,7 @@ register_cuda_sig("r4dxb_trellis_gemv_mma", _I, [_P, _P, _P, _P, _P, _P, _P, _F,
 # Which weight-streaming kernel serves T <= 8 rows: "simt" = CUDA-core decode + fp16 FMA (trellis_gemv.cu), "mma" = code values
 # written to tensor memory and contracted by tcgen05.mma kind::f16 (trellis_gemv_mma.cu), "auto" (the default) = decode in
 # registers for mma.sync (one row: for fp16 FMA) where rows and weights are many enough (trellis_gemv_rows.cu; us at 2 / 4 / 8 rows on gate_up
-# 52 / 52 / 54 against 66 / 78 / 94 for the better of the other two), else by row count one of the other two.
+# 50 / 50 / 54 against 64 / 78 / 94 for the better of the other two), else by row count one of the other two.
 GEMV_IMPL = os.environ.get("R4DXB_GEMV", "auto")
 
 
