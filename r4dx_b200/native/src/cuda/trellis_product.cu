@@ -122,6 +122,13 @@ __device__ __forceinline__ __nv_bfloat16* OutRow(const ProductArgs& a, int t, in
   return a.y + static_cast<size_t>(t) * a.N + nb * 128;
 }
 
+// The rows of a tile whose wait ran out: NaN instead of what they held before.
+template <bool kGrouped>
+__device__ __noinline__ void FillNan(const ProductArgs& a, int t0, int t_end) {
+  for (int t = t0 + (threadIdx.x >> 5); t < t_end; t += blockDim.x >> 5)
+    *reinterpret_cast<uint2*>(OutRow<kGrouped>(a, t, blockIdx.x) + (threadIdx.x & 31) * 4) = make_uint2(0x7FC07FC0u, 0x7FC07FC0u);
+}
+
 template <int KB, int TN, int DW, bool kPair, bool kGrouped>
 __global__ void __launch_bounds__((DW + 3) * 32, DW == 8 ? 2 : 1)
 TrellisProductKernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ ProductArgs a) {
@@ -488,9 +495,7 @@ TrellisProductKernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_co
   ptx::TcFenceBefore();
   __syncthreads();
   if (*abort_flag != 0) {
-    // a wait ran out: NaN instead of what the rows held before
-    for (int t = t0 + warp; t < min(t0 + TN, t_end); t += DW + 3)
-      *reinterpret_cast<uint2*>(OutRow<kGrouped>(a, t, nb) + lane * 4) = make_uint2(0x7FC07FC0u, 0x7FC07FC0u);
+    FillNan<kGrouped>(a, t0, min(t0 + TN, t_end));
     // give copies that may still be in flight time to land before the shared memory goes away
     for (int i = 0; i < 64; ++i) __nanosleep(1000);
     if (threadIdx.x == 0) atomicExch(a.status, *abort_flag);
