@@ -239,7 +239,7 @@ ROWS_MIN_WORK = 3 << 24
 # per launch instead of once per CTA.  us of a captured step of the 27B geometry (8 layers, 8192 tokens of context), one-row products on
 # the CUDA cores / on the rows kernel from 64M / from 29M weights: 1282 / 1150 / 1120.  Launches of fewer weights keep the bits they had,
 # which a test compares; for them the rows kernel alone is slower (8192 x 2048 13.9 and 15.3 us), though a step of a small model, whose
-# next product waits for the transform in every CTA, would gain (16 steps of four layers of width 1024: 2914 -> 2692 us).
+# next product waits for the transform in every CTA, would gain (16 steps of four layers of width 1024: 2842 -> 2630 us).
 ROWS_MIN_ROWS = 2
 ONE_ROW_MIN_WEIGHTS = 7 << 22
 # CTAs that run at a time with one to an SM, by cluster size: 48 clusters of three take two waves, and so on
